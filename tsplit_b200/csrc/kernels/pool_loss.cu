@@ -11,6 +11,7 @@
 // Roles in the reference: cudnnPoolingForward/Backward (src/ops/CudnnMaxPool.cu,
 // CudnnAvgPool.cu) and the <<<1,1024>>> kernels of src/ops/Softmax.cu:3-22 and
 // src/ops/SoftmaxCrossEntropy.cu:5-104.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include "scratch.h"
 #include <float.h>
@@ -21,6 +22,8 @@
 #define TSB_ERR_UNSUPPORTED 2
 #define TSB_ERR_LAUNCH 3
 #define TSB_ERR_OOM 5
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -82,6 +85,75 @@ __global__ void pool_fwd(const float* __restrict__ x, float* __restrict__ y, con
     }
     *reinterpret_cast<float4*>(y + n * p.ysn + oy * p.ysh + ox * p.ysw + c) = acc;
   }
+}
+
+// Average pooling over large windows (the global pool in front of a classifier).  One thread per output and four
+// channels leaves n * C / 1024 blocks that walk the window one load at a time; here a block of 32 pixel lanes x 8
+// channel vectors (128-byte segments) reads the window with four loads in flight per thread, and a cluster of up to 8
+// blocks shares one window, joined through distributed shared memory in a fixed order, so one launch both fills the
+// chip and stays deterministic.  Bound by DRAM.  Whole training
+// steps: VGG's first block before a 112 x 112 pool of 64 channels, batch 16: 4998 -> 1552 us; a 56 x 56 pool of 256
+// channels, batch 32: 1570 -> 844 us; 17 x 17 of 256 channels, batch 32: 338 -> 292 us.
+constexpr int WIN_COLS = 8, WIN_LANES = 32;
+__global__ void __launch_bounds__(WIN_COLS * WIN_LANES) avg_pool_window(const float* __restrict__ x,
+                                                                        float* __restrict__ y, const PoolP p) {
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ float4 sh[WIN_LANES][WIN_COLS];
+  const int cx = threadIdx.x % WIN_COLS, lane = threadIdx.x / WIN_COLS;
+  const int splits = (int)cl.num_blocks(), part = (int)cl.block_rank();
+  const int c = (blockIdx.y * WIN_COLS + cx) * 4;
+  long long r = blockIdx.x / splits;
+  const int ox = (int)(r % p.ow); r /= p.ow;
+  const int oy = (int)(r % p.oh);
+  const int n = (int)(r / p.oh);
+  const int y0 = max(oy * p.stride - p.pad, 0), y1 = min(oy * p.stride - p.pad + p.kh, p.h);
+  const int x0 = max(ox * p.stride - p.pad, 0), x1 = min(ox * p.stride - p.pad + p.kw, p.w);
+  const int ww = max(x1 - x0, 0), pixels = ww * max(y1 - y0, 0);
+  const int per = (pixels + splits - 1) / splits, end = min(pixels, (part + 1) * per);
+  float4 a[4] = {};
+  if (c < p.c) {
+    const float* base = x + n * p.xsn + c;
+    for (int i = part * per + lane; i < end; i += 4 * WIN_LANES) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int q = i + u * WIN_LANES, qy = q / ww, qx = q - qy * ww;
+        v[u] = q < end ? __ldg(reinterpret_cast<const float4*>(base + (y0 + qy) * p.xsh + (x0 + qx) * p.xsw))
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { a[u].x += v[u].x; a[u].y += v[u].y; a[u].z += v[u].z; a[u].w += v[u].w; }
+    }
+  }
+  sh[lane][cx] = make_float4((a[0].x + a[1].x) + (a[2].x + a[3].x), (a[0].y + a[1].y) + (a[2].y + a[3].y),
+                             (a[0].z + a[1].z) + (a[2].z + a[3].z), (a[0].w + a[1].w) + (a[2].w + a[3].w));
+  for (int o = WIN_LANES / 2; o > 0; o >>= 1) {
+    __syncthreads();
+    if (lane < o) {
+      const float4 u = sh[lane][cx], v = sh[lane + o][cx];
+      sh[lane][cx] = make_float4(u.x + v.x, u.y + v.y, u.z + v.z, u.w + v.w);
+    }
+  }
+  cl.sync();
+  if (part == 0 && lane == 0 && c < p.c) {
+    float4 t = sh[0][cx];
+    for (int j = 1; j < splits; ++j) {
+      const float4 u = *cl.map_shared_rank(&sh[0][cx], j);
+      t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
+    }
+    const float s = 1.f / (float)(p.kh * p.kw);
+    *reinterpret_cast<float4*>(y + n * p.ysn + oy * p.ysh + ox * p.ysw + c) =
+        make_float4(t.x * s, t.y * s, t.z * s, t.w * s);
+  }
+  cl.sync();                       // a block's shared memory stays until block 0 has read it
+}
+
+// Blocks per window: doubled (up to the portable cluster size) while fewer than four blocks per SM are in flight and
+// a block would still have two rounds of its four loads.
+int window_splits(long long blocks, int pixels) {
+  int s = 1;
+  while (s < 8 && blocks * s < 4ll * sm_count() && pixels / (2 * s) >= 8 * WIN_LANES) s *= 2;
+  return s;
 }
 
 __device__ __forceinline__ int ceil_div_pos(int a, int b) { return a <= 0 ? 0 : (a + b - 1) / b; }
@@ -790,6 +862,24 @@ int tsb_pool_fwd(int kind, const float* x, float* y, int n, int c, int h, int w,
   if ((c % 4) || (xsw % 4) || (ysw % 4)) return TSB_ERR_UNSUPPORTED;
   PoolP p{n, c, h, w, oh, ow, kh, kw, pad, stride, xsn, xsh, xsw, ysn, ysh, ysw};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // windows of a warp's width of pixels or more: block-per-window form (below that its lanes idle)
+  const long long outs = (long long)n * oh * ow;
+  const int cblocks = (c / 4 + WIN_COLS - 1) / WIN_COLS;
+  if (kind == 1 && kh * kw >= WIN_LANES && outs > 0 && outs * 8 < (1ll << 31) && cblocks <= 65535) {
+    const int splits = window_splits(outs * cblocks, kh * kw);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(outs * splits), (unsigned)cblocks);
+    cfg.blockDim = dim3(WIN_COLS * WIN_LANES);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)splits;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, avg_pool_window, x, y, (const PoolP)p);
+    return done();
+  }
   const int grid = ew_grid((long long)n * oh * ow * (c / 4));
   if (kind == 0) pool_fwd<0><<<grid, 256, 0, st>>>(x, y, p);
   else pool_fwd<1><<<grid, 256, 0, st>>>(x, y, p);
