@@ -23,6 +23,7 @@
 
 #include "tc_common.cuh"
 #include "scratch.h"
+#include "launch.cuh"
 
 using namespace tsb;
 
@@ -215,6 +216,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tsb_launch::enter();              // barriers and TMEM are set up under the tail of the previous kernel
 
   const long long items = (long long)p.tiles_m * p.tiles_n * p.taps * p.splits;
   // which shared-memory operand the TMA fills / the gather warps fill
@@ -798,6 +800,7 @@ conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tsb_launch::enter();              // barriers and TMEM are set up under the tail of the previous kernel
 
   const int ptm = (p.M + 255) / 256, ptn = (p.NC + BN - 1) / BN;
   const int items = ptm * ptn;
@@ -973,6 +976,7 @@ conv_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tsb_launch::enter();              // barriers and TMEM are set up under the tail of the previous kernel
 
   const int ptm = (p.M + 255) / 256, ptn = (p.NC + P2_BN - 1) / P2_BN;
   const int tiles = ptm * ptn;
@@ -1116,6 +1120,7 @@ conv_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
 // Eight times the arithmetic, but on the tensor cores at full rate instead of on the gather path.
 __global__ void stem_pack_filters(const float* __restrict__ w, long long so, long long sc, long long sh,
                                   long long sw, float* __restrict__ out, int O, int C, int KH, int KW, int pw) {
+  tsb_launch::enter();
   const long long total = 8ll * O * KH * 3 * 32;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -1137,6 +1142,7 @@ __global__ void stem_pack_filters(const float* __restrict__ w, long long so, lon
 __global__ void stem_unpack_filter_grads(const float* __restrict__ gp, float* __restrict__ dw, long long so,
                                          long long sc, long long sh, long long sw, int O, int C, int KH, int KW,
                                          int pw) {
+  tsb_launch::enter();
   const int total = O * KH * KW * C;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int c = i % C;
@@ -1161,6 +1167,7 @@ __global__ void stem_unpack_filter_grads(const float* __restrict__ gp, float* __
 // zeros cost s*s times the arithmetic of the strided layer, but on the TMA kernels.
 __global__ void upsample_zero_insert(const float* __restrict__ dy, float* __restrict__ up, int N, int OH, int OW,
                                      int O, int Hup, int Wup, int stride) {
+  tsb_launch::enter();
   const int O4 = O >> 2;
   const long long total = (long long)N * Hup * Wup * O4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -1207,6 +1214,7 @@ bool parity_axis(int H, int OH, int K, int pad, int a, ParityAxis* d) {
 // out[c][Ta-1-ta][Tb-1-tb][o] = w[o][2ta + ra][2tb + rb][c]: the class's sub-filter, flipped and transposed.
 __global__ void parity_filters(const float* __restrict__ w, float* __restrict__ out, int O, int C, int KH, int KW,
                                int ra, int Ta, int rb, int Tb) {
+  tsb_launch::enter();
   __shared__ float tile[32][33];
   const int ta = blockIdx.z / Tb, tb = blockIdx.z - ta * Tb;
   const int ftap = (Ta - 1 - ta) * Tb + (Tb - 1 - tb);
@@ -1232,6 +1240,7 @@ struct ParityParts {
 };
 
 __global__ void parity_interleave(const ParityParts pp, float* __restrict__ dx, int N, int H, int W, int C) {
+  tsb_launch::enter();
   const int C4 = C >> 2;
   const long long total = (long long)N * H * W * C4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -1252,6 +1261,7 @@ __global__ void parity_interleave(const ParityParts pp, float* __restrict__ dx, 
 
 __global__ void conv_splitk_reduce(const float* __restrict__ ws, float* __restrict__ out, int splits,
                                    long long per_split, int accumulate) {
+  tsb_launch::enter();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < per_split;
        i += (long long)gridDim.x * blockDim.x) {
     float acc = 0.f;
@@ -1264,6 +1274,7 @@ __global__ void conv_splitk_reduce(const float* __restrict__ ws, float* __restri
 // One 32x32 tile of the (o, c) plane of one tap per block, transposed through shared memory.
 __global__ void flip_transpose_filters(const float* __restrict__ w, float* __restrict__ out, int O, int C, int KH,
                                        int KW) {
+  tsb_launch::enter();
   __shared__ float tile[32][33];
   const int tap = blockIdx.z, kh = tap / KW, kw = tap - kh * KW;
   const int ftap = (KH - 1 - kh) * KW + (KW - 1 - kw);
@@ -1329,7 +1340,7 @@ int launch(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo
   cudaMemsetAsync(prof, 0, 16 * sizeof(unsigned long long), st);
   ConvParams pp = p;
   pp.prof = prof;
-  kern<<<grid, threads, C::SMEM_BYTES, st>>>(tm, tmi, tmo, pp);
+  tsb_launch::launch(kern, grid, threads, C::SMEM_BYTES, st, tm, tmi, tmo, pp);
   unsigned long long h[16];
   cudaMemcpyAsync(h, prof, sizeof(h), cudaMemcpyDeviceToHost, st);
   cudaStreamSynchronize(st);
@@ -1342,7 +1353,7 @@ int launch(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo
           h[2] / kbs / grid, h[13] / kbs / grid, h[14] / kbs / grid, h[5] / kbs / grid, h[4] / kbs / grid, h[9] / kbs / grid, h[6] / kbs / grid,
           h[12] / kbs / grid, h[11] / kbs / grid);
 #else
-  kern<<<grid, threads, C::SMEM_BYTES, st>>>(tm, tmi, tmo, p);
+  tsb_launch::launch(kern, grid, threads, C::SMEM_BYTES, st, tm, tmi, tmo, p);
 #endif
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
@@ -1372,19 +1383,8 @@ int launch_fwd_pair_bn(const CUtensorMap& tm, const CUtensorMap& tmi, const CUte
   long long pairs = sm_count() / 2;
   if (pairs > items) pairs = items;
   if (p.stats && pairs > ptn) pairs -= pairs % ptn;              // every pair then sees one column tile only
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * pairs));
-  cfg.blockDim = dim3(192);
-  cfg.dynamicSmemBytes = PC::SMEM_BYTES;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm, tmi, tmo, p);
+  cudaError_t e = tsb_launch::launch_cluster(2u, kern, dim3((unsigned)(2 * pairs)), dim3(192), PC::SMEM_BYTES, st,
+                                             tm, tmi, tmo, p);
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
 
@@ -1406,19 +1406,9 @@ int launch_wgrad_pair(const CUtensorMap& tm, const CUtensorMap& tmi, const ConvP
   const long long items = (long long)((p.M + 255) / 256) * ((p.NC + P2_BN - 1) / P2_BN) * p.splits;
   long long pairs = sm_count() / 2;
   if (pairs > items) pairs = items;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * pairs));
-  cfg.blockDim = dim3(288);
-  cfg.dynamicSmemBytes = P2_SMEM_BYTES;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, conv_wgrad_pair_kernel, tm, tmi, p);
+  cudaError_t e = tsb_launch::launch_cluster(2u, conv_wgrad_pair_kernel, dim3((unsigned)(2 * pairs)), dim3(288),
+                                             P2_SMEM_BYTES, st,
+                                             tm, tmi, p);
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
 
@@ -1561,7 +1551,7 @@ int run_dgrad_parity(float* dx, const float* w, const float* dy, int N, int C, i
       float* wk = wt + (size_t)k * (wmax / sizeof(float));
       float* part = reinterpret_cast<float*>(reinterpret_cast<char*>(parts) + poff[k]);
       dim3 grid((C + 31) / 32, (O + 31) / 32, A.T * B.T);
-      parity_filters<<<grid, dim3(32, 8), 0, st>>>(w, wk, O, C, KH, KW, A.r, A.T, B.r, B.T);
+      tsb_launch::launch(parity_filters, grid, dim3(32, 8), 0, st, w, wk, O, C, KH, KW, A.r, A.T, B.r, B.T);
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
       const int rc = run_forward(dy, wk, part, N, O, OH, OW, C, A.T, B.T, A.R, B.R, A.pad_lead, B.pad_lead, 1, st,
@@ -1572,7 +1562,7 @@ int run_dgrad_parity(float* dx, const float* w, const float* dy, int N, int C, i
   const long long work = (long long)N * H * W * (C / 4);
   long long blocks = (work + 255) / 256;
   if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-  parity_interleave<<<(unsigned)blocks, 256, 0, st>>>(pp, dx, N, H, W, C);
+  tsb_launch::launch(parity_interleave, (unsigned)blocks, 256, 0, st, pp, dx, N, H, W, C);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
   return TSB_OK;
@@ -1613,7 +1603,7 @@ int tsb_conv2d(int kind, float* x, float* w, float* y, int N, int C, int H, int 
     float* wt = get_ws(st, 1, wbytes, size_t(16) << 20);
     if (!wt) return TSB_ERR_OOM;
     dim3 grid((C + 31) / 32, (O + 31) / 32, KH * KW);
-    flip_transpose_filters<<<grid, dim3(32, 8), 0, st>>>(w, wt, O, C, KH, KW);
+    tsb_launch::launch(flip_transpose_filters, grid, dim3(32, 8), 0, st, w, wt, O, C, KH, KW);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
     rc = run_forward(y, wt, x, N, O, OH, OW, C, KH, KW, H, W, KH - 1 - ph, KW - 1 - pw, 1, st);
@@ -1630,11 +1620,11 @@ int tsb_conv2d(int kind, float* x, float* w, float* y, int N, int C, int H, int 
     float* up = get_ws(st, 2, ubytes, size_t(64) << 20);
     if (!wt || !up) return TSB_ERR_OOM;
     dim3 grid((C + 31) / 32, (O + 31) / 32, KH * KW);
-    flip_transpose_filters<<<grid, dim3(32, 8), 0, st>>>(w, wt, O, C, KH, KW);
+    tsb_launch::launch(flip_transpose_filters, grid, dim3(32, 8), 0, st, w, wt, O, C, KH, KW);
     const long long work = (long long)N * Hup * Wup * (O / 4);
     long long blocks = (work + 255) / 256;
     if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-    upsample_zero_insert<<<(unsigned)blocks, 256, 0, st>>>(y, up, N, OH, OW, O, Hup, Wup, stride);
+    tsb_launch::launch(upsample_zero_insert, (unsigned)blocks, 256, 0, st, y, up, N, OH, OW, O, Hup, Wup, stride);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
     rc = run_forward(up, wt, x, N, O, Hup, Wup, C, KH, KW, H, W, KH - 1 - ph, KW - 1 - pw, 1, st);
@@ -1725,7 +1715,7 @@ int tsb_conv2d(int kind, float* x, float* w, float* y, int N, int C, int H, int 
       const long long per_split = (long long)O * KH * KW * C;
       int blocks = (int)((per_split + 255) / 256);
       if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-      conv_splitk_reduce<<<blocks, 256, 0, st>>>(p.ws, p.out, p.splits, per_split, 0);
+      tsb_launch::launch(conv_splitk_reduce, blocks, 256, 0, st, p.ws, p.out, p.splits, per_split, 0);
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
     }
@@ -1762,8 +1752,8 @@ int tsb_stem_pack_filters(const float* w, long long so, long long sc, long long 
                           int O, int C, int KH, int KW, int pw, void* stream) {
   if (C > 4 || KW > 9 || pw > 8 || KW - 1 - pw > 8) return TSB_ERR_UNSUPPORTED;
   const long long total = 8ll * O * KH * 3 * 32;
-  stem_pack_filters<<<(unsigned)((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      w, so, sc, sh, sw, packed, O, C, KH, KW, pw);
+  tsb_launch::launch(stem_pack_filters, (unsigned)((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), w,
+                     so, sc, sh, sw, packed, O, C, KH, KW, pw);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
@@ -1772,8 +1762,8 @@ int tsb_stem_unpack_filter_grads(const float* packed, float* dw, long long so, l
                                  long long sw, int O, int C, int KH, int KW, int pw, void* stream) {
   if (C > 4 || KW > 9 || pw > 8 || KW - 1 - pw > 8) return TSB_ERR_UNSUPPORTED;
   const int total = O * KH * KW * C;
-  stem_unpack_filter_grads<<<(total + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      packed, dw, so, sc, sh, sw, O, C, KH, KW, pw);
+  tsb_launch::launch(stem_unpack_filter_grads, (total + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream), packed,
+                     dw, so, sc, sh, sw, O, C, KH, KW, pw);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }

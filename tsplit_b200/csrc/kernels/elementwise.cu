@@ -12,6 +12,7 @@
 // ReduceSumAxisZero,Conv2dBroadcast,Conv2dReduceSum}.cu
 #include <cuda_runtime.h>
 #include "scratch.h"
+#include "launch.cuh"
 #include <stdint.h>
 
 #define TSB_OK 0
@@ -63,48 +64,71 @@ __device__ __forceinline__ float bin(float a, float b) {
   }
 }
 
+// Streaming kernels: a block takes one tile of 2 x 256 float4 and ends.  A grid of a few blocks per SM that strides
+// through the tensor loses a tenth or more of the bandwidth, and so does a loop around the tile even where it runs
+// once (the loads of a tile no longer start together).  Chains over random data, 131 M floats times a constant:
+// strided 179 us, tile in a loop 163, tile without one 151.7, one float4 a thread 156; 25.7 M floats: 34.3, 33.6, 31.2, 31.9 us;
+// 4.2 M floats (in L2): 4.47, 4.63, 3.80, 4.07 us.
+constexpr int TILE4 = 2 * 256;
+
 template <int OP>
-__global__ void unary_flat(const float* __restrict__ x, float* __restrict__ y, long long n, float a) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) unary_flat(const float* __restrict__ x, float* __restrict__ y, long long n,
+                                                  float a) {
+  tsb_launch::enter();
   const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
   if (vec) {
-    const long long n4 = n >> 2;
-    for (long long j = i; j < n4; j += stride) {
-      float4 v = OP == UN_FILL ? make_float4(0, 0, 0, 0) : reinterpret_cast<const float4*>(x)[j];
-      v.x = un<OP>(v.x, a); v.y = un<OP>(v.y, a); v.z = un<OP>(v.z, a); v.w = un<OP>(v.w, a);
-      reinterpret_cast<float4*>(y)[j] = v;
-    }
-    for (long long j = (n4 << 2) + i; j < n; j += stride) y[j] = un<OP>(OP == UN_FILL ? 0.f : x[j], a);
+    const long long n4 = n >> 2, j = blockIdx.x * (long long)TILE4 + threadIdx.x;
+    float4 v[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (OP != UN_FILL && j + u * 256 < n4) v[u] = __ldg(reinterpret_cast<const float4*>(x) + j + u * 256);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (j + u * 256 < n4) {
+        if (OP == UN_FILL) v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        reinterpret_cast<float4*>(y)[j + u * 256] =
+            make_float4(un<OP>(v[u].x, a), un<OP>(v[u].y, a), un<OP>(v[u].z, a), un<OP>(v[u].w, a));
+      }
+    const long long tail = (n4 << 2) + threadIdx.x;
+    if (blockIdx.x == 0 && tail < n) y[tail] = un<OP>(OP == UN_FILL ? 0.f : x[tail], a);
   } else {
-    for (; i < n; i += stride) y[i] = un<OP>(OP == UN_FILL ? 0.f : x[i], a);
+    const long long e0 = blockIdx.x * (4ll * TILE4), e1 = min(n, e0 + 4 * TILE4);
+    for (long long i = e0 + threadIdx.x; i < e1; i += 256) y[i] = un<OP>(OP == UN_FILL ? 0.f : x[i], a);
   }
 }
 
 template <int OP>
-__global__ void binary_flat(const float* __restrict__ p, const float* __restrict__ q, float* __restrict__ y,
-                            long long n) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) binary_flat(const float* __restrict__ p, const float* __restrict__ q,
+                                                   float* __restrict__ y, long long n) {
+  tsb_launch::enter();
   const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(q) |
                      reinterpret_cast<uintptr_t>(y)) & 15) == 0;
   if (vec) {
-    const long long n4 = n >> 2;
-    for (long long j = i; j < n4; j += stride) {
-      const float4 a = reinterpret_cast<const float4*>(p)[j];
-      const float4 b = reinterpret_cast<const float4*>(q)[j];
-      float4 o;
-      o.x = bin<OP>(a.x, b.x); o.y = bin<OP>(a.y, b.y); o.z = bin<OP>(a.z, b.z); o.w = bin<OP>(a.w, b.w);
-      reinterpret_cast<float4*>(y)[j] = o;
-    }
-    for (long long j = (n4 << 2) + i; j < n; j += stride) y[j] = bin<OP>(p[j], q[j]);
+    const long long n4 = n >> 2, j = blockIdx.x * (long long)TILE4 + threadIdx.x;
+    float4 a[2], b[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (j + u * 256 < n4) {
+        a[u] = __ldg(reinterpret_cast<const float4*>(p) + j + u * 256);
+        b[u] = __ldg(reinterpret_cast<const float4*>(q) + j + u * 256);
+      }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (j + u * 256 < n4)
+        reinterpret_cast<float4*>(y)[j + u * 256] =
+            make_float4(bin<OP>(a[u].x, b[u].x), bin<OP>(a[u].y, b[u].y), bin<OP>(a[u].z, b[u].z),
+                        bin<OP>(a[u].w, b[u].w));
+    const long long tail = (n4 << 2) + threadIdx.x;
+    if (blockIdx.x == 0 && tail < n) y[tail] = bin<OP>(p[tail], q[tail]);
   } else {
-    for (; i < n; i += stride) y[i] = bin<OP>(p[i], q[i]);
+    const long long e0 = blockIdx.x * (4ll * TILE4), e1 = min(n, e0 + 4 * TILE4);
+    for (long long i = e0 + threadIdx.x; i < e1; i += 256) y[i] = bin<OP>(p[i], q[i]);
   }
 }
 
 __global__ void where_flat(const float* __restrict__ c, const float* __restrict__ a, const float* __restrict__ b,
                            float* __restrict__ y, long long n) {
+  tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
     y[i] = c[i] != 0.f ? a[i] : b[i];
@@ -112,14 +136,23 @@ __global__ void where_flat(const float* __restrict__ c, const float* __restrict_
 
 // y[r, c] = x[r, c] + b[c] on a dense row-major [rows, cols] view, 16 bytes per thread (the bias of a
 // dense layer added without materialising the broadcast).
-__global__ void bias_add_v4(const float4* __restrict__ x, const float4* __restrict__ b, float4* __restrict__ y,
+__global__ void __launch_bounds__(256) bias_add_v4(const float4* __restrict__ x, const float4* __restrict__ b, float4* __restrict__ y,
                             long long n4, unsigned cols4) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += stride) {
-    const unsigned c = (n4 >> 32) == 0 ? (unsigned)i % cols4 : (unsigned)(i % cols4);
-    const float4 v = x[i], w = __ldg(b + c);
-    y[i] = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+  tsb_launch::enter();
+  const long long i = blockIdx.x * (long long)TILE4 + threadIdx.x;
+  float4 v[2], w[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const long long j = i + u * 256;
+    if (j < n4) {
+      v[u] = __ldg(x + j);
+      w[u] = __ldg(b + ((n4 >> 32) == 0 ? (unsigned)j % cols4 : (unsigned)(j % cols4)));
+    }
   }
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (i + u * 256 < n4)
+      y[i + u * 256] = make_float4(v[u].x + w[u].x, v[u].y + w[u].y, v[u].z + w[u].z, v[u].w + w[u].w);
 }
 
 // index decomposition: the LAST dim varies fastest across threads
@@ -188,6 +221,7 @@ __device__ __forceinline__ void offsets3(const Dims& d, long long idx, long long
 // index walk as unary_strided, but in units of 16 bytes.  `d` holds the shape and strides already
 // divided by four in the innermost dimension / for the outer strides.
 __global__ void copy_strided_v4(const float4* __restrict__ x, float4* __restrict__ y, const Dims d, long long n4) {
+  tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += stride) {
     long long ox, oy;
@@ -199,6 +233,7 @@ __global__ void copy_strided_v4(const float4* __restrict__ x, float4* __restrict
 template <int OP>
 __global__ void unary_strided(const float* __restrict__ x, float* __restrict__ y, const Dims d, long long n,
                               float a) {
+  tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
     long long ox, oy;
@@ -213,6 +248,7 @@ __global__ void unary_strided(const float* __restrict__ x, float* __restrict__ y
 __global__ void copy_tiled(const float* __restrict__ x, float* __restrict__ y, long long outer, long long R,
                            long long Cc, long long xs_outer, long long xs_r, long long xs_c, long long ys_outer,
                            long long ys_r, long long ys_c) {
+  tsb_launch::enter();
   // source is contiguous along c (xs_c == 1), destination along r (ys_r == 1)
   __shared__ float tile[32][33];
   const long long tiles_r = (R + 31) / 32, tiles_c = (Cc + 31) / 32;
@@ -238,6 +274,7 @@ __global__ void copy_tiled(const float* __restrict__ x, float* __restrict__ y, l
 template <int OP>
 __global__ void binary_strided(const float* __restrict__ p, const float* __restrict__ q, float* __restrict__ y,
                                const Dims d, long long n) {
+  tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
     long long oa, ob, oy;
@@ -252,6 +289,7 @@ template <int OP>
 __global__ void binary_rows(const float* __restrict__ p, const float* __restrict__ q, float* __restrict__ y,
                             const Dims o, long long outer, int inner, long long sa, long long sb,
                             long long sy) {
+  tsb_launch::enter();
   for (long long r = blockIdx.x * (long long)blockDim.y + threadIdx.y; r < outer;
        r += (long long)gridDim.x * blockDim.y) {
     long long oa, ob, oy;
@@ -264,6 +302,7 @@ __global__ void binary_rows(const float* __restrict__ p, const float* __restrict
 template <int OP>
 __global__ void unary_rows(const float* __restrict__ x, float* __restrict__ y, const Dims o, long long outer,
                            int inner, float a, long long sx, long long sy) {
+  tsb_launch::enter();
   for (long long r = blockIdx.x * (long long)blockDim.y + threadIdx.y; r < outer;
        r += (long long)gridDim.x * blockDim.y) {
     long long ox, oy;
@@ -282,6 +321,7 @@ struct RDims {
 };
 __global__ void reduce_sum_kernel(const float* __restrict__ x, float* __restrict__ y, const RDims d,
                                   long long nkeep, long long nred) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -314,6 +354,7 @@ __global__ void reduce_sum_kernel(const float* __restrict__ x, float* __restrict
 // cols, two-stage and deterministic.
 __global__ void colsum_partial(const float* __restrict__ x, float* __restrict__ part, long long rows,
                                long long cols, long long ld, int chunks) {
+  tsb_launch::enter();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int ch = blockIdx.y;
   if (c >= cols) return;
@@ -326,6 +367,7 @@ __global__ void colsum_partial(const float* __restrict__ x, float* __restrict__ 
 // 16-byte variant: a thread owns four adjacent columns and keeps four rows in flight.
 __global__ void colsum_partial_v4(const float4* __restrict__ x, float4* __restrict__ part, long long rows,
                                   int cols4, long long ld4, int chunks) {
+  tsb_launch::enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int ch = blockIdx.y;
   if (c >= cols4) return;
@@ -352,6 +394,7 @@ __global__ void colsum_partial_v4(const float4* __restrict__ x, float4* __restri
 // Second stage for many chunks: 32 columns x 8 chunk lanes per block, lanes joined in a fixed order.
 __global__ void colsum_final_lanes(const float* __restrict__ part, float* __restrict__ y, long long cols, int chunks,
                                    long long ys) {
+  tsb_launch::enter();
   __shared__ float sh[8][33];
   const long long c = blockIdx.x * 32ll + threadIdx.x;
   float acc = 0.f;
@@ -368,6 +411,7 @@ __global__ void colsum_final_lanes(const float* __restrict__ part, float* __rest
 }
 __global__ void colsum_final(const float* __restrict__ part, float* __restrict__ y, long long cols, int chunks,
                              long long ys) {
+  tsb_launch::enter();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= cols) return;
   float acc = 0.f;
@@ -388,6 +432,9 @@ int grid_for(long long work_items, int threads) {
   if (blocks > cap) blocks = cap;
   return blocks < 1 ? 1 : (int)blocks;
 }
+
+// Blocks of a streaming kernel over n floats (at most 2^31 - 1 of them: 4e12 floats).
+unsigned tiles_for(long long n) { return (unsigned)((n + 4 * TILE4 - 1) / (4 * TILE4)); }
 
 int done() {
   cudaError_t e = cudaGetLastError();
@@ -417,24 +464,24 @@ dim3 rows_grid(long long outer, int inner) {
 }
 
 #define UN_CASE(OPC) \
-  case OPC: unary_flat<OPC><<<grid, 256, 0, st>>>(x, y, n, alpha); break;
+  case OPC: tsb_launch::launch(unary_flat<OPC>, grid, 256, 0, st, x, y, n, alpha); break;
 #define UNR_CASE(OPC) \
-  case OPC: unary_rows<OPC><<<rgrid, dim3(32, 8), 0, st>>>(x, y, dr, outer, inner, alpha, xs[nd - 1], ys[nd - 1]); break;
+  case OPC: tsb_launch::launch(unary_rows<OPC>, rgrid, dim3(32, 8), 0, st, x, y, dr, outer, inner, alpha, xs[nd - 1], ys[nd - 1]); break;
 #define BINR_CASE(OPC) \
-  case OPC: binary_rows<OPC><<<rgrid, dim3(32, 8), 0, st>>>(a, b, y, dr, outer, inner, as[nd - 1], bs[nd - 1], ys[nd - 1]); break;
+  case OPC: tsb_launch::launch(binary_rows<OPC>, rgrid, dim3(32, 8), 0, st, a, b, y, dr, outer, inner, as[nd - 1], bs[nd - 1], ys[nd - 1]); break;
 #define UNS_CASE(OPC) \
-  case OPC: unary_strided<OPC><<<grid, 256, 0, st>>>(x, y, d, n, alpha); break;
+  case OPC: tsb_launch::launch(unary_strided<OPC>, grid, 256, 0, st, x, y, d, n, alpha); break;
 #define BIN_CASE(OPC) \
-  case OPC: binary_flat<OPC><<<grid, 256, 0, st>>>(a, b, y, n); break;
+  case OPC: tsb_launch::launch(binary_flat<OPC>, grid, 256, 0, st, a, b, y, n); break;
 #define BINS_CASE(OPC) \
-  case OPC: binary_strided<OPC><<<grid, 256, 0, st>>>(a, b, y, d, n); break;
+  case OPC: tsb_launch::launch(binary_strided<OPC>, grid, 256, 0, st, a, b, y, d, n); break;
 
 extern "C" {
 
 int tsb_ew_unary(int op, const float* x, float* y, long long n, float alpha, void* stream) {
   if (n <= 0) return TSB_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = grid_for((n + 3) / 4, 256);
+  const unsigned grid = tiles_for(n);
   switch (op) {
     UN_CASE(UN_COPY) UN_CASE(UN_RELU) UN_CASE(UN_SIGMOID) UN_CASE(UN_TANH) UN_CASE(UN_SQRT) UN_CASE(UN_RSQRT)
     UN_CASE(UN_NEG) UN_CASE(UN_ADDC) UN_CASE(UN_MULC) UN_CASE(UN_CDIV) UN_CASE(UN_FILL)
@@ -446,7 +493,7 @@ int tsb_ew_unary(int op, const float* x, float* y, long long n, float alpha, voi
 int tsb_ew_binary(int op, const float* a, const float* b, float* y, long long n, void* stream) {
   if (n <= 0) return TSB_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = grid_for((n + 3) / 4, 256);
+  const unsigned grid = tiles_for(n);
   switch (op) {
     BIN_CASE(BIN_ADD) BIN_CASE(BIN_MUL) BIN_CASE(BIN_DIV) BIN_CASE(BIN_RELU_GRAD) BIN_CASE(BIN_SUB)
     BIN_CASE(BIN_ADD_RELU) BIN_CASE(BIN_RELU_GRAD_OUT)
@@ -457,7 +504,7 @@ int tsb_ew_binary(int op, const float* a, const float* b, float* y, long long n,
 
 int tsb_where(const float* c, const float* a, const float* b, float* y, long long n, void* stream) {
   if (n <= 0) return TSB_OK;
-  where_flat<<<grid_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(c, a, b, y, n);
+  tsb_launch::launch(where_flat, grid_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream), c, a, b, y, n);
   return done();
 }
 
@@ -490,7 +537,7 @@ int tsb_strided_unary(int op, const float* x, float* y, int nd, const long long*
       v.shape[nd - 1] = shape[cd] / 4; v.s0[nd - 1] = 1; v.s1[nd - 1] = 1;
       for (int i = 0; i < nd - 1; ++i) { v.s0[i] /= 4; v.s1[i] /= 4; }
       const long long n4 = n / 4;
-      copy_strided_v4<<<grid_for(n4, 256), 256, 0, st>>>(reinterpret_cast<const float4*>(x),
+      tsb_launch::launch(copy_strided_v4, grid_for(n4, 256), 256, 0, st, reinterpret_cast<const float4*>(x),
                                                           reinterpret_cast<float4*>(y), v, n4);
       return done();
     }
@@ -504,7 +551,8 @@ int tsb_strided_unary(int op, const float* x, float* y, int nd, const long long*
       if (nd == 3) { const int od = rdim == 0 ? 1 : 0; outer = shape[od]; xso = xs[od]; yso = ys[od]; }
       const long long tiles = outer * ((shape[rdim] + 31) / 32) * ((shape[nd - 1] + 31) / 32);
       int grid = tiles > 148ll * 16 ? 148 * 16 : (int)tiles;
-      copy_tiled<<<grid, dim3(32, 8), 0, st>>>(x, y, outer, shape[rdim], shape[nd - 1], xso, xs[rdim], 1, yso, 1,
+      tsb_launch::launch(copy_tiled, grid, dim3(32, 8), 0, st, x, y, outer, shape[rdim], shape[nd - 1], xso, xs[rdim],
+                         1, yso, 1,
                                                ys[nd - 1]);
       return done();
     }
@@ -518,7 +566,8 @@ int tsb_strided_unary(int op, const float* x, float* y, int nd, const long long*
       // roles: r = last dim (dst-contiguous), c = cdim (src-contiguous)
       const long long tiles = outer * ((shape[nd - 1] + 31) / 32) * ((shape[cdim] + 31) / 32);
       int grid = tiles > 148ll * 16 ? 148 * 16 : (int)tiles;
-      copy_tiled<<<grid, dim3(32, 8), 0, st>>>(x, y, outer, shape[nd - 1], shape[cdim], xso, xs[nd - 1], 1, yso, 1,
+      tsb_launch::launch(copy_tiled, grid, dim3(32, 8), 0, st, x, y, outer, shape[nd - 1], shape[cdim], xso,
+                         xs[nd - 1], 1, yso, 1,
                                                ys[cdim]);
       return done();
     }
@@ -551,8 +600,9 @@ int tsb_bias_add(const float* x, const float* b, float* y, long long rows, long 
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(y)) & 15))
     return TSB_ERR_UNSUPPORTED;
   const long long n4 = rows * (cols / 4);
-  bias_add_v4<<<grid_for(n4, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const float4*>(x), reinterpret_cast<const float4*>(b), reinterpret_cast<float4*>(y), n4,
+  tsb_launch::launch(bias_add_v4, tiles_for(4 * n4), 256, 0, static_cast<cudaStream_t>(stream),
+                     reinterpret_cast<const float4*>(x), reinterpret_cast<const float4*>(b),
+                     reinterpret_cast<float4*>(y), n4,
       (unsigned)(cols / 4));
   return done();
 }
@@ -613,20 +663,22 @@ int tsb_reduce_sum(const float* x, float* y, int nk, const long long* kshape, co
         const int chunks = (int)(want < cmax ? want : cmax);
         const int cols4 = (int)(nkeep / 4);
         dim3 g1((unsigned)((cols4 + 127) / 128), chunks);
-        colsum_partial_v4<<<g1, 128, 0, st>>>(reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(part),
+        tsb_launch::launch(colsum_partial_v4, g1, 128, 0, st, reinterpret_cast<const float4*>(x),
+                           reinterpret_cast<float4*>(part),
                                               nred, cols4, rxs[0] / 4, chunks);
-        colsum_final_lanes<<<(unsigned)((nkeep + 31) / 32), dim3(32, 8), 0, st>>>(part, y, nkeep, chunks, kys[0]);
+        tsb_launch::launch(colsum_final_lanes, (unsigned)((nkeep + 31) / 32), dim3(32, 8), 0, st, part, y, nkeep,
+                           chunks, kys[0]);
         return done();
       }
       int chunks = (int)(nred / 64 < 64 ? (nred / 64 < 1 ? 1 : nred / 64) : 64);
       dim3 g1((unsigned)((nkeep + 127) / 128), chunks);
-      colsum_partial<<<g1, 128, 0, st>>>(x, part, nred, nkeep, rxs[0], chunks);
-      colsum_final<<<(unsigned)((nkeep + 127) / 128), 128, 0, st>>>(part, y, nkeep, chunks, kys[0]);
+      tsb_launch::launch(colsum_partial, g1, 128, 0, st, x, part, nred, nkeep, rxs[0], chunks);
+      tsb_launch::launch(colsum_final, (unsigned)((nkeep + 127) / 128), 128, 0, st, part, y, nkeep, chunks, kys[0]);
       return done();
     }
   }
   const int grid = grid_for(nkeep * 32, 256);
-  reduce_sum_kernel<<<grid, 256, 0, st>>>(x, y, d, nkeep, nred);
+  tsb_launch::launch(reduce_sum_kernel, grid, 256, 0, st, x, y, d, nkeep, nred);
   return done();
 }
 

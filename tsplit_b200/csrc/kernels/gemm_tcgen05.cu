@@ -16,6 +16,7 @@
 // (src/ops/MatrixMult.cu:4-72, src/ops/BatchMatrixMult.cu:4-43).
 #include "tc_common.cuh"
 #include "scratch.h"
+#include "launch.cuh"
 
 #include <mutex>
 #include <unordered_map>
@@ -135,6 +136,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tsb_launch::enter();              // barriers and TMEM are set up under the tail of the previous kernel
 
   const int tiles = p.tiles_m * p.tiles_n;
   const long long items = (long long)tiles * p.batch * p.splits;
@@ -366,6 +368,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   cluster_sync_all();                                 // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tsb_launch::enter();              // barriers and TMEM are set up under the tail of the previous kernel
 
   const int ptm = (p.m + 255) / 256, ptn = (p.n + P2_BN - 1) / P2_BN;
   const int tiles = ptm * ptn;
@@ -498,6 +501,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 __global__ void splitk_reduce_kernel(const float* __restrict__ ws, float* __restrict__ c, int splits,
                                      long long per_split, int m, int n, long long ldc, long long sc,
                                      int accumulate) {
+  tsb_launch::enter();
   const long long total = per_split;   // = batch * m * n
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -516,6 +520,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, float* __rest
 __global__ void gemm_simt_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
                                  int m, int n, int k, long long lda, long long ldb, long long ldc, int ta, int tb,
                                  long long sa, long long sb, long long sc, int accumulate) {
+  tsb_launch::enter();
   __shared__ float as[16][17], bs[16][17];
   const int bz = blockIdx.z;
   a += bz * sa; b += bz * sb; c += bz * sc;
@@ -745,7 +750,7 @@ int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
   }
   const long long items = (long long)p.tiles_m * p.tiles_n * p.batch * p.splits;
   const int grid = (int)(items < sm_count() ? items : sm_count());
-  kern<<<grid, 192, C::SMEM_BYTES, st>>>(ta, tb, p);
+  tsb_launch::launch(kern, grid, 192, C::SMEM_BYTES, st, ta, tb, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
@@ -771,19 +776,8 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& 
   const long long items = (long long)((p.m + 255) / 256) * ((p.n + P2_BN - 1) / P2_BN) * p.batch;
   long long pairs = sm_count() / 2;
   if (pairs > items) pairs = items;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * pairs));
-  cfg.blockDim = dim3(192);
-  cfg.dynamicSmemBytes = P2_SMEM_BYTES;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
+  cudaError_t e = tsb_launch::launch_cluster(2u, kern, dim3((unsigned)(2 * pairs)), dim3(192), P2_SMEM_BYTES, st, ta,
+                                             tb, p);
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
 
@@ -791,6 +785,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& 
 // scratch array with the row stride rounded up (pad columns zero), so that TMA can address it.
 __global__ void pad_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int batch, int rows,
                                 int cols, long long lds, long long ss, long long ldd, long long sd) {
+  tsb_launch::enter();
   const long long total = (long long)batch * rows * ldd;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -870,7 +865,8 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
         const long long total = (long long)batch * rows_a * lda2;
         long long blocks = (total + 255) / 256;
         if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-        pad_rows_kernel<<<(unsigned)blocks, 256, 0, st>>>(a, buf, batch, rows_a, cols_a, lda, batch > 1 ? sa : 0, lda2,
+        tsb_launch::launch(pad_rows_kernel, (unsigned)blocks, 256, 0, st, a, buf, batch, rows_a, cols_a, lda,
+                           batch > 1 ? sa : 0, lda2,
                                                          sa2);
         ap = buf;
       }
@@ -884,7 +880,8 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
         const long long total = (long long)batch * rows_b * ldb2;
         long long blocks = (total + 255) / 256;
         if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-        pad_rows_kernel<<<(unsigned)blocks, 256, 0, st>>>(b, buf, batch, rows_b, cols_b, ldb, batch > 1 ? sb : 0, ldb2,
+        tsb_launch::launch(pad_rows_kernel, (unsigned)blocks, 256, 0, st, b, buf, batch, rows_b, cols_b, ldb,
+                           batch > 1 ? sb : 0, ldb2,
                                                          sb2);
         bp = buf;
       }
@@ -901,7 +898,7 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
               m, n, k, lda, ldb, trans_a, trans_b, batch, sa, sb, (int)(reinterpret_cast<uintptr_t>(a) & 15),
               (int)(reinterpret_cast<uintptr_t>(b) & 15));
     dim3 blk(16, 16), grd((n + 15) / 16, (m + 15) / 16, batch);
-    gemm_simt_kernel<<<grd, blk, 0, st>>>(a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, sa, sb, sc,
+    tsb_launch::launch(gemm_simt_kernel, grd, blk, 0, st, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, sa, sb, sc,
                                           accumulate);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
@@ -998,7 +995,8 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
     const long long per_split = (long long)batch * m * n;
     int blocks = (int)((per_split + 255) / 256);
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-    splitk_reduce_kernel<<<blocks, 256, 0, st>>>(p.ws, c, p.splits, per_split, m, n, ldc, sc, accumulate);
+    tsb_launch::launch(splitk_reduce_kernel, blocks, 256, 0, st, p.ws, c, p.splits, per_split, m, n, ldc, sc,
+                       accumulate);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
   }

@@ -1,0 +1,55 @@
+// Kernel launches that overlap the tail of the kernel before them (programmatic dependent launch).
+//
+// A training step of this library is a chain of some hundred to some thousand kernels on one stream, most of them a
+// few microseconds long, so the time between one kernel's last block and the next one's first instruction is a large
+// part of it.  Every kernel here is launched with the programmatic-serialisation attribute and begins with enter():
+// its blocks may be placed, and barriers and TMEM set up, while the previous kernel drains; they wait until that
+// kernel has completed and its writes are visible.  Because every kernel waits, completion stays in stream order; a
+// copy, an event or a kernel of another library in between is ordered in full as before.  Stream capture keeps the
+// attribute as a programmatic edge.  Captured steps: LSTM, 2428 kernels: 6718 -> 5535 us (2.77 -> 2.28 us a kernel);
+// a 1x7 / 7x1 convolution pair at 17 x 17: 292 -> 275 us; a small Transformer: 808 -> 716 us.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace tsb_launch {
+
+// Wait for the kernel before this one.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Let the kernel after this one take the places that are free (it waits for this one's end in wait_previous).
+__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A kernel of few blocks allows it as soon as it runs itself.  A larger one leaves it to its blocks' ends: blocks that
+// are placed while some SMs are still busy crowd on the others, and a grid that should spread over the chip runs
+// unbalanced (ResNet-50, batch 32, 8650 us before: all kernels allowing 8594 us, up to 100 blocks 8617, up to 32 or 16
+// 8455; the LSTM step is 5680 us when its one-block products do not, and 5525 us for any of the limits).
+constexpr unsigned FEW_BLOCKS = 32;
+__device__ __forceinline__ void enter() {
+  wait_previous();
+  if (gridDim.x * gridDim.y * gridDim.z <= FEW_BLOCKS) allow_next();
+}
+
+// cluster: blocks per cluster along x (0: no cluster).  Errors are left for cudaGetLastError, as with <<<>>>.
+template <class... P, class... A>
+cudaError_t launch_cluster(unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                           A&&... args) {
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <class... P, class... A>
+cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  return launch_cluster(0u, kernel, grid, block, smem, st, static_cast<A&&>(args)...);
+}
+
+}  // namespace tsb_launch

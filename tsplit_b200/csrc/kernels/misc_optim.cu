@@ -6,6 +6,7 @@
 // CuSparseCsrmm.cu (legacy cuSPARSE) and Optimizers.cu:3-149 (one launch per
 // parameter tensor there, one launch per 64 tensors here).
 #include <cuda_runtime.h>
+#include "launch.cuh"
 #include <stdint.h>
 
 #define TSB_OK 0
@@ -36,6 +37,7 @@ int done() {
 }
 
 __global__ void one_hot_kernel(const float* __restrict__ idx, float* __restrict__ y, long long n, long long k) {
+  tsb_launch::enter();
   const long long total = n * k;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -47,6 +49,7 @@ __global__ void one_hot_kernel(const float* __restrict__ idx, float* __restrict_
 // Rows that are a multiple of four classes long: one block row-slice per row, 16-byte stores, no division
 // per element (grid.y walks the rows, grid.x * blockDim.x the 4-class groups of a row).
 __global__ void one_hot_rows_v4(const float* __restrict__ idx, float4* __restrict__ y, long long n, int k4) {
+  tsb_launch::enter();
   for (long long r = blockIdx.y; r < n; r += gridDim.y) {
     const long long id = (long long)idx[r];
     float4* yr = y + r * k4;
@@ -60,6 +63,7 @@ __global__ void one_hot_rows_v4(const float* __restrict__ idx, float4* __restric
 
 __global__ void embedding_kernel(const float* __restrict__ table, const float* __restrict__ idx,
                                  float* __restrict__ y, long long n, long long vocab, long long dim) {
+  tsb_launch::enter();
   const long long total = n * dim;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -71,6 +75,7 @@ __global__ void embedding_kernel(const float* __restrict__ table, const float* _
 
 __global__ void embedding_grad_kernel(const float* __restrict__ g, const float* __restrict__ idx,
                                       float* __restrict__ dtable, long long n, long long vocab, long long dim) {
+  tsb_launch::enter();
   const long long total = n * dim;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -96,6 +101,7 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
 __global__ void dropout_kernel(const float* __restrict__ x, float* __restrict__ y, long long n, float keep,
                                unsigned long long seed, const unsigned long long* __restrict__ step_dev,
                                unsigned long long offset) {
+  tsb_launch::enter();
   if (step_dev) seed = (seed + 0x632BE5ABull * *step_dev) & 0x7FFFFFFFFFFFFFFFull;
   const float inv = 1.f / keep;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -107,6 +113,7 @@ __global__ void dropout_kernel(const float* __restrict__ x, float* __restrict__ 
 __global__ void csrmm_kernel(const float* __restrict__ vals, const float* __restrict__ rowptr,
                              const float* __restrict__ colidx, long long nrow, const float* __restrict__ dense,
                              float* __restrict__ out, long long ncols) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   if (row >= nrow) return;
@@ -121,6 +128,7 @@ __global__ void csrmm_kernel(const float* __restrict__ vals, const float* __rest
 __global__ void csrmm_t_kernel(const float* __restrict__ vals, const float* __restrict__ rowptr,
                                const float* __restrict__ colidx, long long nrow, const float* __restrict__ dense,
                                float* __restrict__ out, long long ncols) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   if (row >= nrow) return;
@@ -132,6 +140,7 @@ __global__ void csrmm_t_kernel(const float* __restrict__ vals, const float* __re
   }
 }
 __global__ void zero_kernel(float* __restrict__ y, long long n) {
+  tsb_launch::enter();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     y[i] = 0.f;
@@ -147,8 +156,12 @@ struct OptArgs {
   long long n[MAX_TENSORS];
   float h[8];
   const float* hdev;     // Adam only, may be null: {beta1^t, beta2^t} kept on the device (see tsb_adam_advance)
+  unsigned first[MAX_TENSORS + 1];   // first block of each tensor: a block updates OPT_TILE elements of one
   int count;
 };
+// (a grid of the largest tensor's blocks times the number of tensors is mostly empty blocks for a network whose
+// parameters differ in size; Adam on 16.4 M: 71.8 -> 68.3 us)
+constexpr int OPT_TILE = 2 * 256 * 4;
 
 template <int KIND>
 __device__ __forceinline__ void opt_one(float& p, float g, float& s1, float& s2, const float* h) {
@@ -175,8 +188,10 @@ __device__ __forceinline__ void opt_one(float& p, float g, float& s1, float& s2,
 
 template <int KIND>
 __global__ void opt_kernel(const OptArgs a) {
-  const int t = blockIdx.y;
-  if (t >= a.count) return;
+  tsb_launch::enter();
+  int t = 0;
+  for (int step = MAX_TENSORS / 2; step > 0; step >>= 1)
+    if (t + step < a.count && a.first[t + step] <= blockIdx.x) t += step;
   float hloc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) hloc[i] = a.h[i];
@@ -186,14 +201,14 @@ __global__ void opt_kernel(const OptArgs a) {
   float* s1 = a.s1[t];
   float* s2 = a.s2[t];
   const long long n = a.n[t];
-  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long nthreads = (long long)gridDim.x * blockDim.x;
+  const long long e0 = (long long)(blockIdx.x - a.first[t]) * OPT_TILE, e1 = min(n, e0 + OPT_TILE);
   // 16 bytes per access when every array of this tensor is 16-byte aligned; scalar tail / fallback
   const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
                      (KIND >= 1 ? reinterpret_cast<uintptr_t>(s1) : 0) |
                      (KIND == 4 ? reinterpret_cast<uintptr_t>(s2) : 0)) & 15) == 0;
-  const long long n4 = vec ? n / 4 : 0;
-  for (long long i = tid; i < n4; i += nthreads) {
+  const long long n4 = vec ? e1 / 4 : e0 / 4;
+#pragma unroll 2
+  for (long long i = e0 / 4 + threadIdx.x; i < n4; i += 256) {
     float4 pv = reinterpret_cast<float4*>(p)[i];
     const float4 gv = reinterpret_cast<const float4*>(g)[i];
     float4 v1 = make_float4(0, 0, 0, 0), v2 = make_float4(0, 0, 0, 0);
@@ -207,7 +222,7 @@ __global__ void opt_kernel(const OptArgs a) {
     if (KIND >= 1) reinterpret_cast<float4*>(s1)[i] = v1;
     if (KIND == 4) reinterpret_cast<float4*>(s2)[i] = v2;
   }
-  for (long long i = n4 * 4 + tid; i < n; i += nthreads) {
+  for (long long i = n4 * 4 + threadIdx.x; i < e1; i += 256) {
     float pv = p[i], v1 = (KIND >= 1) ? s1[i] : 0.f, v2 = (KIND == 4) ? s2[i] : 0.f;
     opt_one<KIND>(pv, g[i], v1, v2, hloc);
     p[i] = pv;
@@ -218,9 +233,10 @@ __global__ void opt_kernel(const OptArgs a) {
 
 // Adam's bias-correction powers live on the device so that a captured step (CUDA graph) advances
 // them by itself: one thread multiplies {beta1^t, beta2^t} by {beta1, beta2} before the update.
-__global__ void step_advance_kernel(unsigned long long* step_dev) { *step_dev += 1ull; }
+__global__ void step_advance_kernel(unsigned long long* step_dev) { tsb_launch::enter(); *step_dev += 1ull; }
 
 __global__ void adam_advance_kernel(float* hdev, float b1, float b2) {
+  tsb_launch::enter();
   hdev[0] *= b1;
   hdev[1] *= b2;
 }
@@ -231,7 +247,7 @@ extern "C" {
 
 int tsb_adam_advance(float* hdev, float b1, float b2, void* stream) {
   if (!hdev) return TSB_ERR_ARG;
-  adam_advance_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(hdev, b1, b2);
+  tsb_launch::launch(adam_advance_kernel, 1, 1, 0, static_cast<cudaStream_t>(stream), hdev, b1, b2);
   return done();
 }
 
@@ -242,25 +258,27 @@ int tsb_one_hot(const float* idx, float* y, long long n, long long k, void* stre
     int gx = (k4 + 255) / 256;
     if (gx > 32) gx = 32;
     long long gy = n < 65535 ? n : 65535;
-    one_hot_rows_v4<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        idx, reinterpret_cast<float4*>(y), n, k4);
+    tsb_launch::launch(one_hot_rows_v4, dim3((unsigned)gx, (unsigned)gy), 256, 0, static_cast<cudaStream_t>(stream),
+                       idx, reinterpret_cast<float4*>(y), n, k4);
     return done();
   }
-  one_hot_kernel<<<ew_grid(n * k), 256, 0, static_cast<cudaStream_t>(stream)>>>(idx, y, n, k);
+  tsb_launch::launch(one_hot_kernel, ew_grid(n * k), 256, 0, static_cast<cudaStream_t>(stream), idx, y, n, k);
   return done();
 }
 
 int tsb_embedding(const float* table, const float* idx, float* y, long long n, long long vocab, long long dim,
                   void* stream) {
   if (n <= 0) return TSB_OK;
-  embedding_kernel<<<ew_grid(n * dim), 256, 0, static_cast<cudaStream_t>(stream)>>>(table, idx, y, n, vocab, dim);
+  tsb_launch::launch(embedding_kernel, ew_grid(n * dim), 256, 0, static_cast<cudaStream_t>(stream), table, idx, y, n,
+                     vocab, dim);
   return done();
 }
 
 int tsb_embedding_grad(const float* g, const float* idx, float* dtable, long long n, long long vocab,
                        long long dim, void* stream) {
   if (n <= 0) return TSB_OK;
-  embedding_grad_kernel<<<ew_grid(n * dim), 256, 0, static_cast<cudaStream_t>(stream)>>>(g, idx, dtable, n, vocab,
+  tsb_launch::launch(embedding_grad_kernel, ew_grid(n * dim), 256, 0, static_cast<cudaStream_t>(stream), g, idx,
+                     dtable, n, vocab,
                                                                                          dim);
   return done();
 }
@@ -269,14 +287,15 @@ int tsb_dropout(const float* x, float* y, long long n, float keep, unsigned long
                 const unsigned long long* step_dev, unsigned long long offset, void* stream) {
   if (n <= 0) return TSB_OK;
   if (!(keep > 0.f)) return TSB_ERR_ARG;
-  dropout_kernel<<<ew_grid(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, n, keep, seed, step_dev, offset);
+  tsb_launch::launch(dropout_kernel, ew_grid(n), 256, 0, static_cast<cudaStream_t>(stream), x, y, n, keep, seed,
+                     step_dev, offset);
   return done();
 }
 
 // ++*step_dev on the stream (one thread): the executor's step counter, advanced at the start of a step
 int tsb_step_advance(unsigned long long* step_dev, void* stream) {
   if (!step_dev) return TSB_ERR_ARG;
-  step_advance_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(step_dev);
+  tsb_launch::launch(step_advance_kernel, 1, 1, 0, static_cast<cudaStream_t>(stream), step_dev);
   return done();
 }
 
@@ -286,11 +305,13 @@ int tsb_csrmm(const float* vals, const float* rowptr, const float* colidx, long 
   if (nrow <= 0 || ncols_dense <= 0) return TSB_ERR_ARG;
   const long long threads = nrow * 32;
   if (!trans_a) {
-    csrmm_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(vals, rowptr, colidx, nrow, dense, out,
+    tsb_launch::launch(csrmm_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, vals, rowptr, colidx, nrow, dense,
+                       out,
                                                                      ncols_dense);
   } else {
-    zero_kernel<<<ew_grid(ncol * ncols_dense), 256, 0, st>>>(out, ncol * ncols_dense);
-    csrmm_t_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(vals, rowptr, colidx, nrow, dense, out,
+    tsb_launch::launch(zero_kernel, ew_grid(ncol * ncols_dense), 256, 0, st, out, ncol * ncols_dense);
+    tsb_launch::launch(csrmm_t_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, vals, rowptr, colidx, nrow,
+                       dense, out,
                                                                        ncols_dense);
   }
   return done();
@@ -311,28 +332,30 @@ int tsb_optimizer_step_dev(int kind, int count, float** params, const float** gr
   OptArgs a;
   a.count = count;
   a.hdev = hyper_dev;
-  long long biggest = 0;
+  long long blocks = 0;
   for (int i = 0; i < count; ++i) {
     a.p[i] = params[i]; a.g[i] = grads[i];
     a.s1[i] = slot1 ? slot1[i] : nullptr;
     a.s2[i] = slot2 ? slot2[i] : nullptr;
     a.n[i] = sizes[i];
-    if (sizes[i] > biggest) biggest = sizes[i];
+    if (sizes[i] < 0) return TSB_ERR_ARG;
+    a.first[i] = (unsigned)blocks;
+    blocks += (sizes[i] + OPT_TILE - 1) / OPT_TILE;
+    if (blocks > 0x7fffffffll) return TSB_ERR_ARG;
     if (kind >= 1 && !a.s1[i]) return TSB_ERR_ARG;
     if (kind == 4 && !a.s2[i]) return TSB_ERR_ARG;
   }
+  a.first[count] = (unsigned)blocks;
   for (int i = 0; i < 8; ++i) a.h[i] = hyper[i];
-  long long bx = (biggest / 4 + 255) / 256;
-  if (bx > 8 * sm_count()) bx = 8 * sm_count();
-  if (bx < 1) bx = 1;
-  dim3 grid((unsigned)bx, count);
+  if (blocks == 0) return TSB_OK;
+  const dim3 grid((unsigned)blocks);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (kind) {
-    case 0: opt_kernel<0><<<grid, 256, 0, st>>>(a); break;
-    case 1: opt_kernel<1><<<grid, 256, 0, st>>>(a); break;
-    case 2: opt_kernel<2><<<grid, 256, 0, st>>>(a); break;
-    case 3: opt_kernel<3><<<grid, 256, 0, st>>>(a); break;
-    default: opt_kernel<4><<<grid, 256, 0, st>>>(a); break;
+    case 0: tsb_launch::launch(opt_kernel<0>, grid, 256, 0, st, a); break;
+    case 1: tsb_launch::launch(opt_kernel<1>, grid, 256, 0, st, a); break;
+    case 2: tsb_launch::launch(opt_kernel<2>, grid, 256, 0, st, a); break;
+    case 3: tsb_launch::launch(opt_kernel<3>, grid, 256, 0, st, a); break;
+    default: tsb_launch::launch(opt_kernel<4>, grid, 256, 0, st, a); break;
   }
   return done();
 }

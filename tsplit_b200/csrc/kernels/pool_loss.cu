@@ -14,6 +14,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include "scratch.h"
+#include "launch.cuh"
 #include <float.h>
 #include <stdint.h>
 
@@ -55,6 +56,7 @@ struct PoolP {
 
 template <int KIND>
 __global__ void pool_fwd(const float* __restrict__ x, float* __restrict__ y, const PoolP p) {
+  tsb_launch::enter();
   const int C4 = p.c >> 2;
   const long long total = (long long)p.n * p.oh * p.ow * C4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -97,6 +99,7 @@ __global__ void pool_fwd(const float* __restrict__ x, float* __restrict__ y, con
 constexpr int WIN_COLS = 8, WIN_LANES = 32;
 __global__ void __launch_bounds__(WIN_COLS * WIN_LANES) avg_pool_window(const float* __restrict__ x,
                                                                         float* __restrict__ y, const PoolP p) {
+  tsb_launch::enter();
   cg::cluster_group cl = cg::this_cluster();
   __shared__ float4 sh[WIN_LANES][WIN_COLS];
   const int cx = threadIdx.x % WIN_COLS, lane = threadIdx.x / WIN_COLS;
@@ -161,6 +164,7 @@ __device__ __forceinline__ int ceil_div_pos(int a, int b) { return a <= 0 ? 0 : 
 template <int KIND>
 __global__ void pool_bwd(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ dy,
                          float* __restrict__ dx, const PoolP p) {
+  tsb_launch::enter();
   const int C4 = p.c >> 2;
   const long long total = (long long)p.n * p.h * p.w * C4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -221,6 +225,7 @@ __global__ void pool_bwd(const float* __restrict__ x, const float* __restrict__ 
 template <int KIND, int K>
 __global__ void pool_bwd_tiled(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dx,
                                const PoolP p) {
+  tsb_launch::enter();
   const int C4 = p.c >> 2;
   const long long total = (long long)p.n * p.oh * p.ow * C4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -275,6 +280,7 @@ __global__ void pool_bwd_tiled(const float* __restrict__ x, const float* __restr
 // After a ReLU most windows tie at zero, which made the scan-for-earlier-maximum form of the general
 // kernel expensive; here every tensor is read once.
 __global__ void pool_argmax(const float* __restrict__ x, unsigned char* __restrict__ idx, const PoolP p) {
+  tsb_launch::enter();
   const int C4 = p.c >> 2;
   const long long total = (long long)p.n * p.oh * p.ow * C4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -306,6 +312,7 @@ __global__ void pool_argmax(const float* __restrict__ x, unsigned char* __restri
 
 __global__ void pool_bwd_from_argmax(const unsigned char* __restrict__ idx, const float* __restrict__ dy,
                                      float* __restrict__ dx, const PoolP p) {
+  tsb_launch::enter();
   const int C4 = p.c >> 2;
   const long long total = (long long)p.n * p.h * p.w * C4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -363,6 +370,7 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
 }
 
 __global__ void softmax_rows(const float* __restrict__ x, float* __restrict__ y, long long rows, long long cols) {
+  tsb_launch::enter();
   __shared__ float sh[8];
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float* xr = x + row * cols;
@@ -382,6 +390,7 @@ __global__ void softmax_rows(const float* __restrict__ x, float* __restrict__ y,
 template <int NV>
 __global__ void __launch_bounds__(256) softmax_warp_rows(const float4* __restrict__ x, float4* __restrict__ y,
                                                          long long rows, int nvec) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -421,6 +430,7 @@ __global__ void __launch_bounds__(256) softmax_warp_rows(const float4* __restric
 template <int NE>
 __global__ void __launch_bounds__(256) softmax_warp_rows_scalar(const float* __restrict__ x, float* __restrict__ y,
                                                                 long long rows, int cols) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -456,6 +466,7 @@ __global__ void __launch_bounds__(256) softmax_grad_warp_rows_scalar(const float
                                                                      const float* __restrict__ dy,
                                                                      float* __restrict__ dx, long long rows,
                                                                      int cols) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -487,6 +498,7 @@ template <int NV>
 __global__ void __launch_bounds__(256) softmax_grad_warp_rows(const float4* __restrict__ y,
                                                               const float4* __restrict__ dy,
                                                               float4* __restrict__ dx, long long rows, int nvec) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -526,6 +538,7 @@ __global__ void __launch_bounds__(256) masked_softmax_warp_rows(const float* __r
                                                                 float* __restrict__ y, long long rows, int cols,
                                                                 long long rows_per_batch, int tq, float scale,
                                                                 int causal) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -577,6 +590,7 @@ __global__ void __launch_bounds__(256) masked_softmax_warp_rows_v4(const float4*
                                                                    float4* __restrict__ y, long long rows, int nvec,
                                                                    long long rows_per_batch, int tq, float scale,
                                                                    int causal) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -643,6 +657,7 @@ __global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows(const float
                                                                      const float* __restrict__ dy,
                                                                      float* __restrict__ dx, long long rows, int cols,
                                                                      float scale) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -674,6 +689,7 @@ __global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows_v4(const fl
                                                                         const float4* __restrict__ dy,
                                                                         float4* __restrict__ dx, long long rows,
                                                                         int nvec, float scale) {
+  tsb_launch::enter();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -705,6 +721,7 @@ __global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows_v4(const fl
 // Any row length: one CTA per row, the second pass finds the row in L2.
 __global__ void softmax_grad_rows(const float* __restrict__ y, const float* __restrict__ dy, float* __restrict__ dx,
                                   long long rows, long long cols) {
+  tsb_launch::enter();
   __shared__ float sh[8];
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float* yr = y + row * cols;
@@ -758,6 +775,7 @@ __device__ __forceinline__ MaxSum row_max_sum(const float4* __restrict__ xr, int
 // rows in flight being kept below its size by the block size chosen at launch).
 __global__ void __launch_bounds__(512) ce_rows_v4(const float4* __restrict__ x, const float4* __restrict__ lab,
                                                   float* __restrict__ row_loss, long long rows, int nvec) {
+  tsb_launch::enter();
   __shared__ float sh[64];
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float4* xr = x + row * nvec;
@@ -778,6 +796,7 @@ __global__ void __launch_bounds__(512) ce_rows_v4(const float4* __restrict__ x, 
 __global__ void __launch_bounds__(512) ce_grad_rows_v4(const float4* __restrict__ x, const float4* __restrict__ lab,
                                                        const float* __restrict__ g, float4* __restrict__ dx,
                                                        long long rows, int nvec) {
+  tsb_launch::enter();
   __shared__ float sh[64];
   const float scale = g[0] / (float)rows;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -801,6 +820,7 @@ __global__ void __launch_bounds__(512) ce_grad_rows_v4(const float4* __restrict_
 
 __global__ void ce_rows(const float* __restrict__ x, const float* __restrict__ lab, float* __restrict__ row_loss,
                         long long rows, long long cols) {
+  tsb_launch::enter();
   __shared__ float sh[8];
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float* xr = x + row * cols;
@@ -820,6 +840,7 @@ __global__ void ce_rows(const float* __restrict__ x, const float* __restrict__ l
 }
 
 __global__ void mean_rows(const float* __restrict__ row_loss, float* __restrict__ out, long long rows) {
+  tsb_launch::enter();
   __shared__ float sh[32];
   float s = 0.f;
   for (long long i = threadIdx.x; i < rows; i += blockDim.x) s += row_loss[i];
@@ -829,6 +850,7 @@ __global__ void mean_rows(const float* __restrict__ row_loss, float* __restrict_
 
 __global__ void ce_grad_rows(const float* __restrict__ x, const float* __restrict__ lab, const float* __restrict__ g,
                              float* __restrict__ dx, long long rows, long long cols) {
+  tsb_launch::enter();
   __shared__ float sh[8];
   const float scale = g[0] / (float)rows;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -862,27 +884,20 @@ int tsb_pool_fwd(int kind, const float* x, float* y, int n, int c, int h, int w,
   if ((c % 4) || (xsw % 4) || (ysw % 4)) return TSB_ERR_UNSUPPORTED;
   PoolP p{n, c, h, w, oh, ow, kh, kw, pad, stride, xsn, xsh, xsw, ysn, ysh, ysw};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // windows of a warp's width of pixels or more: block-per-window form (below that its lanes idle)
+  // Large windows whose outputs leave the one-thread-per-output form on less than a quarter of the SMs (8 x 8 windows:
+  // 8 images of 1536 channels, 12 blocks: 10.3 -> 4.6 us; 32 of 2048, 64 blocks: 10.3 us and 12.7 us with a block per
+  // window, and 28.7 against 89.7 us for 256 images).
   const long long outs = (long long)n * oh * ow;
   const int cblocks = (c / 4 + WIN_COLS - 1) / WIN_COLS;
-  if (kind == 1 && kh * kw >= WIN_LANES && outs > 0 && outs * 8 < (1ll << 31) && cblocks <= 65535) {
+  if (kind == 1 && kh * kw >= 2 * WIN_LANES && outs > 0 && outs * (c / 4) < 64ll * sm_count() && cblocks <= 65535) {
     const int splits = window_splits(outs * cblocks, kh * kw);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(outs * splits), (unsigned)cblocks);
-    cfg.blockDim = dim3(WIN_COLS * WIN_LANES);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)splits;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, avg_pool_window, x, y, (const PoolP)p);
+    tsb_launch::launch_cluster((unsigned)splits, avg_pool_window, dim3((unsigned)(outs * splits), (unsigned)cblocks),
+                               dim3(WIN_COLS * WIN_LANES), 0, st, x, y, p);
     return done();
   }
   const int grid = ew_grid((long long)n * oh * ow * (c / 4));
-  if (kind == 0) pool_fwd<0><<<grid, 256, 0, st>>>(x, y, p);
-  else pool_fwd<1><<<grid, 256, 0, st>>>(x, y, p);
+  if (kind == 0) tsb_launch::launch(pool_fwd<0>, grid, 256, 0, st, x, y, p);
+  else tsb_launch::launch(pool_fwd<1>, grid, 256, 0, st, x, y, p);
   return done();
 }
 
@@ -895,10 +910,10 @@ int tsb_pool_bwd(int kind, const float* x, const float* y, const float* dy, floa
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (kh == stride && kw == stride && pad == 0 && oh * stride == h && ow * stride == w && (stride == 2 || stride == 3)) {
     const int tg = ew_grid((long long)n * oh * ow * (c / 4));
-    if (kind == 0 && stride == 2) pool_bwd_tiled<0, 2><<<tg, 256, 0, st>>>(x, dy, dx, p);
-    else if (kind == 0) pool_bwd_tiled<0, 3><<<tg, 256, 0, st>>>(x, dy, dx, p);
-    else if (stride == 2) pool_bwd_tiled<1, 2><<<tg, 256, 0, st>>>(x, dy, dx, p);
-    else pool_bwd_tiled<1, 3><<<tg, 256, 0, st>>>(x, dy, dx, p);
+    if (kind == 0 && stride == 2) tsb_launch::launch(pool_bwd_tiled<0, 2>, tg, 256, 0, st, x, dy, dx, p);
+    else if (kind == 0) tsb_launch::launch(pool_bwd_tiled<0, 3>, tg, 256, 0, st, x, dy, dx, p);
+    else if (stride == 2) tsb_launch::launch(pool_bwd_tiled<1, 2>, tg, 256, 0, st, x, dy, dx, p);
+    else tsb_launch::launch(pool_bwd_tiled<1, 3>, tg, 256, 0, st, x, dy, dx, p);
     return done();
   }
   const int grid = ew_grid((long long)n * h * w * (c / 4));
@@ -907,13 +922,13 @@ int tsb_pool_bwd(int kind, const float* x, const float* y, const float* dy, floa
     // buffer per device: pooling backward passes of one device must not overlap on different streams)
     unsigned char* idx = argmax_scratch((size_t)n * oh * ow * c);
     if (idx) {
-      pool_argmax<<<ew_grid((long long)n * oh * ow * (c / 4)), 256, 0, st>>>(x, idx, p);
-      pool_bwd_from_argmax<<<grid, 256, 0, st>>>(idx, dy, dx, p);
+      tsb_launch::launch(pool_argmax, ew_grid((long long)n * oh * ow * (c / 4)), 256, 0, st, x, idx, p);
+      tsb_launch::launch(pool_bwd_from_argmax, grid, 256, 0, st, idx, dy, dx, p);
       return done();
     }
   }
-  if (kind == 0) pool_bwd<0><<<grid, 256, 0, st>>>(x, y, dy, dx, p);
-  else pool_bwd<1><<<grid, 256, 0, st>>>(x, y, dy, dx, p);
+  if (kind == 0) tsb_launch::launch(pool_bwd<0>, grid, 256, 0, st, x, y, dy, dx, p);
+  else tsb_launch::launch(pool_bwd<1>, grid, 256, 0, st, x, y, dy, dx, p);
   return done();
 }
 
@@ -926,25 +941,25 @@ int tsb_softmax(const float* x, float* y, long long rows, long long cols, void* 
     const int wgrid = (int)(blocks < 148 * 8 ? blocks : 148 * 8);
     const float4* xv = reinterpret_cast<const float4*>(x);
     float4* yv = reinterpret_cast<float4*>(y);
-    if (nvec <= 32) softmax_warp_rows<1><<<wgrid, 256, 0, st>>>(xv, yv, rows, nvec);
-    else if (nvec <= 64) softmax_warp_rows<2><<<wgrid, 256, 0, st>>>(xv, yv, rows, nvec);
-    else if (nvec <= 128) softmax_warp_rows<4><<<wgrid, 256, 0, st>>>(xv, yv, rows, nvec);
-    else softmax_warp_rows<8><<<wgrid, 256, 0, st>>>(xv, yv, rows, nvec);
+    if (nvec <= 32) tsb_launch::launch(softmax_warp_rows<1>, wgrid, 256, 0, st, xv, yv, rows, nvec);
+    else if (nvec <= 64) tsb_launch::launch(softmax_warp_rows<2>, wgrid, 256, 0, st, xv, yv, rows, nvec);
+    else if (nvec <= 128) tsb_launch::launch(softmax_warp_rows<4>, wgrid, 256, 0, st, xv, yv, rows, nvec);
+    else tsb_launch::launch(softmax_warp_rows<8>, wgrid, 256, 0, st, xv, yv, rows, nvec);
     return done();
   }
   if (cols <= 1024) {
     const long long blocks = (rows + 7) / 8;
     const int wgrid = (int)(blocks < 148 * 8 ? blocks : 148 * 8);
     const int c = (int)cols;
-    if (c <= 64) softmax_warp_rows_scalar<2><<<wgrid, 256, 0, st>>>(x, y, rows, c);
-    else if (c <= 128) softmax_warp_rows_scalar<4><<<wgrid, 256, 0, st>>>(x, y, rows, c);
-    else if (c <= 256) softmax_warp_rows_scalar<8><<<wgrid, 256, 0, st>>>(x, y, rows, c);
-    else if (c <= 512) softmax_warp_rows_scalar<16><<<wgrid, 256, 0, st>>>(x, y, rows, c);
-    else softmax_warp_rows_scalar<32><<<wgrid, 256, 0, st>>>(x, y, rows, c);
+    if (c <= 64) tsb_launch::launch(softmax_warp_rows_scalar<2>, wgrid, 256, 0, st, x, y, rows, c);
+    else if (c <= 128) tsb_launch::launch(softmax_warp_rows_scalar<4>, wgrid, 256, 0, st, x, y, rows, c);
+    else if (c <= 256) tsb_launch::launch(softmax_warp_rows_scalar<8>, wgrid, 256, 0, st, x, y, rows, c);
+    else if (c <= 512) tsb_launch::launch(softmax_warp_rows_scalar<16>, wgrid, 256, 0, st, x, y, rows, c);
+    else tsb_launch::launch(softmax_warp_rows_scalar<32>, wgrid, 256, 0, st, x, y, rows, c);
     return done();
   }
   const int grid = (int)(rows < 148 * 16 ? rows : 148 * 16);
-  softmax_rows<<<grid, cols >= 1024 ? 256 : 128, 0, st>>>(x, y, rows, cols);
+  tsb_launch::launch(softmax_rows, grid, cols >= 1024 ? 256 : 128, 0, st, x, y, rows, cols);
   return done();
 }
 
@@ -958,25 +973,25 @@ int tsb_softmax_grad(const float* y, const float* dy, float* dx, long long rows,
     const float4* yv = reinterpret_cast<const float4*>(y);
     const float4* gv = reinterpret_cast<const float4*>(dy);
     float4* dv = reinterpret_cast<float4*>(dx);
-    if (nvec <= 32) softmax_grad_warp_rows<1><<<wgrid, 256, 0, st>>>(yv, gv, dv, rows, nvec);
-    else if (nvec <= 64) softmax_grad_warp_rows<2><<<wgrid, 256, 0, st>>>(yv, gv, dv, rows, nvec);
-    else if (nvec <= 128) softmax_grad_warp_rows<4><<<wgrid, 256, 0, st>>>(yv, gv, dv, rows, nvec);
-    else softmax_grad_warp_rows<8><<<wgrid, 256, 0, st>>>(yv, gv, dv, rows, nvec);
+    if (nvec <= 32) tsb_launch::launch(softmax_grad_warp_rows<1>, wgrid, 256, 0, st, yv, gv, dv, rows, nvec);
+    else if (nvec <= 64) tsb_launch::launch(softmax_grad_warp_rows<2>, wgrid, 256, 0, st, yv, gv, dv, rows, nvec);
+    else if (nvec <= 128) tsb_launch::launch(softmax_grad_warp_rows<4>, wgrid, 256, 0, st, yv, gv, dv, rows, nvec);
+    else tsb_launch::launch(softmax_grad_warp_rows<8>, wgrid, 256, 0, st, yv, gv, dv, rows, nvec);
     return done();
   }
   if (cols <= 1024) {
     const long long blocks = (rows + 7) / 8;
     const int wgrid = (int)(blocks < 148 * 8 ? blocks : 148 * 8);
     const int c = (int)cols;
-    if (c <= 64) softmax_grad_warp_rows_scalar<2><<<wgrid, 256, 0, st>>>(y, dy, dx, rows, c);
-    else if (c <= 128) softmax_grad_warp_rows_scalar<4><<<wgrid, 256, 0, st>>>(y, dy, dx, rows, c);
-    else if (c <= 256) softmax_grad_warp_rows_scalar<8><<<wgrid, 256, 0, st>>>(y, dy, dx, rows, c);
-    else if (c <= 512) softmax_grad_warp_rows_scalar<16><<<wgrid, 256, 0, st>>>(y, dy, dx, rows, c);
-    else softmax_grad_warp_rows_scalar<32><<<wgrid, 256, 0, st>>>(y, dy, dx, rows, c);
+    if (c <= 64) tsb_launch::launch(softmax_grad_warp_rows_scalar<2>, wgrid, 256, 0, st, y, dy, dx, rows, c);
+    else if (c <= 128) tsb_launch::launch(softmax_grad_warp_rows_scalar<4>, wgrid, 256, 0, st, y, dy, dx, rows, c);
+    else if (c <= 256) tsb_launch::launch(softmax_grad_warp_rows_scalar<8>, wgrid, 256, 0, st, y, dy, dx, rows, c);
+    else if (c <= 512) tsb_launch::launch(softmax_grad_warp_rows_scalar<16>, wgrid, 256, 0, st, y, dy, dx, rows, c);
+    else tsb_launch::launch(softmax_grad_warp_rows_scalar<32>, wgrid, 256, 0, st, y, dy, dx, rows, c);
     return done();
   }
   const int grid = (int)(rows < 148 * 16 ? rows : 148 * 16);
-  softmax_grad_rows<<<grid, cols >= 1024 ? 256 : 128, 0, st>>>(y, dy, dx, rows, cols);
+  tsb_launch::launch(softmax_grad_rows, grid, cols >= 1024 ? 256 : 128, 0, st, y, dy, dx, rows, cols);
   return done();
 }
 
@@ -995,7 +1010,8 @@ int tsb_masked_softmax(const float* x, const float* key_tokens, float* y, long l
     const float4* xv = reinterpret_cast<const float4*>(x);
     const float4* kv = reinterpret_cast<const float4*>(key_tokens);
     float4* yv = reinterpret_cast<float4*>(y);
-#define TSB_MSV(NV) masked_softmax_warp_rows_v4<NV><<<wgrid, 256, 0, st>>>(xv, kv, yv, rows, nvec, rows_per_batch, tq, scale, causal)
+#define TSB_MSV(NV) tsb_launch::launch(masked_softmax_warp_rows_v4<NV>, wgrid, 256, 0, st, xv, kv, yv, rows, nvec, \
+                                       rows_per_batch, tq, scale, causal)
     if (nvec <= 32) TSB_MSV(1);
     else if (nvec <= 64) TSB_MSV(2);
     else if (nvec <= 128) TSB_MSV(4);
@@ -1003,7 +1019,8 @@ int tsb_masked_softmax(const float* x, const float* key_tokens, float* y, long l
 #undef TSB_MSV
     return done();
   }
-#define TSB_MSM(NE) masked_softmax_warp_rows<NE><<<wgrid, 256, 0, st>>>(x, key_tokens, y, rows, c, rows_per_batch, tq, scale, causal)
+#define TSB_MSM(NE) tsb_launch::launch(masked_softmax_warp_rows<NE>, wgrid, 256, 0, st, x, key_tokens, y, rows, c, \
+                                       rows_per_batch, tq, scale, causal)
   if (c <= 64) TSB_MSM(2);
   else if (c <= 128) TSB_MSM(4);
   else if (c <= 256) TSB_MSM(8);
@@ -1026,7 +1043,8 @@ int tsb_scaled_softmax_grad(const float* y, const float* dy, float* dx, long lon
     const float4* yv = reinterpret_cast<const float4*>(y);
     const float4* gv = reinterpret_cast<const float4*>(dy);
     float4* dv = reinterpret_cast<float4*>(dx);
-#define TSB_SSV(NV) scaled_softmax_grad_warp_rows_v4<NV><<<wgrid, 256, 0, st>>>(yv, gv, dv, rows, nvec, scale)
+#define TSB_SSV(NV) tsb_launch::launch(scaled_softmax_grad_warp_rows_v4<NV>, wgrid, 256, 0, st, yv, gv, dv, rows, \
+                                       nvec, scale)
     if (nvec <= 32) TSB_SSV(1);
     else if (nvec <= 64) TSB_SSV(2);
     else if (nvec <= 128) TSB_SSV(4);
@@ -1034,7 +1052,7 @@ int tsb_scaled_softmax_grad(const float* y, const float* dy, float* dx, long lon
 #undef TSB_SSV
     return done();
   }
-#define TSB_SSG(NE) scaled_softmax_grad_warp_rows<NE><<<wgrid, 256, 0, st>>>(y, dy, dx, rows, c, scale)
+#define TSB_SSG(NE) tsb_launch::launch(scaled_softmax_grad_warp_rows<NE>, wgrid, 256, 0, st, y, dy, dx, rows, c, scale)
   if (c <= 64) TSB_SSG(2);
   else if (c <= 128) TSB_SSG(4);
   else if (c <= 256) TSB_SSG(8);
@@ -1051,14 +1069,14 @@ int tsb_softmax_ce(const float* x, const float* labels, float* loss, long long r
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = (int)(rows < 148 * 16 ? rows : 148 * 16);
   if (cols >= 512 && cols % 4 == 0 && cols / 4 < (1ll << 30) && aligned16(x) && aligned16(labels)) {
-    ce_rows_v4<<<grid, cols >= 8192 ? 512 : 256, 0, st>>>(reinterpret_cast<const float4*>(x),
+    tsb_launch::launch(ce_rows_v4, grid, cols >= 8192 ? 512 : 256, 0, st, reinterpret_cast<const float4*>(x),
                                                          reinterpret_cast<const float4*>(labels), rl, rows,
                                                          (int)(cols / 4));
-    mean_rows<<<1, 1024, 0, st>>>(rl, loss, rows);
+    tsb_launch::launch(mean_rows, 1, 1024, 0, st, rl, loss, rows);
     return done();
   }
-  ce_rows<<<grid, cols >= 1024 ? 256 : 128, 0, st>>>(x, labels, rl, rows, cols);
-  mean_rows<<<1, 1024, 0, st>>>(rl, loss, rows);
+  tsb_launch::launch(ce_rows, grid, cols >= 1024 ? 256 : 128, 0, st, x, labels, rl, rows, cols);
+  tsb_launch::launch(mean_rows, 1, 1024, 0, st, rl, loss, rows);
   return done();
 }
 
@@ -1067,12 +1085,13 @@ int tsb_softmax_ce_grad(const float* x, const float* labels, const float* g, flo
   if (rows <= 0 || cols <= 0) return TSB_ERR_ARG;
   const int grid = (int)(rows < 148 * 16 ? rows : 148 * 16);
   if (cols >= 512 && cols % 4 == 0 && cols / 4 < (1ll << 30) && aligned16(x) && aligned16(labels) && aligned16(dx)) {
-    ce_grad_rows_v4<<<grid, cols >= 8192 ? 512 : 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const float4*>(x), reinterpret_cast<const float4*>(labels), g,
+    tsb_launch::launch(ce_grad_rows_v4, grid, cols >= 8192 ? 512 : 256, 0, static_cast<cudaStream_t>(stream),
+                       reinterpret_cast<const float4*>(x), reinterpret_cast<const float4*>(labels), g,
         reinterpret_cast<float4*>(dx), rows, (int)(cols / 4));
     return done();
   }
-  ce_grad_rows<<<grid, cols >= 1024 ? 256 : 128, 0, static_cast<cudaStream_t>(stream)>>>(x, labels, g, dx, rows,
+  tsb_launch::launch(ce_grad_rows, grid, cols >= 1024 ? 256 : 128, 0, static_cast<cudaStream_t>(stream), x, labels, g,
+                     dx, rows,
                                                                                          cols);
   return done();
 }
