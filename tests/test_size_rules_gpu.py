@@ -66,3 +66,41 @@ def test_optimizer_tiles_of_many_tensors():
         # two products, an addition and an update in fp32, contracted or not: a few units in the last place of values < 8
         torch.testing.assert_close(v.t, v1, rtol=0, atol=2e-6)
         torch.testing.assert_close(p.t, p0 + v1, rtol=0, atol=4e-6)
+
+
+# launches whose tiles are narrowed: one tile, a ragged one, the last number of wide tiles that is halved and the first
+# that is not, and a batch; every combination of transposed operands
+@pytest.mark.parametrize("m,n,k,batch", [(64, 256, 96, 1), (130, 300, 70, 1), (5, 129, 40, 1), (128 * 74, 256, 32, 1),
+                                         (128 * 74 + 4, 256, 32, 1), (36, 132, 64, 20)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+def test_gemm_tiles_of_small_launches(m, n, k, batch, ta, tb):
+    a, b = _rand(batch, k, m) if ta else _rand(batch, m, k), _rand(batch, n, k, seed=1) if tb else _rand(batch, k, n, seed=1)
+    c = torch.full((batch, m, n), 9.0, device="cuda")
+    ctx = ndarray.gpu(0)
+    G.gemm(ndarray.from_tensor(a, ctx), ndarray.from_tensor(b, ctx), ndarray.from_tensor(c, ctx), ta, tb, _stream(),
+           batch=batch, m=m, n=n, k=k, sa=m * k, sb=n * k, sc=m * n, lda=a.shape[2], ldb=b.shape[2], ldc=n)
+    x, y = (a.transpose(1, 2) if ta else a).double(), (b.transpose(1, 2) if tb else b).double()
+    # an operand cut to 10 mantissa bits is at most 2^-10 off, so a product is 2^-9 of its magnitude; fp32 sums add less
+    assert torch.all((c.double() - x @ y).abs() <= 2.2e-3 * (x.abs() @ y.abs()) + 1e-6)
+
+
+# the same for convolutions: 7 x 7 pixels of 512 channels (4 x 2 wide tiles), a ragged width, 37 and 38 tiles of a batch
+@pytest.mark.parametrize("n,c,hw,o,k", [(8, 64, 7, 512, 3), (2, 32, 9, 200, 1), (37, 32, 11, 256, 1), (38, 32, 11, 256, 3)])
+def test_convolution_tiles_of_small_launches(n, c, hw, o, k):
+    x, w, dy = _rand(n, c, hw, hw), _rand(o, c, k, k, seed=1), _rand(n, o, hw, hw, seed=2)
+    y, dx = _arr(torch.zeros(n, o, hw, hw, device="cuda")), _arr(torch.zeros(n, c, hw, hw, device="cuda"))
+    conv = torch.nn.functional.conv2d
+    grad = torch.nn.grad.conv2d_input
+    part = ndarray.empty((2 * G.CONV_STAT_MAX_CHUNKS * o,), ndarray.gpu(0), use_pool=False)
+    chunks = G.conv2d_fwd_stats(_arr(x), _arr(w), y, k // 2, k // 2, 1, part, _stream())
+    xd, wd, dyd = x.double(), w.double(), dy.double()
+    assert torch.all((y.t.double() - conv(xd, wd, padding=k // 2)).abs()
+                     <= 2.2e-3 * conv(xd.abs(), wd.abs(), padding=k // 2) + 1e-6)
+    G.conv2d(1, dx, _arr(w), _arr(dy), k // 2, k // 2, 1, _stream())
+    assert torch.all((dx.t.double() - grad(x.shape, wd, dyd, padding=k // 2)).abs()
+                     <= 2.2e-3 * grad(x.shape, wd.abs(), dyd.abs(), padding=k // 2) + 1e-6)
+    if chunks:                         # the column sums are those of the rounded outputs, in fp32
+        planes = part.t.view(2, G.CONV_STAT_MAX_CHUNKS, o)[:, :chunks].double().sum(1)
+        ys = y.t.double()
+        torch.testing.assert_close(planes[0], ys.sum((0, 2, 3)), rtol=0, atol=1e-5 * float(ys.abs().sum((0, 2, 3)).max()))
+        torch.testing.assert_close(planes[1], ys.square().sum((0, 2, 3)), rtol=1e-5, atol=1e-5)

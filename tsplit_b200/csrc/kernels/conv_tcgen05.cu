@@ -1457,7 +1457,7 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
   if (!p.status) return TSB_ERR_LAUNCH;
   p.src = src; p.out = out; p.M = N * OH * OW; p.NC = O; p.ldc = O;
   p.kblocks = (p.K + BK - 1) / BK;
-  const int bn = O > 128 ? 256 : (O > 64 ? 128 : 64);
+  int bn = O > 128 ? 256 : (O > 64 ? 128 : 64);
   p.tiles_m = (p.M + BM - 1) / BM;
   p.tiles_n = (p.NC + bn - 1) / bn;
   CUtensorMap tm, tmi;
@@ -1497,6 +1497,14 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
         }
       }
       return launch_fwd_pair(bn, tmh, tmi, tmo, p, st);
+    }
+    const int nbn = tsb_host::narrow_tile(bn, (long long)p.tiles_m * p.tiles_n, sm_count());
+    if (nbn != bn) {
+      bn = nbn;
+      p.tiles_n = (p.NC + bn - 1) / bn;
+      bx[1] = (uint32_t)bn;
+      rc = tsb_host::make_tmap_f32(&tm, wts, 2, d, s, bx, false);
+      if (rc) return rc;
     }
     if (stats) {                // same grid arithmetic as launch<>
       const long long items = (long long)p.tiles_m * p.tiles_n;

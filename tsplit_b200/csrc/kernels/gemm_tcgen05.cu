@@ -903,7 +903,7 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
   }
-  const int bn = n > 128 ? 256 : (n > 64 ? 128 : 64);
+  int bn = n > 128 ? 256 : (n > 64 ? 128 : 64);
   GemmParams p;
   p.c = c; p.m = m; p.n = n; p.k = k; p.batch = batch; p.ldc = ldc; p.sc = sc;
   p.accumulate = accumulate;
@@ -943,6 +943,10 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
     const bool enabled = !(e && e[0] == '0');
     use_pair = enabled && bn == 256 && p.splits == 1 && m >= 256 && pair_items * 4 >= sm_count() &&
                (!trans_a || m % 32 == 0) && (trans_b || n % 32 == 0);
+  }
+  if (!use_pair) {          // (the K ranges stay those of the wide tile: results do not depend on the choice)
+    bn = tsb_host::narrow_tile(bn, (long long)p.tiles_m * p.tiles_n * batch * p.splits, sm_count());
+    p.tiles_n = (n + bn - 1) / bn;
   }
   const uint32_t bbox = use_pair ? P2_BNH : (uint32_t)bn;   // columns of B that one CTA stages
   // tensor maps (dims innermost first)
