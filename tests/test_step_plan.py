@@ -1,0 +1,207 @@
+"""The issue order of the keep-all executors on the GPU, interpreted on the host: programs of element-wise operators,
+views and joint copies give what the node-by-node NumPy oracle gives, and nothing moves past an update."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tsplit_b200 import gpu_ops as ad, ndarray, optimizer
+from tsplit_b200.executors import step_plan
+from tsplit_b200.models import lstm, mlp, resnet, transformer
+from tsplit_b200.ops import _gpu as G
+
+_UN = {G.UN_COPY: lambda x, a: x, G.UN_RELU: lambda x, a: np.maximum(x, 0), G.UN_SIGMOID: lambda x, a: 1 / (1 + np.exp(-x)),
+       G.UN_TANH: lambda x, a: np.tanh(x), G.UN_SQRT: lambda x, a: np.sqrt(x), G.UN_RSQRT: lambda x, a: 1 / np.sqrt(x),
+       G.UN_NEG: lambda x, a: -x, G.UN_ADDC: lambda x, a: x + a, G.UN_MULC: lambda x, a: x * a, G.UN_CDIV: lambda x, a: a / x}
+_BIN = {G.BIN_ADD: np.add, G.BIN_MUL: np.multiply, G.BIN_DIV: np.divide, G.BIN_SUB: np.subtract,
+        G.BIN_RELU_GRAD: lambda x, g: np.where(x > 0, g, np.where(x == 0, 0.5 * g, 0)),
+        G.BIN_ADD_RELU: lambda x, y: np.maximum(x + y, 0), G.BIN_RELU_GRAD_OUT: lambda y, g: np.where(y > 0, g, 0)}
+
+
+def _at(address, n):
+    return np.ctypeslib.as_array((ctypes.c_float * int(n)).from_address(address))
+
+
+def _pointwise(inputs, kinds, code, alpha, outs, slots, n, cols, stream):
+    assert len(inputs) <= step_plan.MAX_IN <= slots + step_plan.MAX_IN and len(outs) <= step_plan.MAX_INS
+    assert slots <= step_plan.MAX_SLOTS and len(inputs) <= slots and n % 4 == 0
+    value = [None] * slots
+    for k, (p, kind) in enumerate(zip(inputs, kinds)):
+        value[k] = _at(p, n).copy() if kind == step_plan.FULL else np.resize(_at(p, cols if kind == step_plan.ROW else 1), n)
+    for k, out in enumerate(outs):
+        op, a, b, dst = code[4 * k:4 * k + 4]
+        if op == G.UN_FILL:
+            v = np.full(n, alpha[k], np.float32)
+        elif op < 32:
+            v = _UN[op](value[a], np.float32(alpha[k])).astype(np.float32)
+        else:
+            v = _BIN[op - 32](value[a], value[b]).astype(np.float32)
+        value[dst] = v
+        if out:
+            _at(out, n)[:] = v
+
+
+class _HostPlan(step_plan.StepPlan):
+    def _node(self, n, vals, stream):
+        out = self.arrays.get(n)
+        ins = [v.numpy_view() if isinstance(v, ndarray.NDArray) else v for v in (vals[i] for i in n.inputs)]
+        n.op.compute(n, ins, out.numpy_view() if out is not None else None, True, None)
+        vals[n] = out
+        for key in ("dscale", "dbias"):
+            if "np_" + key in getattr(n, "state", {}):
+                n.state[key] = ndarray.array(n.state["np_" + key], ndarray.cpu(0))
+
+
+def _run(monkeypatch, nodes, feed, steps=1):
+    monkeypatch.setattr(G, "pointwise", _pointwise)
+    monkeypatch.setattr(G, "multi_copy", lambda s, d, st: [x.numpy_view().__setitem__(Ellipsis, y.numpy_view()) for x, y in zip(d, s)])
+    ex = ad.Executor(nodes, ctx=ndarray.cpu(0))
+    fed = {k: ndarray.array(v, ndarray.cpu(0)) for k, v in feed.items()}
+    shapes = {k: v.shape for k, v in fed.items()}
+    ex.infer_shape(shapes)
+    ex.memory_plan(shapes)
+    plan = _HostPlan(ex, set(fed))
+    for _ in range(steps):
+        vals = dict(fed)
+        plan.run(ex, vals)
+    return plan, [np.array(vals[n].numpy_view()) if isinstance(vals[n], ndarray.NDArray) else vals[n] for n in nodes]
+
+
+def _compare(monkeypatch, build, steps=1, least=0):
+    nodes, feed = build()
+    ex = ad.Executor(nodes)
+    for _ in range(steps):
+        want = ex.run(feed)
+    nodes, feed = build()
+    plan, got = _run(monkeypatch, nodes, feed, steps)
+    assert sum(1 for a in plan.actions if a[0] == "program") >= least
+    for w, g in zip(want, got):
+        if w is not None:
+            # the oracle and the interpreter round alike, but for the order in which gradients meet
+            np.testing.assert_allclose(g, w, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(w).max())))
+    return plan
+
+
+def _model(m, batch):
+    x, y = m.synthetic_batch(batch)
+    opt = optimizer.SGDOptimizer(0.1)
+    train = opt.minimize(m.loss)
+    return [m.loss, m.y, train] + m.variables, {m.X: x, m.y_: y}
+
+
+@pytest.mark.parametrize("name,least", [("lstm", 6), ("mlp", 0), ("resnet", 1), ("transformer", 2)])
+def test_models(monkeypatch, name, least):
+    def build():
+        if name == "transformer":
+            t = transformer(vocab_size=40, d_model=16, num_heads=2, d_ff=32, num_blocks=1, maxlen1=6, maxlen2=7, batch_size=3)
+            return [t.loss, t.logits] + ad.gradients(t.loss, t.variables), t.synthetic_batch()
+        m = {"lstm": lambda: lstm(steps=4, features=8, hidden=12, num_classes=5), "mlp": lambda: mlp((20, 12, 8, 4)),
+             "resnet": lambda: resnet(26, num_classes=4, image=32, width_div=16)}[name]()
+        return _model(m, 4)
+    plan = _compare(monkeypatch, build, steps=1, least=least)
+    if name == "resnet":
+        assert any(a[0] == "copies" and len(a[1]) > 10 for a in plan.actions)
+
+
+def _arrays(*shapes):
+    r = np.random.RandomState(0)
+    return [r.standard_normal(s).astype(np.float32) for s in shapes]
+
+
+@pytest.mark.parametrize("shape", [(4, 8), (3, 5), (2, 3, 4), (1, 1), (2, 4, 3, 2)])
+def test_forms_of_operands(monkeypatch, shape):
+    """Whole operands, a row, a number first and second, the same operand twice, results that are kept, read by a
+    reduction in the middle of a chain, and read through reshapes; sizes that are no multiple of four run node by node."""
+    xv, zv, bv, sv = _arrays(shape, shape, shape[-1:], (1,))
+
+    def build():
+        x, z, b = (ad.Variable(k) for k in "xzb")
+        s = ad.Variable("s", value=sv, trainable=False)
+        a = ad.relu_op(x + ad.broadcasttoTF_op(b, x))
+        c = ad.mul_op(a, a) + z
+        kept = ad.sigmoid_op(c)
+        total = ad.reduce_sum_op(kept, list(range(len(shape))))         # (1,): read back as a number
+        by_number = ad.mul_op(total, ad.tanh_op(c)) + ad.mul_op(kept, s)
+        flat = ad.array_reshape_op(ad.tanh_op(c), (-1,))
+        e = ad.array_reshape_op(ad.mul_byconst_op(flat, 0.5), shape) + kept
+        out = ad.array_reshape_op(e, (-1, 1))
+        grads = ad.gradients(ad.reduce_sum_op(ad.mul_op(out, out), [0, 1]), [x, z, b])
+        return [kept, out, flat, e, by_number] + grads, {x: xv, z: zv, b: bv, s: sv}
+    _compare(monkeypatch, build)
+
+
+def test_long_chains_are_cut(monkeypatch):
+    """More operators, inputs and live values than one program holds."""
+    vals = _arrays(*[(8, 4)] * 40)
+
+    def build():
+        xs = [ad.Variable("x%d" % i) for i in range(40)]
+        ys = [ad.tanh_op(x) for x in xs]
+        acc = ys[0]
+        for i in range(1, 40):
+            acc = ad.add_op(ad.mul_op(acc, ys[i]), ys[(7 * i) % 40])
+        return [acc], dict(zip(xs, vals))
+    _compare(monkeypatch, build, least=2)
+
+
+def test_order_around_an_update(monkeypatch):
+    """Values computed from a parameter before its update and after it, over three steps."""
+    wv, xv = _arrays((8, 4), (2, 8))
+
+    def build():
+        x, w = ad.Variable("x"), ad.Variable("w", value=wv.copy())
+        before = ad.mul_byconst_op(w, 2.0)
+        y = ad.matmul_op(x, ad.relu_op(w))
+        loss = ad.reduce_sum_op(ad.mul_op(y, y), [0, 1])
+        train = optimizer.SGDOptimizer(0.05).minimize(loss)
+        after = ad.addbyconst_op(ad.mul_byconst_op(w, 3.0), 1.0)
+        return [loss, before, train, after], {x: xv}
+    _compare(monkeypatch, build, steps=3)
+
+
+def test_a_feed_in_another_layout_runs_node_by_node(monkeypatch):
+    xv, zv = _arrays((4, 8), (4, 8))
+    x, z = ad.Variable("x"), ad.Variable("z")
+    out = ad.relu_op(ad.mul_op(x, z))
+    plan, got = _run(monkeypatch, [out], {x: xv, z: zv})
+    assert [a[0] for a in plan.actions] == ["program"]
+    import torch
+    vals = {x: ndarray.from_tensor(torch.from_numpy(np.ascontiguousarray(xv.T)).t(), ndarray.cpu(0)),
+            z: ndarray.array(zv, ndarray.cpu(0))}
+    plan.run(type("E", (), {"stream": None})(), vals)
+    np.testing.assert_array_equal(vals[out].numpy_view(), got[0])
+
+
+# one group of four; a row length that is no power of two; the last size of the short blocks and the first of the long
+# ones; a tensor past the limit for many values
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 4), (3, 20), (64 * 148, 4), (64 * 148 + 1, 4), (2049, 4096)])
+def test_programs_give_the_bits_of_the_single_kernels(shape):
+    import torch
+    ctx = ndarray.gpu(0)
+    xv, zv, bv = _arrays(shape, shape, shape[-1:])
+    x, z, b = (ad.Variable(k) for k in "xzb")
+    s = ad.Variable("s", value=np.full((1,), 0.75, np.float32), trainable=False)
+    a = ad.relu_op(x + ad.broadcasttoTF_op(b, x))
+    c = ad.sigmoid_op(ad.mul_op(a, z)) + ad.tanh_op(ad.div_op(z, ad.addbyconst_op(ad.mul_op(x, x), 1.0)))
+    d = ad.add_relu_op(ad.opposite_op(c), ad.mul_op(ad.sqrt_op(ad.mul_op(z, z)), s))
+    e = ad.relu_gradient_op(d, ad.div_const_op(2.0, ad.addbyconst_op(a, 1.5)))
+    f = ad.relu_out_gradient_op(a, ad.mul_byconst_op(e, 0.3)) + ad.array_reshape_op(ad.array_reshape_op(d, (-1,)), shape)
+    nodes = [a, c, f, ad.rsqrt_op(ad.addbyconst_op(ad.mul_op(f, f), 0.5))]
+    ex = ad.Executor(nodes, ctx=ctx)
+    feed = {k: ndarray.array(v, ctx, use_pool=False) for k, v in ((x, xv), (z, zv), (b, bv))}
+    got = [o.t.clone() for o in ex.run(feed)]
+    plan = ex._step_plan
+    assert any(k == "program" for k, _ in plan.actions)
+    vals = dict(feed)
+    vals[s] = s.tensor_value
+    for kind, what in plan.actions:
+        for n in [m for m, _ in what.members] if kind == "program" else [what]:
+            if kind == "view":
+                vals[n] = plan.arrays[n]
+            else:
+                plan.arrays[n].t.fill_(-1.0)
+                plan._node(n, vals, ex.stream)
+    ex.stream.sync()
+    for n, g in zip(nodes, got):
+        assert torch.equal(vals[n].t, g), n.desc

@@ -140,6 +140,7 @@ class Executor(object):
         self.use_graph = bool(use_graph) and self.on_device
         self._graph = None
         self._graph_feed_arrs = None
+        self._step_plan = None            # issue order of a step on the GPU (step_plan.py), built per feed shape
         # a CPU-context executor can replay its step from the native tape too (use_graph="tape"): every operator
         # of the step must have a host kernel (csrc/runtime/cpu_ops.cc), else it keeps its Python loop
         self.cpu_tape = use_graph == "tape" and ctx is not None and ctx.device_type == 1
@@ -164,6 +165,7 @@ class Executor(object):
 
     def memory_plan(self, feed_shapes):
         """One array per computed node, kept until the feed shapes change."""
+        self._step_plan = None
         self.node_to_arr_map = {}
         for node, shape in self.node_to_shape_map.items():
             if node in feed_shapes or isinstance(node.op, PlaceholderOp) or shape is None:
@@ -289,7 +291,13 @@ class Executor(object):
 
     def _run_eager(self, node_to_val):
         self._advance_device_step()
-        host_like = not self.on_device
+        if self.on_device:
+            if self._step_plan is None:
+                from .step_plan import StepPlan
+                self._step_plan = StepPlan(self, set(node_to_val))
+            self._step_plan.run(self, node_to_val)
+            self._last_vals = node_to_val
+            return
         for node in self.topo_order:
             if node in node_to_val:
                 continue
@@ -301,13 +309,10 @@ class Executor(object):
                 out = np.empty(self.node_to_shape_map[node], dtype=np.float32) \
                     if self.node_to_shape_map[node] is not None else None
                 node.op.compute(node, ins, out, True, None)
-            elif host_like:
+            else:
                 out = self.node_to_arr_map.get(node)
                 node.op.compute(node, [self._val(i) for i in ins],
                                 out.numpy_view() if out is not None else None, True, self.stream)
-            else:
-                out = self.node_to_arr_map.get(node)
-                node.op.compute(node, ins, out, False, self.stream)
             node_to_val[node] = out
         self._last_vals = node_to_val
 

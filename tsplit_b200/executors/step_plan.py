@@ -1,0 +1,331 @@
+"""The order in which the keep-all executors issue a step on the GPU, worked out once per feed shape.
+
+Three things are taken out of the node-by-node loop, none of which changes a value:
+
+* element-wise operators over the same elements are collected and run as one ``tsb_pointwise`` program, at the first
+  node that needs one of their results; results that nobody outside the program reads are not stored;
+* a reshape of a row-major array is a view of it;
+* the small parameter gradients that a normalisation operator hands out from its own buffers are copied in one launch.
+
+Element-wise nodes are taken as soon as their inputs are there, the others in creation order, and nothing moves past a
+node with effects of its own (an optimizer update, a collective, a swap).  The memory-planning executors have
+schedules of their own and do not use this.
+"""
+from __future__ import annotations
+
+import heapq
+
+from .. import ndarray
+from ..ops import _gpu as G
+from ..ops.elementwise import _Binary, _Unary, _is_scalar_shape
+from ..ops.misc import PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
+from ..ops.norm import BatchNormGradScaleOp
+from ..ops.shape import AddBroadcastOp, ReshapeOp, ReshapeGradientOp
+
+FULL, ROW, SCALAR = 0, 1, 2
+_BINARY = 32                       # instruction code of binary operator 0
+MAX_IN, MAX_INS, MAX_SLOTS = 32, 64, 48
+#: value slots of a program over a tensor that does not fit in L2: more of them leave too few threads to cover DRAM
+MAX_SLOTS_LARGE, LARGE = 12, 8 << 20
+
+
+def _key(arr):
+    """What two arrays share when element i of one belongs to element i of the other in memory order."""
+    t = arr.t
+    if t.is_contiguous():
+        return ("rows", t.numel())
+    return (arr.shape, arr.strides) if arr.is_dense() else None
+
+
+def _code(node):
+    op = node.op
+    if isinstance(op, AddBroadcastOp):
+        return _BINARY + G.BIN_ADD, 0.0
+    if isinstance(op, _FillLike):
+        return G.UN_FILL, float(op.value)
+    if isinstance(op, _Binary):
+        return _BINARY + op.gpu_code, 0.0
+    return op.gpu_code, 0.0 if node.const_attr is None else float(node.const_attr)
+
+
+class Program(object):
+    """Element-wise nodes collected so far (``members``, in order) and what they read from outside."""
+
+    def __init__(self, key, numel):
+        self.key, self.numel = key, numel
+        self.members, self.values, self.inputs = [], {}, []      # values: node -> index of its instruction
+        self.kinds, self.slot_of_input, self.cols = [], {}, 0
+
+    def close(self, stored):
+        """Assigns value slots (``stored``: the members whose results are read outside)."""
+        last = {}
+        for k, (node, ins) in enumerate(self.members):
+            for ref in ins:
+                last[ref] = k
+        n_in = len(self.inputs)
+        free, used = [], n_in
+        where = {("in", j): j for j in range(n_in)}
+        code, self.alpha, self.out = [], [], []
+        for k, (node, ins) in enumerate(self.members):
+            op, alpha = _code(node)
+            at = [where[ref] for ref in ins]
+            for ref in dict.fromkeys(ins):
+                if last[ref] == k:
+                    free.append(where[ref])          # an instruction reads its operands before it writes
+            if free:
+                dst = free.pop()
+            else:
+                dst, used = used, used + 1
+            where[("val", k)] = dst
+            if ("val", k) not in last:
+                free.append(dst)
+            a = at[0] if at else 0
+            code += [op, a, at[1] if len(at) > 1 else a, dst]
+            self.alpha.append(alpha)
+            self.out.append(node if node in stored else None)
+        self.slots = max(used, 1)
+        self.code = bytes(code)
+        return self.slots
+
+    def run(self, vals, arrays, stream):
+        """False when an input is not laid out as planned (a feed may be): the caller runs the nodes one by one."""
+        ptrs = []
+        for node, kind in zip(self.inputs, self.kinds):
+            v = vals[node]
+            if kind == FULL:
+                if _key(v) != self.key:
+                    return False
+            elif not v.is_contiguous():
+                return False
+            p = v.ptr
+            if kind != SCALAR and p & 15:
+                return False
+            ptrs.append(p)
+        outs = [arrays[n].ptr if n is not None else 0 for n in self.out]
+        if any(p & 15 for p in outs):
+            return False
+        G.pointwise(ptrs, self.kinds, self.code, self.alpha, outs, self.slots, self.numel, self.cols, stream)
+        return True
+
+
+class StepPlan(object):
+    def __init__(self, ex, fed):
+        self.arrays = ex.node_to_arr_map
+        self.shapes = ex.node_to_shape_map
+        self.placeholders = [n for n in ex.topo_order if isinstance(n.op, PlaceholderOp) and n not in fed]
+        self.evals = set(ex.eval_node_list)
+        self.external = set(self.placeholders) | set(fed)
+        self.users = {}
+        for n in ex.topo_order:
+            if n not in self.external:
+                for i in n.inputs:
+                    self.users.setdefault(i, []).append(n)
+        self.root = {}                    # view -> the node whose array it looks at
+        self.actions = []
+        self.open = {}                    # key -> Program that still collects
+        self.home = {}                    # node -> its open Program
+        self.copies = []
+        segment = []
+        for n in ex.topo_order:
+            if n in self.external:
+                continue
+            if self._has_effects(n):
+                self._schedule(segment)
+                segment = []
+                self._flush_all()
+                self.actions.append(("node", n))
+            else:
+                segment.append(n)
+        self._schedule(segment)
+        self._flush_all()
+
+    @staticmethod
+    def _has_effects(n):
+        return (not type(n.op).__module__.startswith("tsplit_b200.ops.") or isinstance(n.op, (SwapInOp, SwapOutOp))
+                or n.phase == "update")
+
+    # -- what a node is -------------------------------------------------------------------
+    def _is_view(self, n):
+        """Row-major reshapes of computed arrays (a result that the caller keeps stays an array of its own)."""
+        if not isinstance(n.op, (ReshapeOp, ReshapeGradientOp)) or n in self.evals:
+            return False
+        src, arr = self.arrays.get(n.inputs[0]), self.arrays.get(n)
+        return (src is not None and arr is not None and n.inputs[0] not in self.evals and src.t.is_contiguous()
+                and arr.t.is_contiguous() and src.t.numel() == arr.t.numel())
+
+    def _operands(self, n):
+        """[(node, kind)] when ``n`` can be part of a program, else None."""
+        arr = self.arrays.get(n)
+        if arr is None or not isinstance(n.op, (_Binary, _Unary, _FillLike, AddBroadcastOp)):
+            return None
+        key, numel = _key(arr), arr.t.numel()
+        if key is None or numel == 0 or numel % 4:
+            return None
+        if isinstance(n.op, _FillLike):
+            return []
+        res = []
+        for j, i in enumerate(n.inputs):
+            shape, src = tuple(self.shapes[i]), self.arrays.get(i)
+            if shape == arr.shape and (src is None or _key(src) == key):
+                res.append((i, FULL))
+            elif isinstance(n.op, AddBroadcastOp) and j == 1:
+                cols = arr.shape[-1]
+                if key[0] != "rows" or cols % 4 or shape[-1] != cols or ndarray._numel(shape) != cols:
+                    return None
+                res.append((i, ROW))
+            elif _is_scalar_shape(shape) and isinstance(n.op, _Binary):
+                res.append((i, SCALAR))
+            else:
+                return None
+        return res
+
+    # -- scheduling ------------------------------------------------------------------------
+    def _schedule(self, nodes):
+        inside = set(nodes)
+        waits = {n: len({i for i in n.inputs if i in inside}) for n in nodes}
+        light, heavy = [], []             # ready nodes: those that cost no launch of their own, the others
+
+        def ready(n):
+            cls = "view" if self._is_view(n) else "copy" if isinstance(n.op, BatchNormGradScaleOp) else None
+            ops = None if cls else self._operands(n)
+            heapq.heappush(light if cls or ops is not None else heavy, (n.id, n, cls, ops))
+        for n in nodes:
+            if waits[n] == 0:
+                ready(n)
+        while light or heavy:
+            if light:
+                _, n, cls, ops = heapq.heappop(light)
+                if cls == "view":
+                    self._view(n)
+                elif cls == "copy":
+                    self._need(n.inputs[0])
+                    self.copies.append(n)
+                else:
+                    self._collect(n, ops)
+            else:
+                _, n, _, _ = heapq.heappop(heavy)
+                for i in n.inputs:
+                    self._need(i)
+                self.actions.append(("node", n))
+            for u in set(self.users.get(n, ())):
+                if u in inside:
+                    waits[u] -= 1
+                    if waits[u] == 0:
+                        ready(u)
+
+    def _view(self, n):
+        src = n.inputs[0]
+        self.root[n] = self.root.get(src, src)
+        base, own = self.arrays[src], self.arrays[n]
+        # (with the strides of the array it replaces: kernels read those of dimensions of one element, too)
+        view = ndarray.NDArray(base.t.as_strided(own.shape, own.strides, base.t.storage_offset()), base.ctx, owns=False)
+        view._base = base                  # the bytes live as long as anything looks at them
+        self.arrays[n] = view
+        self.actions.append(("view", n))
+
+    def _need(self, i):
+        """``i``'s array is read by something outside its program: run that now."""
+        i = self.root.get(i, i)
+        if i in self.home:
+            self._flush(self.home[i])
+        elif i in self.copies:
+            self._flush_copies()
+
+    def _collect(self, n, operands):
+        arr = self.arrays[n]
+        key = _key(arr)
+        prog = self.open.get(key)
+        roots = [self.root.get(i, i) for i, _ in operands]
+        for i, r, (_, kind) in zip(n.inputs, roots, operands):
+            if prog is None or self.home.get(r) is not prog or kind != FULL:
+                self._need(i)              # computed by another program, or read in another way than its values lie
+        prog = self.open.get(key)          # (the call above may have run it)
+        new = [r for r in dict.fromkeys(roots) if prog is None or self.home.get(r) is not prog]
+        limit = MAX_SLOTS_LARGE if arr.t.numel() >= LARGE else MAX_SLOTS
+        cols = arr.shape[-1] if any(k == ROW for _, k in operands) else 0
+        if prog is not None and (len(prog.inputs) + len(new) > min(MAX_IN, limit - 4) or len(prog.members) >= MAX_INS
+                                 or (cols and prog.cols and prog.cols != cols) or self._slots_with(prog, n) > limit):
+            self._flush(prog)
+            prog = None
+        if prog is None:
+            prog = self.open[key] = Program(key, arr.t.numel())
+        refs = []
+        for r, (_, kind) in zip(roots, operands):
+            if self.home.get(r) is prog and kind == FULL:
+                refs.append(("val", prog.values[r]))
+                continue
+            if (r, kind) not in prog.slot_of_input:
+                prog.slot_of_input[(r, kind)] = len(prog.inputs)
+                prog.inputs.append(r)
+                prog.kinds.append(kind)
+            refs.append(("in", prog.slot_of_input[(r, kind)]))
+        prog.cols = prog.cols or cols
+        prog.values[n] = len(prog.members)
+        prog.members.append((n, refs))
+        self.home[n] = prog
+
+    def _slots_with(self, prog, n):
+        """Upper bound of the slots after one more member: every value still read later holds one."""
+        inside = {m for m, _ in prog.members}
+        inside.add(n)
+        live = sum(1 for m, _ in prog.members if any(u not in inside for u in self.users.get(m, ())))
+        return len(prog.inputs) + live + 3
+
+    def _flush(self, prog):
+        del self.open[prog.key]
+        members = [m for m, _ in prog.members]
+        inside = set(members)
+        for m in members:
+            del self.home[m]
+
+        def read_outside(m):
+            return m in self.evals or any(u not in inside for u in self.users.get(m, ()))
+        # (views count as outside: their readers are)
+        stored = {m for m in members if read_outside(m)}
+        if len(members) == 1 or prog.close(stored) > MAX_SLOTS:
+            self.actions += [("node", m) for m in members]
+        else:
+            self.actions.append(("program", prog))
+
+    def _flush_copies(self):
+        for lo in range(0, len(self.copies), 64):
+            self.actions.append(("copies", self.copies[lo:lo + 64]))
+        self.copies = []
+
+    def _flush_all(self):
+        for prog in list(self.open.values()):
+            self._flush(prog)
+        self._flush_copies()
+
+    # -- execution --------------------------------------------------------------------------
+    def run(self, ex, vals):
+        for n in self.placeholders:
+            vals[n] = ex._placeholder_value(n)
+        stream = ex.stream
+        for what, x in self.actions:
+            if what == "node":
+                self._node(x, vals, stream)
+            elif what == "view":
+                vals[x] = self.arrays[x]
+            elif what == "program":
+                if x.run(vals, self.arrays, stream):
+                    for m, _ in x.members:
+                        vals[m] = self.arrays[m]
+                else:
+                    for m, _ in x.members:
+                        self._node(m, vals, stream)
+            else:
+                src = [n.inputs[0].state[n.op.key] for n in x]
+                dst = [self.arrays[n] for n in x]
+                if all(a.is_dense() and a.same_layout(b) for a, b in zip(src, dst)):
+                    G.multi_copy(src, dst, stream)
+                    for n in x:
+                        vals[n] = self.arrays[n]
+                else:
+                    for n in x:
+                        self._node(n, vals, stream)
+
+    def _node(self, n, vals, stream):
+        out = self.arrays.get(n)
+        n.op.compute(n, [vals[i] for i in n.inputs], out, False, stream)
+        vals[n] = out

@@ -163,6 +163,24 @@ def binary_dev_scalar(code, a, scalar, y, stream, scalar_first=False):
         binary_bcast(code, a.ptr, a.strides, scalar.ptr, zero, y, stream)
 
 
+def pointwise(inputs, kinds, code, alpha, outs, slots, n, cols, stream):
+    """One launch of a program of element-wise operators (see ``csrc/kernels/pointwise_program.cu``): ``inputs`` /
+    ``outs`` are device addresses (an out of 0: the value is not stored), ``code`` four bytes an instruction."""
+    ni, no = len(inputs), len(outs)
+    rc = lib().tsb_pointwise(c_int(ni), (c_void_p * max(ni, 1))(*inputs), (c_int * max(ni, 1))(*kinds), c_int(no),
+                             ctypes.c_char_p(code), (c_float * no)(*alpha), (c_void_p * no)(*outs), c_int(slots),
+                             c_int64(n), c_int64(cols), _s(stream))
+    _check(rc, "pointwise")
+
+
+def multi_copy(srcs, dsts, stream):
+    """Up to 64 short dense arrays copied in one launch."""
+    n = len(srcs)
+    rc = lib().tsb_multi_copy(c_int(n), (c_void_p * n)(*[a.ptr for a in srcs]), (c_void_p * n)(*[a.ptr for a in dsts]),
+                              (c_int64 * n)(*[_numel(a.shape) for a in srcs]), _s(stream))
+    _check(rc, "multi_copy")
+
+
 def where(c, a, b, y, stream):
     assert _flat_ok(c, a, b, y), "where: operands must share one dense layout"
     _check(lib().tsb_where(_p(c), _p(a), _p(b), _p(y), c_int64(_numel(y.shape)), _s(stream)), "where")
