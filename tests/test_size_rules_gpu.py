@@ -104,3 +104,33 @@ def test_convolution_tiles_of_small_launches(n, c, hw, o, k):
         ys = y.t.double()
         torch.testing.assert_close(planes[0], ys.sum((0, 2, 3)), rtol=0, atol=1e-5 * float(ys.abs().sum((0, 2, 3)).max()))
         torch.testing.assert_close(planes[1], ys.square().sum((0, 2, 3)), rtol=1e-5, atol=1e-5)
+
+
+# the shortest long row, the last that is not staged, the first and the last that are and the first past them; fewer
+# rows than blocks and more; an id outside the classes
+@pytest.mark.parametrize("cols", [512, 8188, 8192, 32000, 51200, 51204])
+@pytest.mark.parametrize("rows", [1, 700])
+def test_cross_entropy_of_long_rows(rows, cols):
+    ctx = ndarray.gpu(0)
+    x = 3 * _rand(rows, cols)
+    ids = torch.randint(0, cols, (rows,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).float()
+    if rows > 1:
+        ids[1], ids[2], ids[3] = cols, 0, cols - 1
+    on, off = np.float32(0.9) + np.float32(0.1 / cols), np.float32(0.1 / cols)
+    lab = torch.full((rows, cols), float(off), device="cuda")
+    inside = ids < cols
+    lab[inside, ids[inside].long()] = float(on)
+    g = torch.full((1,), 0.5, device="cuda")
+    dense, smooth = [[torch.zeros(1, device="cuda"), torch.zeros(rows, cols, device="cuda")] for _ in range(2)]
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    G.softmax_ce(a(x), a(lab), a(dense[0]), _stream())
+    G.softmax_ce_grad(a(x), a(lab), a(g), a(dense[1]), _stream())
+    assert G.softmax_ce_smooth(a(x), a(ids), float(on), float(off), a(smooth[0]), _stream())
+    assert G.softmax_ce_grad_smooth(a(x), a(ids), float(on), float(off), a(g), a(smooth[1]), _stream())
+    assert torch.equal(dense[1], smooth[1])
+    lp = torch.log_softmax(x.double(), 1)
+    ref = -(lab.double() * lp).sum(1).mean().reshape(1)
+    # fp32 sums of some 10^4 terms of one sign per row, and the fast exponential's 2^-21
+    for loss in (dense[0], smooth[0]):
+        torch.testing.assert_close(loss.double(), ref, rtol=2e-5, atol=1e-5)
+    torch.testing.assert_close(dense[1].double(), (lp.exp() - lab.double()) * 0.5 / rows, rtol=1e-4, atol=1e-6 * 0.5 / rows)

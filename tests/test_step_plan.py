@@ -52,8 +52,24 @@ class _HostPlan(step_plan.StepPlan):
                 n.state[key] = ndarray.array(n.state["np_" + key], ndarray.cpu(0))
 
 
-def _run(monkeypatch, nodes, feed, steps=1):
+def _smooth(grad, taken):
+    """``softmax_ce_smooth`` / ``softmax_ce_grad_smooth`` in NumPy; ``taken``: False as for a shape it does not cover."""
+    def run(logits, ids, on, off, *rest):
+        if not taken:
+            return False
+        x, out = logits.numpy_view(), rest[1 if grad else 0].numpy_view()
+        lab = np.where(np.arange(x.shape[1])[None, :] == ids.numpy_view().reshape(-1, 1), np.float32(on), np.float32(off))
+        p = np.exp(x - x.max(1, keepdims=True))
+        p /= p.sum(1, keepdims=True)
+        out[...] = (p - lab) * rest[0].numpy_view() / x.shape[0] if grad else np.mean(-(lab * np.log(p)).sum(1))
+        return True
+    return run
+
+
+def _run(monkeypatch, nodes, feed, steps=1, taken=True):
     monkeypatch.setattr(G, "pointwise", _pointwise)
+    monkeypatch.setattr(G, "softmax_ce_smooth", _smooth(False, taken))
+    monkeypatch.setattr(G, "softmax_ce_grad_smooth", _smooth(True, taken))
     monkeypatch.setattr(G, "multi_copy", lambda s, d, st: [x.numpy_view().__setitem__(Ellipsis, y.numpy_view()) for x, y in zip(d, s)])
     ex = ad.Executor(nodes, ctx=ndarray.cpu(0))
     fed = {k: ndarray.array(v, ndarray.cpu(0)) for k, v in feed.items()}
@@ -67,13 +83,13 @@ def _run(monkeypatch, nodes, feed, steps=1):
     return plan, [np.array(vals[n].numpy_view()) if isinstance(vals[n], ndarray.NDArray) else vals[n] for n in nodes]
 
 
-def _compare(monkeypatch, build, steps=1, least=0):
+def _compare(monkeypatch, build, steps=1, least=0, taken=True):
     nodes, feed = build()
     ex = ad.Executor(nodes)
     for _ in range(steps):
         want = ex.run(feed)
     nodes, feed = build()
-    plan, got = _run(monkeypatch, nodes, feed, steps)
+    plan, got = _run(monkeypatch, nodes, feed, steps, taken)
     assert sum(1 for a in plan.actions if a[0] == "program") >= least
     for w, g in zip(want, got):
         if w is not None:
@@ -170,6 +186,38 @@ def test_a_feed_in_another_layout_runs_node_by_node(monkeypatch):
             z: ndarray.array(zv, ndarray.cpu(0))}
     plan.run(type("E", (), {"stream": None})(), vals)
     np.testing.assert_array_equal(vals[out].numpy_view(), got[0])
+
+
+@pytest.mark.parametrize("form", ["plain", "smooth", "shifted twice", "kept", "read elsewhere", "two losses", "fed"])
+@pytest.mark.parametrize("taken", [True, False])
+def test_labels_from_ids(monkeypatch, form, taken):
+    """One-hot labels that only cross-entropies read are not made; all others are."""
+    xv, yv = _arrays((6, 12), (6, 12))
+    ids = np.array([[0, 3, 11], [5, 5, 2]], np.float32)
+
+    def build():
+        x, y, i = (ad.Variable(k) for k in "xyi")
+        lab = ad.array_reshape_op(ad.one_hot_op(i, 12), (-1, 12))
+        if form != "plain":
+            lab = ad.addbyconst_op(ad.mul_byconst_op(lab, 0.9), 0.1 / 12)
+        if form == "shifted twice":
+            lab = ad.mul_byconst_op(ad.addbyconst_op(lab, 0.25), 0.5)
+        loss = ad.softmaxcrossentropy_op(x, lab)
+        nodes = [loss] + ad.gradients(loss, [x])
+        feed = {x: xv, i: ids}
+        if form == "kept":
+            nodes.append(lab)
+        if form == "read elsewhere":
+            nodes.append(ad.reduce_sum_op(lab, [0]))
+        if form == "two losses":
+            feed[y] = yv
+            nodes.append(ad.softmaxcrossentropy_op(y, lab))
+        if form == "fed":
+            feed[lab] = np.abs(yv)
+        return nodes, feed
+    plan = _compare(monkeypatch, build, taken=taken)
+    made = form in ("kept", "read elsewhere", "fed")
+    assert sum(1 for a in plan.actions if a[0] == "smooth") == (0 if made else 3 if form == "two losses" else 2)
 
 
 # one group of four; a row length that is no power of two; the last size of the short blocks and the first of the long

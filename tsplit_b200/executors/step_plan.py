@@ -1,11 +1,12 @@
 """The order in which the keep-all executors issue a step on the GPU, worked out once per feed shape.
 
-Three things are taken out of the node-by-node loop, none of which changes a value:
+Four things are taken out of the node-by-node loop, none of which changes a value:
 
 * element-wise operators over the same elements are collected and run as one ``tsb_pointwise`` program, at the first
   node that needs one of their results; results that nobody outside the program reads are not stored;
 * a reshape of a row-major array is a view of it;
-* the small parameter gradients that a normalisation operator hands out from its own buffers are copied in one launch.
+* the small parameter gradients that a normalisation operator hands out from its own buffers are copied in one launch;
+* one-hot labels, scaled and shifted (label smoothing), that only a cross-entropy reads are not made: it takes the ids.
 
 Element-wise nodes are taken as soon as their inputs are there, the others in creation order, and nothing moves past a
 node with effects of its own (an optimizer update, a collective, a swap).  The memory-planning executors have
@@ -15,10 +16,13 @@ from __future__ import annotations
 
 import heapq
 
+import numpy as np
+
 from .. import ndarray
 from ..ops import _gpu as G
-from ..ops.elementwise import _Binary, _Unary, _is_scalar_shape
-from ..ops.misc import PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
+from ..ops.elementwise import AddConstOp, MulConstOp, _Binary, _Unary, _is_scalar_shape
+from ..ops.loss import SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp
+from ..ops.misc import OneHotOp, PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
 from ..ops.norm import BatchNormGradScaleOp
 from ..ops.shape import AddBroadcastOp, ReshapeOp, ReshapeGradientOp
 
@@ -120,6 +124,10 @@ class StepPlan(object):
             if n not in self.external:
                 for i in n.inputs:
                     self.users.setdefault(i, []).append(n)
+        self.smooth, self.elided = {}, set()
+        for n in ex.topo_order:
+            if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
+                self._smooth_labels(n)
         self.root = {}                    # view -> the node whose array it looks at
         self.actions = []
         self.open = {}                    # key -> Program that still collects
@@ -179,6 +187,40 @@ class StepPlan(object):
                 return None
         return res
 
+    def _smooth_labels(self, ce):
+        """When ``ce``'s labels are ``one_hot(ids) * a + b`` (any number of constants, reshapes that keep the classes)
+        and nothing but cross-entropies over them reads any of it: remember ids and the two values."""
+        labels = cur = ce.inputs[1]
+        chain, consts = [], []
+        while True:
+            if cur in self.external or cur in self.evals or self._has_effects(cur) or self.arrays.get(cur) is None:
+                return
+            chain.append(cur)
+            if isinstance(cur.op, OneHotOp):
+                break
+            if isinstance(cur.op, (AddConstOp, MulConstOp)):
+                consts.append((isinstance(cur.op, MulConstOp), np.float32(cur.const_attr)))
+            elif not (isinstance(cur.op, ReshapeOp) and self.arrays[cur].t.is_contiguous()):
+                return
+            cur = cur.inputs[0]
+            if tuple(self.shapes[cur])[-1:] != tuple(self.shapes[labels])[-1:]:
+                return
+        readers = [u for u in self.users.get(labels, ())]
+        if len(self.shapes[labels]) != 2 or not all(
+                isinstance(u.op, (SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp)) and u.inputs[1] is labels
+                and u.inputs.count(labels) == 1 for u in readers):
+            return
+        if any(u not in chain for m in chain[1:] for u in self.users.get(m, ())):
+            return
+        values = []
+        for v in (np.float32(1), np.float32(0)):
+            for mul, c in reversed(consts):
+                v = np.float32(v * c) if mul else np.float32(v + c)
+            values.append(float(v))
+        self.elided.update(chain)
+        for u in readers:
+            self.smooth[u] = (cur.inputs[0], values[0], values[1], chain[::-1])
+
     # -- scheduling ------------------------------------------------------------------------
     def _schedule(self, nodes):
         inside = set(nodes)
@@ -186,7 +228,7 @@ class StepPlan(object):
         light, heavy = [], []             # ready nodes: those that cost no launch of their own, the others
 
         def ready(n):
-            cls = "view" if self._is_view(n) else "copy" if isinstance(n.op, BatchNormGradScaleOp) else None
+            cls = "elided" if n in self.elided else "view" if self._is_view(n) else "copy" if isinstance(n.op, BatchNormGradScaleOp) else None
             ops = None if cls else self._operands(n)
             heapq.heappush(light if cls or ops is not None else heavy, (n.id, n, cls, ops))
         for n in nodes:
@@ -195,7 +237,9 @@ class StepPlan(object):
         while light or heavy:
             if light:
                 _, n, cls, ops = heapq.heappop(light)
-                if cls == "view":
+                if cls == "elided":
+                    pass
+                elif cls == "view":
                     self._view(n)
                 elif cls == "copy":
                     self._need(n.inputs[0])
@@ -206,7 +250,9 @@ class StepPlan(object):
                 _, n, _, _ = heapq.heappop(heavy)
                 for i in n.inputs:
                     self._need(i)
-                self.actions.append(("node", n))
+                if n in self.smooth:
+                    self._need(self.smooth[n][0])
+                self.actions.append(("smooth" if n in self.smooth else "node", n))
             for u in set(self.users.get(n, ())):
                 if u in inside:
                     waits[u] -= 1
@@ -307,6 +353,8 @@ class StepPlan(object):
                 self._node(x, vals, stream)
             elif what == "view":
                 vals[x] = self.arrays[x]
+            elif what == "smooth":
+                self._smooth(x, vals, stream)
             elif what == "program":
                 if x.run(vals, self.arrays, stream):
                     for m, _ in x.members:
@@ -324,6 +372,20 @@ class StepPlan(object):
                 else:
                     for n in x:
                         self._node(n, vals, stream)
+
+    def _smooth(self, n, vals, stream):
+        ids, on, off, chain = self.smooth[n]
+        x, i, out = vals[n.inputs[0]], vals[ids], self.arrays[n]
+        ok = x.is_contiguous() and i.is_contiguous() and out.is_contiguous()
+        if ok and isinstance(n.op, SoftmaxCrossEntropyOp):
+            ok = G.softmax_ce_smooth(x, i, on, off, out, stream)
+        elif ok:
+            ok = G.softmax_ce_grad_smooth(x, i, on, off, vals[n.inputs[2]], out, stream)
+        if ok:
+            vals[n] = out
+            return
+        for m in chain + [n]:
+            self._node(m, vals, stream)
 
     def _node(self, n, vals, stream):
         out = self.arrays.get(n)

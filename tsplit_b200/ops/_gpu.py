@@ -241,6 +241,25 @@ def softmax_ce_grad(logits, labels, g, dx, stream):
                                      _s(stream)), "softmax_ce_grad")
 
 
+def softmax_ce_smooth(logits, ids, on, off, loss, stream):
+    """``softmax_ce`` with labels that are ``on`` at a row's class id and ``off`` elsewhere; False: not this shape."""
+    rows, cols = logits.shape
+    rc = lib().tsb_softmax_ce_smooth(_p(logits), _p(ids), c_float(on), c_float(off), _p(loss), c_int64(rows),
+                                     c_int64(cols), _s(stream))
+    if rc != 2:
+        _check(rc, "softmax_ce_smooth")
+    return rc == 0
+
+
+def softmax_ce_grad_smooth(logits, ids, on, off, g, dx, stream):
+    rows, cols = logits.shape
+    rc = lib().tsb_softmax_ce_grad_smooth(_p(logits), _p(ids), c_float(on), c_float(off), _p(g), _p(dx), c_int64(rows),
+                                          c_int64(cols), _s(stream))
+    if rc != 2:
+        _check(rc, "softmax_ce_grad_smooth")
+    return rc == 0
+
+
 def one_hot(idx, y, num_classes, stream):
     _check(lib().tsb_one_hot(_p(idx), _p(y), c_int64(_numel(idx.shape)), c_int64(num_classes), _s(stream)),
            "one_hot")
