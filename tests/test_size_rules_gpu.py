@@ -134,3 +134,22 @@ def test_cross_entropy_of_long_rows(rows, cols):
     for loss in (dense[0], smooth[0]):
         torch.testing.assert_close(loss.double(), ref, rtol=2e-5, atol=1e-5)
     torch.testing.assert_close(dense[1].double(), (lp.exp() - lab.double()) * 0.5 / rows, rtol=1e-4, atol=1e-6 * 0.5 / rows)
+
+
+# outputs that leave by TMA store: ragged rows and columns of a block, one column block and many, batches, several
+# splits; and those whose strides or sums do not allow it (a row of 130 + 1 floats, a base 4 bytes in, accumulation)
+@pytest.mark.parametrize("m,n,k,batch,ldc,shift,accumulate", [
+    (129, 68, 40, 1, 68, 0, False), (300, 260, 64, 3, 260, 0, False), (31, 12, 33, 5, 16, 0, False),
+    (64, 256, 1024, 1, 256, 0, False), (512, 520, 96, 1, 640, 0, False), (130, 100, 64, 2, 131, 0, False),
+    (130, 100, 64, 2, 132, 1, False), (130, 100, 64, 2, 132, 0, True), (1, 4, 4, 1, 4, 0, False)])
+def test_gemm_output_forms(m, n, k, batch, ldc, shift, accumulate):
+    ctx = ndarray.gpu(0)
+    a, b = _rand(batch, m, k), _rand(batch, k, n, seed=1)
+    room = torch.full((shift + batch * m * ldc + 8,), 2.0, device="cuda")
+    c = room[shift:shift + batch * m * ldc].view(batch, m, ldc)
+    G.gemm(ndarray.from_tensor(a, ctx), ndarray.from_tensor(b, ctx), ndarray.from_tensor(c, ctx), False, False, _stream(),
+           batch=batch, m=m, n=n, k=k, sa=m * k, sb=n * k, sc=m * ldc, lda=k, ldb=n, ldc=ldc, accumulate=accumulate)
+    x, y = a.double(), b.double()
+    want = x @ y + (2.0 if accumulate else 0.0)
+    assert torch.all((c[:, :, :n].double() - want).abs() <= 2.2e-3 * (x.abs() @ y.abs()) + 1e-6)
+    assert torch.all(c[:, :, n:] == 2) and torch.all(room[:shift] == 2) and torch.all(room[shift + batch * m * ldc:] == 2)
