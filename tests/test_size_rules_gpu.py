@@ -153,3 +153,21 @@ def test_gemm_output_forms(m, n, k, batch, ldc, shift, accumulate):
     want = x @ y + (2.0 if accumulate else 0.0)
     assert torch.all((c[:, :, :n].double() - want).abs() <= 2.2e-3 * (x.abs() @ y.abs()) + 1e-6)
     assert torch.all(c[:, :, n:] == 2) and torch.all(room[:shift] == 2) and torch.all(room[shift + batch * m * ldc:] == 2)
+
+
+# overlapping windows: tiles cut at both edges, one tile, windows that skip pixels, several channel blocks with a ragged
+# one, padding as wide as the window allows, and windows too large for a tile's shared memory (two passes)
+@pytest.mark.parametrize("n,c,h,w,k,pad,stride", [(2, 4, 17, 33, 3, 1, 2), (1, 36, 16, 16, 3, 1, 2), (1, 8, 15, 31, 3, 0, 2),
+                                                  (2, 8, 20, 18, 3, 1, 1), (1, 8, 35, 20, 2, 0, 3), (1, 64, 9, 40, 5, 2, 2),
+                                                  (1, 4, 24, 24, 9, 4, 1), (1, 4, 40, 40, 15, 7, 1), (3, 4, 1, 1, 1, 0, 1)])
+def test_max_pool_gradient_tiles(n, c, h, w, k, pad, stride):
+    x = torch.round(_rand(n, c, h, w) * 2) / 2                       # ties on purpose: the first maximum takes all
+    ref_x = x.double().requires_grad_()
+    ref_y = torch.nn.functional.max_pool2d(ref_x, k, stride, pad)
+    dy = torch.round(_rand(*ref_y.shape, seed=1) * 8) / 8            # sums of eighths are exact
+    y, dx = _arr(ref_y.detach().float()), _arr(torch.full_like(x, 7.0))
+    G.pool_grad(0, _arr(x), y, _arr(dy), dx, k, k, pad, stride, _stream())
+    # torch gives a tie to the last or first maximum depending on the layout, so the oracle is the library's own
+    from tsplit_b200.ops.pool import np_max_pool_grad
+    want = np_max_pool_grad(x.cpu().numpy(), ref_y.detach().cpu().numpy(), dy.cpu().numpy(), k, k, pad, stride)
+    assert torch.equal(dx.t.cpu(), torch.from_numpy(want))
