@@ -66,8 +66,18 @@ def _smooth(grad, taken):
     return run
 
 
+def _gemm_group(products, ta, tb, stream):
+    assert 2 <= len(products) <= step_plan.MAX_GROUP
+    for a, b, c, m, n, k in products:
+        x, y = a.numpy_view(), b.numpy_view()
+        c.numpy_view()[...] = np.matmul(x.T if ta else x, y.T if tb else y)
+        assert c.shape == (m, n) and k <= step_plan.GROUP_K
+    return True
+
+
 def _run(monkeypatch, nodes, feed, steps=1, taken=True):
     monkeypatch.setattr(G, "pointwise", _pointwise)
+    monkeypatch.setattr(G, "gemm_group", _gemm_group if taken else lambda *a: False)
     monkeypatch.setattr(G, "softmax_ce_smooth", _smooth(False, taken))
     monkeypatch.setattr(G, "softmax_ce_grad_smooth", _smooth(True, taken))
     monkeypatch.setattr(G, "multi_copy", lambda s, d, st: [x.numpy_view().__setitem__(Ellipsis, y.numpy_view()) for x, y in zip(d, s)])
@@ -115,6 +125,7 @@ def test_models(monkeypatch, name, least):
              "resnet": lambda: resnet(26, num_classes=4, image=32, width_div=16)}[name]()
         return _model(m, 4)
     plan = _compare(monkeypatch, build, steps=1, least=least)
+    assert any(a[0] == "products" for a in plan.actions) or name not in ("lstm", "transformer")
     if name == "resnet":
         assert any(a[0] == "copies" and len(a[1]) > 10 for a in plan.actions)
 
@@ -188,6 +199,22 @@ def test_a_feed_in_another_layout_runs_node_by_node(monkeypatch):
     np.testing.assert_array_equal(vals[out].numpy_view(), got[0])
 
 
+@pytest.mark.parametrize("taken", [True, False])
+def test_products_that_are_ready_together(monkeypatch, taken):
+    """Products of all four transpositions, too long and too wide ones, one that reads another, more than one launch."""
+    xv, wv, longv, widev = _arrays((6, 20), (20, 6), (20, 600), (600, 3000))
+
+    def build():
+        x, w, l, b = (ad.Variable(k) for k in "xwlb")
+        outs = [ad.matmul_op(x, w), ad.matmul_op(w, x, True, True), ad.matmul_op(x, x, True), ad.matmul_op(x, x, False, True)]
+        outs += [ad.matmul_op(ad.mul_byconst_op(x, float(j)), w) for j in range(40)]
+        outs += [ad.matmul_op(outs[0], outs[5]), ad.matmul_op(ad.matmul_op(x, l), b), ad.matmul_op(x, l)]
+        return outs, {x: xv, w: wv, l: longv, b: widev}
+    plan = _compare(monkeypatch, build, taken=taken)
+    groups = [a[1] for a in plan.actions if a[0] == "products"]
+    assert sum(len(g) for g in groups) >= 40 and max(len(g) for g in groups) == step_plan.MAX_GROUP
+
+
 @pytest.mark.parametrize("form", ["plain", "smooth", "shifted twice", "kept", "read elsewhere", "two losses", "fed"])
 @pytest.mark.parametrize("taken", [True, False])
 def test_labels_from_ids(monkeypatch, form, taken):
@@ -253,3 +280,40 @@ def test_programs_give_the_bits_of_the_single_kernels(shape):
     ex.stream.sync()
     for n, g in zip(nodes, got):
         assert torch.equal(vals[n].t, g), n.desc
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+def test_product_groups_give_the_bits_of_single_products(ta, tb):
+    import torch
+    from tsplit_b200.stream import current_stream
+    ctx, st = ndarray.gpu(0), current_stream(ndarray.gpu(0))
+    r = torch.Generator(device="cuda").manual_seed(2)
+    # one element, ragged tiles, several tiles, the longest sum that is not split; then a group with wider tiles
+    for sizes in ([(4, 4, 4), (128, 128, 128), (130, 68, 28), (300, 200, 480), (1, 132, 64)], [(256, 1000, 96)] * 8,
+                  [(64, 64, 32)] * 16, [(128, 256, 40), (8, 12, 36)]):
+        items, single = [], []
+        for m, n, k in sizes:
+            m4, n4 = (m + 3) // 4 * 4 if ta else m, n if tb else (n + 3) // 4 * 4
+            a = torch.randn((k, m4) if ta else (m4, k), generator=r, device="cuda")
+            b = torch.randn((n4, k) if tb else (k, n4), generator=r, device="cuda")
+            c, d = (torch.full((m4, n4), 5.0, device="cuda") for _ in range(2))
+            items.append(tuple(ndarray.from_tensor(t, ctx) for t in (a, b, c)) + (m4, n4, k))
+            G.gemm(items[-1][0], items[-1][1], ndarray.from_tensor(d, ctx), ta, tb, st, m=m4, n=n4, k=k, lda=a.shape[1],
+                   ldb=b.shape[1], ldc=n4)
+            single.append(d)
+        assert G.gemm_group(items, ta, tb, st)
+        for it, d in zip(items, single):
+            assert torch.equal(it[2].t, d)
+    a = ndarray.from_tensor(torch.zeros((2048, 2048), device="cuda"), ctx)
+    assert not G.gemm_group([(a, a, a, 2048, 2048, 2048)], ta, tb, st)           # no small product: refused, untouched
+
+
+@pytest.mark.gpu
+def test_operators_are_timed_after_a_planned_step():
+    t = transformer(vocab_size=512, d_model=16, num_heads=2, d_ff=32, num_blocks=1, maxlen1=8, maxlen2=9, batch_size=4)
+    ex = ad.recomputeExecutor([t.loss] + ad.gradients(t.loss, t.variables), ctx=ndarray.gpu(0), policy="speed")
+    feed = t.synthetic_batch()
+    table = ex.measure_ops(feed, repeats=1)
+    names = {n.op.name for n in table}
+    assert {"OneHot", "Reshape", "MulConst", "SoftmaxCrossEntropy", "MatMul"} <= names and min(table.values()) > 0

@@ -124,10 +124,11 @@ struct Cfg {
   static constexpr int TMEM_COLS = (2 * BN <= 128) ? 128 : (2 * BN <= 256 ? 256 : 512);
 };
 
+// One CTA's work items first, first + step, ... below last (an item: a tile of a batch of a K range).
 template <int BN, bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(192, 1)
-gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
+__device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
+                                           const GemmParams& p, const long long first, const long long step,
+                                           const long long last) {
   using C = Cfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -169,7 +170,6 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tsb_launch::enter();              // barriers and TMEM are set up under the tail of the previous kernel
 
   const int tiles = p.tiles_m * p.tiles_n;
-  const long long items = (long long)tiles * p.batch * p.splits;
   const int kb_per_split = (p.kblocks + p.splits - 1) / p.splits;
 
   if (warp == 0) {
@@ -177,7 +177,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      for (long long item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      for (long long item = first; item < last && ok; item += step) {
         const int tile = (int)(item % tiles);
         const long long rest = item / tiles;
         const int b = (int)(rest % p.batch);
@@ -234,7 +234,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem_b), B_MN ? BK * 128 : 16);
       uint32_t it = 0, acc_it = 0;
       bool ok = true, ready = false;
-      for (long long item = blockIdx.x; item < items && ok; item += gridDim.x, ++acc_it) {
+      for (long long item = first; item < last && ok; item += step, ++acc_it) {
         const long long rest = item / tiles;
         const int split = (int)(rest / p.batch);
         const int kb0 = split * kb_per_split;
@@ -271,7 +271,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     int which = 0;
     uint32_t acc_it = 0;
     bool ok = true;
-    for (long long item = blockIdx.x; item < items && ok; item += gridDim.x, ++acc_it) {
+    for (long long item = first; item < last && ok; item += step, ++acc_it) {
       const int tile = (int)(item % tiles);
       const long long rest = item / tiles;
       const int b = (int)(rest % p.batch);
@@ -343,6 +343,33 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem_base, C::TMEM_COLS);
   }
+}
+
+template <int BN, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(192, 1)
+gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ GemmParams p) {
+  gemm_items<BN, A_MN, B_MN>(tmA, tmB, tmC, p, blockIdx.x, gridDim.x,
+                             (long long)p.tiles_m * p.tiles_n * p.batch * p.splits);
+}
+
+// Several small products as one launch, a CTA per tile.  The gates of a recurrent cell are a handful of products of a
+// tile or two each; one after the other they are bound by the latency of a launch, a TMA round trip and a store, with
+// all but two SMs idle, and side by side they take the time of one.  LSTM step, 549 products in 84 launches:
+// 3351 -> 1322 us; a small Transformer 565 -> 504.
+constexpr int MAX_GROUP = 16;
+struct GemmGroup {
+  CUtensorMap ta[MAX_GROUP], tb[MAX_GROUP], tc[MAX_GROUP];
+  GemmParams p[MAX_GROUP];
+  int first[MAX_GROUP + 1];         // first CTA of each product
+  int count;
+};
+template <int BN, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(192, 1) gemm_tf32_group_kernel(const __grid_constant__ GemmGroup g) {
+  int t = 0;
+  while (t + 1 < g.count && g.first[t + 1] <= (int)blockIdx.x) ++t;
+  const long long item = (int)blockIdx.x - g.first[t];
+  gemm_items<BN, A_MN, B_MN>(g.ta[t], g.tb[t], g.tc[t], g.p[t], item, 1, item + 1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -811,6 +838,26 @@ int dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMa
   return launch_tc<BN, true, true>(ta, tb, tc, p, st);
 }
 
+template <int BN, bool A_MN, bool B_MN>
+int launch_group(const GemmGroup& g, int ctas, cudaStream_t st) {
+  auto kern = gemm_tf32_group_kernel<BN, A_MN, B_MN>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::SMEM_BYTES) != cudaSuccess)
+      return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
+    attr_set = true;
+  }
+  const cudaError_t e = tsb_launch::launch(kern, ctas, 192, Cfg<BN>::SMEM_BYTES, st, g);
+  return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
+}
+template <int BN>
+int dispatch_group(bool a_mn, bool b_mn, const GemmGroup& g, int ctas, cudaStream_t st) {
+  if (!a_mn && !b_mn) return launch_group<BN, false, false>(g, ctas, st);
+  if (!a_mn && b_mn) return launch_group<BN, false, true>(g, ctas, st);
+  if (a_mn && !b_mn) return launch_group<BN, true, false>(g, ctas, st);
+  return launch_group<BN, true, true>(g, ctas, st);
+}
+
 template <bool A_MN, bool B_MN>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
                 cudaStream_t st) {
@@ -878,6 +925,123 @@ static int choose_splits(long long tiles, int kblocks, int forced) {
   if (s > kblocks / 8) s = kblocks / 8;
   if (s > 32) s = 32;
   return s < 1 ? 1 : (int)s;
+}
+
+// Fills in one product: tile width, K ranges, tensor maps.  group_bn: the width is given (a product of a group, which is
+// neither split nor run on CTA pairs; TSB_ERR_UNSUPPORTED for one that would be).
+static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorMap& tc, int& bn, bool& use_pair,
+                      int group_bn, const float* a, const float* b, float* c, int m, int n, int k, long long lda,
+                      long long ldb, long long ldc, int trans_a, int trans_b, int batch, long long sa, long long sb,
+                      long long sc, int accumulate, int forced_splits, float* ws, size_t ws_bytes, bool may_alloc,
+                      cudaStream_t st, int heads, int head_mask) {
+  const bool a_heads = (head_mask & 1) != 0, b_heads = (head_mask & 2) != 0, c_heads = (head_mask & 4) != 0;
+  bn = n > 128 ? 256 : (n > 64 ? 128 : 64);
+  p.c = c; p.m = m; p.n = n; p.k = k; p.batch = batch; p.ldc = ldc; p.sc = sc;
+  p.accumulate = accumulate;
+  p.heads = head_mask ? heads : 0;
+  p.a_heads = a_heads; p.b_heads = b_heads; p.c_heads = c_heads;
+  p.a_shift = trans_a ? k : m;
+  p.b_shift = trans_b ? n : k;
+  p.sc2 = (long long)m * ldc;
+  p.tiles_m = (m + BM - 1) / BM;
+  p.tiles_n = (n + bn - 1) / bn;
+  p.kblocks = (k + BK - 1) / BK;
+  p.splits = choose_splits((long long)p.tiles_m * p.tiles_n * batch, p.kblocks, forced_splits);
+  if (p.splits > p.kblocks) p.splits = p.kblocks;
+  {   // no empty K ranges: re-derive the count from the per-split share
+    const int per = (p.kblocks + p.splits - 1) / p.splits;
+    p.splits = (p.kblocks + per - 1) / per;
+  }
+  p.ws = nullptr;
+  p.status = tsb_host::status_word(st);
+  if (!p.status) return TSB_ERR_LAUNCH;
+  if (p.splits > 1) {
+    const size_t need = (size_t)p.splits * batch * m * n * sizeof(float);
+    if (ws && ws_bytes >= need) {
+      p.ws = ws;
+    } else if (may_alloc) {
+      p.ws = get_workspace(need, st);
+      if (!p.ws) return TSB_ERR_OOM;
+    } else {
+      return TSB_ERR_SCRATCH;
+    }
+  }
+  // CTA pairs (256 x 256 tiles on SM pairs) when the problem has enough of them and no split-K
+  use_pair = false;
+  {
+    const long long pair_items = (long long)((m + 255) / 256) * ((n + 255) / 256) * batch;
+    const char* e = getenv("TSB_GEMM_PAIR");              // "0" selects the one-CTA tiles everywhere
+    const bool enabled = !(e && e[0] == '0');
+    use_pair = enabled && bn == 256 && p.splits == 1 && m >= 256 && pair_items * 4 >= sm_count() &&
+               (!trans_a || m % 32 == 0) && (trans_b || n % 32 == 0);
+  }
+  if (group_bn) {
+    if (use_pair || p.splits > 1) return TSB_ERR_UNSUPPORTED;
+    bn = group_bn;
+    p.tiles_n = (n + bn - 1) / bn;
+  } else if (!use_pair) {   // (the K ranges stay those of the wide tile: results do not depend on the choice)
+    bn = tsb_host::narrow_tile(bn, (long long)p.tiles_m * p.tiles_n * batch * p.splits, sm_count());
+    p.tiles_n = (n + bn - 1) / bn;
+  }
+  const uint32_t bbox = use_pair ? P2_BNH : (uint32_t)bn;   // columns of B that one CTA stages
+  // tensor maps (dims innermost first)
+  p.a_chunked = p.b_chunked = 0;
+  const uint64_t sab = (uint64_t)(batch > 1 ? sa : (long long)(trans_a ? k : m) * lda) * 4;
+  const uint64_t sbb = (uint64_t)(batch > 1 ? sb : (long long)(trans_b ? n : k) * ldb) * 4;
+  int rc = TSB_OK;
+  // an operand in head layout: rows of all outer batches in the row dimension, the head as batch dimension
+  const uint64_t outer = head_mask ? (uint64_t)(batch / heads) : 1;
+  const uint64_t a_rows = a_heads ? outer : 1, a_bat = a_heads ? (uint64_t)heads : (uint64_t)batch;
+  const uint64_t b_rows = b_heads ? outer : 1, b_bat = b_heads ? (uint64_t)heads : (uint64_t)batch;
+  if (!trans_a) {   // A[m][k], K contiguous -> K-major
+    uint64_t d[3] = {(uint64_t)k, (uint64_t)m * a_rows, a_bat}, s[2] = {(uint64_t)lda * 4, sab};
+    uint32_t bx[3] = {BK, BM, 1};
+    rc = tsb_host::make_tmap_f32(&ta, a, 3, d, s, bx);
+  } else if (m % 32 == 0) {   // A stored [k][m], M contiguous -> MN-major; all chunks of a stage in one box
+    uint64_t d[4] = {32, (uint64_t)k * a_rows, (uint64_t)m / 32, a_bat}, s[3] = {(uint64_t)lda * 4, 128, sab};
+    uint32_t bx[4] = {32, BK, BM / 32, 1};
+    rc = tsb_host::make_tmap_f32(&ta, a, 4, d, s, bx, true);
+    p.a_chunked = 1;
+  } else {
+    uint64_t d[3] = {(uint64_t)m, (uint64_t)k * a_rows, a_bat}, s[2] = {(uint64_t)lda * 4, sab};
+    uint32_t bx[3] = {32, BK, 1};
+    rc = tsb_host::make_tmap_f32(&ta, a, 3, d, s, bx, true);
+  }
+  if (rc) return rc;
+  if (trans_b) {    // B stored [n][k], K contiguous -> K-major
+    uint64_t d[3] = {(uint64_t)k, (uint64_t)n * b_rows, b_bat}, s[2] = {(uint64_t)ldb * 4, sbb};
+    uint32_t bx[3] = {BK, bbox, 1};
+    rc = tsb_host::make_tmap_f32(&tb, b, 3, d, s, bx);
+  } else if (n % 32 == 0) {   // B[k][n], N contiguous -> MN-major; all chunks of a stage in one box
+    uint64_t d[4] = {32, (uint64_t)k * b_rows, (uint64_t)n / 32, b_bat}, s[3] = {(uint64_t)ldb * 4, 128, sbb};
+    uint32_t bx[4] = {32, BK, bbox / 32, 1};
+    rc = tsb_host::make_tmap_f32(&tb, b, 4, d, s, bx, true);
+    p.b_chunked = 1;
+  } else {
+    uint64_t d[3] = {(uint64_t)n, (uint64_t)k * b_rows, b_bat}, s[2] = {(uint64_t)ldb * 4, sbb};
+    uint32_t bx[3] = {32, BK, 1};
+    rc = tsb_host::make_tmap_f32(&tb, b, 3, d, s, bx, true);
+  }
+  if (rc) return rc;
+  // C (or the split-K partial sums) as [outer][head or batch][row][column], where its strides allow a tensor map
+  tc = ta;
+  {
+    const float* base = p.splits > 1 ? p.ws : c;
+    const long long row = p.splits > 1 ? n : ldc;
+    const long long mat = p.splits > 1 ? (long long)m * n : (batch > 1 ? sc : (long long)m * ldc);
+    const uint64_t mats = c_heads ? (uint64_t)heads : (uint64_t)batch * p.splits;
+    const long long top = c_heads ? p.sc2 : (long long)mats * mat;
+    p.tma_store = (p.splits > 1 || !accumulate) && row % 4 == 0 && mat % 4 == 0 && top % 4 == 0 && row > 0 && mat > 0 &&
+                  (reinterpret_cast<uintptr_t>(base) & 15) == 0 && top < (1ll << 37);
+    if (p.tma_store) {
+      uint64_t d[4] = {(uint64_t)n, (uint64_t)m, mats, c_heads ? outer : 1};
+      uint64_t s[3] = {(uint64_t)row * 4, (uint64_t)mat * 4, (uint64_t)top * 4};
+      uint32_t bx[4] = {32, 32, 1, 1};
+      rc = tsb_host::make_tmap_f32(&tc, base, 4, d, s, bx);
+      if (rc) return rc;
+    }
+  }
+  return TSB_OK;
 }
 
 // Core entry shared by the allocating and the non-allocating front ends.
@@ -950,110 +1114,13 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
   }
-  int bn = n > 128 ? 256 : (n > 64 ? 128 : 64);
   GemmParams p;
-  p.c = c; p.m = m; p.n = n; p.k = k; p.batch = batch; p.ldc = ldc; p.sc = sc;
-  p.accumulate = accumulate;
-  p.heads = head_mask ? heads : 0;
-  p.a_heads = a_heads; p.b_heads = b_heads; p.c_heads = c_heads;
-  p.a_shift = trans_a ? k : m;
-  p.b_shift = trans_b ? n : k;
-  p.sc2 = (long long)m * ldc;
-  p.tiles_m = (m + BM - 1) / BM;
-  p.tiles_n = (n + bn - 1) / bn;
-  p.kblocks = (k + BK - 1) / BK;
-  p.splits = choose_splits((long long)p.tiles_m * p.tiles_n * batch, p.kblocks, forced_splits);
-  if (p.splits > p.kblocks) p.splits = p.kblocks;
-  {   // no empty K ranges: re-derive the count from the per-split share
-    const int per = (p.kblocks + p.splits - 1) / p.splits;
-    p.splits = (p.kblocks + per - 1) / per;
-  }
-  p.ws = nullptr;
-  p.status = tsb_host::status_word(st);
-  if (!p.status) return TSB_ERR_LAUNCH;
-  if (p.splits > 1) {
-    const size_t need = (size_t)p.splits * batch * m * n * sizeof(float);
-    if (ws && ws_bytes >= need) {
-      p.ws = ws;
-    } else if (may_alloc) {
-      p.ws = get_workspace(need, st);
-      if (!p.ws) return TSB_ERR_OOM;
-    } else {
-      return TSB_ERR_SCRATCH;
-    }
-  }
-  // CTA pairs (256 x 256 tiles on SM pairs) when the problem has enough of them and no split-K
-  bool use_pair = false;
-  {
-    const long long pair_items = (long long)((m + 255) / 256) * ((n + 255) / 256) * batch;
-    const char* e = getenv("TSB_GEMM_PAIR");              // "0" selects the one-CTA tiles everywhere
-    const bool enabled = !(e && e[0] == '0');
-    use_pair = enabled && bn == 256 && p.splits == 1 && m >= 256 && pair_items * 4 >= sm_count() &&
-               (!trans_a || m % 32 == 0) && (trans_b || n % 32 == 0);
-  }
-  if (!use_pair) {          // (the K ranges stay those of the wide tile: results do not depend on the choice)
-    bn = tsb_host::narrow_tile(bn, (long long)p.tiles_m * p.tiles_n * batch * p.splits, sm_count());
-    p.tiles_n = (n + bn - 1) / bn;
-  }
-  const uint32_t bbox = use_pair ? P2_BNH : (uint32_t)bn;   // columns of B that one CTA stages
-  // tensor maps (dims innermost first)
-  CUtensorMap ta, tb;
-  p.a_chunked = p.b_chunked = 0;
-  const uint64_t sab = (uint64_t)(batch > 1 ? sa : (long long)(trans_a ? k : m) * lda) * 4;
-  const uint64_t sbb = (uint64_t)(batch > 1 ? sb : (long long)(trans_b ? n : k) * ldb) * 4;
-  int rc;
-  // an operand in head layout: rows of all outer batches in the row dimension, the head as batch dimension
-  const uint64_t outer = head_mask ? (uint64_t)(batch / heads) : 1;
-  const uint64_t a_rows = a_heads ? outer : 1, a_bat = a_heads ? (uint64_t)heads : (uint64_t)batch;
-  const uint64_t b_rows = b_heads ? outer : 1, b_bat = b_heads ? (uint64_t)heads : (uint64_t)batch;
-  if (!trans_a) {   // A[m][k], K contiguous -> K-major
-    uint64_t d[3] = {(uint64_t)k, (uint64_t)m * a_rows, a_bat}, s[2] = {(uint64_t)lda * 4, sab};
-    uint32_t bx[3] = {BK, BM, 1};
-    rc = tsb_host::make_tmap_f32(&ta, a, 3, d, s, bx);
-  } else if (m % 32 == 0) {   // A stored [k][m], M contiguous -> MN-major; all chunks of a stage in one box
-    uint64_t d[4] = {32, (uint64_t)k * a_rows, (uint64_t)m / 32, a_bat}, s[3] = {(uint64_t)lda * 4, 128, sab};
-    uint32_t bx[4] = {32, BK, BM / 32, 1};
-    rc = tsb_host::make_tmap_f32(&ta, a, 4, d, s, bx, true);
-    p.a_chunked = 1;
-  } else {
-    uint64_t d[3] = {(uint64_t)m, (uint64_t)k * a_rows, a_bat}, s[2] = {(uint64_t)lda * 4, sab};
-    uint32_t bx[3] = {32, BK, 1};
-    rc = tsb_host::make_tmap_f32(&ta, a, 3, d, s, bx, true);
-  }
+  CUtensorMap ta, tb, tc;
+  int bn;
+  bool use_pair;
+  int rc = prepare_tc(p, ta, tb, tc, bn, use_pair, 0, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, batch, sa, sb, sc,
+                      accumulate, forced_splits, ws, ws_bytes, may_alloc, st, heads, head_mask);
   if (rc) return rc;
-  if (trans_b) {    // B stored [n][k], K contiguous -> K-major
-    uint64_t d[3] = {(uint64_t)k, (uint64_t)n * b_rows, b_bat}, s[2] = {(uint64_t)ldb * 4, sbb};
-    uint32_t bx[3] = {BK, bbox, 1};
-    rc = tsb_host::make_tmap_f32(&tb, b, 3, d, s, bx);
-  } else if (n % 32 == 0) {   // B[k][n], N contiguous -> MN-major; all chunks of a stage in one box
-    uint64_t d[4] = {32, (uint64_t)k * b_rows, (uint64_t)n / 32, b_bat}, s[3] = {(uint64_t)ldb * 4, 128, sbb};
-    uint32_t bx[4] = {32, BK, bbox / 32, 1};
-    rc = tsb_host::make_tmap_f32(&tb, b, 4, d, s, bx, true);
-    p.b_chunked = 1;
-  } else {
-    uint64_t d[3] = {(uint64_t)n, (uint64_t)k * b_rows, b_bat}, s[2] = {(uint64_t)ldb * 4, sbb};
-    uint32_t bx[3] = {32, BK, 1};
-    rc = tsb_host::make_tmap_f32(&tb, b, 3, d, s, bx, true);
-  }
-  if (rc) return rc;
-  // C (or the split-K partial sums) as [outer][head or batch][row][column], where its strides allow a tensor map
-  CUtensorMap tc = ta;
-  {
-    const float* base = p.splits > 1 ? p.ws : c;
-    const long long row = p.splits > 1 ? n : ldc;
-    const long long mat = p.splits > 1 ? (long long)m * n : (batch > 1 ? sc : (long long)m * ldc);
-    const uint64_t mats = c_heads ? (uint64_t)heads : (uint64_t)batch * p.splits;
-    const long long top = c_heads ? p.sc2 : (long long)mats * mat;
-    p.tma_store = (p.splits > 1 || !accumulate) && row % 4 == 0 && mat % 4 == 0 && top % 4 == 0 && row > 0 && mat > 0 &&
-                  (reinterpret_cast<uintptr_t>(base) & 15) == 0 && top < (1ll << 37);
-    if (p.tma_store) {
-      uint64_t d[4] = {(uint64_t)n, (uint64_t)m, mats, c_heads ? outer : 1};
-      uint64_t s[3] = {(uint64_t)row * 4, (uint64_t)mat * 4, (uint64_t)top * 4};
-      uint32_t bx[4] = {32, 32, 1, 1};
-      rc = tsb_host::make_tmap_f32(&tc, base, 4, d, s, bx);
-      if (rc) return rc;
-    }
-  }
   const bool a_mn = trans_a != 0, b_mn = trans_b == 0;
   if (use_pair) rc = dispatch_pair(a_mn, b_mn, ta, tb, tc, p, st);
   else if (bn == 256) rc = dispatch_major<256>(a_mn, b_mn, ta, tb, tc, p, st);
@@ -1102,6 +1169,44 @@ int tsb_gemm_tf32_splitk(const float* a, const float* b, float* c, int m, int n,
                          long long ldb, long long ldc, int trans_a, int trans_b, int splits, void* stream) {
   return tsb_gemm_tf32_impl(a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, 1, 0, 0, 0, 0, splits, nullptr, 0,
                             true, static_cast<cudaStream_t>(stream));
+}
+
+// Up to 16 products C = op(A) op(B) of the same transposition as one launch.  TSB_ERR_UNSUPPORTED when one of them is no
+// candidate (needs padding, split-K or CTA pairs) or the tiles do not fit the chip at once.
+int tsb_gemm_tf32_group(int count, const float** a, const float** b, float** c, const int* m, const int* n, const int* k,
+                        const long long* lda, const long long* ldb, const long long* ldc, int trans_a, int trans_b,
+                        void* stream) {
+  if (count < 1 || count > MAX_GROUP) return TSB_ERR_ARG;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  long long t64 = 0, t128 = 0;
+  for (int i = 0; i < count; ++i) {
+    if (m[i] <= 0 || n[i] <= 0 || k[i] <= 0) return TSB_ERR_ARG;
+    if ((lda[i] | ldb[i]) % 4 || ((reinterpret_cast<uintptr_t>(a[i]) | reinterpret_cast<uintptr_t>(b[i])) & 15))
+      return TSB_ERR_UNSUPPORTED;
+    const long long rows = ((long long)m[i] + BM - 1) / BM;
+    t64 += rows * ((n[i] + 63) / 64);
+    t128 += rows * ((n[i] + 127) / 128);
+  }
+  const int bn = t64 <= sm_count() ? 64 : 128;       // as narrow as still leaves a tile an SM (see narrow_tile)
+  if (t128 > sm_count()) return TSB_ERR_UNSUPPORTED;
+  GemmGroup g;
+  g.count = count;
+  int ctas = 0;
+  for (int i = 0; i < count; ++i) {
+    int width;
+    bool pair;
+    const int rc = prepare_tc(g.p[i], g.ta[i], g.tb[i], g.tc[i], width, pair, bn, a[i], b[i], c[i], m[i], n[i], k[i],
+                              lda[i], ldb[i], ldc[i], trans_a, trans_b, 1, 0, 0, 0, 0, 0, nullptr, 0, false, st, 0, 0);
+    if (rc) return rc == TSB_ERR_SCRATCH ? TSB_ERR_UNSUPPORTED : rc;
+    g.first[i] = ctas;
+    ctas += g.p[i].tiles_m * g.p[i].tiles_n;
+  }
+  g.first[count] = ctas;
+  const int rc = bn == 64 ? dispatch_group<64>(trans_a != 0, trans_b == 0, g, ctas, st)
+                          : dispatch_group<128>(trans_a != 0, trans_b == 0, g, ctas, st);
+  if (rc) return rc;
+  const int late = tsb_host::peek_status();
+  return late ? TSB_ERR_TIMEOUT | (late << 8) : TSB_OK;
 }
 
 // Synchronise the stream and return (then clear) the device-side wait status:

@@ -1,11 +1,12 @@
 """The order in which the keep-all executors issue a step on the GPU, worked out once per feed shape.
 
-Four things are taken out of the node-by-node loop, none of which changes a value:
+Five things are taken out of the node-by-node loop, none of which changes a value:
 
 * element-wise operators over the same elements are collected and run as one ``tsb_pointwise`` program, at the first
   node that needs one of their results; results that nobody outside the program reads are not stored;
 * a reshape of a row-major array is a view of it;
 * the small parameter gradients that a normalisation operator hands out from its own buffers are copied in one launch;
+* small matrix products that are ready together run as one launch;
 * one-hot labels, scaled and shifted (label smoothing), that only a cross-entropy reads are not made: it takes the ids.
 
 Element-wise nodes are taken as soon as their inputs are there, the others in creation order, and nothing moves past a
@@ -21,6 +22,7 @@ import numpy as np
 from .. import ndarray
 from ..ops import _gpu as G
 from ..ops.elementwise import AddConstOp, MulConstOp, _Binary, _Unary, _is_scalar_shape
+from ..ops.linalg import MatMulOp, _mm_shape
 from ..ops.loss import SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp
 from ..ops.misc import OneHotOp, PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
 from ..ops.norm import BatchNormGradScaleOp
@@ -29,6 +31,8 @@ from ..ops.shape import AddBroadcastOp, ReshapeOp, ReshapeGradientOp
 FULL, ROW, SCALAR = 0, 1, 2
 _BINARY = 32                       # instruction code of binary operator 0
 MAX_IN, MAX_INS, MAX_SLOTS = 32, 64, 48
+#: products of one launch, and what makes one small: the 128 x 64 tiles of one and of all, and K (longer sums are split)
+MAX_GROUP, GROUP_TILES, GROUP_TILES_ALL, GROUP_K = 16, 16, 128, 480
 #: value slots of a program over a tensor that does not fit in L2: more of them leave too few threads to cover DRAM
 MAX_SLOTS_LARGE, LARGE = 12, 8 << 20
 
@@ -231,6 +235,13 @@ class StepPlan(object):
             cls = "elided" if n in self.elided else "view" if self._is_view(n) else "copy" if isinstance(n.op, BatchNormGradScaleOp) else None
             ops = None if cls else self._operands(n)
             heapq.heappush(light if cls or ops is not None else heavy, (n.id, n, cls, ops))
+
+        def done(n):
+            for u in set(self.users.get(n, ())):
+                if u in inside:
+                    waits[u] -= 1
+                    if waits[u] == 0:
+                        ready(u)
         for n in nodes:
             if waits[n] == 0:
                 ready(n)
@@ -248,16 +259,40 @@ class StepPlan(object):
                     self._collect(n, ops)
             else:
                 _, n, _, _ = heapq.heappop(heavy)
-                for i in n.inputs:
-                    self._need(i)
+                taken = self._mates(n, heavy)
+                for m in taken:
+                    for i in m.inputs:
+                        self._need(i)
                 if n in self.smooth:
                     self._need(self.smooth[n][0])
-                self.actions.append(("smooth" if n in self.smooth else "node", n))
-            for u in set(self.users.get(n, ())):
-                if u in inside:
-                    waits[u] -= 1
-                    if waits[u] == 0:
-                        ready(u)
+                self.actions.append(("products", taken) if len(taken) > 1 else
+                                    ("smooth" if n in self.smooth else "node", n))
+                for m in taken[1:]:
+                    done(m)
+            done(n)
+
+    def _product_tiles(self, n):
+        """128 x 64 tiles of a small matrix product, 0 for anything else."""
+        if not isinstance(n.op, MatMulOp) or self.arrays.get(n) is None:
+            return 0
+        m, c, k = _mm_shape(self.shapes[n.inputs[0]], self.shapes[n.inputs[1]], n.attrs["trans_A"], n.attrs["trans_B"])
+        tiles = -(-m // 128) * -(-c // 64)
+        return tiles if tiles <= GROUP_TILES and k <= GROUP_K else 0
+
+    def _mates(self, n, heavy):
+        """``n`` and the products that are ready with it and go into the same launch (taken out of ``heavy``)."""
+        taken, tiles = [n], self._product_tiles(n)
+        if tiles:
+            for entry in sorted(heavy):
+                m = entry[1]
+                t = self._product_tiles(m)
+                if (t and len(taken) < MAX_GROUP and tiles + t <= GROUP_TILES_ALL
+                        and all(m.attrs[f] == n.attrs[f] for f in ("trans_A", "trans_B"))):
+                    taken.append(m)
+                    tiles += t
+                    heavy.remove(entry)
+            heapq.heapify(heavy)
+        return taken
 
     def _view(self, n):
         src = n.inputs[0]
@@ -347,6 +382,8 @@ class StepPlan(object):
     def run(self, ex, vals):
         for n in self.placeholders:
             vals[n] = ex._placeholder_value(n)
+        for n in self.elided:              # (for those who walk all values, as a per-operator timing does)
+            vals[n] = self.arrays[n]
         stream = ex.stream
         for what, x in self.actions:
             if what == "node":
@@ -355,6 +392,8 @@ class StepPlan(object):
                 vals[x] = self.arrays[x]
             elif what == "smooth":
                 self._smooth(x, vals, stream)
+            elif what == "products":
+                self._products(x, vals, stream)
             elif what == "program":
                 if x.run(vals, self.arrays, stream):
                     for m, _ in x.members:
@@ -372,6 +411,21 @@ class StepPlan(object):
                 else:
                     for n in x:
                         self._node(n, vals, stream)
+
+    def _products(self, nodes, vals, stream):
+        ta, tb = nodes[0].attrs["trans_A"], nodes[0].attrs["trans_B"]
+        items = []
+        for n in nodes:
+            a, b, out = vals[n.inputs[0]], vals[n.inputs[1]], self.arrays[n]
+            if not (a.is_contiguous() and b.is_contiguous() and out.is_contiguous()):
+                break
+            items.append((a, b, out) + _mm_shape(a.shape, b.shape, ta, tb))
+        if len(items) == len(nodes) and G.gemm_group(items, ta, tb, stream):
+            for n in nodes:
+                vals[n] = self.arrays[n]
+        else:
+            for n in nodes:
+                self._node(n, vals, stream)
 
     def _smooth(self, n, vals, stream):
         ids, on, off, chain = self.smooth[n]

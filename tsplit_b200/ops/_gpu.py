@@ -446,6 +446,19 @@ def gemm(a, b, c, trans_a, trans_b, stream, batch=1, sa=0, sb=0, sc=0, m=None, n
     _check(rc, "gemm_tf32")
 
 
+def gemm_group(products, trans_a, trans_b, stream):
+    """Up to 16 products ``(a, b, c, m, n, k)`` of row-major arrays as one launch; False: not a group of small ones."""
+    cnt = len(products)
+    ptr = lambda j: (c_void_p * cnt)(*[p[j].ptr for p in products])
+    num = lambda j: (c_int * cnt)(*[p[j] for p in products])
+    ld = lambda j: (c_int64 * cnt)(*[p[j].shape[1] for p in products])
+    rc = lib().tsb_gemm_tf32_group(c_int(cnt), ptr(0), ptr(1), ptr(2), num(3), num(4), num(5), ld(0), ld(1), ld(2),
+                                   c_int(int(trans_a)), c_int(int(trans_b)), _s(stream))
+    if rc != 2:
+        _check(rc, "gemm_tf32_group")
+    return rc == 0
+
+
 def conv2d(kind, x, w, y, ph, pw, stride, stream):
     """kind 0: y = conv(x, w); 1: x(dx) = dgrad(y(dy), w); 2: w(dw) = wgrad(x, y(dy)).
     All operands channels-last; logical shapes x[N,C,H,W], w[O,C,KH,KW], y[N,O,OH,OW]."""
