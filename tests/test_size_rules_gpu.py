@@ -171,3 +171,22 @@ def test_max_pool_gradient_tiles(n, c, h, w, k, pad, stride):
     from tsplit_b200.ops.pool import np_max_pool_grad
     want = np_max_pool_grad(x.cpu().numpy(), ref_y.detach().cpu().numpy(), dy.cpu().numpy(), k, k, pad, stride)
     assert torch.equal(dx.t.cpu(), torch.from_numpy(want))
+
+
+# column sums in one launch: a single row, remainders of the 32 lanes and of the four loads, ragged columns, the last row
+# count; the next one takes two stages
+@pytest.mark.parametrize("rows,cols", [(1, 4), (2, 33), (31, 7), (33, 64), (129, 100), (512, 1024), (513, 32)])
+def test_column_sums_of_few_rows(rows, cols):
+    x = _rand(rows, cols + 3)[:, :cols]
+    y = torch.zeros(cols, device="cuda")
+    ctx = ndarray.gpu(0)
+    G.reduce_sum(x.data_ptr(), [rows, cols], [cols + 3, 1], [0], ndarray.from_tensor(y, ctx), _stream())
+    # fp32 sums of at most 513 terms, sixteen or fewer of them in a row: some 30 roundings of partial sums
+    bound = 32 * 2.0 ** -24 * x.double().abs().sum(0) + 1e-6
+    assert torch.all((y.double() - x.double().sum(0)).abs() <= bound)
+    if 1 < rows <= 512:
+        items = [(ndarray.from_tensor(x.contiguous(), ctx), ndarray.from_tensor(torch.zeros(cols, device="cuda"), ctx)),
+                 (ndarray.from_tensor(_rand(3, 5), ctx), ndarray.from_tensor(torch.zeros(5, device="cuda"), ctx))]
+        assert G.colsum_group(items, _stream())
+        assert torch.equal(items[0][1].t, y)
+        torch.testing.assert_close(items[1][1].t, items[1][0].t.sum(0), rtol=0, atol=1e-6)

@@ -75,9 +75,18 @@ def _gemm_group(products, ta, tb, stream):
     return True
 
 
+def _colsum_group(items, stream):
+    assert 2 <= len(items) <= step_plan.MAX_GROUP
+    for x, y in items:
+        assert len(x.shape) == 2 and x.shape[0] <= step_plan.GROUP_ROWS
+        y.numpy_view()[...] = x.numpy_view().sum(0).reshape(y.shape)
+    return True
+
+
 def _run(monkeypatch, nodes, feed, steps=1, taken=True):
     monkeypatch.setattr(G, "pointwise", _pointwise)
     monkeypatch.setattr(G, "gemm_group", _gemm_group if taken else lambda *a: False)
+    monkeypatch.setattr(G, "colsum_group", _colsum_group if taken else lambda *a: False)
     monkeypatch.setattr(G, "softmax_ce_smooth", _smooth(False, taken))
     monkeypatch.setattr(G, "softmax_ce_grad_smooth", _smooth(True, taken))
     monkeypatch.setattr(G, "multi_copy", lambda s, d, st: [x.numpy_view().__setitem__(Ellipsis, y.numpy_view()) for x, y in zip(d, s)])
@@ -213,6 +222,21 @@ def test_products_that_are_ready_together(monkeypatch, taken):
     plan = _compare(monkeypatch, build, taken=taken)
     groups = [a[1] for a in plan.actions if a[0] == "products"]
     assert sum(len(g) for g in groups) >= 40 and max(len(g) for g in groups) == step_plan.MAX_GROUP
+
+
+@pytest.mark.parametrize("taken", [True, False])
+def test_sums_that_are_ready_together(monkeypatch, taken):
+    """Column sums with and without the reduced dimension kept, sums over other axes and over too many rows."""
+    xv, yv, longv = _arrays((6, 20), (5, 6, 8), (600, 4))
+
+    def build():
+        x, y, l = (ad.Variable(k) for k in "xyl")
+        outs = [ad.reduce_sum_op(ad.mul_byconst_op(x, float(j + 1)), [0]) for j in range(20)]
+        outs += [ad.reduce_sum_op(x, [0], True), ad.reduce_sum_op(x, [1]), ad.reduce_sum_op(x, [0, 1]),
+                 ad.reduce_sum_op(y, [0, 1]), ad.reduce_sum_op(l, [0])]
+        return outs, {x: xv, y: yv, l: longv}
+    plan = _compare(monkeypatch, build, taken=taken)
+    assert [len(a[1]) for a in plan.actions if a[0] == "sums"] == [16, 5]
 
 
 @pytest.mark.parametrize("form", ["plain", "smooth", "shifted twice", "kept", "read elsewhere", "two losses", "fed"])

@@ -6,7 +6,7 @@ Five things are taken out of the node-by-node loop, none of which changes a valu
   node that needs one of their results; results that nobody outside the program reads are not stored;
 * a reshape of a row-major array is a view of it;
 * the small parameter gradients that a normalisation operator hands out from its own buffers are copied in one launch;
-* small matrix products that are ready together run as one launch;
+* small matrix products that are ready together run as one launch, and so do column sums of a few rows;
 * one-hot labels, scaled and shifted (label smoothing), that only a cross-entropy reads are not made: it takes the ids.
 
 Element-wise nodes are taken as soon as their inputs are there, the others in creation order, and nothing moves past a
@@ -26,13 +26,15 @@ from ..ops.linalg import MatMulOp, _mm_shape
 from ..ops.loss import SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp
 from ..ops.misc import OneHotOp, PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
 from ..ops.norm import BatchNormGradScaleOp
-from ..ops.shape import AddBroadcastOp, ReshapeOp, ReshapeGradientOp
+from ..ops.shape import AddBroadcastOp, ReduceSumOp, ReshapeOp, ReshapeGradientOp
 
 FULL, ROW, SCALAR = 0, 1, 2
 _BINARY = 32                       # instruction code of binary operator 0
 MAX_IN, MAX_INS, MAX_SLOTS = 32, 64, 48
 #: products of one launch, and what makes one small: the 128 x 64 tiles of one and of all, and K (longer sums are split)
 MAX_GROUP, GROUP_TILES, GROUP_TILES_ALL, GROUP_K = 16, 16, 128, 480
+#: rows of a column sum that is taken together with others
+GROUP_ROWS = 512
 #: value slots of a program over a tensor that does not fit in L2: more of them leave too few threads to cover DRAM
 MAX_SLOTS_LARGE, LARGE = 12, 8 << 20
 
@@ -265,31 +267,37 @@ class StepPlan(object):
                         self._need(i)
                 if n in self.smooth:
                     self._need(self.smooth[n][0])
-                self.actions.append(("products", taken) if len(taken) > 1 else
+                self.actions.append((self._group(n)[0][0], taken) if len(taken) > 1 else
                                     ("smooth" if n in self.smooth else "node", n))
                 for m in taken[1:]:
                     done(m)
             done(n)
 
-    def _product_tiles(self, n):
-        """128 x 64 tiles of a small matrix product, 0 for anything else."""
-        if not isinstance(n.op, MatMulOp) or self.arrays.get(n) is None:
-            return 0
-        m, c, k = _mm_shape(self.shapes[n.inputs[0]], self.shapes[n.inputs[1]], n.attrs["trans_A"], n.attrs["trans_B"])
-        tiles = -(-m // 128) * -(-c // 64)
-        return tiles if tiles <= GROUP_TILES and k <= GROUP_K else 0
+    def _group(self, n):
+        """(kind, blocks) of an operator small enough to share a launch with others of its kind, else None."""
+        if self.arrays.get(n) is None:
+            return None
+        if isinstance(n.op, MatMulOp):
+            ta, tb = n.attrs["trans_A"], n.attrs["trans_B"]
+            m, c, k = _mm_shape(self.shapes[n.inputs[0]], self.shapes[n.inputs[1]], ta, tb)
+            tiles = -(-m // 128) * -(-c // 64)
+            return (("products", bool(ta), bool(tb)), tiles) if tiles <= GROUP_TILES and k <= GROUP_K else None
+        if isinstance(n.op, ReduceSumOp):
+            shape, axes = self.shapes[n.inputs[0]], n.attrs["axes"]
+            if len(shape) == 2 and list(axes) == [0] and 1 < shape[0] <= GROUP_ROWS and shape[1] <= 1024:
+                return ("sums",), 1
+        return None
 
     def _mates(self, n, heavy):
-        """``n`` and the products that are ready with it and go into the same launch (taken out of ``heavy``)."""
-        taken, tiles = [n], self._product_tiles(n)
-        if tiles:
+        """``n`` and the operators that are ready with it and go into the same launch (taken out of ``heavy``)."""
+        taken, own = [n], self._group(n)
+        if own:
+            kind, blocks = own
             for entry in sorted(heavy):
-                m = entry[1]
-                t = self._product_tiles(m)
-                if (t and len(taken) < MAX_GROUP and tiles + t <= GROUP_TILES_ALL
-                        and all(m.attrs[f] == n.attrs[f] for f in ("trans_A", "trans_B"))):
-                    taken.append(m)
-                    tiles += t
+                other = self._group(entry[1])
+                if (other and other[0] == kind and len(taken) < MAX_GROUP and blocks + other[1] <= GROUP_TILES_ALL):
+                    taken.append(entry[1])
+                    blocks += other[1]
                     heavy.remove(entry)
             heapq.heapify(heavy)
         return taken
@@ -394,6 +402,8 @@ class StepPlan(object):
                 self._smooth(x, vals, stream)
             elif what == "products":
                 self._products(x, vals, stream)
+            elif what == "sums":
+                self._sums(x, vals, stream)
             elif what == "program":
                 if x.run(vals, self.arrays, stream):
                     for m, _ in x.members:
@@ -421,6 +431,15 @@ class StepPlan(object):
                 break
             items.append((a, b, out) + _mm_shape(a.shape, b.shape, ta, tb))
         if len(items) == len(nodes) and G.gemm_group(items, ta, tb, stream):
+            for n in nodes:
+                vals[n] = self.arrays[n]
+        else:
+            for n in nodes:
+                self._node(n, vals, stream)
+
+    def _sums(self, nodes, vals, stream):
+        items = [(vals[n.inputs[0]], self.arrays[n]) for n in nodes]
+        if all(x.is_contiguous() and y.is_contiguous() for x, y in items) and G.colsum_group(items, stream):
             for n in nodes:
                 vals[n] = self.arrays[n]
         else:

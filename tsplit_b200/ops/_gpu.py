@@ -203,6 +203,19 @@ def reduce_sum(x_ptr, x_shape, x_strides, axes, y, stream):
     _check(rc, "reduce_sum")
 
 
+def colsum_group(items, stream):
+    """Column sums ``(x [rows, cols], y [cols])`` of up to 16 row-major arrays as one launch; False: too many rows."""
+    cnt = len(items)
+    rc = lib().tsb_colsum_group(c_int(cnt), (c_void_p * cnt)(*[x.ptr for x, _ in items]),
+                                (c_void_p * cnt)(*[y.ptr for _, y in items]),
+                                (c_int * cnt)(*[x.shape[0] for x, _ in items]),
+                                (c_int * cnt)(*[x.shape[1] for x, _ in items]),
+                                (c_int64 * cnt)(*[x.shape[1] for x, _ in items]), _s(stream))
+    if rc != 2:
+        _check(rc, "colsum_group")
+    return rc == 0
+
+
 def softmax(x, y, stream):
     rows, cols = _numel(x.shape[:-1]), x.shape[-1]
     _check(lib().tsb_softmax(_p(x), _p(y), c_int64(rows), c_int64(cols), _s(stream)), "softmax")
