@@ -588,6 +588,20 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, float* __rest
   }
 }
 
+// The same with 16-byte lanes, for rows of whole float4 on both sides.
+__global__ void __launch_bounds__(256) splitk_reduce_v4(const float4* __restrict__ ws, float4* __restrict__ c, int splits,
+                                                        long long per_split4, int m, int n4, long long ldc4,
+                                                        long long sc4, int accumulate) {
+  tsb_launch::enter();
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  if (i >= per_split4) return;
+  const float4 acc = tsb::sum_splits(ws + i, splits, per_split4);
+  const long long row = i / n4;
+  float4* dst = c + row / m * sc4 + row % m * ldc4 + (i - row * n4);
+  float4 o = accumulate ? *dst : make_float4(0.f, 0.f, 0.f, 0.f);
+  *dst = accumulate ? make_float4(o.x + acc.x, o.y + acc.y, o.z + acc.z, o.w + acc.w) : acc;
+}
+
 // Plain SIMT fallback for shapes the tensor-map rules exclude (leading dimension
 // not a multiple of 4 floats, unaligned base).  Tiny problems only.
 __global__ void gemm_simt_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
@@ -1129,6 +1143,15 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
   if (rc) return rc;
   if (p.splits > 1) {
     const long long per_split = (long long)batch * m * n;
+    if (n % 4 == 0 && ldc % 4 == 0 && (batch == 1 || sc % 4 == 0) && (reinterpret_cast<uintptr_t>(c) & 15) == 0) {
+      tsb_launch::launch(splitk_reduce_v4, dim3((unsigned)((per_split / 4 + 255) / 256)), 256, 0, st,
+                         reinterpret_cast<const float4*>(p.ws), reinterpret_cast<float4*>(c), p.splits, per_split / 4, m,
+                         n / 4, ldc / 4, batch > 1 ? sc / 4 : 0, accumulate);
+      const cudaError_t e4 = cudaGetLastError();
+      if (e4 != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e4 << 8);
+      const int late4 = tsb_host::peek_status();
+      return late4 ? TSB_ERR_TIMEOUT | (late4 << 8) : TSB_OK;
+    }
     int blocks = (int)((per_split + 255) / 256);
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
     tsb_launch::launch(splitk_reduce_kernel, blocks, 256, 0, st, p.ws, c, p.splits, per_split, m, n, ldc, sc,

@@ -262,6 +262,21 @@ __host__ __device__ constexpr uint32_t make_idesc_tf32(int M, int N, int a_mn_ma
          ((uint32_t)(M >> 4) << 24);
 }
 
+// Sum of `splits` partial results, four floats of each, in their order; eight loads in flight.
+__device__ __forceinline__ float4 sum_splits(const float4* __restrict__ ws, int splits, long long per_split4) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = 0; s < splits; s += 8) {
+    float4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s + u < splits) v[u] = __ldcs(ws + (s + u) * per_split4);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s + u < splits) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
+  }
+  return acc;
+}
+
 }  // namespace tsb
 
 namespace tsb {
