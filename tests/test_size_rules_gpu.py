@@ -190,3 +190,43 @@ def test_column_sums_of_few_rows(rows, cols):
         assert G.colsum_group(items, _stream())
         assert torch.equal(items[0][1].t, y)
         torch.testing.assert_close(items[1][1].t, items[1][0].t.sum(0), rtol=0, atol=1e-6)
+
+
+# rows of one vector, a lane's remainder, each register count's last and first, the longest kept row and longer ones, a
+# ragged one and one that is not aligned
+@pytest.mark.parametrize("d,shift", [(4, 0), (128, 0), (132, 0), (260, 0), (516, 0), (1024, 0), (1028, 0), (30, 0), (64, 1)])
+@pytest.mark.parametrize("rows", [1, 77])
+def test_layer_norm_gradient_of_rows(d, shift, rows):
+    ctx = ndarray.gpu(0)
+    flat = lambda seed: _rand(rows * d + shift, seed=seed)[shift:].view(rows, d)
+    x, dy, dx = flat(1), flat(2), flat(3)
+    scale = _rand(d, seed=4) + 1
+    mean, inv = x.mean(1), 1 / torch.sqrt(x.var(1, unbiased=False) + 1e-5)
+    ds, db = torch.zeros(d, device="cuda"), torch.zeros(d, device="cuda")
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    G.layer_norm_grad(a(dy), a(x), a(scale), a(mean), a(inv), a(dx), a(ds), a(db), _stream())
+    xd, g = x.double(), dy.double() * scale.double()
+    xn = (xd - mean.double()[:, None]) * inv.double()[:, None]
+    want = inv.double()[:, None] * (g - g.mean(1, keepdim=True) - xn * (g * xn).mean(1, keepdim=True))
+    # a dozen fp32 roundings of terms that are at most the largest of the row
+    bound = 16 * 2.0 ** -23 * inv.double()[:, None] * (g.abs().amax(1, keepdim=True) * (1 + xn.abs().amax(1, keepdim=True) ** 2))
+    assert torch.all((dx.double() - want).abs() <= bound + 1e-6)
+
+
+@pytest.mark.parametrize("n,vocab,dim", [(1, 3, 4), (700, 5, 512), (33, 40, 6), (64, 9, 132)])
+def test_embedding_gradient_of_repeated_ids(n, vocab, dim):
+    ctx = ndarray.gpu(0)
+    ids = torch.randint(-1, vocab + 1, (n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).float()
+    g = torch.round(_rand(n, dim) * 8) / 8                              # sums of eighths are exact in any order
+    table = torch.zeros(vocab, dim, device="cuda")
+    G.embedding_grad(ndarray.from_tensor(g, ctx), ndarray.from_tensor(ids, ctx), ndarray.from_tensor(table, ctx), _stream())
+    inside = (ids >= 0) & (ids < vocab)
+    assert torch.equal(table, torch.zeros_like(table).index_add_(0, ids[inside].long(), g[inside]))
+
+
+@pytest.mark.parametrize("rows,cols", [(514, 4), (1023, 36), (8160, 512), (20000, 1000), (600, 16500)])
+def test_column_sums_of_many_rows(rows, cols):
+    x, y = _rand(rows, cols), torch.zeros(cols, device="cuda")
+    G.reduce_sum(x.data_ptr(), [rows, cols], [cols, 1], [0], ndarray.from_tensor(y, ndarray.gpu(0)), _stream())
+    # pairwise joins of partial sums of at most some eighty terms
+    assert torch.all((y.double() - x.double().sum(0)).abs() <= 96 * 2.0 ** -24 * x.double().abs().sum(0))

@@ -295,7 +295,7 @@ def test_programs_give_the_bits_of_the_single_kernels(shape):
     vals = dict(feed)
     vals[s] = s.tensor_value
     for kind, what in plan.actions:
-        for n in [m for m, _ in what.members] if kind == "program" else [what]:
+        for n in what.members if kind == "program" else [what]:
             if kind == "view":
                 vals[n] = plan.arrays[n]
             else:
