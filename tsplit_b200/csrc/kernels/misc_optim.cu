@@ -85,6 +85,19 @@ __global__ void embedding_grad_kernel(const float* __restrict__ g, const float* 
   }
 }
 
+// Rows of whole float4: one 16-byte reduction instead of four.  Bound by reductions that meet in the
+// rows of frequent ids (8192 tokens x 512 over 1000 words: 24.7 -> 22.1 us).
+__global__ void __launch_bounds__(256) embedding_grad_v4(const float4* __restrict__ g, const float* __restrict__ idx,
+                                                         float4* __restrict__ dtable, long long n4, long long vocab,
+                                                         unsigned dim4) {
+  tsb_launch::enter();
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  if (i >= n4) return;
+  const long long r = (n4 >> 32) == 0 ? (long long)((unsigned)i / dim4) : i / dim4;
+  const long long id = (long long)idx[r];
+  if (id >= 0 && id < vocab) atomicAdd(dtable + id * dim4 + (i - r * dim4), __ldg(g + i));
+}
+
 // splitmix64 of (seed, element index): the keep decision is a pure function of both
 __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned long long i) {
   unsigned long long x = i + seed * 0x9E3779B97F4A7C15ull;
@@ -277,6 +290,14 @@ int tsb_embedding(const float* table, const float* idx, float* y, long long n, l
 int tsb_embedding_grad(const float* g, const float* idx, float* dtable, long long n, long long vocab,
                        long long dim, void* stream) {
   if (n <= 0) return TSB_OK;
+  if (n > 0 && dim > 0 && dim % 4 == 0 && dim < (1ll << 32) && n * dim < (1ll << 40) &&
+      ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(dtable)) & 15) == 0) {
+    const long long n4 = n * (dim / 4);
+    tsb_launch::launch(embedding_grad_v4, dim3((unsigned)((n4 + 255) / 256)), 256, 0, static_cast<cudaStream_t>(stream),
+                       reinterpret_cast<const float4*>(g), idx, reinterpret_cast<float4*>(dtable), n4, vocab,
+                       (unsigned)(dim / 4));
+    return done();
+  }
   tsb_launch::launch(embedding_grad_kernel, ew_grid(n * dim), 256, 0, static_cast<cudaStream_t>(stream), g, idx,
                      dtable, n, vocab,
                                                                                          dim);
