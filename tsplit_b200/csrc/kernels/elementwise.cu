@@ -362,23 +362,27 @@ __global__ void colsum_partial_v4(const float4* __restrict__ x, float4* __restri
       make_float4((a0.x + a1.x) + (a2.x + a3.x), (a0.y + a1.y) + (a2.y + a3.y), (a0.z + a1.z) + (a2.z + a3.z),
                   (a0.w + a1.w) + (a2.w + a3.w));
 }
-// Second stage for many chunks: 32 columns x 8 chunk lanes per block, lanes joined in a fixed order.
-__global__ void colsum_final_lanes(const float* __restrict__ part, float* __restrict__ y, long long cols, int chunks,
-                                   long long ys) {
+// Second stage: 32 columns x 32 chunk lanes per block, eight loads in flight, lanes joined in a fixed order (256 chunks
+// of 512 columns: 3.4 us with 8 lanes, 2.9 now).
+__global__ void __launch_bounds__(1024) colsum_final_lanes(const float* __restrict__ part, float* __restrict__ y,
+                                                           long long cols, int chunks, long long ys) {
   tsb_launch::enter();
-  __shared__ float sh[8][33];
+  __shared__ float sh[32][33];
   const long long c = blockIdx.x * 32ll + threadIdx.x;
   float acc = 0.f;
   if (c < cols)
-    for (int ch = threadIdx.y; ch < chunks; ch += 8) acc += part[(long long)ch * cols + c];
-  sh[threadIdx.y][threadIdx.x] = acc;
-  __syncthreads();
-  if (threadIdx.y == 0 && c < cols) {
-    float t = 0.f;
+    for (int ch = threadIdx.y; ch < chunks; ch += 256) {
+      float v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) t += sh[j][threadIdx.x];
-    y[c * ys] = t;
+      for (int u = 0; u < 8; ++u) v[u] = ch + 32 * u < chunks ? part[(long long)(ch + 32 * u) * cols + c] : 0.f;
+      acc += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
+  sh[threadIdx.y][threadIdx.x] = acc;
+  for (int o = 16; o > 0; o >>= 1) {
+    __syncthreads();
+    if (threadIdx.y < o) sh[threadIdx.y][threadIdx.x] += sh[threadIdx.y + o][threadIdx.x];
   }
+  if (threadIdx.y == 0 && c < cols) y[c * ys] = sh[0][threadIdx.x];
 }
 __global__ void colsum_final(const float* __restrict__ part, float* __restrict__ y, long long cols, int chunks,
                              long long ys) {
@@ -678,7 +682,7 @@ int tsb_reduce_sum(const float* x, float* y, int nk, const long long* kshape, co
         tsb_launch::launch(colsum_partial_v4, g1, 128, 0, st, reinterpret_cast<const float4*>(x),
                            reinterpret_cast<float4*>(part),
                                               nred, cols4, rxs[0] / 4, chunks);
-        tsb_launch::launch(colsum_final_lanes, (unsigned)((nkeep + 31) / 32), dim3(32, 8), 0, st, part, y, nkeep,
+        tsb_launch::launch(colsum_final_lanes, (unsigned)((nkeep + 31) / 32), dim3(32, 32), 0, st, part, y, nkeep,
                            chunks, kys[0]);
         return done();
       }

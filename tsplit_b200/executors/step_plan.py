@@ -95,6 +95,8 @@ class Program(object):
             self.out.append(node if node in stored else None)
         self.slots = max(used, 1)
         self.code = bytes(code)
+        self.members = [m for m, _ in self.members]
+        del self.values, self.slot_of_input                 # needed while collecting only
         return self.slots
 
     def run(self, vals, arrays, stream):
@@ -152,6 +154,7 @@ class StepPlan(object):
                 segment.append(n)
         self._schedule(segment)
         self._flush_all()
+        del self.users, self.shapes, self.external, self.root, self.open, self.home, self.copies     # planning only
 
     @staticmethod
     def _has_effects(n):
@@ -234,7 +237,8 @@ class StepPlan(object):
         light, heavy = [], []             # ready nodes: those that cost no launch of their own, the others
 
         def ready(n):
-            cls = "elided" if n in self.elided else "view" if self._is_view(n) else "copy" if isinstance(n.op, BatchNormGradScaleOp) else None
+            cls = ("elided" if n in self.elided else "view" if self._is_view(n) else
+                   "copy" if isinstance(n.op, BatchNormGradScaleOp) else None)
             ops = None if cls else self._operands(n)
             heapq.heappush(light if cls or ops is not None else heavy, (n.id, n, cls, ops))
 
@@ -406,10 +410,10 @@ class StepPlan(object):
                 self._sums(x, vals, stream)
             elif what == "program":
                 if x.run(vals, self.arrays, stream):
-                    for m, _ in x.members:
+                    for m in x.members:
                         vals[m] = self.arrays[m]
                 else:
-                    for m, _ in x.members:
+                    for m in x.members:
                         self._node(m, vals, stream)
             else:
                 src = [n.inputs[0].state[n.op.key] for n in x]
