@@ -1381,8 +1381,8 @@ int launch_fwd_pair_bn(const CUtensorMap& tm, const CUtensorMap& tmi, const CUte
   long long pairs = sm_count() / 2;
   if (pairs > items) pairs = items;
   if (p.stats && pairs > ptn) pairs -= pairs % ptn;              // every pair then sees one column tile only
-  cudaError_t e = tsb_launch::launch_cluster(2u, kern, dim3((unsigned)(2 * pairs)), dim3(192), PC::SMEM_BYTES, st,
-                                             tm, tmi, tmo, p);
+  cudaError_t e = tsb_launch::launch_cluster(2u, kern, dim3((unsigned)(2 * pairs)), dim3(192), PC::SMEM_BYTES, st, tm,
+                                             tmi, tmo, p);
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
 
@@ -1405,8 +1405,7 @@ int launch_wgrad_pair(const CUtensorMap& tm, const CUtensorMap& tmi, const ConvP
   long long pairs = sm_count() / 2;
   if (pairs > items) pairs = items;
   cudaError_t e = tsb_launch::launch_cluster(2u, conv_wgrad_pair_kernel, dim3((unsigned)(2 * pairs)), dim3(288),
-                                             P2_SMEM_BYTES, st,
-                                             tm, tmi, p);
+                                             P2_SMEM_BYTES, st, tm, tmi, p);
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
 
@@ -1720,7 +1719,8 @@ int tsb_conv2d(int kind, float* x, float* w, float* y, int N, int C, int H, int 
     if (p.splits > 1) {
       const long long per_split4 = (long long)O * KH * KW * C / 4;
       tsb_launch::launch(conv_splitk_reduce, dim3((unsigned)((per_split4 + 255) / 256)), 256, 0, st,
-                         reinterpret_cast<const float4*>(p.ws), reinterpret_cast<float4*>(p.out), p.splits, per_split4);
+                         reinterpret_cast<const float4*>(p.ws), reinterpret_cast<float4*>(p.out), p.splits,
+                         per_split4);
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
     }

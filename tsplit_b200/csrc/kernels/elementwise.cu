@@ -548,7 +548,7 @@ int tsb_strided_unary(int op, const float* x, float* y, int nd, const long long*
       for (int i = 0; i < nd - 1; ++i) { v.s0[i] /= 4; v.s1[i] /= 4; }
       const long long n4 = n / 4;
       tsb_launch::launch(copy_strided_v4, grid_for(n4, 256), 256, 0, st, reinterpret_cast<const float4*>(x),
-                                                          reinterpret_cast<float4*>(y), v, n4);
+                         reinterpret_cast<float4*>(y), v, n4);
       return done();
     }
   }
@@ -562,8 +562,7 @@ int tsb_strided_unary(int op, const float* x, float* y, int nd, const long long*
       const long long tiles = outer * ((shape[rdim] + 31) / 32) * ((shape[nd - 1] + 31) / 32);
       int grid = tiles > 148ll * 16 ? 148 * 16 : (int)tiles;
       tsb_launch::launch(copy_tiled, grid, dim3(32, 8), 0, st, x, y, outer, shape[rdim], shape[nd - 1], xso, xs[rdim],
-                         1, yso, 1,
-                                               ys[nd - 1]);
+                         1, yso, 1, ys[nd - 1]);
       return done();
     }
   }
@@ -577,8 +576,7 @@ int tsb_strided_unary(int op, const float* x, float* y, int nd, const long long*
       const long long tiles = outer * ((shape[nd - 1] + 31) / 32) * ((shape[cdim] + 31) / 32);
       int grid = tiles > 148ll * 16 ? 148 * 16 : (int)tiles;
       tsb_launch::launch(copy_tiled, grid, dim3(32, 8), 0, st, x, y, outer, shape[nd - 1], shape[cdim], xso,
-                         xs[nd - 1], 1, yso, 1,
-                                               ys[cdim]);
+                         xs[nd - 1], 1, yso, 1, ys[cdim]);
       return done();
     }
   }
@@ -612,8 +610,7 @@ int tsb_bias_add(const float* x, const float* b, float* y, long long rows, long 
   const long long n4 = rows * (cols / 4);
   tsb_launch::launch(bias_add_v4, tiles_for(4 * n4), 256, 0, static_cast<cudaStream_t>(stream),
                      reinterpret_cast<const float4*>(x), reinterpret_cast<const float4*>(b),
-                     reinterpret_cast<float4*>(y), n4,
-      (unsigned)(cols / 4));
+                     reinterpret_cast<float4*>(y), n4, (unsigned)(cols / 4));
   return done();
 }
 
@@ -680,8 +677,7 @@ int tsb_reduce_sum(const float* x, float* y, int nk, const long long* kshape, co
         const int cols4 = (int)(nkeep / 4);
         dim3 g1((unsigned)((cols4 + 127) / 128), chunks);
         tsb_launch::launch(colsum_partial_v4, g1, 128, 0, st, reinterpret_cast<const float4*>(x),
-                           reinterpret_cast<float4*>(part),
-                                              nred, cols4, rxs[0] / 4, chunks);
+                           reinterpret_cast<float4*>(part), nred, cols4, rxs[0] / 4, chunks);
         tsb_launch::launch(colsum_final_lanes, (unsigned)((nkeep + 31) / 32), dim3(32, 32), 0, st, part, y, nkeep,
                            chunks, kys[0]);
         return done();

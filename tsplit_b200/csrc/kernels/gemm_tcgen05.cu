@@ -1091,8 +1091,7 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
         long long blocks = (total + 255) / 256;
         if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
         tsb_launch::launch(pad_rows_kernel, (unsigned)blocks, 256, 0, st, a, buf, batch, rows_a, cols_a, lda,
-                           batch > 1 ? sa : 0, lda2,
-                                                         sa2);
+                           batch > 1 ? sa : 0, lda2, sa2);
         ap = buf;
       }
     }
@@ -1106,8 +1105,7 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
         long long blocks = (total + 255) / 256;
         if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
         tsb_launch::launch(pad_rows_kernel, (unsigned)blocks, 256, 0, st, b, buf, batch, rows_b, cols_b, ldb,
-                           batch > 1 ? sb : 0, ldb2,
-                                                         sb2);
+                           batch > 1 ? sb : 0, ldb2, sb2);
         bp = buf;
       }
     }
@@ -1123,8 +1121,8 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
               m, n, k, lda, ldb, trans_a, trans_b, batch, sa, sb, (int)(reinterpret_cast<uintptr_t>(a) & 15),
               (int)(reinterpret_cast<uintptr_t>(b) & 15));
     dim3 blk(16, 16), grd((n + 15) / 16, (m + 15) / 16, batch);
-    tsb_launch::launch(gemm_simt_kernel, grd, blk, 0, st, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, sa, sb, sc,
-                                          accumulate);
+    tsb_launch::launch(gemm_simt_kernel, grd, blk, 0, st, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, sa, sb,
+                       sc, accumulate);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
   }
@@ -1145,8 +1143,8 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
     const long long per_split = (long long)batch * m * n;
     if (n % 4 == 0 && ldc % 4 == 0 && (batch == 1 || sc % 4 == 0) && (reinterpret_cast<uintptr_t>(c) & 15) == 0) {
       tsb_launch::launch(splitk_reduce_v4, dim3((unsigned)((per_split / 4 + 255) / 256)), 256, 0, st,
-                         reinterpret_cast<const float4*>(p.ws), reinterpret_cast<float4*>(c), p.splits, per_split / 4, m,
-                         n / 4, ldc / 4, batch > 1 ? sc / 4 : 0, accumulate);
+                         reinterpret_cast<const float4*>(p.ws), reinterpret_cast<float4*>(c), p.splits, per_split / 4,
+                         m, n / 4, ldc / 4, batch > 1 ? sc / 4 : 0, accumulate);
       const cudaError_t e4 = cudaGetLastError();
       if (e4 != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e4 << 8);
       const int late4 = tsb_host::peek_status();

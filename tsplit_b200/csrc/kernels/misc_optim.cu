@@ -293,14 +293,13 @@ int tsb_embedding_grad(const float* g, const float* idx, float* dtable, long lon
   if (n > 0 && dim > 0 && dim % 4 == 0 && dim < (1ll << 32) && n * dim < (1ll << 40) &&
       ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(dtable)) & 15) == 0) {
     const long long n4 = n * (dim / 4);
-    tsb_launch::launch(embedding_grad_v4, dim3((unsigned)((n4 + 255) / 256)), 256, 0, static_cast<cudaStream_t>(stream),
-                       reinterpret_cast<const float4*>(g), idx, reinterpret_cast<float4*>(dtable), n4, vocab,
-                       (unsigned)(dim / 4));
+    tsb_launch::launch(embedding_grad_v4, dim3((unsigned)((n4 + 255) / 256)), 256, 0,
+                       static_cast<cudaStream_t>(stream), reinterpret_cast<const float4*>(g), idx,
+                       reinterpret_cast<float4*>(dtable), n4, vocab, (unsigned)(dim / 4));
     return done();
   }
   tsb_launch::launch(embedding_grad_kernel, ew_grid(n * dim), 256, 0, static_cast<cudaStream_t>(stream), g, idx,
-                     dtable, n, vocab,
-                                                                                         dim);
+                     dtable, n, vocab, dim);
   return done();
 }
 
@@ -327,13 +326,11 @@ int tsb_csrmm(const float* vals, const float* rowptr, const float* colidx, long 
   const long long threads = nrow * 32;
   if (!trans_a) {
     tsb_launch::launch(csrmm_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, vals, rowptr, colidx, nrow, dense,
-                       out,
-                                                                     ncols_dense);
+                       out, ncols_dense);
   } else {
     tsb_launch::launch(zero_kernel, ew_grid(ncol * ncols_dense), 256, 0, st, out, ncol * ncols_dense);
     tsb_launch::launch(csrmm_t_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, vals, rowptr, colidx, nrow,
-                       dense, out,
-                                                                       ncols_dense);
+                       dense, out, ncols_dense);
   }
   return done();
 }

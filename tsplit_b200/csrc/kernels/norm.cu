@@ -510,12 +510,10 @@ int tsb_bn_forward(const float* x, const float* scale, const float* bias, float*
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<0>, sg.grid, STAT_THREADS, 0, st, x, nullptr, nullptr, nullptr, part, rows, (int)C,
                      ldx, 0, sg.chunks, sg.cw, nullptr, nullptr, PLANE_FLOATS);
-  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C,
-                     (double)rows, eps, momentum, save_mean,
-                                                         save_invstd, run_mean, run_var, PLANE_FLOATS);
-  tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y,
-                     rows, (int)C,
-                                                        ldx, ldy, relu);
+  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C, (double)rows,
+                     eps, momentum, save_mean, save_invstd, run_mean, run_var, PLANE_FLOATS);
+  tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y, rows,
+                     (int)C, ldx, ldy, relu);
   return done();
 }
 
@@ -529,11 +527,9 @@ int tsb_bn_forward_from_partials(const float* part, int chunks, long long plane,
   if (rows <= 0 || C <= 0 || chunks <= 0 || !part) return TSB_ERR_ARG;
   if ((C % 4) || (ldx % 4) || (ldy % 4)) return TSB_ERR_UNSUPPORTED;
   tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, chunks, (int)C, (double)rows,
-                     eps, momentum,
-                                                                 save_mean, save_invstd, run_mean, run_var, plane);
-  tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y,
-                     rows, (int)C,
-                                                        ldx, ldy, relu);
+                     eps, momentum, save_mean, save_invstd, run_mean, run_var, plane);
+  tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y, rows,
+                     (int)C, ldx, ldy, relu);
   return done();
 }
 
@@ -546,9 +542,8 @@ int tsb_bn_apply(const float* x, const float* scale, const float* bias, float* y
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows <= 0 || C <= 0) return TSB_ERR_ARG;
   if ((C % 4) || (ldx % 4) || (ldy % 4)) return TSB_ERR_UNSUPPORTED;
-  tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y,
-                     rows, (int)C,
-                                                        ldx, ldy, relu);
+  tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y, rows,
+                     (int)C, ldx, ldy, relu);
   return done();
 }
 
@@ -568,12 +563,10 @@ int tsb_bn_forward_static(const float* x, const float* scale, const float* bias,
   // same call, so nothing in the shared array has to be cleared between calls
   tsb_launch::launch(col_partial<0>, sg.grid, STAT_THREADS, 0, st, x, nullptr, nullptr, nullptr, part, rows, (int)C,
                      ldx, 0, sg.chunks, sg.cw, nullptr, nullptr, PLANE_FLOATS);
-  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C,
-                     (double)rows, eps, momentum, save_mean,
-                                                         save_invstd, run_mean, run_var, PLANE_FLOATS);
-  tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y,
-                     rows, (int)C,
-                                                        ldx, ldy, relu);
+  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C, (double)rows,
+                     eps, momentum, save_mean, save_invstd, run_mean, run_var, PLANE_FLOATS);
+  tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y, rows,
+                     (int)C, ldx, ldy, relu);
   return done();
 }
 
@@ -587,13 +580,11 @@ int tsb_bn_backward(const float* dy, const float* x, const float* scale, const f
   if (!part) return TSB_ERR_OOM;
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<1>, sg.grid, STAT_THREADS, 0, st, dy, x, save_mean, save_invstd, part, rows, (int)C,
-                     lddy, ldx, sg.chunks,
-                                                   sg.cw, nullptr, nullptr, PLANE_FLOATS);
+                     lddy, ldx, sg.chunks, sg.cw, nullptr, nullptr, PLANE_FLOATS);
   tsb_launch::launch(bn_finalize_bwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C, dscale,
                      dbias, PLANE_FLOATS);
   tsb_launch::launch(bn_apply_bwd, apply_grid(rows, C), 256, 0, st, dy, x, scale, save_mean, save_invstd, dscale,
-                     dbias, dx,
-                                                        rows, (int)C, lddy, ldx, lddx, 1.f / (float)rows, nullptr);
+                     dbias, dx, rows, (int)C, lddy, ldx, lddx, 1.f / (float)rows, nullptr);
   return done();
 }
 
@@ -610,13 +601,11 @@ int tsb_bn_relu_backward(const float* dy, const float* x, const float* scale, co
   if (!part) return TSB_ERR_OOM;
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<1>, sg.grid, STAT_THREADS, 0, st, dy, x, save_mean, save_invstd, part, rows, (int)C,
-                     lddy, ldx, sg.chunks,
-                                                   sg.cw, scale, bias, PLANE_FLOATS);
+                     lddy, ldx, sg.chunks, sg.cw, scale, bias, PLANE_FLOATS);
   tsb_launch::launch(bn_finalize_bwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C, dscale,
                      dbias, PLANE_FLOATS);
   tsb_launch::launch(bn_apply_bwd, apply_grid(rows, C), 256, 0, st, dy, x, scale, save_mean, save_invstd, dscale,
-                     dbias, dx,
-                                                        rows, (int)C, lddy, ldx, lddx, 1.f / (float)rows, bias);
+                     dbias, dx, rows, (int)C, lddy, ldx, lddx, 1.f / (float)rows, bias);
   return done();
 }
 
@@ -635,8 +624,8 @@ int tsb_bn_stats_partial(const float* x, float* part, long long plane, int chunk
   const StatGeom sg = stat_geom(rows, (int)C, chunk_cap);
   if ((long long)(chunk_offset + sg.chunks) * C > plane) return TSB_ERR_SCRATCH;
   tsb_launch::launch(col_partial<0>, sg.grid, STAT_THREADS, 0, st, x, nullptr, nullptr, nullptr,
-                     part + (long long)chunk_offset * C,
-                                                   rows, (int)C, ldx, 0, sg.chunks, sg.cw, nullptr, nullptr, plane);
+                     part + (long long)chunk_offset * C, rows, (int)C, ldx, 0, sg.chunks, sg.cw, nullptr, nullptr,
+                     plane);
   *chunks_out = sg.chunks;
   return done();
 }
@@ -647,8 +636,7 @@ int tsb_bn_stats_finalize(const float* part, long long plane, int chunks, double
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (chunks <= 0 || C <= 0 || count <= 0 || !part) return TSB_ERR_ARG;
   tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, chunks, (int)C, count, eps,
-                     momentum, mean,
-                                                                 invstd, run_mean, run_var, plane);
+                     momentum, mean, invstd, run_mean, run_var, plane);
   return done();
 }
 
@@ -663,8 +651,8 @@ int tsb_bn_bwd_partial(const float* dy, const float* x, const float* mean, const
   const StatGeom sg = stat_geom(rows, (int)C, chunk_cap);
   if ((long long)(chunk_offset + sg.chunks) * C > plane) return TSB_ERR_SCRATCH;
   tsb_launch::launch(col_partial<1>, sg.grid, STAT_THREADS, 0, st, dy, x, mean, invstd,
-                     part + (long long)chunk_offset * C, rows,
-                                                   (int)C, lddy, ldx, sg.chunks, sg.cw, rscale, rbias, plane);
+                     part + (long long)chunk_offset * C, rows, (int)C, lddy, ldx, sg.chunks, sg.cw, rscale, rbias,
+                     plane);
   *chunks_out = sg.chunks;
   return done();
 }
@@ -686,8 +674,7 @@ int tsb_bn_bwd_apply(const float* dy, const float* x, const float* scale, const 
   if (rows <= 0 || C <= 0 || total_count <= 0) return TSB_ERR_ARG;
   if ((C % 4) || (ldx % 4) || (lddy % 4) || (lddx % 4)) return TSB_ERR_UNSUPPORTED;
   tsb_launch::launch(bn_apply_bwd, apply_grid(rows, C), 256, 0, st, dy, x, scale, mean, invstd, dscale, dbias, dx,
-                     rows, (int)C,
-                                                        lddy, ldx, lddx, (float)(1.0 / total_count), rbias);
+                     rows, (int)C, lddy, ldx, lddx, (float)(1.0 / total_count), rbias);
   return done();
 }
 
@@ -713,14 +700,13 @@ int tsb_layer_norm_grad(const float* dy, const float* x, const float* scale, con
   const int d4 = (int)(D / 4);
   if (D % 4 == 0 && D <= 1024 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) |
                                    reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(scale)) & 15) == 0) {
-    tsb_launch::launch(d4 <= 32 ? ln_bwd_dx_v4<1> : d4 <= 64 ? ln_bwd_dx_v4<2> : d4 <= 128 ? ln_bwd_dx_v4<4>
-                                                                                           : ln_bwd_dx_v4<8>,
+    tsb_launch::launch(d4 <= 32 ? ln_bwd_dx_v4<1> : d4 <= 64 ? ln_bwd_dx_v4<2> : d4 <= 128 ? ln_bwd_dx_v4<4> : ln_bwd_dx_v4<8>,
                        (unsigned)((threads + 255) / 256), 256, 0, st, reinterpret_cast<const float4*>(dy),
                        reinterpret_cast<const float4*>(x), reinterpret_cast<const float4*>(scale), mean, invstd,
                        reinterpret_cast<float4*>(dx), rows, d4);
   } else {
     tsb_launch::launch(ln_bwd_dx, (unsigned)((threads + 255) / 256), 256, 0, st, dy, x, scale, mean, invstd, dx, rows,
-                     (int)D);
+                       (int)D);
   }
   int chunks = (int)((rows + 31) / 32);
   if (chunks > MAX_CHUNKS) chunks = MAX_CHUNKS;
@@ -734,10 +720,9 @@ int tsb_layer_norm_grad(const float* dy, const float* x, const float* scale, con
     chunks = (int)(c4 < 1 ? 1 : c4);
     dim3 grid4((unsigned)((D4 + bt - 1) / bt), chunks);
     tsb_launch::launch(ln_bwd_params_partial_v4, grid4, bt, 0, st, reinterpret_cast<const float4*>(dy),
-                                                   reinterpret_cast<const float4*>(x), mean, invstd, part, rows, D4,
-                                                   chunks);
-    tsb_launch::launch(bn_finalize_bwd, fin_blocks(D), dim3(32, FIN_LANES), 0, st, part, chunks, (int)D, dscale,
-                       dbias, PLANE_FLOATS);
+                       reinterpret_cast<const float4*>(x), mean, invstd, part, rows, D4, chunks);
+    tsb_launch::launch(bn_finalize_bwd, fin_blocks(D), dim3(32, FIN_LANES), 0, st, part, chunks, (int)D, dscale, dbias,
+                       PLANE_FLOATS);
     return done();
   }
   dim3 grid((unsigned)((D + 127) / 128), chunks);

@@ -1267,8 +1267,7 @@ int tsb_softmax_ce_grad(const float* x, const float* labels, const float* g, flo
                        rows, (int)(cols / 4));
   }
   tsb_launch::launch(ce_grad_rows, grid, cols >= 1024 ? 256 : 128, 0, static_cast<cudaStream_t>(stream), x, labels, g,
-                     dx, rows,
-                                                                                         cols);
+                     dx, rows, cols);
   return done();
 }
 
