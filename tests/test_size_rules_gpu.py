@@ -224,6 +224,17 @@ def test_embedding_gradient_of_repeated_ids(n, vocab, dim):
     assert torch.equal(table, torch.zeros_like(table).index_add_(0, ids[inside].long(), g[inside]))
 
 
+@pytest.mark.parametrize("n,vocab,dim", [(1, 3, 4), (700, 5, 512), (33, 40, 6), (129, 9, 12)])
+def test_embedding_rows(n, vocab, dim):
+    ctx = ndarray.gpu(0)
+    ids = torch.randint(-1, vocab + 1, (n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)).float()
+    table, y = _rand(vocab, dim), torch.full((n + 1, dim), 7.0, device="cuda")
+    G.embedding(ndarray.from_tensor(table, ctx), ndarray.from_tensor(ids, ctx), ndarray.from_tensor(y[:n], ctx), _stream())
+    inside = ((ids >= 0) & (ids < vocab))[:, None]                       # other ids give rows of zeros
+    assert torch.equal(y[:n], torch.where(inside, table[ids.long().clamp(0, vocab - 1)], torch.zeros((), device="cuda")))
+    assert torch.all(y[n] == 7)
+
+
 @pytest.mark.parametrize("rows,cols", [(514, 4), (1023, 36), (8160, 512), (20000, 1000), (600, 16500)])
 def test_column_sums_of_many_rows(rows, cols):
     x, y = _rand(rows, cols), torch.zeros(cols, device="cuda")
