@@ -136,6 +136,47 @@ def test_cross_entropy_of_long_rows(rows, cols):
     torch.testing.assert_close(dense[1].double(), (lp.exp() - lab.double()) * 0.5 / rows, rtol=1e-4, atol=1e-6 * 0.5 / rows)
 
 
+# masked classes (the lowest float, a common mask value, minus infinity): two of them, half of them, all of one thread's, and
+# the labelled one; the loss from ids is finite, infinite or NaN where the one from dense labels is
+@pytest.mark.parametrize("masked", ["two", "half", "a thread's", "the label"])
+@pytest.mark.parametrize("value", [float(np.finfo(np.float32).min), -1e9, float("-inf")])
+@pytest.mark.parametrize("cols", [512, 8192, 32000])
+def test_cross_entropy_with_masked_classes(cols, value, masked):
+    ctx = ndarray.gpu(0)
+    rows = 5
+    ids = torch.tensor([0., 7., cols - 1, cols // 2, cols], device="cuda")             # the last one: no class
+    x = 3 * _rand(rows, cols)
+    if masked == "two":
+        x[:, 3], x[:, cols - 3] = value, value
+    elif masked == "half":
+        x[:, 1::2] = value
+    elif masked == "a thread's":
+        x[:, 8:12] = value
+        x[:, 8 + 4 * 256:12 + 4 * 256] = value
+        x[:, 8 + 4 * 512::4 * 512] = value
+    else:
+        x[torch.arange(4), ids[:4].long()] = value
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    g = torch.ones(1, device="cuda")
+    for on, off in ((1.0, 0.0), (float(np.float32(0.9) + np.float32(0.1 / cols)), float(np.float32(0.1 / cols)))):
+        lab = torch.full((rows, cols), off, device="cuda")
+        lab[torch.arange(4), ids[:4].long()] = on
+        for r in range(rows):                                                          # each row's loss by itself
+            dense, smooth, row, i = torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda"), x[r:r + 1], ids[r:r + 1]
+            G.softmax_ce(a(row), a(lab[r:r + 1]), a(dense), _stream())
+            assert G.softmax_ce_smooth(a(row), a(i), on, off, a(smooth), _stream())
+            lp = torch.log_softmax(row.double(), 1)
+            want = -(lab[r:r + 1].double() * lp).sum().float()
+            _stream().sync()
+            for loss in (dense, smooth):               # fp32 sums of terms of one sign, as in the test above
+                torch.testing.assert_close(loss[0], want, rtol=2e-5, atol=2e-5, equal_nan=True)
+        dd, ds = torch.zeros(rows, cols, device="cuda"), torch.ones(rows, cols, device="cuda")
+        G.softmax_ce_grad(a(x), a(lab), a(g), a(dd), _stream())
+        assert G.softmax_ce_grad_smooth(a(x), a(ids), on, off, a(g), a(ds), _stream())
+        _stream().sync()
+        assert torch.equal(dd, ds)
+
+
 # outputs that leave by TMA store: ragged rows and columns of a block, one column block and many, batches, several
 # splits; and those whose strides or sums do not allow it (a row of 130 + 1 floats, a base 4 bytes in, accumulation)
 @pytest.mark.parametrize("m,n,k,batch,ldc,shift,accumulate", [
