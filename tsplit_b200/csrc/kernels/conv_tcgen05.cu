@@ -1118,7 +1118,7 @@ conv_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
 // convolution with 32 input and 8*O output channels whose filters are mostly zero:
 //   w'[(po, o)][kh][dx + 1][(pi, c)] = w[o][kh][kw][c]  with  kw = 8 * dx + pi - po + pw,  if 0 <= kw < KW.
 // Eight times the arithmetic, but on the tensor cores at full rate instead of on the gather path.
-__global__ void stem_pack_filters(const float* __restrict__ w, long long so, long long sc, long long sh,
+__global__ void stem_pack_filters(const float* w, long long so, long long sc, long long sh,
                                   long long sw, float* __restrict__ out, int O, int C, int KH, int KW, int pw) {
   tsb_launch::enter();
   const long long total = 8ll * O * KH * 3 * 32;
@@ -1139,7 +1139,7 @@ __global__ void stem_pack_filters(const float* __restrict__ w, long long so, lon
 }
 
 // dw[o][kh][kw][c] = sum of the packed gradient entries that alias this filter tap
-__global__ void stem_unpack_filter_grads(const float* __restrict__ gp, float* __restrict__ dw, long long so,
+__global__ void stem_unpack_filter_grads(const float* gp, float* __restrict__ dw, long long so,
                                          long long sc, long long sh, long long sw, int O, int C, int KH, int KW,
                                          int pw) {
   tsb_launch::enter();
@@ -1165,7 +1165,7 @@ __global__ void stem_unpack_filter_grads(const float* __restrict__ gp, float* __
 // Strided dgrad runs as a stride-1 forward convolution over dy with zeros inserted between its
 // pixels: up[n][s*i][s*j][:] = dy[n][i][j][:], zero elsewhere (Hup x Wup positions).  The inserted
 // zeros cost s*s times the arithmetic of the strided layer, but on the TMA kernels.
-__global__ void upsample_zero_insert(const float* __restrict__ dy, float* __restrict__ up, int N, int OH, int OW,
+__global__ void upsample_zero_insert(const float* dy, float* __restrict__ up, int N, int OH, int OW,
                                      int O, int Hup, int Wup, int stride) {
   tsb_launch::enter();
   const int O4 = O >> 2;
@@ -1212,7 +1212,7 @@ bool parity_axis(int H, int OH, int K, int pad, int a, ParityAxis* d) {
 }
 
 // out[c][Ta-1-ta][Tb-1-tb][o] = w[o][2ta + ra][2tb + rb][c]: the class's sub-filter, flipped and transposed.
-__global__ void parity_filters(const float* __restrict__ w, float* __restrict__ out, int O, int C, int KH, int KW,
+__global__ void parity_filters(const float* w, float* __restrict__ out, int O, int C, int KH, int KW,
                                int ra, int Ta, int rb, int Tb) {
   tsb_launch::enter();
   __shared__ float tile[32][33];
@@ -1261,7 +1261,7 @@ __global__ void parity_interleave(const ParityParts pp, float* __restrict__ dx, 
 
 // (Channel counts are multiples of four, so filters are whole float4.)  Eight partial sums in flight per thread instead
 // of one float after another: ResNet-50 step, 53 of them, 7912 -> 7713 us.
-__global__ void __launch_bounds__(256) conv_splitk_reduce(const float4* __restrict__ ws, float4* __restrict__ out,
+__global__ void __launch_bounds__(256) conv_splitk_reduce(const float4* ws, float4* __restrict__ out,
                                                           int splits, long long per_split4) {
   tsb_launch::enter();
   const long long i = blockIdx.x * 256ll + threadIdx.x;
@@ -1270,7 +1270,7 @@ __global__ void __launch_bounds__(256) conv_splitk_reduce(const float4* __restri
 
 // Filters for stride-1 dgrad run through the forward kernel: out[c][KH-1-kh][KW-1-kw][o] = w[o][kh][kw][c].
 // One 32x32 tile of the (o, c) plane of one tap per block, transposed through shared memory.
-__global__ void flip_transpose_filters(const float* __restrict__ w, float* __restrict__ out, int O, int C, int KH,
+__global__ void flip_transpose_filters(const float* w, float* __restrict__ out, int O, int C, int KH,
                                        int KW) {
   tsb_launch::enter();
   __shared__ float tile[32][33];

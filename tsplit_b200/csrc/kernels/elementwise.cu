@@ -23,6 +23,8 @@
 
 namespace {
 
+using tsb_launch::load;
+
 using namespace tsb_pw;
 
 constexpr int MAXD = 8;
@@ -43,7 +45,7 @@ struct Dims {
 constexpr int TILE4 = 2 * 256;
 
 template <int OP>
-__global__ void __launch_bounds__(256) unary_flat(const float* __restrict__ x, float* __restrict__ y, long long n,
+__global__ void __launch_bounds__(256) unary_flat(const float* x, float* __restrict__ y, long long n,
                                                   float a) {
   tsb_launch::enter();
   const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
@@ -52,7 +54,7 @@ __global__ void __launch_bounds__(256) unary_flat(const float* __restrict__ x, f
     float4 v[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u)
-      if (OP != UN_FILL && j + u * 256 < n4) v[u] = __ldg(reinterpret_cast<const float4*>(x) + j + u * 256);
+      if (OP != UN_FILL && j + u * 256 < n4) v[u] = load(reinterpret_cast<const float4*>(x) + j + u * 256);
 #pragma unroll
     for (int u = 0; u < 2; ++u)
       if (j + u * 256 < n4) {
@@ -69,7 +71,7 @@ __global__ void __launch_bounds__(256) unary_flat(const float* __restrict__ x, f
 }
 
 template <int OP>
-__global__ void __launch_bounds__(256) binary_flat(const float* __restrict__ p, const float* __restrict__ q,
+__global__ void __launch_bounds__(256) binary_flat(const float* p, const float* q,
                                                    float* __restrict__ y, long long n) {
   tsb_launch::enter();
   const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(q) |
@@ -80,8 +82,8 @@ __global__ void __launch_bounds__(256) binary_flat(const float* __restrict__ p, 
 #pragma unroll
     for (int u = 0; u < 2; ++u)
       if (j + u * 256 < n4) {
-        a[u] = __ldg(reinterpret_cast<const float4*>(p) + j + u * 256);
-        b[u] = __ldg(reinterpret_cast<const float4*>(q) + j + u * 256);
+        a[u] = load(reinterpret_cast<const float4*>(p) + j + u * 256);
+        b[u] = load(reinterpret_cast<const float4*>(q) + j + u * 256);
       }
 #pragma unroll
     for (int u = 0; u < 2; ++u)
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(256) binary_flat(const float* __restrict__ p, 
   }
 }
 
-__global__ void where_flat(const float* __restrict__ c, const float* __restrict__ a, const float* __restrict__ b,
+__global__ void where_flat(const float* c, const float* a, const float* b,
                            float* __restrict__ y, long long n) {
   tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -107,7 +109,7 @@ __global__ void where_flat(const float* __restrict__ c, const float* __restrict_
 
 // y[r, c] = x[r, c] + b[c] on a dense row-major [rows, cols] view, 16 bytes per thread (the bias of a
 // dense layer added without materialising the broadcast).
-__global__ void __launch_bounds__(256) bias_add_v4(const float4* __restrict__ x, const float4* __restrict__ b, float4* __restrict__ y,
+__global__ void __launch_bounds__(256) bias_add_v4(const float4* x, const float4* b, float4* __restrict__ y,
                             long long n4, unsigned cols4) {
   tsb_launch::enter();
   const long long i = blockIdx.x * (long long)TILE4 + threadIdx.x;
@@ -116,8 +118,8 @@ __global__ void __launch_bounds__(256) bias_add_v4(const float4* __restrict__ x,
   for (int u = 0; u < 2; ++u) {
     const long long j = i + u * 256;
     if (j < n4) {
-      v[u] = __ldg(x + j);
-      w[u] = __ldg(b + ((n4 >> 32) == 0 ? (unsigned)j % cols4 : (unsigned)(j % cols4)));
+      v[u] = load(x + j);
+      w[u] = load(b + ((n4 >> 32) == 0 ? (unsigned)j % cols4 : (unsigned)(j % cols4)));
     }
   }
 #pragma unroll
@@ -191,7 +193,7 @@ __device__ __forceinline__ void offsets3(const Dims& d, long long idx, long long
 // (a channel range of a channels-last tensor: concat / slice along channels, padded feeds): the same
 // index walk as unary_strided, but in units of 16 bytes.  `d` holds the shape and strides already
 // divided by four in the innermost dimension / for the outer strides.
-__global__ void copy_strided_v4(const float4* __restrict__ x, float4* __restrict__ y, const Dims d, long long n4) {
+__global__ void copy_strided_v4(const float4* x, float4* __restrict__ y, const Dims d, long long n4) {
   tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += stride) {
@@ -202,7 +204,7 @@ __global__ void copy_strided_v4(const float4* __restrict__ x, float4* __restrict
 }
 
 template <int OP>
-__global__ void unary_strided(const float* __restrict__ x, float* __restrict__ y, const Dims d, long long n,
+__global__ void unary_strided(const float* x, float* __restrict__ y, const Dims d, long long n,
                               float a) {
   tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -216,7 +218,7 @@ __global__ void unary_strided(const float* __restrict__ x, float* __restrict__ y
 // 2-D tiled transpose-copy through shared memory for the common "two dims whose
 // fast axis differs between source and destination" case (NCHW <-> NHWC,
 // matrix transpose): both the read and the write are coalesced.
-__global__ void copy_tiled(const float* __restrict__ x, float* __restrict__ y, long long outer, long long R,
+__global__ void copy_tiled(const float* x, float* __restrict__ y, long long outer, long long R,
                            long long Cc, long long xs_outer, long long xs_r, long long xs_c, long long ys_outer,
                            long long ys_r, long long ys_c) {
   tsb_launch::enter();
@@ -243,7 +245,7 @@ __global__ void copy_tiled(const float* __restrict__ x, float* __restrict__ y, l
 }
 
 template <int OP>
-__global__ void binary_strided(const float* __restrict__ p, const float* __restrict__ q, float* __restrict__ y,
+__global__ void binary_strided(const float* p, const float* q, float* __restrict__ y,
                                const Dims d, long long n) {
   tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -257,7 +259,7 @@ __global__ void binary_strided(const float* __restrict__ p, const float* __restr
 // Row forms of the strided kernels for a long innermost dimension: a warp walks one row, so the outer
 // index is decomposed once per row instead of once per element.  Block = 32 lanes x 8 rows.
 template <int OP>
-__global__ void binary_rows(const float* __restrict__ p, const float* __restrict__ q, float* __restrict__ y,
+__global__ void binary_rows(const float* p, const float* q, float* __restrict__ y,
                             const Dims o, long long outer, int inner, long long sa, long long sb,
                             long long sy) {
   tsb_launch::enter();
@@ -271,7 +273,7 @@ __global__ void binary_rows(const float* __restrict__ p, const float* __restrict
   }
 }
 template <int OP>
-__global__ void unary_rows(const float* __restrict__ x, float* __restrict__ y, const Dims o, long long outer,
+__global__ void unary_rows(const float* x, float* __restrict__ y, const Dims o, long long outer,
                            int inner, float a, long long sx, long long sy) {
   tsb_launch::enter();
   for (long long r = blockIdx.x * (long long)blockDim.y + threadIdx.y; r < outer;
@@ -290,7 +292,7 @@ struct RDims {
   long long rshape[MAXD], rxs[MAXD];
   int nk, nr;
 };
-__global__ void reduce_sum_kernel(const float* __restrict__ x, float* __restrict__ y, const RDims d,
+__global__ void reduce_sum_kernel(const float* x, float* __restrict__ y, const RDims d,
                                   long long nkeep, long long nred) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;
@@ -323,7 +325,7 @@ __global__ void reduce_sum_kernel(const float* __restrict__ x, float* __restrict
 // Column sums of a row-major [rows, cols] view with cols contiguous (the
 // "reduce over leading dims" case: bias gradients, axis-0 sums): coalesced along
 // cols, two-stage and deterministic.
-__global__ void colsum_partial(const float* __restrict__ x, float* __restrict__ part, long long rows,
+__global__ void colsum_partial(const float* x, float* __restrict__ part, long long rows,
                                long long cols, long long ld, int chunks) {
   tsb_launch::enter();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -336,7 +338,7 @@ __global__ void colsum_partial(const float* __restrict__ x, float* __restrict__ 
   part[(long long)ch * cols + c] = acc;
 }
 // 16-byte variant: a thread owns four adjacent columns and keeps four rows in flight.
-__global__ void colsum_partial_v4(const float4* __restrict__ x, float4* __restrict__ part, long long rows,
+__global__ void colsum_partial_v4(const float4* x, float4* __restrict__ part, long long rows,
                                   int cols4, long long ld4, int chunks) {
   tsb_launch::enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -347,15 +349,15 @@ __global__ void colsum_partial_v4(const float4* __restrict__ x, float4* __restri
   float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0, a2 = a0, a3 = a0;
   long long r = r0;
   for (; r + 3 < r1; r += 4) {
-    const float4 v0 = __ldg(x + r * ld4 + c), v1 = __ldg(x + (r + 1) * ld4 + c), v2 = __ldg(x + (r + 2) * ld4 + c),
-                 v3 = __ldg(x + (r + 3) * ld4 + c);
+    const float4 v0 = load(x + r * ld4 + c), v1 = load(x + (r + 1) * ld4 + c), v2 = load(x + (r + 2) * ld4 + c),
+                 v3 = load(x + (r + 3) * ld4 + c);
     a0.x += v0.x; a0.y += v0.y; a0.z += v0.z; a0.w += v0.w;
     a1.x += v1.x; a1.y += v1.y; a1.z += v1.z; a1.w += v1.w;
     a2.x += v2.x; a2.y += v2.y; a2.z += v2.z; a2.w += v2.w;
     a3.x += v3.x; a3.y += v3.y; a3.z += v3.z; a3.w += v3.w;
   }
   for (; r < r1; ++r) {
-    const float4 v = __ldg(x + r * ld4 + c);
+    const float4 v = load(x + r * ld4 + c);
     a0.x += v.x; a0.y += v.y; a0.z += v.z; a0.w += v.w;
   }
   part[(long long)ch * cols4 + c] =
@@ -364,7 +366,7 @@ __global__ void colsum_partial_v4(const float4* __restrict__ x, float4* __restri
 }
 // Second stage: 32 columns x 32 chunk lanes per block, eight loads in flight, lanes joined in a fixed order (256 chunks
 // of 512 columns: 3.4 us with 8 lanes, 2.9 now).
-__global__ void __launch_bounds__(1024) colsum_final_lanes(const float* __restrict__ part, float* __restrict__ y,
+__global__ void __launch_bounds__(1024) colsum_final_lanes(const float* part, float* __restrict__ y,
                                                            long long cols, int chunks, long long ys) {
   tsb_launch::enter();
   __shared__ float sh[32][33];
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(1024) colsum_final_lanes(const float* __restri
   }
   if (threadIdx.y == 0 && c < cols) y[c * ys] = sh[0][threadIdx.x];
 }
-__global__ void colsum_final(const float* __restrict__ part, float* __restrict__ y, long long cols, int chunks,
+__global__ void colsum_final(const float* part, float* __restrict__ y, long long cols, int chunks,
                              long long ys) {
   tsb_launch::enter();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -419,7 +421,7 @@ __global__ void __launch_bounds__(1024) colsum_group(const __grid_constant__ Col
     for (int r = threadIdx.y; r < rows; r += 128) {
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (r + 32 * u < rows) a[u] += __ldg(x + (r + 32 * u) * ld);
+        if (r + 32 * u < rows) a[u] += load(x + (r + 32 * u) * ld);
     }
   sh[threadIdx.y][threadIdx.x] = (a[0] + a[1]) + (a[2] + a[3]);
   for (int o = 16; o > 0; o >>= 1) {

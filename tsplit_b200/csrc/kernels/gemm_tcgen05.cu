@@ -571,7 +571,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 }
 
 // Deterministic split-K reduction: c (+)= sum_s ws[s]
-__global__ void splitk_reduce_kernel(const float* __restrict__ ws, float* __restrict__ c, int splits,
+__global__ void splitk_reduce_kernel(const float* ws, float* __restrict__ c, int splits,
                                      long long per_split, int m, int n, long long ldc, long long sc,
                                      int accumulate) {
   tsb_launch::enter();
@@ -589,7 +589,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, float* __rest
 }
 
 // The same with 16-byte lanes, for rows of whole float4 on both sides (5.6 -> 4.4 us each in a Transformer block).
-__global__ void __launch_bounds__(256) splitk_reduce_v4(const float4* __restrict__ ws, float4* __restrict__ c, int splits,
+__global__ void __launch_bounds__(256) splitk_reduce_v4(const float4* ws, float4* __restrict__ c, int splits,
                                                         long long per_split4, int m, int n4, long long ldc4,
                                                         long long sc4, int accumulate) {
   tsb_launch::enter();
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_v4(const float4* __restrict
 
 // Plain SIMT fallback for shapes the tensor-map rules exclude (leading dimension
 // not a multiple of 4 floats, unaligned base).  Tiny problems only.
-__global__ void gemm_simt_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
+__global__ void gemm_simt_kernel(const float* a, const float* b, float* __restrict__ c,
                                  int m, int n, int k, long long lda, long long ldb, long long ldc, int ta, int tb,
                                  long long sa, long long sb, long long sc, int accumulate) {
   tsb_launch::enter();
@@ -891,7 +891,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
 
 // Copy of a [batch][rows][cols] operand whose row stride is not a multiple of four floats into a
 // scratch array with the row stride rounded up (pad columns zero), so that TMA can address it.
-__global__ void pad_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int batch, int rows,
+__global__ void pad_rows_kernel(const float* src, float* __restrict__ dst, int batch, int rows,
                                 int cols, long long lds, long long ss, long long ldd, long long sd) {
   tsb_launch::enter();
   const long long total = (long long)batch * rows * ldd;

@@ -6,8 +6,17 @@
 // its blocks may be placed, and barriers and TMEM set up, while the previous kernel drains; they wait until that
 // kernel has completed and its writes are visible.  Because every kernel waits, completion stays in stream order; a
 // copy, an event or a kernel of another library in between is ordered in full as before.  Stream capture keeps the
-// attribute as a programmatic edge.  Captured steps: LSTM, 2428 kernels: 6718 -> 5535 us (2.77 -> 2.28 us a kernel);
-// a 1x7 / 7x1 convolution pair at 17 x 17: 292 -> 275 us; a small Transformer: 808 -> 716 us.
+// attribute as a programmatic edge.
+//
+// A kernel thus begins before its inputs are written.  Loads through the read-only path (ld.global.nc: __ldg, or what
+// nvcc makes of a `const T* __restrict__` parameter) want data that nothing writes while the kernel lives, and
+// may be moved above the wait or served from a line that was cached before it.  So kernels launched from here
+// take the pointers they read without __restrict__ and use ordinary loads, which stay behind the wait; pointers that
+// they write keep __restrict__, so loads may still pass stores.  A plain load costs the same: 137 M floats times a
+// constant 161.5 us through the read-only path and 161.9 without, the sum of two such tensors 234.3 and 235.5.
+//
+// Captured steps: LSTM, 2428 kernels: 6718 -> 5535 us (2.77 -> 2.28 us a kernel); a 1x7 / 7x1 convolution pair at 17 x 17:
+// 292 -> 275 us; a small Transformer: 808 -> 716 us.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -26,6 +35,10 @@ __device__ __forceinline__ void enter() {
   wait_previous();
   if (gridDim.x * gridDim.y * gridDim.z <= FEW_BLOCKS) allow_next();
 }
+
+// An ordinary (coherent) load of data that an earlier kernel may have written.
+template <class T>
+__device__ __forceinline__ T load(const T* p) { return *p; }
 
 // cluster: blocks per cluster along x (0: no cluster).  Errors are left for cudaGetLastError, as with <<<>>>.
 template <class... P, class... A>

@@ -15,6 +15,8 @@
 
 namespace {
 
+using tsb_launch::load;
+
 int sm_count() {
   static int n = 0;
   if (!n) {
@@ -36,7 +38,7 @@ int done() {
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
 
-__global__ void one_hot_kernel(const float* __restrict__ idx, float* __restrict__ y, long long n, long long k) {
+__global__ void one_hot_kernel(const float* idx, float* __restrict__ y, long long n, long long k) {
   tsb_launch::enter();
   const long long total = n * k;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -48,7 +50,7 @@ __global__ void one_hot_kernel(const float* __restrict__ idx, float* __restrict_
 
 // Rows that are a multiple of four classes long: one block row-slice per row, 16-byte stores, no division
 // per element (grid.y walks the rows, grid.x * blockDim.x the 4-class groups of a row).
-__global__ void one_hot_rows_v4(const float* __restrict__ idx, float4* __restrict__ y, long long n, int k4) {
+__global__ void one_hot_rows_v4(const float* idx, float4* __restrict__ y, long long n, int k4) {
   tsb_launch::enter();
   for (long long r = blockIdx.y; r < n; r += gridDim.y) {
     const long long id = (long long)idx[r];
@@ -61,7 +63,7 @@ __global__ void one_hot_rows_v4(const float* __restrict__ idx, float4* __restric
   }
 }
 
-__global__ void embedding_kernel(const float* __restrict__ table, const float* __restrict__ idx,
+__global__ void embedding_kernel(const float* table, const float* idx,
                                  float* __restrict__ y, long long n, long long vocab, long long dim) {
   tsb_launch::enter();
   const long long total = n * dim;
@@ -75,7 +77,7 @@ __global__ void embedding_kernel(const float* __restrict__ table, const float* _
 
 // Rows of whole float4: two 16-byte loads in flight and a 32-bit division per thread instead of a 64-bit one per float.
 // 8192 tokens x 512: 12.4 -> 5.6 us.
-__global__ void __launch_bounds__(256) embedding_v4(const float4* __restrict__ table, const float* __restrict__ idx,
+__global__ void __launch_bounds__(256) embedding_v4(const float4* table, const float* idx,
                                                     float4* __restrict__ y, long long n4, long long vocab,
                                                     unsigned dim4) {
   tsb_launch::enter();
@@ -87,8 +89,8 @@ __global__ void __launch_bounds__(256) embedding_v4(const float4* __restrict__ t
     v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (j < n4) {
       const long long r = (n4 >> 32) == 0 ? (long long)((unsigned)j / dim4) : j / dim4;
-      const long long id = (long long)__ldg(idx + r);
-      if (id >= 0 && id < vocab) v[u] = __ldg(table + id * dim4 + (j - r * dim4));
+      const long long id = (long long)load(idx + r);
+      if (id >= 0 && id < vocab) v[u] = load(table + id * dim4 + (j - r * dim4));
     }
   }
 #pragma unroll
@@ -96,7 +98,7 @@ __global__ void __launch_bounds__(256) embedding_v4(const float4* __restrict__ t
     if (i + u * 256 < n4) y[i + u * 256] = v[u];
 }
 
-__global__ void embedding_grad_kernel(const float* __restrict__ g, const float* __restrict__ idx,
+__global__ void embedding_grad_kernel(const float* g, const float* idx,
                                       float* __restrict__ dtable, long long n, long long vocab, long long dim) {
   tsb_launch::enter();
   const long long total = n * dim;
@@ -110,7 +112,7 @@ __global__ void embedding_grad_kernel(const float* __restrict__ g, const float* 
 
 // Rows of whole float4: one 16-byte reduction instead of four.  Bound by reductions that meet in the
 // rows of frequent ids (8192 tokens x 512 over 1000 words: 24.7 -> 22.1 us).
-__global__ void __launch_bounds__(256) embedding_grad_v4(const float4* __restrict__ g, const float* __restrict__ idx,
+__global__ void __launch_bounds__(256) embedding_grad_v4(const float4* g, const float* idx,
                                                          float4* __restrict__ dtable, long long n4, long long vocab,
                                                          unsigned dim4) {
   tsb_launch::enter();
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(256) embedding_grad_v4(const float4* __restric
   if (i >= n4) return;
   const long long r = (n4 >> 32) == 0 ? (long long)((unsigned)i / dim4) : i / dim4;
   const long long id = (long long)idx[r];
-  if (id >= 0 && id < vocab) atomicAdd(dtable + id * dim4 + (i - r * dim4), __ldg(g + i));
+  if (id >= 0 && id < vocab) atomicAdd(dtable + id * dim4 + (i - r * dim4), load(g + i));
 }
 
 // splitmix64 of (seed, element index): the keep decision is a pure function of both
@@ -134,8 +136,8 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
 // step replayed from a CUDA graph still draws a new mask; the seed is mixed exactly as on the host.
 // offset: index of x[0] in the whole tensor when x is a batch piece of it (the mask is a function of the
 // element's index in the WHOLE tensor, so a tensor computed piece by piece gets the same mask).
-__global__ void dropout_kernel(const float* __restrict__ x, float* __restrict__ y, long long n, float keep,
-                               unsigned long long seed, const unsigned long long* __restrict__ step_dev,
+__global__ void dropout_kernel(const float* x, float* __restrict__ y, long long n, float keep,
+                               unsigned long long seed, const unsigned long long* step_dev,
                                unsigned long long offset) {
   tsb_launch::enter();
   if (step_dev) seed = (seed + 0x632BE5ABull * *step_dev) & 0x7FFFFFFFFFFFFFFFull;
@@ -146,8 +148,8 @@ __global__ void dropout_kernel(const float* __restrict__ x, float* __restrict__ 
 }
 
 // out[r, :] = sum_j vals[j] * dense[col[j], :]   (one warp per sparse row)
-__global__ void csrmm_kernel(const float* __restrict__ vals, const float* __restrict__ rowptr,
-                             const float* __restrict__ colidx, long long nrow, const float* __restrict__ dense,
+__global__ void csrmm_kernel(const float* vals, const float* rowptr,
+                             const float* colidx, long long nrow, const float* dense,
                              float* __restrict__ out, long long ncols) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;
@@ -161,8 +163,8 @@ __global__ void csrmm_kernel(const float* __restrict__ vals, const float* __rest
   }
 }
 // out[col[j], :] += vals[j] * dense[r, :]   (transposed sparse operand; out pre-zeroed)
-__global__ void csrmm_t_kernel(const float* __restrict__ vals, const float* __restrict__ rowptr,
-                               const float* __restrict__ colidx, long long nrow, const float* __restrict__ dense,
+__global__ void csrmm_t_kernel(const float* vals, const float* rowptr,
+                               const float* colidx, long long nrow, const float* dense,
                                float* __restrict__ out, long long ncols) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;

@@ -27,6 +27,8 @@
 
 namespace {
 
+using tsb_launch::load;
+
 constexpr int MAX_CHUNKS = 128;
 constexpr long long PLANE_FLOATS = (long long)MAX_CHUNKS * 8192;   // one partial plane: chunks x channels
 constexpr long long SCRATCH_FLOATS = 2 * PLANE_FLOATS;              // two planes (up to 8192 channels at MAX_CHUNKS)
@@ -83,10 +85,10 @@ __device__ __forceinline__ float4 relu_mask(float4 g, const float4 x, const floa
 
 template <int MODE>
 __global__ void __launch_bounds__(STAT_THREADS)
-col_partial(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ mean,
-            const float* __restrict__ invstd, float* __restrict__ part, long long rows, int C,
-            long long lda, long long ldb, int chunks, int cw, const float* __restrict__ rscale = nullptr,
-            const float* __restrict__ rbias = nullptr, long long plane = PLANE_FLOATS) {
+col_partial(const float* a, const float* b, const float* mean,
+            const float* invstd, float* __restrict__ part, long long rows, int C,
+            long long lda, long long ldb, int chunks, int cw, const float* rscale = nullptr,
+            const float* rbias = nullptr, long long plane = PLANE_FLOATS) {
   tsb_launch::enter();
   __shared__ float4 s0[STAT_THREADS], s1[STAT_THREADS];
   const int rl = STAT_THREADS / cw;               // row lanes
@@ -159,7 +161,7 @@ col_partial(const float* __restrict__ a, const float* __restrict__ b, const floa
 // x FIN_LANES lanes; lane y adds chunks y, y+FIN_LANES, ... (four independent loads in flight),
 // lane 0 then adds the lane sums.
 constexpr int FIN_LANES = 32;
-__device__ __forceinline__ void reduce_partials(const float* __restrict__ part, int chunks, int C, int c,
+__device__ __forceinline__ void reduce_partials(const float* part, int chunks, int C, int c,
                                                 double& s, double& ss, long long plane = PLANE_FLOATS) {
   __shared__ double sh0[FIN_LANES][33], sh1[FIN_LANES][33];
   double a = 0.0, b = 0.0;
@@ -191,7 +193,7 @@ __device__ __forceinline__ void reduce_partials(const float* __restrict__ part, 
 }
 
 // Forward finalise: mean / invstd from the partial sums (+ running statistics).  Block (32, FIN_LANES).
-__global__ void bn_finalize_fwd(const float* __restrict__ part, int chunks, int C, double count, float eps,
+__global__ void bn_finalize_fwd(const float* part, int chunks, int C, double count, float eps,
                                 float momentum, float* __restrict__ mean, float* __restrict__ invstd,
                                 float* __restrict__ run_mean, float* __restrict__ run_var,
                                 long long plane = PLANE_FLOATS) {
@@ -211,7 +213,7 @@ __global__ void bn_finalize_fwd(const float* __restrict__ part, int chunks, int 
   }
 }
 
-__global__ void bn_finalize_bwd(const float* __restrict__ part, int chunks, int C, float* __restrict__ dscale,
+__global__ void bn_finalize_bwd(const float* part, int chunks, int C, float* __restrict__ dscale,
                                 float* __restrict__ dbias, long long plane = PLANE_FLOATS) {
   tsb_launch::enter();
   const int c = blockIdx.x * 32 + threadIdx.x;
@@ -238,9 +240,9 @@ __device__ __forceinline__ void row_col(long long i, int C4, long long total, lo
   }
 }
 
-__global__ void __launch_bounds__(256) bn_apply_fwd(const float* __restrict__ x, const float* __restrict__ scale,
-                             const float* __restrict__ bias, const float* __restrict__ mean,
-                             const float* __restrict__ invstd, float* __restrict__ y, long long rows, int C,
+__global__ void __launch_bounds__(256) bn_apply_fwd(const float* x, const float* scale,
+                             const float* bias, const float* mean,
+                             const float* invstd, float* __restrict__ y, long long rows, int C,
                              long long ldx, long long ldy, int relu) {
   tsb_launch::enter();
   const long long total = rows * (C >> 2), i = blockIdx.x * (long long)APPLY_TILE + threadIdx.x;
@@ -251,15 +253,15 @@ __global__ void __launch_bounds__(256) bn_apply_fwd(const float* __restrict__ x,
   for (int u = 0; u < 2; ++u)
     if (i + u * 256 < total) {
       row_col(i + u * 256, C >> 2, total, r[u], c[u]);
-      v[u] = __ldg(reinterpret_cast<const float4*>(x + r[u] * ldx + c[u]));
+      v[u] = load(reinterpret_cast<const float4*>(x + r[u] * ldx + c[u]));
     }
 #pragma unroll
   for (int u = 0; u < 2; ++u)
     if (i + u * 256 < total) {
-      const float4 mu = __ldg(reinterpret_cast<const float4*>(mean + c[u]));
-      const float4 is = __ldg(reinterpret_cast<const float4*>(invstd + c[u]));
-      const float4 g = __ldg(reinterpret_cast<const float4*>(scale + c[u]));
-      const float4 b = __ldg(reinterpret_cast<const float4*>(bias + c[u]));
+      const float4 mu = load(reinterpret_cast<const float4*>(mean + c[u]));
+      const float4 is = load(reinterpret_cast<const float4*>(invstd + c[u]));
+      const float4 g = load(reinterpret_cast<const float4*>(scale + c[u]));
+      const float4 b = load(reinterpret_cast<const float4*>(bias + c[u]));
       float4 o;
       o.x = (v[u].x - mu.x) * is.x * g.x + b.x; o.y = (v[u].y - mu.y) * is.y * g.y + b.y;
       o.z = (v[u].z - mu.z) * is.z * g.z + b.z; o.w = (v[u].w - mu.w) * is.w * g.w + b.w;
@@ -268,12 +270,12 @@ __global__ void __launch_bounds__(256) bn_apply_fwd(const float* __restrict__ x,
     }
 }
 
-__global__ void __launch_bounds__(256) bn_apply_bwd(const float* __restrict__ dy, const float* __restrict__ x,
-                             const float* __restrict__ scale, const float* __restrict__ mean,
-                             const float* __restrict__ invstd, const float* __restrict__ dscale,
-                             const float* __restrict__ dbias, float* __restrict__ dx, long long rows, int C,
+__global__ void __launch_bounds__(256) bn_apply_bwd(const float* dy, const float* x,
+                             const float* scale, const float* mean,
+                             const float* invstd, const float* dscale,
+                             const float* dbias, float* __restrict__ dx, long long rows, int C,
                              long long lddy, long long ldx, long long lddx, float inv_count,
-                             const float* __restrict__ rbias = nullptr) {
+                             const float* rbias = nullptr) {
   tsb_launch::enter();
   const long long total = rows * (C >> 2), i = blockIdx.x * (long long)APPLY_TILE + threadIdx.x;
   long long r[2];
@@ -283,19 +285,19 @@ __global__ void __launch_bounds__(256) bn_apply_bwd(const float* __restrict__ dy
   for (int u = 0; u < 2; ++u)
     if (i + u * 256 < total) {
       row_col(i + u * 256, C >> 2, total, r[u], c[u]);
-      g[u] = __ldg(reinterpret_cast<const float4*>(dy + r[u] * lddy + c[u]));
-      v[u] = __ldg(reinterpret_cast<const float4*>(x + r[u] * ldx + c[u]));
+      g[u] = load(reinterpret_cast<const float4*>(dy + r[u] * lddy + c[u]));
+      v[u] = load(reinterpret_cast<const float4*>(x + r[u] * ldx + c[u]));
     }
 #pragma unroll
   for (int u = 0; u < 2; ++u)
     if (i + u * 256 < total) {
-      const float4 mu = __ldg(reinterpret_cast<const float4*>(mean + c[u]));
-      const float4 is = __ldg(reinterpret_cast<const float4*>(invstd + c[u]));
-      const float4 sc = __ldg(reinterpret_cast<const float4*>(scale + c[u]));
+      const float4 mu = load(reinterpret_cast<const float4*>(mean + c[u]));
+      const float4 is = load(reinterpret_cast<const float4*>(invstd + c[u]));
+      const float4 sc = load(reinterpret_cast<const float4*>(scale + c[u]));
       if (rbias)                                                                                  // fused ReLU
-        g[u] = relu_mask(g[u], v[u], mu, is, sc, __ldg(reinterpret_cast<const float4*>(rbias + c[u])));
-      const float4 ds = __ldg(reinterpret_cast<const float4*>(dscale + c[u]));
-      const float4 db = __ldg(reinterpret_cast<const float4*>(dbias + c[u]));
+        g[u] = relu_mask(g[u], v[u], mu, is, sc, load(reinterpret_cast<const float4*>(rbias + c[u])));
+      const float4 ds = load(reinterpret_cast<const float4*>(dscale + c[u]));
+      const float4 db = load(reinterpret_cast<const float4*>(dbias + c[u]));
       float4 o;
       o.x = sc.x * is.x * (g[u].x - db.x * inv_count - (v[u].x - mu.x) * is.x * ds.x * inv_count);
       o.y = sc.y * is.y * (g[u].y - db.y * inv_count - (v[u].y - mu.y) * is.y * ds.y * inv_count);
@@ -354,7 +356,7 @@ inline unsigned fin_blocks(long long C) { return (unsigned)((C + 31) / 32); }
 unsigned apply_grid(long long rows, long long C) { return (unsigned)((rows * (C / 4) + APPLY_TILE - 1) / APPLY_TILE); }
 
 // ------------------------------------------------------------------ layer norm (one warp per row)
-__global__ void ln_fwd(const float* __restrict__ x, const float* __restrict__ scale, const float* __restrict__ bias,
+__global__ void ln_fwd(const float* x, const float* scale, const float* bias,
                        float* __restrict__ y, float* __restrict__ mean, float* __restrict__ invstd, long long rows,
                        int D, float eps) {
   tsb_launch::enter();
@@ -374,8 +376,8 @@ __global__ void ln_fwd(const float* __restrict__ x, const float* __restrict__ sc
   for (int i = lane; i < D; i += 32) yr[i] = (xr[i] - m) * is * scale[i] + bias[i];
 }
 
-__global__ void ln_bwd_dx(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ scale,
-                          const float* __restrict__ mean, const float* __restrict__ invstd, float* __restrict__ dx,
+__global__ void ln_bwd_dx(const float* dy, const float* x, const float* scale,
+                          const float* mean, const float* invstd, float* __restrict__ dx,
                           long long rows, int D) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;
@@ -400,9 +402,9 @@ __global__ void ln_bwd_dx(const float* __restrict__ dy, const float* __restrict_
 // 16-byte variant for rows of up to 128 * NV floats: the row stays in registers between the sums and the result, so dy
 // and x are read once.  Bound by DRAM.  8192 x 512: 11.8 -> 9.1 us.
 template <int NV>
-__global__ void __launch_bounds__(256) ln_bwd_dx_v4(const float4* __restrict__ dy, const float4* __restrict__ x,
-                                                    const float4* __restrict__ scale, const float* __restrict__ mean,
-                                                    const float* __restrict__ invstd, float4* __restrict__ dx,
+__global__ void __launch_bounds__(256) ln_bwd_dx_v4(const float4* dy, const float4* x,
+                                                    const float4* scale, const float* mean,
+                                                    const float* invstd, float4* __restrict__ dx,
                                                     long long rows, int D4) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(256) ln_bwd_dx_v4(const float4* __restrict__ d
   for (int v = 0; v < NV; ++v) {
     const int i = lane + 32 * v;
     g[v] = h[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < D4) { g[v] = __ldg(dy + row * D4 + i); h[v] = __ldg(x + row * D4 + i); }
+    if (i < D4) { g[v] = load(dy + row * D4 + i); h[v] = load(x + row * D4 + i); }
   }
   const float m = mean[row], is = invstd[row];
   float s1 = 0.f, s2 = 0.f;
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(256) ln_bwd_dx_v4(const float4* __restrict__ d
   for (int v = 0; v < NV; ++v) {
     const int i = lane + 32 * v;
     if (i >= D4) continue;
-    const float4 sc = __ldg(scale + i);
+    const float4 sc = load(scale + i);
     g[v].x *= sc.x; g[v].y *= sc.y; g[v].z *= sc.z; g[v].w *= sc.w;
     h[v].x = (h[v].x - m) * is; h[v].y = (h[v].y - m) * is; h[v].z = (h[v].z - m) * is; h[v].w = (h[v].w - m) * is;
     s1 += (g[v].x + g[v].y) + (g[v].z + g[v].w);
@@ -441,8 +443,8 @@ __global__ void __launch_bounds__(256) ln_bwd_dx_v4(const float4* __restrict__ d
 }
 
 // column sums for dscale / dbias of layer norm: partials over row chunks
-__global__ void ln_bwd_params_partial(const float* __restrict__ dy, const float* __restrict__ x,
-                                      const float* __restrict__ mean, const float* __restrict__ invstd,
+__global__ void ln_bwd_params_partial(const float* dy, const float* x,
+                                      const float* mean, const float* invstd,
                                       float* __restrict__ part, long long rows, int D, int chunks) {
   tsb_launch::enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -461,8 +463,8 @@ __global__ void ln_bwd_params_partial(const float* __restrict__ dy, const float*
 }
 
 // 16-byte variant (D a multiple of 4): a thread owns four adjacent columns, two rows in flight.
-__global__ void ln_bwd_params_partial_v4(const float4* __restrict__ dy, const float4* __restrict__ x,
-                                         const float* __restrict__ mean, const float* __restrict__ invstd,
+__global__ void ln_bwd_params_partial_v4(const float4* dy, const float4* x,
+                                         const float* mean, const float* invstd,
                                          float* __restrict__ part, long long rows, int D4, int chunks) {
   tsb_launch::enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -473,9 +475,9 @@ __global__ void ln_bwd_params_partial_v4(const float4* __restrict__ dy, const fl
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, a2 = a, b2 = a;
   long long r = r0;
   for (; r + 1 < r1; r += 2) {
-    const float4 g0 = __ldg(dy + r * D4 + c), g1 = __ldg(dy + (r + 1) * D4 + c);
-    const float4 v0 = __ldg(x + r * D4 + c), v1 = __ldg(x + (r + 1) * D4 + c);
-    const float m0 = __ldg(mean + r), m1 = __ldg(mean + r + 1), i0 = __ldg(invstd + r), i1 = __ldg(invstd + r + 1);
+    const float4 g0 = load(dy + r * D4 + c), g1 = load(dy + (r + 1) * D4 + c);
+    const float4 v0 = load(x + r * D4 + c), v1 = load(x + (r + 1) * D4 + c);
+    const float m0 = load(mean + r), m1 = load(mean + r + 1), i0 = load(invstd + r), i1 = load(invstd + r + 1);
     a.x += g0.x; a.y += g0.y; a.z += g0.z; a.w += g0.w;
     a2.x += g1.x; a2.y += g1.y; a2.z += g1.z; a2.w += g1.w;
     b.x += g0.x * (v0.x - m0) * i0; b.y += g0.y * (v0.y - m0) * i0;
@@ -484,8 +486,8 @@ __global__ void ln_bwd_params_partial_v4(const float4* __restrict__ dy, const fl
     b2.z += g1.z * (v1.z - m1) * i1; b2.w += g1.w * (v1.w - m1) * i1;
   }
   for (; r < r1; ++r) {
-    const float4 g0 = __ldg(dy + r * D4 + c), v0 = __ldg(x + r * D4 + c);
-    const float m0 = __ldg(mean + r), i0 = __ldg(invstd + r);
+    const float4 g0 = load(dy + r * D4 + c), v0 = load(x + r * D4 + c);
+    const float m0 = load(mean + r), i0 = load(invstd + r);
     a.x += g0.x; a.y += g0.y; a.z += g0.z; a.w += g0.w;
     b.x += g0.x * (v0.x - m0) * i0; b.y += g0.y * (v0.y - m0) * i0;
     b.z += g0.z * (v0.z - m0) * i0; b.w += g0.w * (v0.w - m0) * i0;

@@ -22,6 +22,8 @@
 
 namespace {
 
+using tsb_launch::load;
+
 using namespace tsb_pw;
 
 constexpr int MAX_IN = 32, MAX_INS = 64, MAX_SLOTS = 48, BINARY = 32;
@@ -58,7 +60,7 @@ __global__ void __launch_bounds__(256) pointwise_program(const __grid_constant__
   if (i >= p.n4) return;
   for (int k = 0; k < p.n_in; ++k) {
     if (p.kind[k] == 2) {
-      const float v = __ldg(p.in[k]);
+      const float v = load(p.in[k]);
       r[k * T] = make_float4(v, v, v, v);
     } else {
       const float4* src = reinterpret_cast<const float4*>(p.in[k]) + (p.kind[k] == 0 ? i : i % p.cols4);

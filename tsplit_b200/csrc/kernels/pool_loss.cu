@@ -28,6 +28,8 @@ namespace cg = cooperative_groups;
 
 namespace {
 
+using tsb_launch::load;
+
 int sm_count() {
   static int n = 0;
   if (!n) {
@@ -55,7 +57,7 @@ struct PoolP {
 };
 
 template <int KIND>
-__global__ void pool_fwd(const float* __restrict__ x, float* __restrict__ y, const PoolP p) {
+__global__ void pool_fwd(const float* x, float* __restrict__ y, const PoolP p) {
   tsb_launch::enter();
   const int C4 = p.c >> 2;
   const long long total = (long long)p.n * p.oh * p.ow * C4;
@@ -97,7 +99,7 @@ __global__ void pool_fwd(const float* __restrict__ x, float* __restrict__ y, con
 // steps: VGG's first block before a 112 x 112 pool of 64 channels, batch 16: 4998 -> 1552 us; a 56 x 56 pool of 256
 // channels, batch 32: 1570 -> 844 us; 17 x 17 of 256 channels, batch 32: 338 -> 292 us.
 constexpr int WIN_COLS = 8, WIN_LANES = 32;
-__global__ void __launch_bounds__(WIN_COLS * WIN_LANES) avg_pool_window(const float* __restrict__ x,
+__global__ void __launch_bounds__(WIN_COLS * WIN_LANES) avg_pool_window(const float* x,
                                                                         float* __restrict__ y, const PoolP p) {
   tsb_launch::enter();
   cg::cluster_group cl = cg::this_cluster();
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(WIN_COLS * WIN_LANES) avg_pool_window(const fl
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int q = i + u * WIN_LANES, qy = q / ww, qx = q - qy * ww;
-        v[u] = q < end ? __ldg(reinterpret_cast<const float4*>(base + (y0 + qy) * p.xsh + (x0 + qx) * p.xsw))
+        v[u] = q < end ? load(reinterpret_cast<const float4*>(base + (y0 + qy) * p.xsh + (x0 + qx) * p.xsw))
                        : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
@@ -162,7 +164,7 @@ int window_splits(long long blocks, int pixels) {
 __device__ __forceinline__ int ceil_div_pos(int a, int b) { return a <= 0 ? 0 : (a + b - 1) / b; }
 
 template <int KIND>
-__global__ void pool_bwd(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ dy,
+__global__ void pool_bwd(const float* x, const float* y, const float* dy,
                          float* __restrict__ dx, const PoolP p) {
   tsb_launch::enter();
   const int C4 = p.c >> 2;
@@ -223,7 +225,7 @@ __global__ void pool_bwd(const float* __restrict__ x, const float* __restrict__ 
 // and writes the K x K input gradients -- x and dx cross HBM once each and y is not read at all.
 // Ties go to the first maximum in scan order, as in the general kernel.
 template <int KIND, int K>
-__global__ void pool_bwd_tiled(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dx,
+__global__ void pool_bwd_tiled(const float* x, const float* dy, float* __restrict__ dx,
                                const PoolP p) {
   tsb_launch::enter();
   const int C4 = p.c >> 2;
@@ -279,7 +281,7 @@ __global__ void pool_bwd_tiled(const float* __restrict__ x, const float* __restr
 //           pixel and whose recorded position is this pixel, in a fixed order.
 // After a ReLU most windows tie at zero, which made the scan-for-earlier-maximum form of the general
 // kernel expensive; here every tensor is read once.
-__global__ void pool_argmax(const float* __restrict__ x, unsigned char* __restrict__ idx, const PoolP p) {
+__global__ void pool_argmax(const float* x, unsigned char* __restrict__ idx, const PoolP p) {
   tsb_launch::enter();
   const int C4 = p.c >> 2;
   const long long total = (long long)p.n * p.oh * p.ow * C4;
@@ -310,7 +312,7 @@ __global__ void pool_argmax(const float* __restrict__ x, unsigned char* __restri
   }
 }
 
-__global__ void pool_bwd_from_argmax(const unsigned char* __restrict__ idx, const float* __restrict__ dy,
+__global__ void pool_bwd_from_argmax(const unsigned char* idx, const float* dy,
                                      float* __restrict__ dx, const PoolP p) {
   tsb_launch::enter();
   const int C4 = p.c >> 2;
@@ -348,7 +350,7 @@ __global__ void pool_bwd_from_argmax(const unsigned char* __restrict__ idx, cons
 // 32 x 112 x 112 x 64, 3 x 3 stride 2: 180 us in two passes -> 94 (127 without the constants); ResNet stem step 795 -> 712.
 // K, S: window and stride as constants (0: from p), which halves the arithmetic of the usual 3 x 3 stride 2.
 template <int T, int K, int S>
-__global__ void __launch_bounds__(256) max_pool_bwd_tile(const float* __restrict__ x, const float* __restrict__ dy,
+__global__ void __launch_bounds__(256) max_pool_bwd_tile(const float* x, const float* dy,
                                                          float* __restrict__ dx, const PoolP p, int tiles_x, int nw) {
   tsb_launch::enter();
   extern __shared__ float4 grad[];                                          // [window][8]
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(256) max_pool_bwd_tile(const float* __restrict
   const bool live = c < p.c;
   for (int w = threadIdx.x >> 3; live && nx > 0 && w < ny * nx; w += 32) {
     const int oy = oy0 + w / nx, ox = ox0 + w % nx;
-    grad[w * 8 + lane] = __ldg(reinterpret_cast<const float4*>(dy + n * p.ysn + oy * p.ysh + ox * p.ysw + c));
+    grad[w * 8 + lane] = load(reinterpret_cast<const float4*>(dy + n * p.ysn + oy * p.ysh + ox * p.ysw + c));
     float4 m = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
     uchar4 q = make_uchar4(255, 255, 255, 255);
 #pragma unroll 3
@@ -375,7 +377,7 @@ __global__ void __launch_bounds__(256) max_pool_bwd_tile(const float* __restrict
       for (int b = 0; b < kw; ++b) {
         const int ix = ox * stride - p.pad + b;
         if ((unsigned)ix >= (unsigned)p.w) continue;
-        const float4 v = __ldg(reinterpret_cast<const float4*>(x + n * p.xsn + iy * p.xsh + ix * p.xsw + c));
+        const float4 v = load(reinterpret_cast<const float4*>(x + n * p.xsn + iy * p.xsh + ix * p.xsw + c));
         const unsigned char at = (unsigned char)(a * kw + b);
         if (v.x > m.x || q.x == 255) { m.x = v.x; q.x = at; }
         if (v.y > m.y || q.y == 255) { m.y = v.y; q.y = at; }
@@ -436,7 +438,7 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
   return r;
 }
 
-__global__ void softmax_rows(const float* __restrict__ x, float* __restrict__ y, long long rows, long long cols) {
+__global__ void softmax_rows(const float* x, float* __restrict__ y, long long rows, long long cols) {
   tsb_launch::enter();
   __shared__ float sh[8];
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -455,7 +457,7 @@ __global__ void softmax_rows(const float* __restrict__ x, float* __restrict__ y,
 // Short rows (cols <= 1024, a multiple of 4): one warp per row, the row held in registers between the
 // maximum, the sum and the store, so it is read once and no block barrier is involved.
 template <int NV>
-__global__ void __launch_bounds__(256) softmax_warp_rows(const float4* __restrict__ x, float4* __restrict__ y,
+__global__ void __launch_bounds__(256) softmax_warp_rows(const float4* x, float4* __restrict__ y,
                                                          long long rows, int nvec) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;
@@ -468,7 +470,7 @@ __global__ void __launch_bounds__(256) softmax_warp_rows(const float4* __restric
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int i = lane + 32 * j;
-      v[j] = i < nvec ? __ldg(xr + i) : make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
+      v[j] = i < nvec ? load(xr + i) : make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
       m = fmaxf(m, fmaxf(fmaxf(v[j].x, v[j].y), fmaxf(v[j].z, v[j].w)));
     }
 #pragma unroll
@@ -495,7 +497,7 @@ __global__ void __launch_bounds__(256) softmax_warp_rows(const float4* __restric
 // The same for rows whose length is no multiple of 4 (or whose base is not 16-byte aligned): scalar,
 // still coalesced, lanes; NE elements per lane.
 template <int NE>
-__global__ void __launch_bounds__(256) softmax_warp_rows_scalar(const float* __restrict__ x, float* __restrict__ y,
+__global__ void __launch_bounds__(256) softmax_warp_rows_scalar(const float* x, float* __restrict__ y,
                                                                 long long rows, int cols) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;
@@ -508,7 +510,7 @@ __global__ void __launch_bounds__(256) softmax_warp_rows_scalar(const float* __r
 #pragma unroll
     for (int j = 0; j < NE; ++j) {
       const int i = lane + 32 * j;
-      v[j] = i < cols ? __ldg(xr + i) : -FLT_MAX;
+      v[j] = i < cols ? load(xr + i) : -FLT_MAX;
       m = fmaxf(m, v[j]);
     }
 #pragma unroll
@@ -529,8 +531,8 @@ __global__ void __launch_bounds__(256) softmax_warp_rows_scalar(const float* __r
 }
 
 template <int NE>
-__global__ void __launch_bounds__(256) softmax_grad_warp_rows_scalar(const float* __restrict__ y,
-                                                                     const float* __restrict__ dy,
+__global__ void __launch_bounds__(256) softmax_grad_warp_rows_scalar(const float* y,
+                                                                     const float* dy,
                                                                      float* __restrict__ dx, long long rows,
                                                                      int cols) {
   tsb_launch::enter();
@@ -545,8 +547,8 @@ __global__ void __launch_bounds__(256) softmax_grad_warp_rows_scalar(const float
 #pragma unroll
     for (int j = 0; j < NE; ++j) {
       const int i = lane + 32 * j;
-      a[j] = i < cols ? __ldg(yr + i) : 0.f;
-      g[j] = i < cols ? __ldg(gr + i) : 0.f;
+      a[j] = i < cols ? load(yr + i) : 0.f;
+      g[j] = i < cols ? load(gr + i) : 0.f;
       s += a[j] * g[j];
     }
 #pragma unroll
@@ -562,8 +564,8 @@ __global__ void __launch_bounds__(256) softmax_grad_warp_rows_scalar(const float
 
 // Softmax backward, dx = y * (dy - sum(dy * y)): one warp per row, y and dy read once.
 template <int NV>
-__global__ void __launch_bounds__(256) softmax_grad_warp_rows(const float4* __restrict__ y,
-                                                              const float4* __restrict__ dy,
+__global__ void __launch_bounds__(256) softmax_grad_warp_rows(const float4* y,
+                                                              const float4* dy,
                                                               float4* __restrict__ dx, long long rows, int nvec) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;
@@ -577,8 +579,8 @@ __global__ void __launch_bounds__(256) softmax_grad_warp_rows(const float4* __re
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int i = lane + 32 * j;
-      a[j] = i < nvec ? __ldg(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      g[j] = i < nvec ? __ldg(gr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      a[j] = i < nvec ? load(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      g[j] = i < nvec ? load(gr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
       s += (a[j].x * g[j].x + a[j].y * g[j].y) + (a[j].z * g[j].z + a[j].w * g[j].w);
     }
 #pragma unroll
@@ -600,8 +602,8 @@ __global__ void __launch_bounds__(256) softmax_grad_warp_rows(const float4* __re
 //   causal: column j of query row q (row % tq) is replaced by -1e9 when j > q
 // Rows are [batch][rows_per_batch] with rows_per_batch = heads * tq.
 template <int NE>
-__global__ void __launch_bounds__(256) masked_softmax_warp_rows(const float* __restrict__ x,
-                                                                const float* __restrict__ key_tokens,
+__global__ void __launch_bounds__(256) masked_softmax_warp_rows(const float* x,
+                                                                const float* key_tokens,
                                                                 float* __restrict__ y, long long rows, int cols,
                                                                 long long rows_per_batch, int tq, float scale,
                                                                 int causal) {
@@ -622,8 +624,8 @@ __global__ void __launch_bounds__(256) masked_softmax_warp_rows(const float* __r
       const int i = lane + 32 * j;
       float t = -FLT_MAX;
       if (i < cols) {
-        t = __ldg(xr + i) * scale;
-        if (kt && __ldg(kt + i) == 0.f) t += -1e9f;
+        t = load(xr + i) * scale;
+        if (kt && load(kt + i) == 0.f) t += -1e9f;
         if (causal && i > q) t = -1e9f;
       }
       v[j] = t;
@@ -652,8 +654,8 @@ __global__ void __launch_bounds__(256) masked_softmax_warp_rows(const float* __r
 
 // The same with 16-byte lanes (cols % 4 == 0, 16-byte aligned rows): NV float4 per lane.
 template <int NV>
-__global__ void __launch_bounds__(256) masked_softmax_warp_rows_v4(const float4* __restrict__ x,
-                                                                   const float4* __restrict__ key_tokens,
+__global__ void __launch_bounds__(256) masked_softmax_warp_rows_v4(const float4* x,
+                                                                   const float4* key_tokens,
                                                                    float4* __restrict__ y, long long rows, int nvec,
                                                                    long long rows_per_batch, int tq, float scale,
                                                                    int causal) {
@@ -672,10 +674,10 @@ __global__ void __launch_bounds__(256) masked_softmax_warp_rows_v4(const float4*
       const int i = lane + 32 * j;
       float4 t = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
       if (i < nvec) {
-        t = __ldg(xr + i);
+        t = load(xr + i);
         t.x *= scale; t.y *= scale; t.z *= scale; t.w *= scale;
         if (kt) {
-          const float4 k = __ldg(kt + i);
+          const float4 k = load(kt + i);
           if (k.x == 0.f) t.x += -1e9f;
           if (k.y == 0.f) t.y += -1e9f;
           if (k.z == 0.f) t.z += -1e9f;
@@ -720,8 +722,8 @@ __global__ void __launch_bounds__(256) masked_softmax_warp_rows_v4(const float4*
 
 // Its backward: dx = scale * y * (dy - sum(dy * y)) (masked positions have y = 0).
 template <int NE>
-__global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows(const float* __restrict__ y,
-                                                                     const float* __restrict__ dy,
+__global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows(const float* y,
+                                                                     const float* dy,
                                                                      float* __restrict__ dx, long long rows, int cols,
                                                                      float scale) {
   tsb_launch::enter();
@@ -736,8 +738,8 @@ __global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows(const float
 #pragma unroll
     for (int j = 0; j < NE; ++j) {
       const int i = lane + 32 * j;
-      a[j] = i < cols ? __ldg(yr + i) : 0.f;
-      g[j] = i < cols ? __ldg(gr + i) : 0.f;
+      a[j] = i < cols ? load(yr + i) : 0.f;
+      g[j] = i < cols ? load(gr + i) : 0.f;
       s += a[j] * g[j];
     }
 #pragma unroll
@@ -752,8 +754,8 @@ __global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows(const float
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows_v4(const float4* __restrict__ y,
-                                                                        const float4* __restrict__ dy,
+__global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows_v4(const float4* y,
+                                                                        const float4* dy,
                                                                         float4* __restrict__ dx, long long rows,
                                                                         int nvec, float scale) {
   tsb_launch::enter();
@@ -768,8 +770,8 @@ __global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows_v4(const fl
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int i = lane + 32 * j;
-      a[j] = i < nvec ? __ldg(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      g[j] = i < nvec ? __ldg(gr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      a[j] = i < nvec ? load(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      g[j] = i < nvec ? load(gr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
       s += (a[j].x * g[j].x + a[j].y * g[j].y) + (a[j].z * g[j].z + a[j].w * g[j].w);
     }
 #pragma unroll
@@ -786,7 +788,7 @@ __global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows_v4(const fl
 }
 
 // Any row length: one CTA per row, the second pass finds the row in L2.
-__global__ void softmax_grad_rows(const float* __restrict__ y, const float* __restrict__ dy, float* __restrict__ dx,
+__global__ void softmax_grad_rows(const float* y, const float* dy, float* __restrict__ dx,
                                   long long rows, long long cols) {
   tsb_launch::enter();
   __shared__ float sh[8];
@@ -828,7 +830,7 @@ __device__ __forceinline__ MaxSum block_max_sum(MaxSum a, float* sh) {
 }
 template <bool STAGED>
 __device__ __forceinline__ MaxSum row_max_sum(const float4* xr, int nvec, float* sh) {
-  auto at = [&](int i) { return STAGED ? xr[i] : __ldg(xr + i); };
+  auto at = [&](int i) { return STAGED ? xr[i] : load(xr + i); };
   MaxSum a{-FLT_MAX, 0.f};
   int i = threadIdx.x;
   for (; i + 3 * (int)blockDim.x < nvec; i += 4 * blockDim.x) {
@@ -872,7 +874,7 @@ __device__ __forceinline__ void staged() { asm volatile("cp.async.wait_all;" :::
 // 4096 x 32000 gradient with labels from ids: 278 us (dense labels, unstaged) -> 193 us; loss 174 -> 96 us in one pass.
 // The whole step of a 32000-word head: 1758 -> 1347 us, the label tensors (one-hot, scaled, shifted) not made at all.
 template <class Labels, bool STAGED>
-__global__ void __launch_bounds__(512) ce_rows_v4(const float4* __restrict__ x, Labels lab,
+__global__ void __launch_bounds__(512) ce_rows_v4(const float4* x, Labels lab,
                                                   float* __restrict__ row_loss, long long rows, int nvec) {
   tsb_launch::enter();
   extern __shared__ float4 row_buf[];
@@ -890,7 +892,7 @@ __global__ void __launch_bounds__(512) ce_rows_v4(const float4* __restrict__ x, 
     float l = 0.f;
     for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
       const float4 t = lab.at(i);
-      const float4 v = STAGED ? xr[i] : __ldg(xr + i);
+      const float4 v = STAGED ? xr[i] : load(xr + i);
       if (next) stage(row_buf + i, next + i);
       l -= (t.x * (v.x - lse) + t.y * (v.y - lse)) + (t.z * (v.z - lse) + t.w * (v.w - lse));
     }
@@ -903,7 +905,7 @@ __global__ void __launch_bounds__(512) ce_rows_v4(const float4* __restrict__ x, 
 // once.  Every logit is weighed before it is added: sums stay as small as those of the two-pass form, and logits at the
 // lowest float (masked classes) under a label of 0 count as 0 there and here.  4096 x 32000: 121 us, 109 with the
 // sum of the bare logits, which overflowed, 164 in two passes.
-__global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* __restrict__ x, SmoothLabels lab,
+__global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* x, SmoothLabels lab,
                                                          float* __restrict__ row_loss, long long rows, int nvec) {
   tsb_launch::enter();
   __shared__ float sh[64];
@@ -922,11 +924,11 @@ __global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* __restric
     };
     int i = threadIdx.x;
     for (; i + 3 * (int)blockDim.x < nvec; i += 4 * blockDim.x) {
-      const float4 v0 = __ldg(xr + i), v1 = __ldg(xr + i + blockDim.x), v2 = __ldg(xr + i + 2 * blockDim.x),
-                   v3 = __ldg(xr + i + 3 * blockDim.x);
+      const float4 v0 = load(xr + i), v1 = load(xr + i + blockDim.x), v2 = load(xr + i + 2 * blockDim.x),
+                   v3 = load(xr + i + 3 * blockDim.x);
       add(v0, i); add(v1, i + blockDim.x); add(v2, i + 2 * blockDim.x); add(v3, i + 3 * blockDim.x);
     }
-    for (; i < nvec; i += blockDim.x) add(__ldg(xr + i), i);
+    for (; i < nvec; i += blockDim.x) add(load(xr + i), i);
     const MaxSum ms = block_max_sum(a, sh);
     tx = block_sum(tx, sh);
     if (threadIdx.x == 0) {
@@ -937,8 +939,8 @@ __global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* __restric
 }
 
 template <class Labels, bool STAGED>
-__global__ void __launch_bounds__(512) ce_grad_rows_v4(const float4* __restrict__ x, Labels lab,
-                                                       const float* __restrict__ g, float4* __restrict__ dx,
+__global__ void __launch_bounds__(512) ce_grad_rows_v4(const float4* x, Labels lab,
+                                                       const float* g, float4* __restrict__ dx,
                                                        long long rows, int nvec) {
   tsb_launch::enter();
   extern __shared__ float4 row_buf[];
@@ -957,7 +959,7 @@ __global__ void __launch_bounds__(512) ce_grad_rows_v4(const float4* __restrict_
     const float inv = 1.f / ms.s, m = ms.m;
     for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
       const float4 t = lab.at(i);
-      const float4 v = STAGED ? xr[i] : __ldg(xr + i);
+      const float4 v = STAGED ? xr[i] : load(xr + i);
       if (next) stage(row_buf + i, next + i);
       float4 o;
       o.x = (__expf(v.x - m) * inv - t.x) * scale;
@@ -969,7 +971,7 @@ __global__ void __launch_bounds__(512) ce_grad_rows_v4(const float4* __restrict_
   }
 }
 
-__global__ void ce_rows(const float* __restrict__ x, const float* __restrict__ lab, float* __restrict__ row_loss,
+__global__ void ce_rows(const float* x, const float* lab, float* __restrict__ row_loss,
                         long long rows, long long cols) {
   tsb_launch::enter();
   __shared__ float sh[8];
@@ -990,7 +992,7 @@ __global__ void ce_rows(const float* __restrict__ x, const float* __restrict__ l
   }
 }
 
-__global__ void mean_rows(const float* __restrict__ row_loss, float* __restrict__ out, long long rows) {
+__global__ void mean_rows(const float* row_loss, float* __restrict__ out, long long rows) {
   tsb_launch::enter();
   __shared__ float sh[32];
   float s = 0.f;
@@ -999,7 +1001,7 @@ __global__ void mean_rows(const float* __restrict__ row_loss, float* __restrict_
   if (threadIdx.x == 0) out[0] = s / (float)rows;
 }
 
-__global__ void ce_grad_rows(const float* __restrict__ x, const float* __restrict__ lab, const float* __restrict__ g,
+__global__ void ce_grad_rows(const float* x, const float* lab, const float* g,
                              float* __restrict__ dx, long long rows, long long cols) {
   tsb_launch::enter();
   __shared__ float sh[8];

@@ -263,7 +263,7 @@ __host__ __device__ constexpr uint32_t make_idesc_tf32(int M, int N, int a_mn_ma
 }
 
 // Sum of `splits` partial results, four floats of each, in their order; eight loads in flight.
-__device__ __forceinline__ float4 sum_splits(const float4* __restrict__ ws, int splits, long long per_split4) {
+__device__ __forceinline__ float4 sum_splits(const float4* ws, int splits, long long per_split4) {
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int s = 0; s < splits; s += 8) {
     float4 v[8];
