@@ -24,6 +24,7 @@
 #include "tc_common.cuh"
 #include "scratch.h"
 #include "launch.cuh"
+#include "smem_limit.h"
 
 using namespace tsb;
 
@@ -1322,12 +1323,8 @@ int launch(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo
   using C = Cfg<BN, IM2COL>;
   auto kern = conv_tf32_kernel<MODE, BN, IM2COL>;
   constexpr int threads = IM2COL ? (MODE == 2 ? 288 : 192) : NUM_THREADS;   // wgrad: three extra producer warps
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess)
-      return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
-    attr_set = true;
-  }
+  static tsb_launch::SmemLimit limit;
+  if (limit.raise(kern, C::SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
   const long long items = (long long)p.tiles_m * p.tiles_n * p.taps * p.splits;
   const long long slots = (long long)sm_count() * C::OCC;
   int grid = (int)(items < slots ? items : slots);
@@ -1370,12 +1367,8 @@ int launch_fwd_pair_bn(const CUtensorMap& tm, const CUtensorMap& tmi, const CUte
                        cudaStream_t st) {
   using PC = PairCfg<BN>;
   auto kern = conv_fwd_pair_kernel<BN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PC::SMEM_BYTES) != cudaSuccess)
-      return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
-    attr_set = true;
-  }
+  static tsb_launch::SmemLimit limit;
+  if (limit.raise(kern, PC::SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
   const int ptn = (p.NC + BN - 1) / BN;
   const long long items = (long long)((p.M + 255) / 256) * ptn;
   long long pairs = sm_count() / 2;
@@ -1394,13 +1387,8 @@ int launch_fwd_pair(int bn, const CUtensorMap& tm, const CUtensorMap& tmi, const
 }
 
 int launch_wgrad_pair(const CUtensorMap& tm, const CUtensorMap& tmi, const ConvParams& p, cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(conv_wgrad_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P2_SMEM_BYTES) !=
-        cudaSuccess)
-      return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
-    attr_set = true;
-  }
+  static tsb_launch::SmemLimit limit;
+  if (limit.raise(conv_wgrad_pair_kernel, P2_SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
   const long long items = (long long)((p.M + 255) / 256) * ((p.NC + P2_BN - 1) / P2_BN) * p.splits;
   long long pairs = sm_count() / 2;
   if (pairs > items) pairs = items;

@@ -17,6 +17,7 @@
 #include "tc_common.cuh"
 #include "scratch.h"
 #include "launch.cuh"
+#include "smem_limit.h"
 
 #include <mutex>
 #include <unordered_map>
@@ -830,12 +831,8 @@ int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& t
               cudaStream_t st) {
   using C = Cfg<BN>;
   auto kern = gemm_tf32_kernel<BN, A_MN, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess)
-      return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
-    attr_set = true;
-  }
+  static tsb_launch::SmemLimit limit;
+  if (limit.raise(kern, C::SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
   const long long items = (long long)p.tiles_m * p.tiles_n * p.batch * p.splits;
   const int grid = (int)(items < sm_count() ? items : sm_count());
   tsb_launch::launch(kern, grid, 192, C::SMEM_BYTES, st, ta, tb, tc, p);
@@ -855,12 +852,8 @@ int dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMa
 template <int BN, bool A_MN, bool B_MN>
 int launch_group(const GemmGroup& g, int ctas, cudaStream_t st) {
   auto kern = gemm_tf32_group_kernel<BN, A_MN, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::SMEM_BYTES) != cudaSuccess)
-      return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
-    attr_set = true;
-  }
+  static tsb_launch::SmemLimit limit;
+  if (limit.raise(kern, Cfg<BN>::SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
   const cudaError_t e = tsb_launch::launch(kern, ctas, 192, Cfg<BN>::SMEM_BYTES, st, g);
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
@@ -876,12 +869,8 @@ template <bool A_MN, bool B_MN>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
                 cudaStream_t st) {
   auto kern = gemm_tf32_pair_kernel<A_MN, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P2_SMEM_BYTES) != cudaSuccess)
-      return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
-    attr_set = true;
-  }
+  static tsb_launch::SmemLimit limit;
+  if (limit.raise(kern, P2_SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
   const long long items = (long long)((p.m + 255) / 256) * ((p.n + P2_BN - 1) / P2_BN) * p.batch;
   long long pairs = sm_count() / 2;
   if (pairs > items) pairs = items;

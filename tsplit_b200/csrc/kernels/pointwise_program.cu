@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "launch.cuh"
+#include "smem_limit.h"
 #include "pointwise.cuh"
 
 #define TSB_OK 0
@@ -156,13 +157,9 @@ int tsb_pointwise(int n_in, const void** in, const int* kind, int n_ins, const u
   // small tensors: short blocks, so that more SMs take part; large ones: a block per 256 groups (see elementwise.cu)
   const int threads = p.n4 <= 64ll * sm_count() ? 64 : 256;
   const size_t smem = (size_t)slots * threads * sizeof(float4);
-  static bool attr_set = false;
-  if (!attr_set) {
-    const cudaError_t e = cudaFuncSetAttribute(pointwise_program, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               MAX_SLOTS * 256 * (int)sizeof(float4));
-    if (e != cudaSuccess) return rc_of(e);
-    attr_set = true;
-  }
+  static tsb_launch::SmemLimit limit;
+  const cudaError_t e = limit.raise(pointwise_program, MAX_SLOTS * 256 * (int)sizeof(float4));
+  if (e != cudaSuccess) return rc_of(e);
   const long long blocks = (p.n4 + threads - 1) / threads;
   if (blocks > 0x7fffffffll) return TSB_ERR_UNSUPPORTED;
   return rc_of(tsb_launch::launch(pointwise_program, dim3((unsigned)blocks), dim3(threads), smem,
