@@ -68,6 +68,24 @@ def test_optimizer_tiles_of_many_tensors():
         torch.testing.assert_close(p.t, p0 + v1, rtol=0, atol=4e-6)
 
 
+@pytest.mark.parametrize("sizes", [[-1, 5, 0, 3000, -2048], [0, -7], [4, -3]])
+def test_optimizer_leaves_tensors_of_no_elements_alone(sizes):
+    """Sizes of zero and below are tensors with nothing to update, not an error."""
+    import ctypes
+    n = len(sizes)
+    ps, gs = ([_rand(max(k, 8), seed=j + 100 * i) for j, k in enumerate(sizes)] for i in range(2))
+    before = [p.clone() for p in ps]
+    ptrs = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() for t in ts])
+    rc = G.lib().tsb_optimizer_step(ctypes.c_int(0), ctypes.c_int(n), ptrs(ps), ptrs(gs), None, None,
+                                    (ctypes.c_int64 * n)(*sizes), (ctypes.c_float * 8)(0.5), ctypes.c_void_p(None))
+    torch.cuda.synchronize()
+    assert rc == 0
+    for k, p, g, p0 in zip(sizes, ps, gs, before):
+        k = max(k, 0)
+        torch.testing.assert_close(p[:k], p0[:k] - 0.5 * g[:k], rtol=0, atol=2e-6)        # (contracted or not)
+        assert torch.equal(p[k:], p0[k:])
+
+
 # launches whose tiles are narrowed: one tile, a ragged one, the last number of wide tiles that is halved and the first
 # that is not, and a batch; every combination of transposed operands
 @pytest.mark.parametrize("m,n,k,batch", [(64, 256, 96, 1), (130, 300, 70, 1), (5, 129, 40, 1), (128 * 74, 256, 32, 1),

@@ -388,10 +388,9 @@ int tsb_optimizer_step_dev(int kind, int count, float** params, const float** gr
     a.p[i] = params[i]; a.g[i] = grads[i];
     a.s1[i] = slot1 ? slot1[i] : nullptr;
     a.s2[i] = slot2 ? slot2[i] : nullptr;
-    a.n[i] = sizes[i];
-    if (sizes[i] < 0) return TSB_ERR_ARG;
+    a.n[i] = sizes[i] > 0 ? sizes[i] : 0;         // nothing to update: no block
     a.first[i] = (unsigned)blocks;
-    blocks += (sizes[i] + OPT_TILE - 1) / OPT_TILE;
+    blocks += (a.n[i] + OPT_TILE - 1) / OPT_TILE;
     if (blocks > 0x7fffffffll) return TSB_ERR_ARG;
     if (kind >= 1 && !a.s1[i]) return TSB_ERR_ARG;
     if (kind == 4 && !a.s2[i]) return TSB_ERR_ARG;
