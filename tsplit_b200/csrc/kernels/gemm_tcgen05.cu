@@ -358,7 +358,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // tile or two each; one after the other they are bound by the latency of a launch, a TMA round trip and a store, with
 // all but two SMs idle, and side by side they take the time of one.  LSTM step, 549 products in 84 launches:
 // 3351 -> 1322 us; a small Transformer 565 -> 504.
-constexpr int MAX_GROUP = 16;
+constexpr int MAX_GROUP = 16, GROUP_BN = 64;      // (the narrowest tile: see narrow_tile)
 struct GemmGroup {
   CUtensorMap ta[MAX_GROUP], tb[MAX_GROUP], tc[MAX_GROUP];
   GemmParams p[MAX_GROUP];
@@ -857,12 +857,11 @@ int launch_group(const GemmGroup& g, int ctas, cudaStream_t st) {
   const cudaError_t e = tsb_launch::launch(kern, ctas, 192, Cfg<BN>::SMEM_BYTES, st, g);
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
-template <int BN>
 int dispatch_group(bool a_mn, bool b_mn, const GemmGroup& g, int ctas, cudaStream_t st) {
-  if (!a_mn && !b_mn) return launch_group<BN, false, false>(g, ctas, st);
-  if (!a_mn && b_mn) return launch_group<BN, false, true>(g, ctas, st);
-  if (a_mn && !b_mn) return launch_group<BN, true, false>(g, ctas, st);
-  return launch_group<BN, true, true>(g, ctas, st);
+  if (!a_mn && !b_mn) return launch_group<GROUP_BN, false, false>(g, ctas, st);
+  if (!a_mn && b_mn) return launch_group<GROUP_BN, false, true>(g, ctas, st);
+  if (a_mn && !b_mn) return launch_group<GROUP_BN, true, false>(g, ctas, st);
+  return launch_group<GROUP_BN, true, true>(g, ctas, st);
 }
 
 template <bool A_MN, bool B_MN>
@@ -1182,38 +1181,34 @@ int tsb_gemm_tf32_splitk(const float* a, const float* b, float* c, int m, int n,
 }
 
 // Up to 16 products C = op(A) op(B) of the same transposition as one launch.  TSB_ERR_UNSUPPORTED when one of them is no
-// candidate (needs padding, split-K or CTA pairs) or the tiles do not fit the chip at once.
+// candidate (needs padding, split-K or CTA pairs) or the tiles are more than two waves.
 int tsb_gemm_tf32_group(int count, const float** a, const float** b, float** c, const int* m, const int* n, const int* k,
                         const long long* lda, const long long* ldb, const long long* ldc, int trans_a, int trans_b,
                         void* stream) {
   if (count < 1 || count > MAX_GROUP) return TSB_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  long long t64 = 0, t128 = 0;
+  long long wide = 0;
   for (int i = 0; i < count; ++i) {
     if (m[i] <= 0 || n[i] <= 0 || k[i] <= 0) return TSB_ERR_ARG;
     if ((lda[i] | ldb[i]) % 4 || ((reinterpret_cast<uintptr_t>(a[i]) | reinterpret_cast<uintptr_t>(b[i])) & 15))
       return TSB_ERR_UNSUPPORTED;
-    const long long rows = ((long long)m[i] + BM - 1) / BM;
-    t64 += rows * ((n[i] + 63) / 64);
-    t128 += rows * ((n[i] + 127) / 128);
+    wide += (((long long)m[i] + BM - 1) / BM) * ((n[i] + 2 * GROUP_BN - 1) / (2 * GROUP_BN));
   }
-  const int bn = t64 <= sm_count() ? 64 : 128;       // as narrow as still leaves a tile an SM (see narrow_tile)
-  if (t128 > sm_count()) return TSB_ERR_UNSUPPORTED;
+  if (wide > sm_count()) return TSB_ERR_UNSUPPORTED;      // (two waves of the narrow tiles at most)
   GemmGroup g;
   g.count = count;
   int ctas = 0;
   for (int i = 0; i < count; ++i) {
     int width;
     bool pair;
-    const int rc = prepare_tc(g.p[i], g.ta[i], g.tb[i], g.tc[i], width, pair, bn, a[i], b[i], c[i], m[i], n[i], k[i],
+    const int rc = prepare_tc(g.p[i], g.ta[i], g.tb[i], g.tc[i], width, pair, GROUP_BN, a[i], b[i], c[i], m[i], n[i], k[i],
                               lda[i], ldb[i], ldc[i], trans_a, trans_b, 1, 0, 0, 0, 0, 0, nullptr, 0, false, st, 0, 0);
     if (rc) return rc == TSB_ERR_SCRATCH ? TSB_ERR_UNSUPPORTED : rc;
     g.first[i] = ctas;
     ctas += g.p[i].tiles_m * g.p[i].tiles_n;
   }
   g.first[count] = ctas;
-  const int rc = bn == 64 ? dispatch_group<64>(trans_a != 0, trans_b == 0, g, ctas, st)
-                          : dispatch_group<128>(trans_a != 0, trans_b == 0, g, ctas, st);
+  const int rc = dispatch_group(trans_a != 0, trans_b == 0, g, ctas, st);
   if (rc) return rc;
   const int late = tsb_host::peek_status();
   return late ? TSB_ERR_TIMEOUT | (late << 8) : TSB_OK;
