@@ -209,6 +209,30 @@ def test_a_feed_in_another_layout_runs_node_by_node(monkeypatch):
 
 
 @pytest.mark.parametrize("taken", [True, False])
+def test_constants_are_read_in_every_step(monkeypatch, taken):
+    """An operator's number (``const_attr``) may change between steps; label smoothing is made of such operators, too."""
+    xv, yv = _arrays((6, 12), (6, 12))
+    x, y, i = (ad.Variable(k) for k in "xyi")
+    scaled = ad.mul_byconst_op(x, 2.0)
+    shifted = ad.addbyconst_op(scaled, 1.0)
+    over = ad.div_const_op(3.0, ad.addbyconst_op(ad.mul_op(shifted, shifted), 0.5))
+    rate = ad.mul_byconst_op(ad.one_hot_op(i, 12), 0.9)
+    floor = ad.addbyconst_op(rate, 0.1 / 12)
+    loss = ad.softmaxcrossentropy_op(y, floor)
+    nodes = [over, loss] + ad.gradients(loss, [y])
+    feed = {x: xv, y: yv, i: np.array([0, 3, 11, 5, 5, 2], np.float32)}
+    plan, first = _run(monkeypatch, nodes, feed, taken=taken)
+    assert {"program", "smooth"} <= {a[0] for a in plan.actions}
+    scaled.const_attr, shifted.const_attr, over.const_attr, rate.const_attr, floor.const_attr = -1.5, 0.25, 7.0, 0.6, 0.4 / 12
+    vals = {k: ndarray.array(v, ndarray.cpu(0)) for k, v in feed.items()}
+    plan.run(type("E", (), {"stream": None})(), vals)
+    want = ad.Executor(nodes).run(feed)
+    for n, w, f in zip(nodes, want, first):
+        assert not np.allclose(f, w, rtol=1e-3)
+        np.testing.assert_allclose(vals[n].numpy_view(), w, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("taken", [True, False])
 def test_products_that_are_ready_together(monkeypatch, taken):
     """Products of all four transpositions, too long and too wide ones, one that reads another, more than one launch."""
     xv, wv, longv, widev = _arrays((6, 20), (20, 6), (20, 600), (600, 3000))

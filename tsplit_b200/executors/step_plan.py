@@ -30,6 +30,7 @@ from ..ops.shape import AddBroadcastOp, ReduceSumOp, ReshapeOp, ReshapeGradientO
 
 FULL, ROW, SCALAR = 0, 1, 2
 _BINARY = 32                       # instruction code of binary operator 0
+_TAKES_NUMBER = (G.UN_ADDC, G.UN_MULC, G.UN_CDIV, G.UN_FILL)
 MAX_IN, MAX_INS, MAX_SLOTS = 32, 64, 48
 #: products of one launch, and what makes one small: the 128 x 64 tiles of one and of all, and K (longer sums are split)
 MAX_GROUP, GROUP_TILES, GROUP_TILES_ALL, GROUP_K = 16, 16, 128, 480
@@ -50,12 +51,19 @@ def _key(arr):
 def _code(node):
     op = node.op
     if isinstance(op, AddBroadcastOp):
-        return _BINARY + G.BIN_ADD, 0.0
+        return _BINARY + G.BIN_ADD
     if isinstance(op, _FillLike):
-        return G.UN_FILL, float(op.value)
+        return G.UN_FILL
     if isinstance(op, _Binary):
-        return _BINARY + op.gpu_code, 0.0
-    return op.gpu_code, 0.0 if node.const_attr is None else float(node.const_attr)
+        return _BINARY + op.gpu_code
+    return op.gpu_code
+
+
+def _constant(node):
+    """The number an operator takes besides its operands, read in every step as the operator itself does."""
+    if isinstance(node.op, _FillLike):
+        return float(node.op.value)
+    return 0.0 if node.const_attr is None else float(node.const_attr)
 
 
 class Program(object):
@@ -75,9 +83,12 @@ class Program(object):
         n_in = len(self.inputs)
         free, used = [], n_in
         where = {("in", j): j for j in range(n_in)}
-        code, self.alpha, self.out = [], [], []
+        code, self.out = [], []
+        self.constants = []                                 # (instruction, node) of those that take a number
         for k, (node, ins) in enumerate(self.members):
-            op, alpha = _code(node)
+            op = _code(node)
+            if op in _TAKES_NUMBER:
+                self.constants.append((k, node))
             at = [where[ref] for ref in ins]
             for ref in dict.fromkeys(ins):
                 if last[ref] == k:
@@ -91,7 +102,6 @@ class Program(object):
                 free.append(dst)
             a = at[0] if at else 0
             code += [op, a, at[1] if len(at) > 1 else a, dst]
-            self.alpha.append(alpha)
             self.out.append(node if node in stored else None)
         self.slots = max(used, 1)
         self.code = bytes(code)
@@ -116,7 +126,10 @@ class Program(object):
         outs = [arrays[n].ptr if n is not None else 0 for n in self.out]
         if any(p & 15 for p in outs):
             return False
-        G.pointwise(ptrs, self.kinds, self.code, self.alpha, outs, self.slots, self.numel, self.cols, stream)
+        alpha = [0.0] * len(outs)
+        for k, node in self.constants:
+            alpha[k] = _constant(node)
+        G.pointwise(ptrs, self.kinds, self.code, alpha, outs, self.slots, self.numel, self.cols, stream)
         return True
 
 
@@ -198,7 +211,7 @@ class StepPlan(object):
 
     def _smooth_labels(self, ce):
         """When ``ce``'s labels are ``one_hot(ids) * a + b`` (any number of constants, reshapes that keep the classes)
-        and nothing but cross-entropies over them reads any of it: remember ids and the two values."""
+        and nothing but cross-entropies over them reads any of it: remember ids and the operators on the way."""
         labels = cur = ce.inputs[1]
         chain, consts = [], []
         while True:
@@ -208,7 +221,7 @@ class StepPlan(object):
             if isinstance(cur.op, OneHotOp):
                 break
             if isinstance(cur.op, (AddConstOp, MulConstOp)):
-                consts.append((isinstance(cur.op, MulConstOp), np.float32(cur.const_attr)))
+                consts.append(cur)
             elif not (isinstance(cur.op, ReshapeOp) and self.arrays[cur].t.is_contiguous()):
                 return
             cur = cur.inputs[0]
@@ -221,14 +234,9 @@ class StepPlan(object):
             return
         if any(u not in chain for m in chain[1:] for u in self.users.get(m, ())):
             return
-        values = []
-        for v in (np.float32(1), np.float32(0)):
-            for mul, c in reversed(consts):
-                v = np.float32(v * c) if mul else np.float32(v + c)
-            values.append(float(v))
         self.elided.update(chain)
         for u in readers:
-            self.smooth[u] = (cur.inputs[0], values[0], values[1], chain[::-1])
+            self.smooth[u] = (cur.inputs[0], consts[::-1], chain[::-1])
 
     # -- scheduling ------------------------------------------------------------------------
     def _schedule(self, nodes):
@@ -451,7 +459,12 @@ class StepPlan(object):
                 self._node(n, vals, stream)
 
     def _smooth(self, n, vals, stream):
-        ids, on, off, chain = self.smooth[n]
+        ids, consts, chain = self.smooth[n]
+        on, off = np.float32(1), np.float32(0)               # what the operators make of a one and of a zero
+        for m in consts:
+            c = np.float32(_constant(m))
+            on, off = (on * c, off * c) if isinstance(m.op, MulConstOp) else (on + c, off + c)
+        on, off = float(on), float(off)
         x, i, out = vals[n.inputs[0]], vals[ids], self.arrays[n]
         ok = x.is_contiguous() and i.is_contiguous() and out.is_contiguous()
         if ok and isinstance(n.op, SoftmaxCrossEntropyOp):
