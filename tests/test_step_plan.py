@@ -295,6 +295,24 @@ def test_labels_from_ids(monkeypatch, form, taken):
     assert sum(1 for a in plan.actions if a[0] == "smooth") == (0 if made else 3 if form == "two losses" else 2)
 
 
+def test_labels_that_are_refused_are_made_once_a_step(monkeypatch):
+    """The loss and its gradient both ask for labels from ids; a class count that the kernels do not cover costs the four
+    operators of the label chain, not eight."""
+    xv, = _arrays((6, 12))
+    x, i = ad.Variable("x"), ad.Variable("i")
+    lab = ad.addbyconst_op(ad.mul_byconst_op(ad.array_reshape_op(ad.one_hot_op(i, 12), (-1, 12)), 0.9), 0.1 / 12)
+    loss = ad.softmaxcrossentropy_op(x, lab)
+    nodes = [loss] + ad.gradients(loss, [x])
+    feed = {x: xv, i: np.array([[0, 3, 11], [5, 5, 2]], np.float32)}
+    ran = []
+    node = _HostPlan._node
+    monkeypatch.setattr(_HostPlan, "_node", lambda self, n, vals, stream: (ran.append(n.op.name), node(self, n, vals, stream)))
+    plan, got = _run(monkeypatch, nodes, feed, steps=2, taken=False)
+    assert [ran.count(k) for k in ("OneHot", "Reshape", "MulConst", "AddConst")] == [2, 2, 2, 2]        # of two steps
+    for w, g in zip(ad.Executor(nodes).run(feed), got):
+        np.testing.assert_allclose(g, w, rtol=1e-5, atol=1e-6)
+
+
 # one group of four; a row length that is no power of two; the last size of the short blocks and the first of the long
 # ones; a tensor past the limit for many values
 @pytest.mark.gpu

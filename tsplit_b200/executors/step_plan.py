@@ -405,13 +405,14 @@ class StepPlan(object):
         for n in self.elided:              # (for those who walk all values, as a per-operator timing does)
             vals[n] = self.arrays[n]
         stream = ex.stream
+        made = set()                       # labels that had to be made after all: once a step, however many read them
         for what, x in self.actions:
             if what == "node":
                 self._node(x, vals, stream)
             elif what == "view":
                 vals[x] = self.arrays[x]
             elif what == "smooth":
-                self._smooth(x, vals, stream)
+                self._smooth(x, vals, stream, made)
             elif what == "products":
                 self._products(x, vals, stream)
             elif what == "sums":
@@ -458,7 +459,7 @@ class StepPlan(object):
             for n in nodes:
                 self._node(n, vals, stream)
 
-    def _smooth(self, n, vals, stream):
+    def _smooth(self, n, vals, stream, made):
         ids, consts, chain = self.smooth[n]
         on, off = np.float32(1), np.float32(0)               # what the operators make of a one and of a zero
         for m in consts:
@@ -474,8 +475,11 @@ class StepPlan(object):
         if ok:
             vals[n] = out
             return
-        for m in chain + [n]:
-            self._node(m, vals, stream)
+        for m in chain:
+            if m not in made:
+                self._node(m, vals, stream)
+        made.update(chain)
+        self._node(n, vals, stream)
 
     def _node(self, n, vals, stream):
         out = self.arrays.get(n)
