@@ -248,6 +248,29 @@ def test_products_that_are_ready_together(monkeypatch, taken):
     assert sum(len(g) for g in groups) >= 40 and max(len(g) for g in groups) == step_plan.MAX_GROUP
 
 
+def test_a_product_that_no_group_takes_leaves_the_others_together(monkeypatch):
+    """Rows of 10 classes have to be padded, so that product runs by itself, not all that are ready with it."""
+    xv, wv, cv = _arrays((6, 20), (20, 8), (20, 10))
+    groups, alone, taken = [], [], _gemm_group
+    node = _HostPlan._node
+
+    def group(products, ta, tb, stream):
+        if any(a.shape[1] % 4 or b.shape[1] % 4 for a, b, *_ in products):
+            return False                                       # as the native entry does, for all of them
+        groups.append(len(products))
+        return taken(products, ta, tb, stream)
+    monkeypatch.setitem(globals(), "_gemm_group", group)
+    monkeypatch.setattr(_HostPlan, "_node", lambda self, n, vals, stream: (alone.append(n.op.name), node(self, n, vals, stream)))
+
+    def build():
+        x, w, c = (ad.Variable(k) for k in "xwc")
+        outs = [ad.matmul_op(ad.mul_byconst_op(x, float(j)), w) for j in range(5)]
+        return outs + [ad.matmul_op(x, c)], {x: xv, w: wv, c: cv}
+    plan = _compare(monkeypatch, build)
+    assert [len(a[1]) for a in plan.actions if a[0] == "products"] == [6]
+    assert groups == [5] and alone.count("MatMul") == 1
+
+
 @pytest.mark.parametrize("taken", [True, False])
 def test_sums_that_are_ready_together(monkeypatch, taken):
     """Column sums with and without the reduced dimension kept, sums over other axes and over too many rows."""

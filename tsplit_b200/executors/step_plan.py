@@ -437,18 +437,20 @@ class StepPlan(object):
 
     def _products(self, nodes, vals, stream):
         ta, tb = nodes[0].attrs["trans_A"], nodes[0].attrs["trans_B"]
-        items = []
+        items, alone = [], []
         for n in nodes:
             a, b, out = vals[n.inputs[0]], vals[n.inputs[1]], self.arrays[n]
-            if not (a.is_contiguous() and b.is_contiguous() and out.is_contiguous()):
-                break
-            items.append((a, b, out) + _mm_shape(a.shape, b.shape, ta, tb))
-        if len(items) == len(nodes) and G.gemm_group(items, ta, tb, stream):
-            for n in nodes:
+            if a.is_contiguous() and b.is_contiguous() and out.is_contiguous() and G.gemm_group_takes(a, b):
+                items.append((n, (a, b, out) + _mm_shape(a.shape, b.shape, ta, tb)))
+            else:
+                alone.append(n)            # (a row of 10 classes needs padding, which a group does not do)
+        if len(items) > 1 and G.gemm_group([i for _, i in items], ta, tb, stream):
+            for n, _ in items:
                 vals[n] = self.arrays[n]
         else:
-            for n in nodes:
-                self._node(n, vals, stream)
+            alone = nodes
+        for n in alone:
+            self._node(n, vals, stream)
 
     def _sums(self, nodes, vals, stream):
         items = [(vals[n.inputs[0]], self.arrays[n]) for n in nodes]

@@ -459,6 +459,11 @@ def gemm(a, b, c, trans_a, trans_b, stream, batch=1, sa=0, sb=0, sc=0, m=None, n
     _check(rc, "gemm_tf32")
 
 
+def gemm_group_takes(a, b):
+    """Whether a product of these operands may be in a group: TMA reads them where they are."""
+    return not ((a.shape[1] | b.shape[1]) & 3 or (a.ptr | b.ptr) & 15)
+
+
 def gemm_group(products, trans_a, trans_b, stream):
     """Up to 16 products ``(a, b, c, m, n, k)`` of row-major arrays as one launch; False: not a group of small ones."""
     cnt = len(products)
