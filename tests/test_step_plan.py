@@ -139,6 +139,43 @@ def test_models(monkeypatch, name, least):
         assert any(a[0] == "copies" and len(a[1]) > 10 for a in plan.actions)
 
 
+@pytest.mark.parametrize("form", ["deep", "wide products", "wide sums", "one value, many readers"])
+def test_planning_takes_time_in_proportion_to_the_graph(form):
+    """The plan is made in the first pass over a feed shape; counted in calls, which do not depend on the machine."""
+    import sys
+
+    def calls(size):
+        x, w, c = ad.Variable("x"), ad.Variable("w"), ad.Variable("c")
+        shapes = {x: (8, 20), w: (20, 20), c: (20,)}
+        if form == "deep":
+            h = x
+            for _ in range(size):
+                h = ad.tanh_op(ad.matmul_op(h, w) + ad.broadcasttoTF_op(c, x))
+            nodes = [h] + ad.gradients(ad.reduce_sum_op(h, [0, 1]), [w, c])
+        elif form == "wide products":
+            nodes = [ad.matmul_op(ad.mul_byconst_op(x, float(j)), w) for j in range(size)]
+        elif form == "wide sums":
+            nodes = [ad.reduce_sum_op(ad.mul_byconst_op(x, float(j)), [0]) for j in range(size)]
+        else:
+            s = ad.tanh_op(x)
+            nodes = [ad.mul_op(s, ad.mul_byconst_op(x, float(j))) for j in range(size)]
+        ex = ad.Executor(nodes, ctx=ndarray.cpu(0))
+        ex.infer_shape(shapes)
+        ex.memory_plan(shapes)
+        count = [0]
+
+        def profile(frame, event, arg):
+            count[0] += event in ("call", "c_call")
+        sys.setprofile(profile)
+        try:
+            step_plan.StepPlan(ex, set(shapes))
+        finally:
+            sys.setprofile(None)
+        return count[0], len(ex.topo_order)
+    (few, n), (many, n4) = calls(100), calls(400)
+    assert many <= 1.15 * few * n4 / n and many <= 90 * n4
+
+
 def _arrays(*shapes):
     r = np.random.RandomState(0)
     return [r.standard_normal(s).astype(np.float32) for s in shapes]

@@ -72,6 +72,7 @@ class Program(object):
     def __init__(self, key, numel):
         self.key, self.numel = key, numel
         self.members, self.values, self.inputs = [], {}, []      # values: node -> index of its instruction
+        self.left, self.live = {}, 0         # member -> its readers outside; members that have such readers
         self.kinds, self.slot_of_input, self.cols = [], {}, 0
 
     def close(self, stored):
@@ -106,7 +107,7 @@ class Program(object):
         self.slots = max(used, 1)
         self.code = bytes(code)
         self.members = [m for m, _ in self.members]
-        del self.values, self.slot_of_input                 # needed while collecting only
+        del self.values, self.slot_of_input, self.left      # needed while collecting only
         return self.slots
 
     def run(self, vals, arrays, stream):
@@ -145,6 +146,7 @@ class StepPlan(object):
             if n not in self.external:
                 for i in n.inputs:
                     self.users.setdefault(i, []).append(n)
+        self.kinds = {}                   # operator type -> _kind
         self.smooth, self.elided = {}, set()
         for n in ex.topo_order:
             if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
@@ -153,7 +155,9 @@ class StepPlan(object):
         self.actions = []
         self.open = {}                    # key -> Program that still collects
         self.home = {}                    # node -> its open Program
-        self.copies = []
+        self.copies, self.copied = [], set()                     # (the same nodes twice)
+        self.layouts = {n: (_key(a), a.t.numel()) for n, a in self.arrays.items()}
+        self.group_of, self.queues, self.gone = {}, {}, set()    # ready operators that may share a launch, see _mates
         segment = []
         for n in ex.topo_order:
             if n in self.external:
@@ -168,16 +172,32 @@ class StepPlan(object):
         self._schedule(segment)
         self._flush_all()
         del self.users, self.shapes, self.external, self.root, self.open, self.home, self.copies     # planning only
+        del self.copied, self.layouts, self.group_of, self.queues, self.gone, self.kinds
 
-    @staticmethod
-    def _has_effects(n):
-        return (not type(n.op).__module__.startswith("tsplit_b200.ops.") or isinstance(n.op, (SwapInOp, SwapOutOp))
-                or n.phase == "update")
+    def _kind(self, n):
+        """What nodes of this operator type may become; "effects": they stay where they are."""
+        op = type(n.op)
+        kind = self.kinds.get(op)
+        if kind is None:
+            kind = "other"
+            if not op.__module__.startswith("tsplit_b200.ops.") or issubclass(op, (SwapInOp, SwapOutOp)):
+                kind = "effects"
+            elif issubclass(op, (ReshapeOp, ReshapeGradientOp)):
+                kind = "view"
+            elif issubclass(op, BatchNormGradScaleOp):
+                kind = "copy"
+            elif issubclass(op, (_Binary, _Unary, _FillLike, AddBroadcastOp)):
+                kind = "element"
+            self.kinds[op] = kind
+        return kind
+
+    def _has_effects(self, n):
+        return n.phase == "update" or self._kind(n) == "effects"
 
     # -- what a node is -------------------------------------------------------------------
     def _is_view(self, n):
         """Row-major reshapes of computed arrays (a result that the caller keeps stays an array of its own)."""
-        if not isinstance(n.op, (ReshapeOp, ReshapeGradientOp)) or n in self.evals:
+        if n in self.evals:
             return False
         src, arr = self.arrays.get(n.inputs[0]), self.arrays.get(n)
         return (src is not None and arr is not None and n.inputs[0] not in self.evals and src.t.is_contiguous()
@@ -185,21 +205,20 @@ class StepPlan(object):
 
     def _operands(self, n):
         """[(node, kind)] when ``n`` can be part of a program, else None."""
-        arr = self.arrays.get(n)
-        if arr is None or not isinstance(n.op, (_Binary, _Unary, _FillLike, AddBroadcastOp)):
+        if n not in self.layouts:
             return None
-        key, numel = _key(arr), arr.t.numel()
+        key, numel = self.layouts[n]
         if key is None or numel == 0 or numel % 4:
             return None
         if isinstance(n.op, _FillLike):
             return []
-        res = []
+        res, shapes, own = [], self.shapes, self.shapes[n]
         for j, i in enumerate(n.inputs):
-            shape, src = tuple(self.shapes[i]), self.arrays.get(i)
-            if shape == arr.shape and (src is None or _key(src) == key):
+            shape, at = shapes[i], self.layouts.get(i)
+            if shape == own and (at is None or at[0] == key):
                 res.append((i, FULL))
             elif isinstance(n.op, AddBroadcastOp) and j == 1:
-                cols = arr.shape[-1]
+                cols = own[-1]
                 if key[0] != "rows" or cols % 4 or shape[-1] != cols or ndarray._numel(shape) != cols:
                     return None
                 res.append((i, ROW))
@@ -241,18 +260,29 @@ class StepPlan(object):
     # -- scheduling ------------------------------------------------------------------------
     def _schedule(self, nodes):
         inside = set(nodes)
-        waits = {n: len({i for i in n.inputs if i in inside}) for n in nodes}
+        waits = {n: sum(1 for i in set(n.inputs) if i in inside) for n in nodes}
+        users = self.users
         light, heavy = [], []             # ready nodes: those that cost no launch of their own, the others
+        self.queues, self.gone = {}, set()
 
         def ready(n):
-            cls = ("elided" if n in self.elided else "view" if self._is_view(n) else
-                   "copy" if isinstance(n.op, BatchNormGradScaleOp) else None)
-            ops = None if cls else self._operands(n)
-            heapq.heappush(light if cls or ops is not None else heavy, (n.id, n, cls, ops))
+            cls, ops = "elided" if n in self.elided else self._kind(n), None
+            if cls == "element":
+                ops = self._operands(n)
+                cls = None if ops is None else cls
+            elif cls == "other" or cls == "view" and not self._is_view(n):
+                cls = None
+            if cls:
+                heapq.heappush(light, (n.id, n, cls, ops))
+                return
+            heapq.heappush(heavy, (n.id, n))
+            group = self.group_of[n] = self._group(n)
+            if group:
+                heapq.heappush(self.queues.setdefault(group[0], []), (n.id, n, group[1]))
 
         def done(n):
-            for u in set(self.users.get(n, ())):
-                if u in inside:
+            for u in set(users.get(n, ())):
+                if u in waits:
                     waits[u] -= 1
                     if waits[u] == 0:
                         ready(u)
@@ -269,17 +299,20 @@ class StepPlan(object):
                 elif cls == "copy":
                     self._need(n.inputs[0])
                     self.copies.append(n)
+                    self.copied.add(n)
                 else:
                     self._collect(n, ops)
             else:
-                _, n, _, _ = heapq.heappop(heavy)
-                taken = self._mates(n, heavy)
+                _, n = heapq.heappop(heavy)
+                if n in self.gone:
+                    continue
+                taken = self._mates(n)
                 for m in taken:
                     for i in m.inputs:
                         self._need(i)
                 if n in self.smooth:
                     self._need(self.smooth[n][0])
-                self.actions.append((self._group(n)[0][0], taken) if len(taken) > 1 else
+                self.actions.append((self.group_of[n][0][0], taken) if len(taken) > 1 else
                                     ("smooth" if n in self.smooth else "node", n))
                 for m in taken[1:]:
                     done(m)
@@ -300,18 +333,23 @@ class StepPlan(object):
                 return ("sums",), 1
         return None
 
-    def _mates(self, n, heavy):
-        """``n`` and the operators that are ready with it and go into the same launch (taken out of ``heavy``)."""
-        taken, own = [n], self._group(n)
+    def _mates(self, n):
+        """``n`` and the operators that are ready with it and go into the same launch: the next ones of its kind, as long
+        as they fit.  They stay in the heap of ready operators and are passed over there (``gone``)."""
+        taken, own = [n], self.group_of[n]
+        self.gone.add(n)
         if own:
             kind, blocks = own
-            for entry in sorted(heavy):
-                other = self._group(entry[1])
-                if (other and other[0] == kind and len(taken) < MAX_GROUP and blocks + other[1] <= GROUP_TILES_ALL):
-                    taken.append(entry[1])
-                    blocks += other[1]
-                    heavy.remove(entry)
-            heapq.heapify(heavy)
+            queue = self.queues[kind]
+            while queue and len(taken) < MAX_GROUP:
+                _, m, more = queue[0]
+                if m not in self.gone:
+                    if blocks + more > GROUP_TILES_ALL:
+                        break
+                    taken.append(m)
+                    self.gone.add(m)
+                    blocks += more
+                heapq.heappop(queue)
         return taken
 
     def _view(self, n):
@@ -329,60 +367,63 @@ class StepPlan(object):
         i = self.root.get(i, i)
         if i in self.home:
             self._flush(self.home[i])
-        elif i in self.copies:
+        elif i in self.copied:
             self._flush_copies()
 
     def _collect(self, n, operands):
-        arr = self.arrays[n]
-        key = _key(arr)
-        prog = self.open.get(key)
-        roots = [self.root.get(i, i) for i, _ in operands]
-        for i, r, (_, kind) in zip(n.inputs, roots, operands):
-            if prog is None or self.home.get(r) is not prog or kind != FULL:
-                self._need(i)              # computed by another program, or read in another way than its values lie
+        key, numel = self.layouts[n]
+        home, prog, cols = self.home, self.open.get(key), 0
+        operands = [(self.root.get(i, i), kind) for i, kind in operands]
+        for r, kind in operands:
+            if kind != FULL or prog is None or home.get(r) is not prog:
+                self._need(r)              # computed by another program, or read in another way than its values lie
+            if kind == ROW:
+                cols = self.shapes[n][-1]
         prog = self.open.get(key)          # (the call above may have run it)
-        new = [r for r in dict.fromkeys(roots) if prog is None or self.home.get(r) is not prog]
-        limit = MAX_SLOTS_LARGE if arr.t.numel() >= LARGE else MAX_SLOTS
-        cols = arr.shape[-1] if any(k == ROW for _, k in operands) else 0
-        if prog is not None and (len(prog.inputs) + len(new) > min(MAX_IN, limit - 4) or len(prog.members) >= MAX_INS
-                                 or (cols and prog.cols and prog.cols != cols) or self._slots_with(prog, n) > limit):
-            self._flush(prog)
-            prog = None
+        if prog is not None:
+            new = len({r for r, _ in operands if home.get(r) is not prog})
+            limit = MAX_SLOTS_LARGE if numel >= LARGE else MAX_SLOTS
+            if (len(prog.inputs) + new > min(MAX_IN, limit - 4) or len(prog.members) >= MAX_INS
+                    or (cols and prog.cols and prog.cols != cols) or self._slots_with(prog, n) > limit):
+                self._flush(prog)
+                prog = None
         if prog is None:
-            prog = self.open[key] = Program(key, arr.t.numel())
+            prog = self.open[key] = Program(key, numel)
         refs = []
-        for r, (_, kind) in zip(roots, operands):
-            if self.home.get(r) is prog and kind == FULL:
+        for r, kind in operands:
+            if home.get(r) is prog:
                 refs.append(("val", prog.values[r]))
                 continue
-            if (r, kind) not in prog.slot_of_input:
-                prog.slot_of_input[(r, kind)] = len(prog.inputs)
+            slot = prog.slot_of_input.get((r, kind))
+            if slot is None:
+                slot = prog.slot_of_input[(r, kind)] = len(prog.inputs)
                 prog.inputs.append(r)
                 prog.kinds.append(kind)
-            refs.append(("in", prog.slot_of_input[(r, kind)]))
+            refs.append(("in", slot))
         prog.cols = prog.cols or cols
         prog.values[n] = len(prog.members)
         prog.members.append((n, refs))
-        self.home[n] = prog
+        home[n] = prog
+        for i in n.inputs:
+            if i in prog.left:
+                prog.left[i] -= 1
+                prog.live -= not prog.left[i]
+        readers = prog.left[n] = len(self.users.get(n, ()))
+        prog.live += readers > 0
 
-    def _slots_with(self, prog, n):
+    @staticmethod
+    def _slots_with(prog, n):
         """Upper bound of the slots after one more member: every value still read later holds one."""
-        inside = {m for m, _ in prog.members}
-        inside.add(n)
-        live = sum(1 for m, _ in prog.members if any(u not in inside for u in self.users.get(m, ())))
-        return len(prog.inputs) + live + 3
+        done = sum(1 for i in set(n.inputs) if prog.left.get(i) == n.inputs.count(i))       # read by nobody after n
+        return len(prog.inputs) + prog.live - done + 3
 
     def _flush(self, prog):
         del self.open[prog.key]
         members = [m for m, _ in prog.members]
-        inside = set(members)
         for m in members:
             del self.home[m]
-
-        def read_outside(m):
-            return m in self.evals or any(u not in inside for u in self.users.get(m, ()))
-        # (views count as outside: their readers are)
-        stored = {m for m in members if read_outside(m)}
+        # (views count as readers outside: theirs are)
+        stored = {m for m in members if m in self.evals or prog.left[m]}
         if len(members) == 1 or prog.close(stored) > MAX_SLOTS:
             self.actions += [("node", m) for m in members]
         else:
@@ -391,7 +432,7 @@ class StepPlan(object):
     def _flush_copies(self):
         for lo in range(0, len(self.copies), 64):
             self.actions.append(("copies", self.copies[lo:lo + 64]))
-        self.copies = []
+        self.copies, self.copied = [], set()
 
     def _flush_all(self):
         for prog in list(self.open.values()):
