@@ -300,3 +300,15 @@ def test_column_sums_of_many_rows(rows, cols):
     G.reduce_sum(x.data_ptr(), [rows, cols], [cols, 1], [0], ndarray.from_tensor(y, ndarray.gpu(0)), _stream())
     # pairwise joins of partial sums of at most some eighty terms
     assert torch.all((y.double() - x.double().sum(0)).abs() <= 96 * 2.0 ** -24 * x.double().abs().sum(0))
+
+
+# few rows of wide arrays: the widths of the single launch and the first past them, for many rows and for few; then many
+# chunks (more than 128) of few columns and of many
+@pytest.mark.parametrize("rows,cols", [(64, 8192), (129, 8192), (129, 8196), (128, 16384), (128, 16388), (63, 16388), (512, 16386),
+                                       (300, 65536), (2, 65536), (4127, 64), (4160, 64), (4200, 4096), (4200, 4100)])
+def test_column_sums_of_wide_arrays(rows, cols):
+    x, y = _rand(rows, cols), torch.zeros(cols, device="cuda")
+    G.reduce_sum(x.data_ptr(), [rows, cols], [cols, 1], [0], ndarray.from_tensor(y, ndarray.gpu(0)), _stream())
+    _stream().sync()
+    # at most some hundred roundings of partial sums in a row
+    assert torch.all((y.double() - x.double().sum(0)).abs() <= 160 * 2.0 ** -24 * x.double().abs().sum(0))

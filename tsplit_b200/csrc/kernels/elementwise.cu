@@ -337,7 +337,8 @@ __global__ void colsum_partial(const float* x, float* __restrict__ part, long lo
   for (long long r = r0; r < r1; ++r) acc += x[r * ld + c];
   part[(long long)ch * cols + c] = acc;
 }
-// 16-byte variant: a thread owns four adjacent columns and keeps four rows in flight.
+// 16-byte variant: a thread owns four adjacent columns and keeps four rows in flight.  (The loop is not unrolled: with the
+// compiler's choice 8192 x 512 is 11.1 us, 9.7 so.)
 __global__ void colsum_partial_v4(const float4* x, float4* __restrict__ part, long long rows,
                                   int cols4, long long ld4, int chunks) {
   tsb_launch::enter();
@@ -348,6 +349,7 @@ __global__ void colsum_partial_v4(const float4* x, float4* __restrict__ part, lo
   const long long r0 = ch * per, r1 = min(rows, r0 + per);
   float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0, a2 = a0, a3 = a0;
   long long r = r0;
+#pragma unroll 1
   for (; r + 3 < r1; r += 4) {
     const float4 v0 = load(x + r * ld4 + c), v1 = load(x + (r + 1) * ld4 + c), v2 = load(x + (r + 2) * ld4 + c),
                  v3 = load(x + (r + 3) * ld4 + c);
@@ -364,8 +366,8 @@ __global__ void colsum_partial_v4(const float4* x, float4* __restrict__ part, lo
       make_float4((a0.x + a1.x) + (a2.x + a3.x), (a0.y + a1.y) + (a2.y + a3.y), (a0.z + a1.z) + (a2.z + a3.z),
                   (a0.w + a1.w) + (a2.w + a3.w));
 }
-// Second stage: 32 columns x 32 chunk lanes per block, eight loads in flight, lanes joined in a fixed order (256 chunks
-// of 512 columns: 3.4 us with 8 lanes, 2.9 now).
+// Second stage of many chunks: 32 columns x 32 chunk lanes per block, eight loads in flight, lanes joined in a fixed order
+// (256 chunks of 512 columns: 3.4 us with 8 lanes, 2.9 now).
 __global__ void __launch_bounds__(1024) colsum_final_lanes(const float* part, float* __restrict__ y,
                                                            long long cols, int chunks, long long ys) {
   tsb_launch::enter();
@@ -386,6 +388,26 @@ __global__ void __launch_bounds__(1024) colsum_final_lanes(const float* part, fl
   }
   if (threadIdx.y == 0 && c < cols) y[c * ys] = sh[0][threadIdx.x];
 }
+// The same for few chunks and for wide arrays, whose blocks alone fill the chip: 8 lanes, one barrier.  Whole sums with 32
+// lanes / 8, us: 8192 x 512 10.5 / 11.1, 8192 x 4096 26.7 / 27.5, 4096 x 2048 11.7 / 11.5, 2048 x 4096 11.8 / 11.0,
+// 8192 x 16384 93.5 / 89.3, 513 x 65536 44.7 / 28.1.
+__global__ void __launch_bounds__(256) colsum_final_wide(const float* part, float* __restrict__ y, long long cols,
+                                                         int chunks, long long ys) {
+  tsb_launch::enter();
+  __shared__ float sh[8][33];
+  const long long c = blockIdx.x * 32ll + threadIdx.x;
+  float acc = 0.f;
+  if (c < cols)
+    for (int ch = threadIdx.y; ch < chunks; ch += 8) acc += part[(long long)ch * cols + c];
+  sh[threadIdx.y][threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < cols) {
+    float t = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) t += sh[j][threadIdx.x];
+    y[c * ys] = t;
+  }
+}
 __global__ void colsum_final(const float* part, float* __restrict__ y, long long cols, int chunks,
                              long long ys) {
   tsb_launch::enter();
@@ -398,9 +420,10 @@ __global__ void colsum_final(const float* part, float* __restrict__ y, long long
 
 // Column sums of a few hundred rows in one launch, of up to 16 arrays at once (the bias gradients of a recurrent cell):
 // 32 columns x 32 row lanes per block, lanes joined in a fixed order.  Such a sum is bound by launch latency, and two
-// stages are two launches.  [128, 128]: 8.2 -> 2.5 us, [512, 512]: 8.3 -> 3.2
-// (two stages take 4.7 for 1024 rows, and their time hardly depends on the rows);
-// LSTM step 1322 -> 937 us (222 launches become 29), small Transformer 504 -> 449.
+// stages are two launches.  [128, 128]: 8.2 -> 2.5 us, [512, 512]: 8.3 -> 3.2; the 222 launches of an LSTM step become 29.
+// The line against the two stages of tsb_reduce_sum (which begin at 64 rows): wide arrays fill the chip there too, with 16
+// bytes a load.  One launch / two, us: 64 x 8192 2.7 / 3.9, 64 x 32768 8.8 / 7.9, 64 x 65536 16.0 / 9.0; 128 x 16384 6.3 / 7.6,
+// 256 x 16384 8.9 / 8.1; 512 x 8192 5.4 / 8.1, 512 x 16384 9.8 / 9.5, 512 x 65536 32.2 / 26.1.
 constexpr int SUM_GROUP = 16, SUM_ROWS = 512;
 struct ColSums {
   const float* x[SUM_GROUP];
@@ -660,7 +683,8 @@ int tsb_reduce_sum(const float* x, float* y, int nk, const long long* kshape, co
   if (nkeep <= 0) return TSB_OK;
   // fast path: kept dims collapse to one contiguous column index and the reduced
   // dims to one row index with a constant stride (e.g. [rows, cols] -> [cols])
-  if (nk == 1 && nr == 1 && kxs[0] == 1 && nkeep <= 65536 && nred > 1 && nred <= SUM_ROWS) {
+  if (nk == 1 && nr == 1 && kxs[0] == 1 && nkeep <= 65536 && nred > 1 && nred <= SUM_ROWS &&
+      (nred < 64 || nkeep <= 8192 || (nkeep <= 16384 && nred <= 128))) {
     ColSums g = {};
     g.x[0] = x; g.y[0] = y; g.ld[0] = rxs[0]; g.ys[0] = kys[0]; g.rows[0] = (int)nred; g.cols[0] = (int)nkeep;
     tsb_launch::launch(colsum_group, dim3((unsigned)((nkeep + 31) / 32)), dim3(32, 32), 0, st, g);
@@ -680,8 +704,9 @@ int tsb_reduce_sum(const float* x, float* y, int nk, const long long* kshape, co
         dim3 g1((unsigned)((cols4 + 127) / 128), chunks);
         tsb_launch::launch(colsum_partial_v4, g1, 128, 0, st, reinterpret_cast<const float4*>(x),
                            reinterpret_cast<float4*>(part), nred, cols4, rxs[0] / 4, chunks);
-        tsb_launch::launch(colsum_final_lanes, (unsigned)((nkeep + 31) / 32), dim3(32, 32), 0, st, part, y, nkeep,
-                           chunks, kys[0]);
+        const bool few = nkeep <= 4096 && chunks > 128;
+        tsb_launch::launch(few ? colsum_final_lanes : colsum_final_wide, (unsigned)((nkeep + 31) / 32),
+                           dim3(32, few ? 32 : 8), 0, st, part, y, nkeep, chunks, kys[0]);
         return done();
       }
       int chunks = (int)(nred / 64 < 64 ? (nred / 64 < 1 ? 1 : nred / 64) : 64);
