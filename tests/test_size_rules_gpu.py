@@ -195,6 +195,27 @@ def test_cross_entropy_with_masked_classes(cols, value, masked):
         assert torch.equal(dd, ds)
 
 
+@pytest.mark.parametrize("offset", [0.0, -37.0, 1000.0])
+@pytest.mark.parametrize("cols", [512, 32000])
+def test_cross_entropy_of_logits_with_a_common_offset(cols, offset):
+    """The loss does not depend on what all logits of a row have in common, and its rounding hardly does."""
+    ctx, rows = ndarray.gpu(0), 64
+    x = _rand(rows, cols) + offset
+    ids = torch.randint(0, cols, (rows,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(8)).float()
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    on, off = float(np.float32(0.9) + np.float32(0.1 / cols)), float(np.float32(0.1 / cols))
+    lab = torch.full((rows, cols), off, device="cuda")
+    lab[torch.arange(rows), ids.long()] = on
+    want = -(lab.double() * torch.log_softmax(x.double(), 1)).sum(1).mean()
+    dense, smooth = torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda")
+    G.softmax_ce(a(x), a(lab), a(dense), _stream())
+    assert G.softmax_ce_smooth(a(x), a(ids), on, off, a(smooth), _stream())
+    _stream().sync()
+    # a logit of 1000 has a unit in the last place of 6e-5; its distance to the row's lse is rounded once, and rows average
+    bound = 8 * 2.0 ** -24 * (float(want) + abs(offset) / 64 ** 0.5)
+    assert abs(float(smooth[0]) - float(want)) <= bound and abs(float(dense[0]) - float(want)) <= bound
+
+
 # outputs that leave by TMA store: ragged rows and columns of a block, one column block and many, batches, several
 # splits; and those whose strides or sums do not allow it (a row of 130 + 1 floats, a base 4 bytes in, accumulation)
 @pytest.mark.parametrize("m,n,k,batch,ldc,shift,accumulate", [

@@ -901,10 +901,12 @@ __global__ void __launch_bounds__(512) ce_rows_v4(const float4* x, Labels lab,
   }
 }
 
-// The loss with labels from ids in one pass: sum t (x - lse) = sum t x - lse sum t over the labels t, so the row is read
-// once.  Every logit is weighed before it is added: sums stay as small as those of the two-pass form, and logits at the
-// lowest float (masked classes) under a label of 0 count as 0 there and here.  4096 x 32000: 121 us, 109 with the
-// sum of the bare logits, which overflowed, 164 in two passes.
+// The loss with labels from ids in one pass: sum t (x - lse) = sum t (x - c) - (lse - c) sum t over the labels t, for any
+// c, so the row is read once.  With the labelled logit as c that class adds nothing, every other one has the weight `off`,
+// and rounding is relative to lse - c, which the loss is made of: a common offset of the logits costs no digits.
+// Every logit is weighed before it is added: logits at the lowest float (masked classes) under a label of 0 count as 0, as
+// in the two-pass form.  No such c (an id outside the classes, a masked or infinite label): 0, and each class its own
+// label.
 __global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* x, SmoothLabels lab,
                                                          float* __restrict__ row_loss, long long rows, int nvec) {
   tsb_launch::enter();
@@ -913,27 +915,32 @@ __global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* x, Smooth
     const float4* xr = x + row * nvec;
     lab.row(row, nvec);
     const bool inside = lab.id >= 0 && lab.id < 4ll * nvec;
-    const int special = inside ? (int)(lab.id >> 2) : -1;                 // the four classes with the id's
-    const float4 l = lab.at(special), o = make_float4(lab.off, lab.off, lab.off, lab.off);
+    const float at_id = inside ? reinterpret_cast<const float*>(xr)[lab.id] : FLT_MAX;
+    const bool usual = fabsf(at_id) < 1e30f;
+    const float c = usual ? at_id : 0.f;
     MaxSum a{-FLT_MAX, 0.f};
-    float tx = 0.f;
-    auto add = [&](const float4 v, int i) {
+    float d = 0.f;
+    auto add = [&](const float4 v, const float4 t) {
       ms_add4(a, v);
-      const float4 t = i == special ? l : o;
-      tx += (t.x * v.x + t.y * v.y) + (t.z * v.z + t.w * v.w);
+      d += (t.x * (v.x - c) + t.y * (v.y - c)) + (t.z * (v.z - c) + t.w * (v.w - c));
     };
     int i = threadIdx.x;
-    for (; i + 3 * (int)blockDim.x < nvec; i += 4 * blockDim.x) {
-      const float4 v0 = load(xr + i), v1 = load(xr + i + blockDim.x), v2 = load(xr + i + 2 * blockDim.x),
-                   v3 = load(xr + i + 3 * blockDim.x);
-      add(v0, i); add(v1, i + blockDim.x); add(v2, i + 2 * blockDim.x); add(v3, i + 3 * blockDim.x);
+    if (usual) {
+      const float4 off = make_float4(lab.off, lab.off, lab.off, lab.off);
+      for (; i + 3 * (int)blockDim.x < nvec; i += 4 * blockDim.x) {
+        const float4 v0 = load(xr + i), v1 = load(xr + i + blockDim.x), v2 = load(xr + i + 2 * blockDim.x),
+                     v3 = load(xr + i + 3 * blockDim.x);
+        add(v0, off); add(v1, off); add(v2, off); add(v3, off);
+      }
+      for (; i < nvec; i += blockDim.x) add(load(xr + i), off);
+    } else {
+      for (; i < nvec; i += blockDim.x) add(load(xr + i), lab.at(i));
     }
-    for (; i < nvec; i += blockDim.x) add(load(xr + i), i);
     const MaxSum ms = block_max_sum(a, sh);
-    tx = block_sum(tx, sh);
+    d = block_sum(d, sh);
     if (threadIdx.x == 0) {
       const float ones = 4.f * (float)nvec * lab.off + (inside ? lab.on - lab.off : 0.f);
-      row_loss[row] = ones * (ms.m + logf(ms.s)) - tx;
+      row_loss[row] = ones * ((ms.m - c) + logf(ms.s)) - d;
     }
   }
 }
