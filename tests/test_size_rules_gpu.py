@@ -323,6 +323,86 @@ def test_column_sums_of_many_rows(rows, cols):
     assert torch.all((y.double() - x.double().sum(0)).abs() <= 96 * 2.0 ** -24 * x.double().abs().sum(0))
 
 
+# rows that stay in registers and rows that do not, at both sides of each line; four-element batches and their rest
+@pytest.mark.parametrize("cols", [1, 3, 127, 129, 511, 1021, 1023, 1025, 2047, 2049])
+def test_cross_entropy_of_short_and_odd_rows(cols):
+    ctx, rows = ndarray.gpu(0), 37
+    x, g = 3 * _rand(rows, cols), torch.full((1,), 0.5, device="cuda")
+    lab = torch.softmax(_rand(rows, cols, seed=1), 1)
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    loss, dx = torch.zeros(1, device="cuda"), torch.full((rows, cols), 9.0, device="cuda")
+    G.softmax_ce(a(x), a(lab), a(loss), _stream())
+    G.softmax_ce_grad(a(x), a(lab), a(g), a(dx), _stream())
+    _stream().sync()
+    lp = torch.log_softmax(x.double(), 1)
+    # fp32 sums of at most some two thousand terms of one sign, and the exponential's 2^-21
+    torch.testing.assert_close(loss[0].double(), -(lab.double() * lp).sum(1).mean(), rtol=2e-5, atol=1e-6)
+    torch.testing.assert_close(dx.double(), (lp.exp() - lab.double()) * 0.5 / rows, rtol=1e-4, atol=1e-6 * 0.5 / rows)
+
+
+@pytest.mark.parametrize("cols", [1, 600, 1000, 1024, 1025, 1200, 5000])
+def test_softmax_rows_and_gradient(cols):
+    ctx, rows = ndarray.gpu(0), 19
+    x, dy = 3 * _rand(rows, cols), _rand(rows, cols, seed=1)
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    y, dx = torch.full_like(x, 9.0), torch.full_like(x, 9.0)
+    G.softmax(a(x), a(y), _stream())
+    G.softmax_grad(a(y), a(dy), a(dx), _stream())
+    _stream().sync()
+    ref = torch.softmax(x.double(), 1)
+    torch.testing.assert_close(y.double(), ref, rtol=1e-4, atol=1e-9)                  # the fast exponential's 2^-21, sums
+    yd = y.double()
+    torch.testing.assert_close(dx.double(), yd * (dy.double() - (yd * dy.double()).sum(1, keepdim=True)), rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("d", [1, 31, 128, 129, 512, 513, 1000, 1024, 1025, 1500])
+def test_layer_norm_rows(d):
+    ctx, rows = ndarray.gpu(0), 13
+    x, scale, bias = _rand(rows, d) + 0.5, _rand(d, seed=1) + 1, _rand(d, seed=2)
+    y, mean, inv = torch.full_like(x, 9.0), torch.zeros(rows, device="cuda"), torch.zeros(rows, device="cuda")
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    G.layer_norm(a(x), a(scale), a(bias), a(y), a(mean), a(inv), 1e-3, _stream())
+    _stream().sync()
+    want = torch.nn.functional.layer_norm(x.double(), (d,), scale.double(), bias.double(), 1e-3)
+    # the variance as a difference of sums of squares: some 2^-20 of the mean square, seen through 1 / sqrt(var + 1e-3)
+    torch.testing.assert_close(y.double(), want, rtol=1e-4, atol=1e-3 if d == 1 else 1e-4)
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 148 * 8 * 256 * 8 - 1, 148 * 8 * 256 * 9 + 3])
+def test_where_and_dropout_cover_the_tensor_once(n):
+    ctx = ndarray.gpu(0)
+    c, p, q = (_rand(n, seed=k) for k in range(3))
+    c[c < 0] = 0
+    out, drop = torch.full((n + 8,), 7.0, device="cuda"), torch.full((n + 8,), 7.0, device="cuda")
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    G.where(a(c), a(p), a(q), a(out[:n]), _stream())
+    G.dropout(a(p), a(drop[:n]), 0.75, 11, _stream())
+    _stream().sync()
+    assert torch.equal(out[:n], torch.where(c != 0, p, q)) and torch.all(out[n:] == 7) and torch.all(drop[n:] == 7)
+    from tsplit_b200.ops.misc import philox_like_mask
+    keep = torch.from_numpy(philox_like_mask((n,), 0.75, 11)).cuda()
+    torch.testing.assert_close(drop[:n], torch.where(keep, p / 0.75, torch.zeros_like(p)), rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("tk", [4, 37, 128, 132, 256, 512, 516, 1000, 1024])
+@pytest.mark.parametrize("keys", [True, False])
+@pytest.mark.parametrize("causal", [0, 1])
+def test_masked_softmax_rows(tk, keys, causal):
+    n, h, tq = 2, 3, 5
+    x = _rand(n, h, tq, tk)
+    k = (torch.arange(tk, device="cuda")[None, :] < torch.tensor([[tk], [max(1, tk // 2)]], device="cuda")).float()
+    a = lambda t: ndarray.from_tensor(t, ndarray.gpu(0))
+    y = torch.full_like(x, 9.0)
+    G.masked_softmax(a(x), a(k) if keys else None, a(y), 0.25, causal, _stream())
+    _stream().sync()
+    t = x.double() * 0.25
+    if keys:
+        t = t + torch.where(k == 0, -1e9, 0.0).double()[:, None, None, :]
+    if causal:
+        t = torch.where(torch.ones(tq, tk, device="cuda").tril() > 0, t, torch.full((), -1e9, dtype=t.dtype, device="cuda"))
+    torch.testing.assert_close(y.double(), torch.softmax(t, -1), rtol=1e-4, atol=1e-8)      # the fast exponential's 2^-21
+
+
 # few rows of wide arrays: the widths of the single launch and the first past them, for many rows and for few; then many
 # chunks (more than 128) of few columns and of many
 @pytest.mark.parametrize("rows,cols", [(64, 8192), (129, 8192), (129, 8196), (128, 16384), (128, 16388), (63, 16388), (512, 16386),

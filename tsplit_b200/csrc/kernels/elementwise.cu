@@ -99,12 +99,21 @@ __global__ void __launch_bounds__(256) binary_flat(const float* p, const float* 
   }
 }
 
-__global__ void where_flat(const float* c, const float* a, const float* b,
-                           float* __restrict__ y, long long n) {
+// (Of a and b only what is taken is read: a mask of one value costs three passes, not four.)
+__global__ void where_flat(const float* c, const float* a, const float* b, float* __restrict__ y, long long n) {
   tsb_launch::enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-    y[i] = c[i] != 0.f ? a[i] : b[i];
+  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (; i + 7 * stride < n; i += 8 * stride) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = c[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = (v[u] != 0.f ? a : b)[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) y[i + u * stride] = v[u];
+  }
+  for (; i < n; i += stride) y[i] = (c[i] != 0.f ? a : b)[i];
 }
 
 // y[r, c] = x[r, c] + b[c] on a dense row-major [rows, cols] view, 16 bytes per thread (the bias of a

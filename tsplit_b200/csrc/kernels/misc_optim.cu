@@ -142,9 +142,10 @@ __global__ void dropout_kernel(const float* x, float* __restrict__ y, long long 
   tsb_launch::enter();
   if (step_dev) seed = (seed + 0x632BE5ABull * *step_dev) & 0x7FFFFFFFFFFFFFFFull;
   const float inv = 1.f / keep;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    y[i] = uniform01(seed, (unsigned long long)i + offset) < keep ? x[i] * inv : 0.f;
+  tsb_launch::read_then_write<8>(
+      blockIdx.x * (long long)blockDim.x + threadIdx.x, n, (long long)gridDim.x * blockDim.x,
+      [&](long long i) { return x[i]; },
+      [&](long long i, float v) { y[i] = uniform01(seed, (unsigned long long)i + offset) < keep ? v * inv : 0.f; });
 }
 
 // out[r, :] = sum_j vals[j] * dense[col[j], :]   (one warp per sparse row)

@@ -373,7 +373,41 @@ __global__ void ln_fwd(const float* x, const float* scale, const float* bias,
   const float is = rsqrtf(var + eps);
   if (lane == 0) { mean[row] = m; invstd[row] = is; }
   float* yr = y + row * D;
-  for (int i = lane; i < D; i += 32) yr[i] = (xr[i] - m) * is * scale[i] + bias[i];
+  tsb_launch::read_then_write<4>(lane, D, 32, [&](int i) { return make_float3(xr[i], scale[i], bias[i]); },
+                                 [&](int i, float3 v) { yr[i] = (v.x - m) * is * v.y + v.z; });
+}
+
+// The same for rows of up to 32 NE floats, which stay in registers between the sums and the result (in the same order).
+template <int NE>
+__global__ void __launch_bounds__(256) ln_fwd_kept(const float* x, const float* scale, const float* bias,
+                                                   float* __restrict__ y, float* __restrict__ mean,
+                                                   float* __restrict__ invstd, long long rows, int D, float eps) {
+  tsb_launch::enter();
+  const int lane = threadIdx.x & 31;
+  const long long row = (blockIdx.x * 256ll + threadIdx.x) >> 5;
+  if (row >= rows) return;
+  float v[NE], s = 0.f, ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NE; ++j) v[j] = lane + 32 * j < D ? load(x + row * D + lane + 32 * j) : 0.f;
+#pragma unroll
+  for (int j = 0; j < NE; ++j) { s += v[j]; ss += v[j] * v[j]; }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { s += __shfl_xor_sync(0xffffffffu, s, o); ss += __shfl_xor_sync(0xffffffffu, ss, o); }
+  const float m = s / D;
+  const float var = fmaxf(ss / D - m * m, 0.f);
+  const float is = rsqrtf(var + eps);
+  if (lane == 0) { mean[row] = m; invstd[row] = is; }
+  float* yr = y + row * D;
+#pragma unroll
+  for (int j = 0; j < NE; j += 4) {
+    float g[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (lane + 32 * (j + u) < D) { g[u] = load(scale + lane + 32 * (j + u)); b[u] = load(bias + lane + 32 * (j + u)); }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (lane + 32 * (j + u) < D) yr[lane + 32 * (j + u)] = (v[j + u] - m) * is * g[u] + b[u];
+  }
 }
 
 __global__ void ln_bwd_dx(const float* dy, const float* x, const float* scale,
@@ -396,7 +430,8 @@ __global__ void ln_bwd_dx(const float* dy, const float* x, const float* scale,
   for (int o = 16; o > 0; o >>= 1) { s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); }
   s1 /= D; s2 /= D;
   float* dr = dx + row * D;
-  for (int i = lane; i < D; i += 32) dr[i] = is * (gr[i] * scale[i] - s1 - (xr[i] - m) * is * s2);
+  tsb_launch::read_then_write<8>(lane, D, 32, [&](int i) { return make_float3(gr[i], scale[i], xr[i]); },
+                                 [&](int i, float3 v) { dr[i] = is * (v.x * v.y - s1 - (v.z - m) * is * s2); });
 }
 
 // 16-byte variant for rows of up to 128 * NV floats: the row stays in registers between the sums and the result, so dy
@@ -685,7 +720,8 @@ int tsb_layer_norm(const float* x, const float* scale, const float* bias, float*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows <= 0 || D <= 0) return TSB_ERR_ARG;
   const long long threads = rows * 32;
-  tsb_launch::launch(ln_fwd, (unsigned)((threads + 255) / 256), 256, 0, st, x, scale, bias, y, mean, invstd, rows,
+  tsb_launch::launch(D <= 128 ? ln_fwd_kept<4> : D <= 512 ? ln_fwd_kept<16> : D <= 1024 ? ln_fwd_kept<32> : ln_fwd,
+                     (unsigned)((threads + 255) / 256), 256, 0, st, x, scale, bias, y, mean, invstd, rows,
                      (int)D, eps);
   return done();
 }

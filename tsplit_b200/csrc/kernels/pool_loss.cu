@@ -450,7 +450,8 @@ __global__ void softmax_rows(const float* x, float* __restrict__ y, long long ro
     for (long long i = threadIdx.x; i < cols; i += blockDim.x) s += __expf(xr[i] - m);
     s = block_sum(s, sh);
     const float inv = 1.f / s;
-    for (long long i = threadIdx.x; i < cols; i += blockDim.x) y[row * cols + i] = __expf(xr[i] - m) * inv;
+    tsb_launch::read_then_write<4>((long long)threadIdx.x, cols, (long long)blockDim.x, [&](long long i) { return xr[i]; },
+                                   [&](long long i, float v) { y[row * cols + i] = __expf(v - m) * inv; });
   }
 }
 
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(256) softmax_warp_rows(const float4* x, float4
 // The same for rows whose length is no multiple of 4 (or whose base is not 16-byte aligned): scalar,
 // still coalesced, lanes; NE elements per lane.
 template <int NE>
-__global__ void __launch_bounds__(256) softmax_warp_rows_scalar(const float* x, float* __restrict__ y,
+__global__ void __launch_bounds__(256, NE == 32 ? 4 : 1) softmax_warp_rows_scalar(const float* x, float* __restrict__ y,
                                                                 long long rows, int cols) {
   tsb_launch::enter();
   const int lane = threadIdx.x & 31;
@@ -667,22 +668,27 @@ __global__ void __launch_bounds__(256) masked_softmax_warp_rows_v4(const float4*
     const float4* xr = x + row * nvec;
     const float4* kt = key_tokens ? key_tokens + (long long)((unsigned)row / (unsigned)rows_per_batch) * nvec : nullptr;
     const int q = (int)((unsigned)row % (unsigned)tq);
-    float4 v[NV];
+    float4 v[NV], keys[NV];                     // all loads first
     float m = -FLT_MAX;
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int i = lane + 32 * j;
-      float4 t = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
+      v[j] = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
+      keys[j] = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (i < nvec) v[j] = load(xr + i);
+      if (i < nvec && kt) keys[j] = load(kt + i);
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + 32 * j;
+      float4 t = v[j];
       if (i < nvec) {
-        t = load(xr + i);
         t.x *= scale; t.y *= scale; t.z *= scale; t.w *= scale;
-        if (kt) {
-          const float4 k = load(kt + i);
-          if (k.x == 0.f) t.x += -1e9f;
-          if (k.y == 0.f) t.y += -1e9f;
-          if (k.z == 0.f) t.z += -1e9f;
-          if (k.w == 0.f) t.w += -1e9f;
-        }
+        const float4 k = keys[j];
+        if (k.x == 0.f) t.x += -1e9f;
+        if (k.y == 0.f) t.y += -1e9f;
+        if (k.z == 0.f) t.z += -1e9f;
+        if (k.w == 0.f) t.w += -1e9f;
         if (causal) {
           const int c = 4 * i;
           if (c > q) t.x = -1e9f;
@@ -798,7 +804,9 @@ __global__ void softmax_grad_rows(const float* y, const float* dy, float* __rest
     float s = 0.f;
     for (long long i = threadIdx.x; i < cols; i += blockDim.x) s += yr[i] * gr[i];
     s = block_sum(s, sh);
-    for (long long i = threadIdx.x; i < cols; i += blockDim.x) dx[row * cols + i] = yr[i] * (gr[i] - s);
+    tsb_launch::read_then_write<4>((long long)threadIdx.x, cols, (long long)blockDim.x,
+                                   [&](long long i) { return make_float2(yr[i], gr[i]); },
+                                   [&](long long i, float2 v) { dx[row * cols + i] = v.x * (v.y - s); });
   }
 }
 
@@ -978,6 +986,26 @@ __global__ void __launch_bounds__(512) ce_grad_rows_v4(const float4* x, Labels l
   }
 }
 
+// Rows of up to KEPT values a thread stay in registers between the passes of the two kernels below.
+constexpr int KEPT = 8;
+__device__ __forceinline__ void keep_row(float (&v)[KEPT], const float* xr, int cols, float rest) {
+#pragma unroll
+  for (int u = 0; u < KEPT; ++u) {
+    const int i = threadIdx.x + u * blockDim.x;
+    v[u] = i < cols ? load(xr + i) : rest;
+  }
+}
+__device__ __forceinline__ MaxSum kept_max_sum(const float (&v)[KEPT], int cols, float* sh) {
+  float m = -FLT_MAX, s = 0.f;
+#pragma unroll
+  for (int u = 0; u < KEPT; ++u) m = fmaxf(m, v[u]);
+  m = block_max(m, sh);
+#pragma unroll
+  for (int u = 0; u < KEPT; ++u)
+    if (threadIdx.x + u * blockDim.x < cols) s += expf(v[u] - m);
+  return {m, block_sum(s, sh)};
+}
+
 __global__ void ce_rows(const float* x, const float* lab, float* __restrict__ row_loss,
                         long long rows, long long cols) {
   tsb_launch::enter();
@@ -985,15 +1013,26 @@ __global__ void ce_rows(const float* x, const float* lab, float* __restrict__ ro
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float* xr = x + row * cols;
     const float* lr = lab + row * cols;
-    float m = -FLT_MAX;
-    for (long long i = threadIdx.x; i < cols; i += blockDim.x) m = fmaxf(m, xr[i]);
-    m = block_max(m, sh);
-    float s = 0.f;
-    for (long long i = threadIdx.x; i < cols; i += blockDim.x) s += expf(xr[i] - m);
-    s = block_sum(s, sh);
-    const float lse = m + logf(s);
     float l = 0.f;
-    for (long long i = threadIdx.x; i < cols; i += blockDim.x) l -= lr[i] * (xr[i] - lse);
+    if (cols <= KEPT * (long long)blockDim.x) {
+      float v[KEPT], t[KEPT];
+      keep_row(v, xr, (int)cols, -FLT_MAX);
+      keep_row(t, lr, (int)cols, 0.f);
+      const MaxSum ms = kept_max_sum(v, (int)cols, sh);
+      const float lse = ms.m + logf(ms.s);
+#pragma unroll
+      for (int u = 0; u < KEPT; ++u)
+        if (threadIdx.x + u * blockDim.x < cols) l -= t[u] * (v[u] - lse);
+    } else {
+      float m = -FLT_MAX;
+      for (long long i = threadIdx.x; i < cols; i += blockDim.x) m = fmaxf(m, xr[i]);
+      m = block_max(m, sh);
+      float s = 0.f;
+      for (long long i = threadIdx.x; i < cols; i += blockDim.x) s += expf(xr[i] - m);
+      s = block_sum(s, sh);
+      const float lse = m + logf(s);
+      for (long long i = threadIdx.x; i < cols; i += blockDim.x) l -= lr[i] * (xr[i] - lse);
+    }
     l = block_sum(l, sh);
     if (threadIdx.x == 0) row_loss[row] = l;
   }
@@ -1015,6 +1054,19 @@ __global__ void ce_grad_rows(const float* x, const float* lab, const float* g,
   const float scale = g[0] / (float)rows;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float* xr = x + row * cols;
+    if (cols <= KEPT * (long long)blockDim.x) {
+      float v[KEPT], t[KEPT];
+      keep_row(v, xr, (int)cols, -FLT_MAX);
+      keep_row(t, lab + row * cols, (int)cols, 0.f);
+      const MaxSum ms = kept_max_sum(v, (int)cols, sh);
+      const float inv = 1.f / ms.s;
+#pragma unroll
+      for (int u = 0; u < KEPT; ++u) {
+        const int i = threadIdx.x + u * blockDim.x;
+        if (i < cols) dx[row * cols + i] = (expf(v[u] - ms.m) * inv - t[u]) * scale;
+      }
+      continue;
+    }
     float m = -FLT_MAX;
     for (long long i = threadIdx.x; i < cols; i += blockDim.x) m = fmaxf(m, xr[i]);
     m = block_max(m, sh);
@@ -1022,8 +1074,9 @@ __global__ void ce_grad_rows(const float* x, const float* lab, const float* g,
     for (long long i = threadIdx.x; i < cols; i += blockDim.x) s += expf(xr[i] - m);
     s = block_sum(s, sh);
     const float inv = 1.f / s;
-    for (long long i = threadIdx.x; i < cols; i += blockDim.x)
-      dx[row * cols + i] = (expf(xr[i] - m) * inv - lab[row * cols + i]) * scale;
+    tsb_launch::read_then_write<4>((long long)threadIdx.x, cols, (long long)blockDim.x,
+                                   [&](long long i) { return make_float2(xr[i], lab[row * cols + i]); },
+                                   [&](long long i, float2 v) { dx[row * cols + i] = (expf(v.x - m) * inv - v.y) * scale; });
   }
 }
 
