@@ -413,3 +413,89 @@ def test_column_sums_of_wide_arrays(rows, cols):
     _stream().sync()
     # at most some hundred roundings of partial sums in a row
     assert torch.all((y.double() - x.double().sum(0)).abs() <= 160 * 2.0 ** -24 * x.double().abs().sum(0))
+
+
+LOWEST = float(np.finfo(np.float32).min)
+
+
+def _first_maximum_gradient(x, dy, k, pad, stride):
+    """The first pixel of a window that nothing after it exceeds takes its gradient; comparisons with NaN are false."""
+    n, c, h, w = x.shape
+    dx = np.zeros_like(x)
+    for b, ch, oy, ox in np.ndindex(dy.shape):
+        best = None
+        for iy in range(max(0, oy * stride - pad), min(h, oy * stride - pad + k)):
+            for ix in range(max(0, ox * stride - pad), min(w, ox * stride - pad + k)):
+                if best is None or x[b, ch, iy, ix] > x[(b, ch) + best]:
+                    best = (iy, ix)
+        dx[(b, ch) + best] += dy[b, ch, oy, ox]
+    return dx
+
+
+# one pass over tiles (with and without the constants of 3 x 3 stride 2), and two passes
+@pytest.mark.parametrize("k,pad,stride", [(3, 1, 2), (2, 0, 1), (15, 7, 1)])
+def test_max_pool_gradient_of_special_values(k, pad, stride):
+    x = _rand(1, 4, 19, 18).cpu().numpy()
+    r = np.random.RandomState(0)
+    for v in (LOWEST, -np.inf, np.inf, np.nan):
+        x[0, r.randint(0, 4, 30), r.randint(0, 19, 30), r.randint(0, 18, 30)] = v
+    x[0, 1, :9, :9], x[0, 2, :9, :9] = LOWEST, -np.inf                       # whole windows of them
+    oh, ow = (19 + 2 * pad - k) // stride + 1, (18 + 2 * pad - k) // stride + 1
+    dy = np.round(_rand(1, 4, oh, ow, seed=1).cpu().numpy() * 8) / 8          # sums of eighths are exact
+    t = lambda a: _arr(torch.from_numpy(a).cuda())
+    dx, y = _arr(torch.full((1, 4, 19, 18), 7.0, device="cuda")), t(np.zeros((1, 4, oh, ow), np.float32))
+    G.pool_grad(0, t(x), y, t(dy), dx, k, k, pad, stride, _stream())
+    _stream().sync()
+    np.testing.assert_array_equal(dx.t.cpu().numpy(), _first_maximum_gradient(x, dy, k, pad, stride))
+
+
+@pytest.mark.parametrize("rows", [2, 63, 64, 512, 513])
+def test_column_sums_of_special_values(rows):
+    x = _rand(rows, 40)
+    x[0, 3], x[rows - 1, 4], x[0, 5], x[rows - 1, 5] = float("inf"), float("-inf"), float("inf"), float("-inf")
+    x[rows // 2, 6] = float("nan")
+    x[0, 7], x[rows - 1, 7] = LOWEST, LOWEST                                  # below the range of fp32
+    x[:, 8] = 0
+    x[0, 8], x[rows - 1, 8] = LOWEST, -LOWEST
+    y = torch.zeros(40, device="cuda")
+    G.reduce_sum(x.data_ptr(), [rows, 40], [40, 1], [0], ndarray.from_tensor(y, ndarray.gpu(0)), _stream())
+    _stream().sync()
+    assert y[3] == float("inf") and y[4] == float("-inf") and torch.isnan(y[5]) and torch.isnan(y[6])
+    assert y[7] == float("-inf") and y[8] == 0
+    assert torch.isfinite(y[[0, 1, 2]]).all() and torch.isfinite(y[9:]).all()
+
+
+# a block per window, several, and a thread per output
+@pytest.mark.parametrize("hw", [8, 57, 7])
+def test_average_pool_of_special_values(hw):
+    x = _rand(2, 8, hw, hw)
+    x[0, 0, 0, 0], x[0, 1, -1, -1], x[1, 2, 3, 3] = float("inf"), float("-inf"), float("nan")
+    x[1, 3, 0, 0], x[1, 3, -1, -1], x[1, 4] = float("inf"), float("-inf"), 0
+    x[1, 4, 0, 0] = LOWEST
+    ref = x.double().mean((2, 3), keepdim=True).float()
+    y = _arr(torch.zeros_like(ref))
+    G.pool(1, _arr(x), y, hw, hw, 0, hw, _stream())
+    _stream().sync()
+    # (sums of at most some hundred terms a lane, pairwise joins)
+    torch.testing.assert_close(y.t, ref, rtol=1e-5, atol=1e-5, equal_nan=True)
+
+
+@pytest.mark.parametrize("d", [64, 1024, 1028, 30])
+def test_layer_norm_gradient_keeps_special_values_in_their_row(d):
+    ctx = ndarray.gpu(0)
+    rows = 9
+    x, dy, scale = _rand(rows, d, seed=1), _rand(rows, d, seed=2), _rand(d, seed=4) + 1
+    mean, inv = x.mean(1), 1 / torch.sqrt(x.var(1, unbiased=False) + 1e-5)
+    a = lambda t: ndarray.from_tensor(t, ctx)
+    outs = []
+    for v in (None, float("nan"), float("inf")):
+        g = dy.clone()
+        if v is not None:
+            g[4, d - 1] = v
+        dx, ds, db = torch.zeros_like(x), torch.zeros(d, device="cuda"), torch.zeros(d, device="cuda")
+        G.layer_norm_grad(a(g), a(x), a(scale), a(mean), a(inv), a(dx), a(ds), a(db), _stream())
+        _stream().sync()
+        outs.append(dx)
+    others = [r for r in range(rows) if r != 4]
+    for dx in outs[1:]:
+        assert torch.equal(dx[others], outs[0][others]) and not torch.isfinite(dx[4]).any()
