@@ -1261,7 +1261,8 @@ __global__ void parity_interleave(const ParityParts pp, float* __restrict__ dx, 
 }
 
 // (Channel counts are multiples of four, so filters are whole float4.)  Eight partial sums in flight per thread instead
-// of one float after another: ResNet-50 step, 53 of them, 7912 -> 7713 us.
+// of one float after another.  Whole filter gradients of 32 images: 512 x 512 x 3 x 3 at 7 x 7 29.2 -> 26.9 us, 512 x 128 at
+// 28 x 28 21.9 -> 20.7, 64 x 64 x 3 x 3 at 56 x 56 38.9 -> 39.0.
 __global__ void __launch_bounds__(256) conv_splitk_reduce(const float4* ws, float4* __restrict__ out,
                                                           int splits, long long per_split4) {
   tsb_launch::enter();

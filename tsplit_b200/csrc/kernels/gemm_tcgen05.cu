@@ -356,8 +356,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 // Several small products as one launch, a CTA per tile.  The gates of a recurrent cell are a handful of products of a
 // tile or two each; one after the other they are bound by the latency of a launch, a TMA round trip and a store, with
-// all but two SMs idle, and side by side they take the time of one.  LSTM step, 549 products in 84 launches:
-// 3351 -> 1322 us; a small Transformer 565 -> 504.
+// all but two SMs idle, and side by side they take the time of one: 16 of 128 x 128 x 128 6.4 us, 5.9 for each by itself.
 constexpr int MAX_GROUP = 16, GROUP_BN = 64;      // (the narrowest tile: see narrow_tile)
 struct GemmGroup {
   CUtensorMap ta[MAX_GROUP], tb[MAX_GROUP], tc[MAX_GROUP];

@@ -2,8 +2,8 @@
 //
 // A training step of this library is a chain of some hundred to some thousand kernels on one stream, most of them a
 // few microseconds long, so the time between one kernel's last block and the next one's first instruction is a large
-// part of it.  Every kernel here is launched with the programmatic-serialisation attribute and begins with enter():
-// its blocks may be placed, and barriers and TMEM set up, while the previous kernel drains; they wait until that
+// part of it.  Every kernel of this folder is launched with the programmatic-serialisation attribute and begins with
+// enter(): its blocks may be placed, and barriers and TMEM set up, while the previous kernel drains; they wait until that
 // kernel has completed and its writes are visible.  Because every kernel waits, completion stays in stream order; a
 // copy, an event or a kernel of another library in between is ordered in full as before.  Stream capture keeps the
 // attribute as a programmatic edge.
@@ -12,8 +12,9 @@
 // nvcc makes of a `const T* __restrict__` parameter) want data that nothing writes while the kernel lives, and
 // may be moved above the wait or served from a line that was cached before it.  So kernels launched from here
 // take the pointers they read without __restrict__ and use ordinary loads, which stay behind the wait; pointers that
-// they write keep __restrict__, so loads may still pass stores.  A plain load costs the same: 137 M floats times a
-// constant 161.5 us through the read-only path and 161.9 without, the sum of two such tensors 234.3 and 235.5.
+// they write keep __restrict__.  A plain load costs the same (137 M floats times a constant 161.5 us through the read-only
+// path and 161.9 without, the sum of two such tensors 234.3 and 235.5), but it stays behind the stores before it, so a
+// kernel reads what it can before it writes (read_then_write below).
 //
 // Captured steps: LSTM, 2428 kernels: 6718 -> 5535 us (2.77 -> 2.28 us a kernel); a 1x7 / 7x1 convolution pair at 17 x 17:
 // 292 -> 275 us; a small Transformer: 808 -> 716 us.

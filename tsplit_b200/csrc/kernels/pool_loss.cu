@@ -95,9 +95,8 @@ __global__ void pool_fwd(const float* x, float* __restrict__ y, const PoolP p) {
 // channels leaves n * C / 1024 blocks that walk the window one load at a time; here a block of 32 pixel lanes x 8
 // channel vectors (128-byte segments) reads the window with four loads in flight per thread, and a cluster of up to 8
 // blocks shares one window, joined through distributed shared memory in a fixed order, so one launch both fills the
-// chip and stays deterministic.  Bound by DRAM.  Whole training
-// steps: VGG's first block before a 112 x 112 pool of 64 channels, batch 16: 4998 -> 1552 us; a 56 x 56 pool of 256
-// channels, batch 32: 1570 -> 844 us; 17 x 17 of 256 channels, batch 32: 338 -> 292 us.
+// chip and stays deterministic.  Bound by DRAM.  16 x 112 x 112 x 64: 3465 us with a thread per output, 20.6 now;
+// 32 x 56 x 56 x 256: 794 and 32.4; 32 x 28 x 28 x 512: 195 and 20.5; 32 x 17 x 17 x 256: 83 and 7.2.
 constexpr int WIN_COLS = 8, WIN_LANES = 32;
 __global__ void __launch_bounds__(WIN_COLS * WIN_LANES) avg_pool_window(const float* x,
                                                                         float* __restrict__ y, const PoolP p) {
@@ -347,7 +346,7 @@ __global__ void pool_bwd_from_argmax(const unsigned char* idx, const float* dy,
 // first maximum of every window that reaches into them (windows on the edge are found by both neighbours), keeps
 // position and gradient in shared memory and gathers from there, in the order of pool_bwd_from_argmax.  x comes from
 // DRAM once and its overlapping reads from L1, and the positions never leave the SM.
-// 32 x 112 x 112 x 64, 3 x 3 stride 2: 180 us in two passes -> 94 (127 without the constants); ResNet stem step 795 -> 712.
+// 32 x 112 x 112 x 64, 3 x 3 stride 2: 180 us in two passes -> 94 (127 without the constants).
 // K, S: window and stride as constants (0: from p), which halves the arithmetic of the usual 3 x 3 stride 2.
 template <int T, int K, int S>
 __global__ void __launch_bounds__(256) max_pool_bwd_tile(const float* x, const float* dy,
@@ -879,8 +878,8 @@ __device__ __forceinline__ void staged() { asm volatile("cp.async.wait_all;" :::
 
 // Long rows, 16-byte lanes.  Two passes over the logits; rows of 32 to 200 KB wait for the second one in shared memory
 // (STAGED): left to L2, most of a 128 KB row is gone by then, with some 600 rows in flight.  Bound by DRAM.
-// 4096 x 32000 gradient with labels from ids: 278 us (dense labels, unstaged) -> 193 us; loss 174 -> 96 us in one pass.
-// The whole step of a 32000-word head: 1758 -> 1347 us, the label tensors (one-hot, scaled, shifted) not made at all.
+// 4096 x 32000 gradient with labels from ids: 278 us (dense labels, unstaged) -> 193 us.  The loss from ids takes one pass
+// (below); the label tensors (one-hot, scaled, shifted) are not made at all.
 template <class Labels, bool STAGED>
 __global__ void __launch_bounds__(512) ce_rows_v4(const float4* x, Labels lab,
                                                   float* __restrict__ row_loss, long long rows, int nvec) {
@@ -914,7 +913,7 @@ __global__ void __launch_bounds__(512) ce_rows_v4(const float4* x, Labels lab,
 // and rounding is relative to lse - c, which the loss is made of: a common offset of the logits costs no digits.
 // Every logit is weighed before it is added: logits at the lowest float (masked classes) under a label of 0 count as 0, as
 // in the two-pass form.  No such c (an id outside the classes, a masked or infinite label): 0, and each class its own
-// label.
+// label.  4096 x 32000 with the mean of the rows: 111 us, bound by DRAM.
 __global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* x, SmoothLabels lab,
                                                          float* __restrict__ row_loss, long long rows, int nvec) {
   tsb_launch::enter();

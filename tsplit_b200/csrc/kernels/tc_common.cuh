@@ -398,10 +398,10 @@ int peek_status();                       // read without synchronising
 
 // Columns per tile of a one-CTA launch whose `tiles` 128 x bn tiles leave at least half of the SMs idle.  Such a launch
 // is bound by what one SM can take from L2: a k-block brings 16 KB of A and bn / 8 KB of B, whatever the number of
-// tiles, so halving bn puts twice the SMs to work at two thirds of the bytes each.  Narrowed while the tiles still fit
-// one per SM; the order of the sums over K does not change.  Captured steps: LSTM (one tile of 128 x 128 a product)
-// 5815 -> 5288 us, MLP 102 -> 86, small Transformer 752 -> 679; the 26- and 49-tile convolutions of ResNet-50, batch 32,
-// 28.4 us each before, 25.0 after.
+// tiles, so halving bn puts twice the SMs to work at two thirds (256 -> 128) or three quarters (128 -> 64) of the bytes
+// each.  Narrowed while the tiles still fit one per SM, also where two CTAs of the narrower tile would fit on one (what
+// lies beyond that line was not measured); the order of the sums over K does not change.  The 26- and 49-tile
+// convolutions of ResNet-50, batch 32, 28.4 us each before, 25.0 after.
 inline int narrow_tile(int bn, long long tiles, int sms) {
   while (bn > 64 && 2 * tiles <= sms) {
     bn /= 2;

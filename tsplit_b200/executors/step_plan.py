@@ -1,6 +1,7 @@
 """The order in which the keep-all executors issue a step on the GPU, worked out once per feed shape.
 
-Five things are taken out of the node-by-node loop, none of which changes a value:
+Five things are taken out of the node-by-node loop.  They change no value, but for the rounding of a loss whose labels
+come from class ids (the last one: the same sum, added up in another order):
 
 * element-wise operators over the same elements are collected and run as one ``tsb_pointwise`` program, at the first
   node that needs one of their results; results that nobody outside the program reads are not stored;
