@@ -1484,6 +1484,7 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
       }
       return launch_fwd_pair(bn, tmh, tmi, tmo, p, st);
     }
+    // few tiles: narrower ones (here only: the gather path below keeps its width, which was not measured)
     const int nbn = tsb_host::narrow_tile(bn, (long long)p.tiles_m * p.tiles_n, sm_count());
     if (nbn != bn) {
       bn = nbn;
