@@ -15,6 +15,7 @@
 // Role in the reference: cublasSgemm / cublasSgemmStridedBatched
 // (src/ops/MatrixMult.cu:4-72, src/ops/BatchMatrixMult.cu:4-43).
 #include "tc_common.cuh"
+#include "gemm_small.h"
 #include "scratch.h"
 #include "launch.cuh"
 #include "smem_limit.h"
@@ -357,7 +358,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // Several small products as one launch, a CTA per tile.  The gates of a recurrent cell are a handful of products of a
 // tile or two each; one after the other they are bound by the latency of a launch, a TMA round trip and a store, with
 // all but two SMs idle, and side by side they take the time of one: 16 of 128 x 128 x 128 6.4 us, 5.9 for each by itself.
-constexpr int MAX_GROUP = 16, GROUP_BN = 64;      // (the narrowest tile: see narrow_tile)
+constexpr int MAX_GROUP = tsb_small::MAX_PRODUCTS, GROUP_BN = 64;      // (the narrowest tile: see narrow_tile)
 struct GemmGroup {
   CUtensorMap ta[MAX_GROUP], tb[MAX_GROUP], tc[MAX_GROUP];
   GemmParams p[MAX_GROUP];
@@ -928,6 +929,99 @@ static int choose_splits(long long tiles, int kblocks, int forced) {
   return s < 1 ? 1 : (int)s;
 }
 
+// K ranges of a product: how many, and k-blocks in each (no empty ones).
+struct KRanges {
+  int kblocks, splits, per;
+};
+static KRanges k_ranges(int m, int n, int k, int batch, int forced) {
+  const int bn = n > 128 ? 256 : (n > 64 ? 128 : 64);
+  KRanges r;
+  r.kblocks = (k + BK - 1) / BK;
+  r.splits = choose_splits((long long)((m + BM - 1) / BM) * ((n + bn - 1) / bn) * batch, r.kblocks, forced);
+  if (r.splits > r.kblocks) r.splits = r.kblocks;
+  r.per = (r.kblocks + r.splits - 1) / r.splits;
+  r.splits = (r.kblocks + r.per - 1) / r.per;
+  return r;
+}
+
+// Tensor map of an operand of `rows` rows (M or N) and k, in boxes of 32 k x `box` rows.  K contiguous: K-major.  Rows
+// contiguous (`mn`): MN-major chunks of 32 rows, all of a box at once where the rows are whole chunks (*chunked).  outer,
+// batch: row blocks and matrices that the map spans (head layout: see GemmParams); strides in bytes.
+// kbox > 1: k-blocks per box (K contiguous: k a multiple of 32).
+static int operand_map(CUtensorMap* out, int* chunked, const float* base, bool mn, int rows, int k, long long ld,
+                       uint64_t outer, uint64_t batch, uint64_t batch_bytes, uint32_t box, uint32_t kbox = 1) {
+  *chunked = mn && rows % 32 == 0;
+  if (!mn && kbox > 1) {
+    uint64_t d[4] = {32, (uint64_t)rows * outer, (uint64_t)k / 32, batch}, s[3] = {(uint64_t)ld * 4, 128, batch_bytes};
+    uint32_t bx[4] = {32, box, kbox, 1};
+    return tsb_host::make_tmap_f32(out, base, 4, d, s, bx);
+  }
+  if (!mn) {
+    uint64_t d[3] = {(uint64_t)k, (uint64_t)rows * outer, batch}, s[2] = {(uint64_t)ld * 4, batch_bytes};
+    uint32_t bx[3] = {BK, box, 1};
+    return tsb_host::make_tmap_f32(out, base, 3, d, s, bx);
+  }
+  if (*chunked) {
+    uint64_t d[4] = {32, (uint64_t)k * outer, (uint64_t)rows / 32, batch}, s[3] = {(uint64_t)ld * 4, 128, batch_bytes};
+    uint32_t bx[4] = {32, BK * kbox, box / 32, 1};
+    return tsb_host::make_tmap_f32(out, base, 4, d, s, bx, true);
+  }
+  uint64_t d[3] = {(uint64_t)rows, (uint64_t)k * outer, batch}, s[2] = {(uint64_t)ld * 4, batch_bytes};
+  uint32_t bx[3] = {32, BK * kbox, 1};
+  return tsb_host::make_tmap_f32(out, base, 3, d, s, bx, true);
+}
+
+// Products for gemm_small.cu: those whose blocks are all resident at once, one or two to an SM as their shared memory
+// allows.  They have each 64 x 32 outputs and all of their K range at hand, so up to there nothing waits for anything
+// but its own operands; in a second wave the wide tiles are ahead.  In a chain of equal products, us here / there:
+// 256 x 256 x 256 2.8 / 5.3, 1024 x 256 x 256 3.6 / 5.4, 128 x 4096 x 128 3.9 / 4.8, 32 of 128 x 128 x 32 3.85 / 4.0,
+// 512 x 512 x 512 (2 ranges) 6.3 / 7.7, 32 x 1000 x 2048 (8 ranges) 6.4 / 7.5; beyond the line 1024 x 1024 x 128 6.1 / 4.9,
+// 512 x 256 x 784 (3 ranges, one block to an SM) 9.6 / 7.9.  The results are the same bit for bit.
+static bool is_small(long long blocks, int kb_per_split) {
+  const int per_sm = 2 * (tsb_small::smem_of(kb_per_split) + (10 << 10)) <= (227 << 10) ? 2 : 1;      // (10 KB: fixed part)
+  return blocks <= (long long)per_sm * sm_count();
+}
+static bool small_form(const KRanges& r, const float* a, const float* b) {
+  return r.splits <= tsb_small::MAX_SPLITS && r.per <= tsb_small::MAX_KBLOCKS &&
+         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+}
+// An operand of such a product, and its tensor map if its strides allow one.
+static int small_operand(tsb_small::Operand* q, CUtensorMap* map, const float* base, bool mn, int rows, int k, long long ld,
+                         long long s, int inner, int batch, bool heads, uint32_t box, int kb_per_split) {
+  q->base = base; q->ld = ld; q->s = s;
+  q->heads = heads;
+  q->shift = heads ? (mn ? k : rows) : 0;
+  q->s2 = heads ? (long long)q->shift * ld : inner * s;
+  q->tma = ld % 4 == 0 && (batch == 1 || s % 4 == 0);
+  q->kbox = !mn && k % BK ? 1 : (kb_per_split < tsb_small::ROUND ? kb_per_split : tsb_small::ROUND);
+  if (!q->tma) return TSB_OK;
+  return operand_map(map, &q->chunked, base, mn, rows, k, ld, heads ? batch / inner : 1, heads ? inner : batch,
+                     (uint64_t)(batch > 1 ? s : (long long)(mn ? k : rows) * ld) * 4, box, q->kbox);
+}
+static int small_product(tsb_small::Product* q, CUtensorMap* ta, CUtensorMap* tb, const float* a, const float* b, float* c,
+                         int m, int n, int k, long long lda, long long ldb, long long ldc, int trans_a, int trans_b, int batch,
+                         long long sa, long long sb, long long sc, int accumulate, int heads, int head_mask, int kb_per_split) {
+  q->inner = heads > 0 ? heads : batch;
+  q->batch = batch;
+  q->c = c; q->ldc = ldc; q->sc = sc;
+  q->sc2 = (head_mask & 4) ? (long long)m * ldc : q->inner * sc;
+  q->m = m; q->n = n; q->k = k;
+  q->accumulate = accumulate;
+  q->kb_per_split = kb_per_split;
+  const int rc = small_operand(&q->a, ta, a, trans_a != 0, m, k, lda, sa, q->inner, batch, (head_mask & 1) != 0, tsb_small::TILE_M, kb_per_split);
+  if (rc) return rc;
+  return small_operand(&q->b, tb, b, trans_b == 0, n, k, ldb, sb, q->inner, batch, (head_mask & 2) != 0, tsb_small::TILE_N, kb_per_split);
+}
+static int run_small(tsb_small::Product* q, const CUtensorMap* ta, const CUtensorMap* tb, int count, int splits, int trans_a,
+                     int trans_b, cudaStream_t st) {
+  int* status = tsb_host::status_word(st);
+  if (!status) return TSB_ERR_LAUNCH;
+  const cudaError_t e = tsb_small::run(q, ta, tb, count, splits, trans_a != 0, trans_b != 0, status, st);
+  if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
+  const int late = tsb_host::peek_status();
+  return late ? TSB_ERR_TIMEOUT | (late << 8) : TSB_OK;
+}
+
 // Fills in one product: tile width, K ranges, tensor maps.  group_bn: the width is given (a product of a group, which is
 // neither split nor run on CTA pairs; TSB_ERR_UNSUPPORTED for one that would be).
 static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorMap& tc, int& bn, bool& use_pair,
@@ -946,13 +1040,9 @@ static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorM
   p.sc2 = (long long)m * ldc;
   p.tiles_m = (m + BM - 1) / BM;
   p.tiles_n = (n + bn - 1) / bn;
-  p.kblocks = (k + BK - 1) / BK;
-  p.splits = choose_splits((long long)p.tiles_m * p.tiles_n * batch, p.kblocks, forced_splits);
-  if (p.splits > p.kblocks) p.splits = p.kblocks;
-  {   // no empty K ranges: re-derive the count from the per-split share
-    const int per = (p.kblocks + p.splits - 1) / p.splits;
-    p.splits = (p.kblocks + per - 1) / per;
-  }
+  const KRanges kr = k_ranges(m, n, k, batch, forced_splits);
+  p.kblocks = kr.kblocks;
+  p.splits = kr.splits;
   p.ws = nullptr;
   p.status = tsb_host::status_word(st);
   if (!p.status) return TSB_ERR_LAUNCH;
@@ -986,7 +1076,6 @@ static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorM
   }
   const uint32_t bbox = use_pair ? P2_BNH : (uint32_t)bn;   // columns of B that one CTA stages
   // tensor maps (dims innermost first)
-  p.a_chunked = p.b_chunked = 0;
   const uint64_t sab = (uint64_t)(batch > 1 ? sa : (long long)(trans_a ? k : m) * lda) * 4;
   const uint64_t sbb = (uint64_t)(batch > 1 ? sb : (long long)(trans_b ? n : k) * ldb) * 4;
   int rc = TSB_OK;
@@ -994,35 +1083,9 @@ static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorM
   const uint64_t outer = head_mask ? (uint64_t)(batch / heads) : 1;
   const uint64_t a_rows = a_heads ? outer : 1, a_bat = a_heads ? (uint64_t)heads : (uint64_t)batch;
   const uint64_t b_rows = b_heads ? outer : 1, b_bat = b_heads ? (uint64_t)heads : (uint64_t)batch;
-  if (!trans_a) {   // A[m][k], K contiguous -> K-major
-    uint64_t d[3] = {(uint64_t)k, (uint64_t)m * a_rows, a_bat}, s[2] = {(uint64_t)lda * 4, sab};
-    uint32_t bx[3] = {BK, BM, 1};
-    rc = tsb_host::make_tmap_f32(&ta, a, 3, d, s, bx);
-  } else if (m % 32 == 0) {   // A stored [k][m], M contiguous -> MN-major; all chunks of a stage in one box
-    uint64_t d[4] = {32, (uint64_t)k * a_rows, (uint64_t)m / 32, a_bat}, s[3] = {(uint64_t)lda * 4, 128, sab};
-    uint32_t bx[4] = {32, BK, BM / 32, 1};
-    rc = tsb_host::make_tmap_f32(&ta, a, 4, d, s, bx, true);
-    p.a_chunked = 1;
-  } else {
-    uint64_t d[3] = {(uint64_t)m, (uint64_t)k * a_rows, a_bat}, s[2] = {(uint64_t)lda * 4, sab};
-    uint32_t bx[3] = {32, BK, 1};
-    rc = tsb_host::make_tmap_f32(&ta, a, 3, d, s, bx, true);
-  }
+  rc = operand_map(&ta, &p.a_chunked, a, trans_a != 0, m, k, lda, a_rows, a_bat, sab, BM);
   if (rc) return rc;
-  if (trans_b) {    // B stored [n][k], K contiguous -> K-major
-    uint64_t d[3] = {(uint64_t)k, (uint64_t)n * b_rows, b_bat}, s[2] = {(uint64_t)ldb * 4, sbb};
-    uint32_t bx[3] = {BK, bbox, 1};
-    rc = tsb_host::make_tmap_f32(&tb, b, 3, d, s, bx);
-  } else if (n % 32 == 0) {   // B[k][n], N contiguous -> MN-major; all chunks of a stage in one box
-    uint64_t d[4] = {32, (uint64_t)k * b_rows, (uint64_t)n / 32, b_bat}, s[3] = {(uint64_t)ldb * 4, 128, sbb};
-    uint32_t bx[4] = {32, BK, bbox / 32, 1};
-    rc = tsb_host::make_tmap_f32(&tb, b, 4, d, s, bx, true);
-    p.b_chunked = 1;
-  } else {
-    uint64_t d[3] = {(uint64_t)n, (uint64_t)k * b_rows, b_bat}, s[2] = {(uint64_t)ldb * 4, sbb};
-    uint32_t bx[3] = {32, BK, 1};
-    rc = tsb_host::make_tmap_f32(&tb, b, 3, d, s, bx, true);
-  }
+  rc = operand_map(&tb, &p.b_chunked, b, trans_b == 0, n, k, ldb, b_rows, b_bat, sbb, bbox);
   if (rc) return rc;
   // C (or the split-K partial sums) as [outer][head or batch][row][column], where its strides allow a tensor map
   tc = ta;
@@ -1055,6 +1118,17 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
   if (heads < 0 || (heads > 0 && (batch % heads) != 0)) return TSB_ERR_ARG;
   if (heads == 0) head_mask = 0;
   const bool a_heads = (head_mask & 1) != 0, b_heads = (head_mask & 2) != 0, c_heads = (head_mask & 4) != 0;
+  if ((forced_splits == 0 || heads > 0) &&
+      !(head_mask && ((a_heads && lda % 4) || (b_heads && ldb % 4)))) {      // (refused below, whatever the size)
+    const KRanges kr = k_ranges(m, n, k, batch, heads > 0 ? 1 : 0);
+    if (small_form(kr, a, b) && is_small(tsb_small::blocks_of(m, n, batch, kr.splits), kr.per)) {
+      tsb_small::Product q = {};
+      CUtensorMap ta, tb;
+      const int rc = small_product(&q, &ta, &tb, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, batch, sa, sb, sc,
+                                   accumulate, heads, head_mask, kr.per);
+      return rc ? rc : run_small(&q, &ta, &tb, 1, kr.splits, trans_a, trans_b, st);
+    }
+  }
   if (head_mask) forced_splits = 1;       // the split-K scratch and its reduction address C by one batch stride
   const bool aligned = (lda % 4 == 0) && (ldb % 4 == 0) && (sa % 4 == 0) && (sb % 4 == 0) &&
                        ((reinterpret_cast<uintptr_t>(a) & 15) == 0) && ((reinterpret_cast<uintptr_t>(b) & 15) == 0);
@@ -1180,15 +1254,35 @@ int tsb_gemm_tf32_splitk(const float* a, const float* b, float* c, int m, int n,
 }
 
 // Up to 16 products C = op(A) op(B) of the same transposition as one launch.  TSB_ERR_UNSUPPORTED when one of them is no
-// candidate (needs padding, split-K or CTA pairs) or the tiles are more than two waves.
+// candidate (rows that TMA cannot read in a group that gemm_small.cu does not take, split-K, CTA pairs) or the tiles are
+// more than two waves.
 int tsb_gemm_tf32_group(int count, const float** a, const float** b, float** c, const int* m, const int* n, const int* k,
                         const long long* lda, const long long* ldb, const long long* ldc, int trans_a, int trans_b,
                         void* stream) {
   if (count < 1 || count > MAX_GROUP) return TSB_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   long long wide = 0;
+  long long blocks = 0;
+  int longest = 1;
+  bool small = true;
   for (int i = 0; i < count; ++i) {
     if (m[i] <= 0 || n[i] <= 0 || k[i] <= 0) return TSB_ERR_ARG;
+    const KRanges kr = k_ranges(m[i], n[i], k[i], 1, 0);
+    small = small && kr.splits == 1 && small_form(kr, a[i], b[i]);
+    blocks += tsb_small::blocks_of(m[i], n[i], 1, 1);
+    if (kr.per > longest) longest = kr.per;
+  }
+  if (small && is_small(blocks, longest)) {
+    tsb_small::Product q[MAX_GROUP] = {};
+    CUtensorMap ta[MAX_GROUP], tb[MAX_GROUP];
+    for (int i = 0; i < count; ++i) {
+      const int rc = small_product(&q[i], &ta[i], &tb[i], a[i], b[i], c[i], m[i], n[i], k[i], lda[i], ldb[i], ldc[i], trans_a,
+                                   trans_b, 1, 0, 0, 0, 0, 0, 0, (k[i] + BK - 1) / BK);
+      if (rc) return rc;
+    }
+    return run_small(q, ta, tb, count, 1, trans_a, trans_b, st);
+  }
+  for (int i = 0; i < count; ++i) {
     if ((lda[i] | ldb[i]) % 4 || ((reinterpret_cast<uintptr_t>(a[i]) | reinterpret_cast<uintptr_t>(b[i])) & 15))
       return TSB_ERR_UNSUPPORTED;
     wide += (((long long)m[i] + BM - 1) / BM) * ((n[i] + 2 * GROUP_BN - 1) / (2 * GROUP_BN));
