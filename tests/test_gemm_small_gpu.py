@@ -60,6 +60,21 @@ def test_bits_of_the_general_path(m, n, k, ta, tb):
     assert lib.tsb_device_status(_stream()) == 0
 
 
+def test_no_store_behind_the_columns_of_the_general_path():
+    lib = _lib()
+    m, n, k, ldc = 300, 1023, 64, 1024                         # more tiles than are resident at once
+    a, b, c = _matrix(m, k, k, 1), _matrix(n, k, k, 2), _matrix(m, n, ldc, 3)
+    before = c.clone()
+    a, m = a.repeat(8, 1), 8 * m
+    c, before = c.repeat(8, 1), before.repeat(8, 1)
+    rc = lib.tsb_gemm_tf32(PTR(a.data_ptr()), PTR(b.data_ptr()), PTR(c.data_ptr()), m, n, k, I64(k), I64(k), I64(ldc), 0, 1, 1,
+                           I64(0), I64(0), I64(0), 0, _stream())
+    assert rc == 0
+    assert torch.equal(c[:, n:], before[:, n:])
+    ref = a.double() @ b.double().t()
+    assert (c[:, :n].double() - ref).norm() < 1e-3 * ref.norm()          # operands are cut to 10 bits
+
+
 @pytest.mark.parametrize("heads,rows,keys,d", [(4, 37, 30, 32), (2, 64, 64, 64), (3, 7, 33, 32)])
 def test_batches_and_head_layout(heads, rows, keys, d):
     """Scores and context of attention: every matrix has the bits of the same product by itself."""
