@@ -50,3 +50,12 @@ def test_average_gradient_without_overlap(n, c, h, w, kh, kw, stride):
     dx = _arr(torch.full((n, c, h, w), 7.0, device="cuda"))
     G.pool_grad(1, None, None, _arr(dy), dx, kh, kw, 0, stride, _stream())
     torch.testing.assert_close(dx.t.double(), ref, rtol=2 ** -22, atol=0)       # one product by a rounded 1 / (kh * kw)
+
+
+@pytest.mark.parametrize("n,c,h,w", [(1, 1, 1, 1), (1, 3, 32, 32), (3, 2, 11, 31), (1, 3, 5, 205), (2, 3, 64, 64)])
+def test_pixels_of_four_channels(n, c, h, w):
+    """One pixel; exactly a block; one pixel more than a block; other remainders."""
+    x = _arr(_rand(n, c, h, w))
+    y = _arr(torch.full((n, 4, h, w), 7.0, device="cuda"))
+    G._to_pixels(x, y, _stream())
+    assert torch.equal(y.t[:, :c], x.t) and not y.t[:, c:].any()

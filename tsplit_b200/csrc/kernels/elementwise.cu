@@ -253,6 +253,31 @@ __global__ void copy_tiled(const float* x, float* __restrict__ y, long long oute
   }
 }
 
+// Pixels of c < 4 channels to pixels of four, zeros behind the c-th: the layout that the convolutions of RGB images read.
+// A block moves 1024 pixels through shared memory, so that reads and the 16-byte writes of a warp are whole lines, with
+// all of a thread's reads in flight.  Bound by DRAM.  32 x 224 x 224 x 3 (45 MB): 21.7 us as a strided copy -> 5.9.
+__global__ void __launch_bounds__(256) pack_pixels(const float* x, float4* __restrict__ y, const int c,
+                                                   const long long pixels) {
+  tsb_launch::enter();
+  __shared__ float sh[3 * 1024];
+  const long long first = blockIdx.x * 1024ll, end = pixels * c;
+  float v[12];
+#pragma unroll
+  for (int u = 0; u < 12; ++u) {
+    const long long i = first * c + u * 256 + threadIdx.x;
+    v[u] = u < 4 * c && i < end ? x[i] : 0.f;
+  }
+#pragma unroll
+  for (int u = 0; u < 12; ++u) sh[u * 256 + threadIdx.x] = v[u];
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int q = u * 256 + threadIdx.x;
+    if (first + q < pixels)
+      y[first + q] = make_float4(sh[q * c], c > 1 ? sh[q * c + 1] : 0.f, c > 2 ? sh[q * c + 2] : 0.f, 0.f);
+  }
+}
+
 template <int OP>
 __global__ void binary_strided(const float* p, const float* q, float* __restrict__ y,
                                const Dims d, long long n) {
@@ -521,6 +546,15 @@ dim3 rows_grid(long long outer, int inner) {
   case OPC: tsb_launch::launch(binary_strided<OPC>, grid, 256, 0, st, a, b, y, d, n); break;
 
 extern "C" {
+
+// y[pixels][4] <- x[pixels][c], zeros in the channels from c on; c < 4.
+int tsb_pack_pixels(const float* x, float* y, int c, long long pixels, void* stream) {
+  if (pixels <= 0) return TSB_OK;
+  if (c < 1 || c > 3 || pixels >= (1ll << 40) || (reinterpret_cast<uintptr_t>(y) & 15)) return TSB_ERR_UNSUPPORTED;
+  tsb_launch::launch(pack_pixels, (unsigned)((pixels + 1023) / 1024), 256, 0, static_cast<cudaStream_t>(stream), x,
+                     reinterpret_cast<float4*>(y), c, pixels);
+  return done();
+}
 
 int tsb_ew_unary(int op, const float* x, float* y, long long n, float alpha, void* stream) {
   if (n <= 0) return TSB_OK;

@@ -566,6 +566,18 @@ def _padded(arr, c4, tag):
     return buf
 
 
+def _to_pixels(x, x4, stream):
+    """``x`` into the first channels of its padded copy."""
+    n, c, h, w = x.shape
+    if x.is_channels_last() and c < 4:
+        rc = lib().tsb_pack_pixels(_p(x), _p(x4), c_int(c), c_int64(n * h * w), _s(stream))
+        if rc == 0:
+            return
+        if rc != 2:      # 2: sizes that the strided copy takes
+            _check(rc, "pack_pixels")
+    copy_raw(x.ptr, x.strides, x4.ptr, x4.strides, x.shape, stream)
+
+
 def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
     """Input-channel count not a multiple of 4 (the RGB stem): run the kernel on
     zero-padded copies of x and w; only the real channels are copied back.
@@ -581,7 +593,7 @@ def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
     x4, w4 = _padded(x, c4, "x"), _padded(w, c4, "w")
     xs, ws = x4.strides, w4.strides
     if kind in (0, 2):
-        copy_raw(x.ptr, x.strides, x4.ptr, xs, x.shape, stream)
+        _to_pixels(x, x4, stream)
     if kind in (0, 1):
         copy_raw(w.ptr, w.strides, w4.ptr, ws, w.shape, stream)
     conv2d(kind, x4, w4, y, ph, pw, stride, stream)
@@ -603,7 +615,7 @@ def _conv2d_packed_stem(kind, x, w, y, ph, pw, stream):
     o, _, kh, kw = w.shape
     _, _, oh, ow = y.shape
     x4 = _padded(x, 4, "x")
-    copy_raw(x.ptr, x.strides, x4.ptr, x4.strides, x.shape, stream)
+    _to_pixels(x, x4, stream)
     key = ("stem_w", (o, kh), x.ctx.device_id)
     packed = _PAD_CACHE.get(key)
     if packed is None:
