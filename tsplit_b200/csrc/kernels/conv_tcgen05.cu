@@ -44,6 +44,7 @@ struct ConvParams {
   float* out;
   float* ws;
   int N, C, H, W, O, KH, KW, OH, OW, ph, pw, stride;
+  int step_w;          // wgrad by TMA: positions of the patch tensor along W per output pixel (the stride, but for strided stems)
   int M;               // GEMM rows
   int NC;              // GEMM columns of one column group
   int K;               // fwd: KH*KW*C
@@ -274,7 +275,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
               tma_load_2d(smem_a + s * A_STAGE_BYTES + c * (BK * 128), &tm, &full[s], w.m0 + c * 32, kb * BK);
           }
         }
-        const int bw = ox * p.stride - p.pw, bh = oy * p.stride - p.ph;
+        const int bw = ox * p.step_w - p.pw, bh = oy * p.stride - p.ph;
 #pragma unroll
         for (int u = 0; u < 2; ++u)
           if (cv[u])
@@ -1402,7 +1403,7 @@ ConvParams base_params(int N, int C, int H, int W, int O, int KH, int KW, int OH
                        int stride) {
   ConvParams p;
   p.N = N; p.C = C; p.H = H; p.W = W; p.O = O; p.KH = KH; p.KW = KW; p.OH = OH; p.OW = OW;
-  p.ph = ph; p.pw = pw; p.stride = stride;
+  p.ph = ph; p.pw = pw; p.stride = p.step_w = stride;
   p.src = nullptr; p.out = nullptr; p.ws = nullptr; p.accumulate = 0; p.splits = 1; p.taps = 1;
   p.K = KH * KW * C; p.ocb = (O + 31) / 32; p.status = nullptr; p.prof = nullptr; p.a3d = 0; p.tma_store = 0; p.stats = nullptr; p.stats_plane = 0;
   p.M = 0; p.NC = 0; p.kblocks = 0; p.tiles_m = 0; p.tiles_n = 0; p.ldc = 0;
@@ -1508,6 +1509,38 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
   }
   if (rc != TSB_ERR_UNSUPPORTED) return rc;
   return launch_bn<0, false>(bn, tm, tm, tmo, p, st);
+}
+
+// K ranges of a filter gradient: its pixel reduction is split so that the work items fill whole waves of CTAs (or pairs).
+int wgrad_splits(long long tiles, int sms, int kblocks) {
+  int splits = 1;
+  double best_eff = 0.0;
+  for (int waves = 1; waves <= 4; ++waves) {
+    int sp = (int)((long long)waves * sms / tiles);
+    if (sp < 1) sp = 1;
+    if (sp > kblocks / 4) sp = kblocks / 4 > 0 ? kblocks / 4 : 1;
+    if (sp > 64) sp = 64;
+    const long long items = tiles * sp;
+    const double eff = (double)items / (double)(((items + sms - 1) / sms) * sms);
+    // prefer more waves only when they are clearly better balanced (each split costs a partial-sum pass)
+    if (eff > best_eff + 0.04) { best_eff = eff; splits = sp; }
+  }
+  return splits;
+}
+
+// Filter gradient of a strided stem (see tsb_stem_wgrad): sum of the K ranges, and from windows of eight pixels to taps.
+__global__ void __launch_bounds__(256) stem_window_grads(const float4* ws, int splits, float* __restrict__ dw, long long so,
+                                                         long long sc, long long sh, long long sw, int O, int C, int KH, int KW) {
+  tsb_launch::enter();
+  const int i = blockIdx.x * 256 + threadIdx.x, per_split4 = O * KH * 8;
+  if (i >= per_split4 || (i & 7) >= KW) return;
+  const float4 v = sum_splits(ws + i, splits, per_split4);
+  const int kw = i & 7, kh = (i >> 3) % KH, o = (i >> 3) / KH;
+  float* dst = dw + o * so + kh * sh + kw * sw;
+  dst[0] = v.x;
+  if (C > 1) dst[sc] = v.y;
+  if (C > 2) dst[2 * sc] = v.z;
+  if (C > 3) dst[3 * sc] = v.w;
 }
 
 // dx[N,H,W,C] = stride-2 dgrad(dy[N,OH,OW,O], w[O,KH,KW,C]) by parity classes (see parity_filters).
@@ -1669,22 +1702,9 @@ int tsb_conv2d(int kind, float* x, float* w, float* y, int N, int C, int H, int 
       const char* e = getenv("TSB_CONV_PAIR");
       use_pair = !(e && e[0] == '0') && p.a3d && O >= 256 && bn == 256;
     }
-    // split the pixel reduction so that the work items fill whole waves of CTAs (or CTA pairs)
     const long long tiles = use_pair ? (long long)((p.M + 255) / 256) * ((p.NC + P2_BN - 1) / P2_BN)
                                      : (long long)p.tiles_m * p.tiles_n * p.taps;
-    const int sms = use_pair ? sm_count() / 2 : sm_count();
-    int splits = 1;
-    double best_eff = 0.0;
-    for (int waves = 1; waves <= 4; ++waves) {
-      int sp = (int)((long long)waves * sms / tiles);
-      if (sp < 1) sp = 1;
-      if (sp > p.kblocks / 4) sp = p.kblocks / 4 > 0 ? p.kblocks / 4 : 1;
-      if (sp > 64) sp = 64;
-      const long long items = tiles * sp;
-      const double eff = (double)items / (double)(((items + sms - 1) / sms) * sms);
-      // prefer more waves only when they are clearly better balanced (each split costs a partial-sum pass)
-      if (eff > best_eff + 0.04) { best_eff = eff; splits = sp; }
-    }
+    const int splits = wgrad_splits(tiles, use_pair ? sm_count() / 2 : sm_count(), p.kblocks);
     const int per = (p.kblocks + splits - 1) / splits;
     p.splits = (p.kblocks + per - 1) / per;
     if (p.splits > 1) {
@@ -1751,6 +1771,67 @@ int tsb_stem_pack_filters(const float* w, long long so, long long sc, long long 
                      so, sc, sh, sw, packed, O, C, KH, KW, pw);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
+}
+
+// Filter gradient of a few-channel convolution of stride > 1 with KH, KW <= 8 (the 7x7 stride-2 stem):
+//   dw[o][c][kh][kw] = sum over output pixels of dy[n][oh][ow][o] * x[n][oh * s - ph + kh][ow * s - pw + kw][c]
+// x is packed to four channels in rows of Wp pixels that begin pw pixels in front of the image, zeros around it
+// (tsb_pack_pixel_rows).  The eight pixels from ow * s on are 32 consecutive floats, so for the TMA unit this is a KH x 1
+// convolution over 32 channels whose positions along a row are s pixels apart and overlap: the patch operand comes as
+// im2col boxes like that of any wide convolution, where the gather path copies 16 bytes at a time.  Pixels and K ranges
+// are taken in the same order as there, so the sums are the same bits.  7x7 stride 2 over 32 x 224 x 224, 64 filters:
+// 170.9 us gathered (64 SMs, bound by the copying warps' instructions) -> 83.7.
+// dw is addressed through element strides (output channel, input channel, kh, kw).
+int tsb_stem_wgrad(const float* xp, const float* dy, float* dw, long long so, long long sc, long long sh, long long sw, int N,
+                   int C, int H, int Wp, int O, int KH, int KW, int OH, int OW, int ph, int stride, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (N <= 0 || stride <= 0 || C < 1 || C > 4) return TSB_ERR_ARG;
+  if (KH > 8 || KW > 8 || O % 4 || (OW - 1) * stride + 8 > Wp || H + 2 * ph < KH || (H + 2 * ph - KH) / stride + 1 != OH ||
+      ((reinterpret_cast<uintptr_t>(xp) | reinterpret_cast<uintptr_t>(dy)) & 15))
+    return TSB_ERR_UNSUPPORTED;
+  if ((long long)N * OH * OW >= (1ll << 31) || (long long)N * H * Wp * 16 < (128 << 10) || (long long)N * H * OW * 128 < (128 << 10))
+    return TSB_ERR_UNSUPPORTED;      // (im2col maps of small tensors: see make_tmap_im2col_f32)
+  const int lower[2] = {0, -ph}, upper[2] = {0, ph - (KH - 1)};
+  const uint64_t strides[3] = {(uint64_t)stride * 16, (uint64_t)Wp * 16, (uint64_t)H * Wp * 16};
+  CUtensorMap tm, tmi;
+  int rc = tsb_host::make_tmap_im2col_f32(&tmi, xp, 32, OW, H, N, lower, upper, 32, BK, 1, stride, true, strides);
+  if (rc) return rc;
+  ConvParams p = base_params(N, 32, H, OW, O, KH, 1, OH, OW, ph, 0, stride);
+  p.step_w = 1;
+  p.status = tsb_host::status_word(st);
+  if (!p.status) return TSB_ERR_LAUNCH;
+  const long long mpix = (long long)N * OH * OW;
+  p.M = O; p.NC = KH * 32; p.ldc = p.NC;
+  p.kblocks = (int)((mpix + BK - 1) / BK);
+  p.tiles_m = (O + BM - 1) / BM;
+  if (O % 32 == 0) {
+    uint64_t d[3] = {32, (uint64_t)mpix, (uint64_t)O / 32}, s[2] = {(uint64_t)O * 4, 128};
+    uint32_t bx[3] = {32, BK, BM / 32};
+    rc = tsb_host::make_tmap_f32(&tm, dy, 3, d, s, bx, true);
+    p.a3d = 1;
+  } else {
+    uint64_t d[2] = {(uint64_t)O, (uint64_t)mpix}, s[1] = {(uint64_t)O * 4};
+    uint32_t bx[2] = {32, BK};
+    rc = tsb_host::make_tmap_f32(&tm, dy, 2, d, s, bx, true);
+  }
+  if (rc) return rc;
+  const int splits = wgrad_splits(p.tiles_m, sm_count(), p.kblocks);      // (of whole column tiles, as the gather path)
+  const int per = (p.kblocks + splits - 1) / splits;
+  p.splits = (p.kblocks + per - 1) / per;
+  p.ws = get_ws(st, 0, (size_t)p.splits * O * p.NC * sizeof(float), size_t(128) << 20);
+  if (!p.ws) return TSB_ERR_OOM;
+  p.out = p.ws;
+  // half the columns per CTA where that puts idle SMs to work: a k-block is bound by what one SM takes from L2
+  const int bn = tsb_host::narrow_tile(p.NC > 128 ? 256 : (p.NC > 64 ? 128 : 64), (long long)p.tiles_m * p.splits, sm_count());
+  p.tiles_n = (p.NC + bn - 1) / bn;
+  rc = launch_bn<2, true>(bn, tm, tmi, tm, p, st);
+  if (rc) return rc;
+  tsb_launch::launch(stem_window_grads, (unsigned)((O * KH * 8 + 255) / 256), 256, 0, st, reinterpret_cast<const float4*>(p.ws),
+                     p.splits, dw, so, sc, sh, sw, O, C, KH, KW);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
+  const int late = tsb_host::peek_status();
+  return late ? TSB_ERR_TIMEOUT | (late << 8) : TSB_OK;
 }
 
 int tsb_stem_unpack_filter_grads(const float* packed, float* dw, long long so, long long sc, long long sh,

@@ -278,6 +278,25 @@ __global__ void __launch_bounds__(256) pack_pixels(const float* x, float4* __res
   }
 }
 
+// The same into rows of `wp` pixels with the image from pixel `left` on and zeros around it: windows of pixels that begin
+// in front of a row or end behind it then read zeros.  32 x 224 x 224 x 3 into rows of 230: 9.0 us from DRAM.
+__global__ void __launch_bounds__(256) pack_pixel_rows(const float* x, float4* __restrict__ y, const int c, const unsigned w,
+                                                       const unsigned wp, const unsigned left, const long long pixels) {
+  tsb_launch::enter();
+  float v[4][3];
+  const long long i0 = blockIdx.x * 1024ll + threadIdx.x;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const long long i = i0 + u * 256, row = (pixels >> 32) == 0 ? (unsigned)i / wp : i / wp;
+    const unsigned at = (unsigned)(i - row * wp) - left;           // (wraps around in front of the image)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[u][k] = k < c && i < pixels && at < w ? x[(row * w + at) * c + k] : 0.f;
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (i0 + u * 256 < pixels) y[i0 + u * 256] = make_float4(v[u][0], v[u][1], v[u][2], 0.f);
+}
+
 template <int OP>
 __global__ void binary_strided(const float* p, const float* q, float* __restrict__ y,
                                const Dims d, long long n) {
@@ -553,6 +572,17 @@ int tsb_pack_pixels(const float* x, float* y, int c, long long pixels, void* str
   if (c < 1 || c > 3 || pixels >= (1ll << 40) || (reinterpret_cast<uintptr_t>(y) & 15)) return TSB_ERR_UNSUPPORTED;
   tsb_launch::launch(pack_pixels, (unsigned)((pixels + 1023) / 1024), 256, 0, static_cast<cudaStream_t>(stream), x,
                      reinterpret_cast<float4*>(y), c, pixels);
+  return done();
+}
+
+// The same for rows of w pixels into rows of wp, the image from pixel `left` on.
+int tsb_pack_pixel_rows(const float* x, float* y, int c, long long rows, int w, int wp, int left, void* stream) {
+  if (rows <= 0 || w <= 0) return TSB_OK;
+  if (c < 1 || c > 3 || left < 0 || wp < left + w || rows >= (1ll << 24) || wp >= (1 << 16) || (reinterpret_cast<uintptr_t>(y) & 15))
+    return TSB_ERR_UNSUPPORTED;
+  const long long pixels = rows * wp;
+  tsb_launch::launch(pack_pixel_rows, (unsigned)((pixels + 1023) / 1024), 256, 0, static_cast<cudaStream_t>(stream), x,
+                     reinterpret_cast<float4*>(y), c, (unsigned)w, (unsigned)wp, (unsigned)left, pixels);
   return done();
 }
 

@@ -703,7 +703,8 @@ int make_tmap_f32_swz(CUtensorMap* out, const void* base, int rank, const uint64
 }
 
 int make_tmap_im2col_f32(CUtensorMap* out, const void* base, int C, int W, int H, int N, const int* lower,
-                         const int* upper, int channels, int pixels, int stride_w, int stride_h, bool atom32) {
+                         const int* upper, int channels, int pixels, int stride_w, int stride_h, bool atom32,
+                         const uint64_t* strides_b) {
   typedef CUresult (*EncodeIm2colFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                      const cuuint64_t*, const int*, const int*, cuuint32_t, cuuint32_t,
                                      const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -723,7 +724,7 @@ int make_tmap_im2col_f32(CUtensorMap* out, const void* base, int C, int W, int H
   for (int i = 0; i < 2; ++i)
     if (lower[i] < -128 || lower[i] > 127 || upper[i] < -128 || upper[i] > 127) return TSB_ERR_UNSUPPORTED;
   struct Key {
-    const void* base; int v[13];
+    const void* base; uint64_t s[3]; int v[13];
     bool operator==(const Key& o) const { return std::memcmp(this, &o, sizeof(Key)) == 0; }
   };
   struct Hash {
@@ -739,6 +740,9 @@ int make_tmap_im2col_f32(CUtensorMap* out, const void* base, int C, int W, int H
   Key key;
   std::memset(&key, 0, sizeof(key));
   key.base = base;
+  const uint64_t dense[3] = {(uint64_t)C * 4, (uint64_t)W * C * 4, (uint64_t)H * W * C * 4};
+  if (!strides_b) strides_b = dense;
+  for (int i = 0; i < 3; ++i) key.s[i] = strides_b[i];
   const int vals[13] = {C, W, H, N, lower[0], lower[1], upper[0], upper[1], channels, pixels, stride_w, stride_h,
                         atom32 ? 1 : 0};
   std::memcpy(key.v, vals, sizeof(vals));
@@ -748,7 +752,7 @@ int make_tmap_im2col_f32(CUtensorMap* out, const void* base, int C, int W, int H
     if (it != cache.end()) { *out = it->second; return TSB_OK; }
   }
   cuuint64_t gd[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-  cuuint64_t gs[3] = {(cuuint64_t)C * 4, (cuuint64_t)W * C * 4, (cuuint64_t)H * W * C * 4};
+  cuuint64_t gs[3] = {strides_b[0], strides_b[1], strides_b[2]};
   cuuint32_t es[4] = {1, (cuuint32_t)stride_w, (cuuint32_t)stride_h, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), gd, gs, lower, upper,
                   (cuuint32_t)channels, (cuuint32_t)pixels, es, CU_TENSOR_MAP_INTERLEAVE_NONE,

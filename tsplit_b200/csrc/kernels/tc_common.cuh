@@ -389,8 +389,10 @@ int make_tmap_f32_swz(CUtensorMap* out, const void* base, int rank, const uint64
 // `pixels` rows of `channels` floats (128-byte rows, 128B swizzle; atom32 as above).  lower/upper
 // are the bounding-box corners in (W, H) order: base positions run from lower to dim-1+upper in
 // steps of `stride`.  Corners must lie in [-128, 127].
+// strides_b: bytes between positions along W, H and N, where they are not those of a dense tensor (positions may overlap).
 int make_tmap_im2col_f32(CUtensorMap* out, const void* base, int C, int W, int H, int N, const int* lower,
-                         const int* upper, int channels, int pixels, int stride_w, int stride_h, bool atom32);
+                         const int* upper, int channels, int pixels, int stride_w, int stride_h, bool atom32,
+                         const uint64_t* strides_b = nullptr);
 
 int* status_word(cudaStream_t stream);   // zeroed device int used by bounded waits (per device)
 int read_status(cudaStream_t stream);    // sync + read + reset; 0 when clean

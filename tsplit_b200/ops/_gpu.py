@@ -590,6 +590,8 @@ def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
     c4 = (c + 3) // 4 * 4
     if kind in (0, 2) and _packed_stem_ok(x, w, y, c4, pw, stride):
         return _conv2d_packed_stem(kind, x, w, y, ph, pw, stream)
+    if kind == 2 and stride > 1 and _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
+        return
     x4, w4 = _padded(x, c4, "x"), _padded(w, c4, "w")
     xs, ws = x4.strides, w4.strides
     if kind in (0, 2):
@@ -601,6 +603,32 @@ def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
         copy_raw(x4.ptr, xs, x.ptr, x.strides, x.shape, stream)
     elif kind == 2:
         copy_raw(w4.ptr, ws, w.ptr, w.strides, w.shape, stream)
+
+
+def _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
+    """Filter gradient of a strided few-channel stem through TMA windows of eight pixels (``tsb_stem_wgrad``); False for
+    a shape it does not cover."""
+    from .. import ndarray
+    n, c, h, wd = x.shape
+    o, _, kh, kw = w.shape
+    _, _, oh, ow = y.shape
+    if c > 3 or kh > 8 or kw > 8 or o % 4 or not x.is_channels_last():
+        return False
+    wp = max((ow - 1) * stride + 8, wd + pw)
+    key = ("windows", (n, h, wp), x.ctx.device_id)
+    xp = _PAD_CACHE.get(key)
+    if xp is None:
+        xp = _PAD_CACHE[key] = ndarray.empty((n * h * wp * 4,), x.ctx, use_pool=False)
+    rc = lib().tsb_pack_pixel_rows(_p(x), _p(xp), c_int(c), c_int64(n * h), c_int(wd), c_int(wp), c_int(pw), _s(stream))
+    if rc == 0:
+        so, sc, sh, sw = w.strides
+        rc = lib().tsb_stem_wgrad(_p(xp), _p(y), _p(w), c_int64(so), c_int64(sc), c_int64(sh), c_int64(sw), c_int(n), c_int(c),
+                                  c_int(h), c_int(wp), c_int(o), c_int(kh), c_int(kw), c_int(oh), c_int(ow), c_int(ph),
+                                  c_int(stride), _s(stream))
+    if rc == 2:          # a size that the gather path takes
+        return False
+    _check(rc, "stem_wgrad")
+    return True
 
 
 def _packed_stem_ok(x, w, y, c4, pw, stride):
