@@ -193,7 +193,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // uniform for the compiler
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -296,7 +296,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
     if (IM2COL && MODE == 0) {
       // forward with both operands by TMA: one im2col box (128 pixels x 32 channels of one filter
       // tap) and one weight box per k-block; k runs over (tap, 32-channel block)
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t it = 0;
         bool ok = true;
         PROF_DECL(tw); PROF_DECL(tt);
@@ -331,8 +331,8 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
         if (!ok) for (int i = 0; i < 64; ++i) __nanosleep(1000);
       }
     } else if (IM2COL && MODE == 2) {
-      if (lane == 0) wgrad_producer(0);
-    } else if (lane == 0) {
+      if (elect_one()) wgrad_producer(0);
+    } else if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       PROF_DECL(tw); PROF_DECL(tt);
@@ -366,7 +366,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr int A_MN = (MODE == 2) ? 1 : 0;
       constexpr int B_MN = (MODE == 0) ? 0 : 1;
       constexpr uint32_t idesc = make_idesc_tf32(BM, BN, A_MN, B_MN);
@@ -378,7 +378,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
       const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem_a), A_MN ? BK * 128 : 16);
       const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem_b), B_MN ? BK * 128 : 16);
       uint32_t it = 0, acc_it = 0;
-      bool ok = true, ready = false;
+      bool ok = true;
       PROF_DECL(mf); PROF_DECL(me); PROF_DECL(mi); PROF_DECL(mt); PROF_DECL(mm); PROF_DECL(mc);
       PROF_BEGIN(mt);
       for (long long item = blockIdx.x; item < items && ok; item += gridDim.x, ++acc_it) {
@@ -394,13 +394,9 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
           const int s = it % C::STAGES;
           const uint32_t ph = (it / C::STAGES) & 1;
           PROF_BEGIN(mf);
-          if (!ready && !mbar_wait(&full[s], ph, p.status, 0x203)) { ok = false; break; }
+          if (!mbar_wait(&full[s], ph, p.status, 0x203)) { ok = false; break; }
           PROF_END(mf);
           PROF_BEGIN(mi);
-          {   // probe the next stage now; the answer arrives while this stage's MMAs are issued
-            const uint32_t it2 = it + 1;
-            ready = mbar_test(&full[it2 % C::STAGES], (it2 / C::STAGES) & 1);
-          }
           tc_fence_after();
           const uint32_t a_lo = a_lo0 + s * (A_STAGE_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + s * (C::B_STAGE_BYTES >> 4);
@@ -522,7 +518,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
     if (warp == 2 && lane == 0) { PROF_FLUSH(11, ew); PROF_FLUSH(12, et); }
   } else if (IM2COL) {
     // ---------------------------------------------------------------- extra TMA producers (wgrad only)
-    if (MODE == 2 && lane == 0) wgrad_producer(warp - 5);
+    if (MODE == 2 && elect_one()) wgrad_producer(warp - 5);
   } else {
     // ---------------------------------------------------------------- gather producers (warps 6..)
     // The loop over k-blocks is kept short on purpose: with few warps per scheduler the chain of
@@ -774,7 +770,7 @@ conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // uniform for the compiler
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -809,7 +805,7 @@ conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       const int cpb = p.C >> 5;
@@ -839,7 +835,7 @@ conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_tf32(256, BN, 0, 0);
       constexpr uint32_t HI = smem_desc_hi(1024);
       constexpr uint32_t KSTEP = (UMMA_K * 4) >> 4;
@@ -951,7 +947,7 @@ conv_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // uniform for the compiler
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -1026,10 +1022,10 @@ conv_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
   };
 
   if (warp == 0) {
-    if (lane == 0) producer(0);
+    if (elect_one()) producer(0);
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_tf32(256, P2_BN, 1, 1);
       constexpr uint32_t HI = smem_desc_hi(512, LAYOUT_SW128_BASE32B);
       constexpr uint32_t KSTEP = 1024 >> 4;
@@ -1101,7 +1097,7 @@ conv_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
       if (lane == 0) mbar_arrive_leader(&tempty[acc]);
     }
   } else {
-    if (lane == 0) producer(warp - 5);      // warps 6, 7, 8: patch chunks 1, 2, 3
+    if (elect_one()) producer(warp - 5);      // warps 6, 7, 8: patch chunks 1, 2, 3
   }
 
   tc_fence_before();
@@ -1466,8 +1462,7 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
     const char* e = getenv("TSB_CONV_PAIR");              // "0" selects the one-CTA tiles everywhere
     const int ptn = (p.NC + bn - 1) / bn;
     const long long pair_items = (long long)((p.M + 255) / 256) * ptn;
-    // narrow tiles measured slower on pairs (one CTA per SM, one issuing thread per two SMs) than on the
-    // one-CTA kernel with two CTAs per SM: 64 -> 64 channels at 224x224, batch 64: 0.90 ms against 0.61 ms
+    // (narrow tiles stay on the one-CTA kernel, whose column statistics come in twice as many chunks)
     if (!(e && e[0] == '0') && bn == 256 && pair_items * 4 >= sm_count()) {
       CUtensorMap tmh;          // filters, bn / 2 rows per CTA
       uint32_t hb[2] = {BK, (uint32_t)bn / 2};

@@ -144,7 +144,7 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // uniform for the compiler
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -176,7 +176,7 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (long long item = first; item < last && ok; item += step) {
@@ -225,7 +225,7 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_tf32(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       // descriptor halves: K-major operands step 32 bytes per MMA inside the 128B swizzle row,
       // MN-major ones (32-byte-atom swizzle, chunks of 32 columns BK*128 bytes apart) 1024 bytes
@@ -235,7 +235,7 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
       const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem_a), A_MN ? BK * 128 : 16);
       const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem_b), B_MN ? BK * 128 : 16);
       uint32_t it = 0, acc_it = 0;
-      bool ok = true, ready = false;
+      bool ok = true;
       for (long long item = first; item < last && ok; item += step, ++acc_it) {
         const long long rest = item / tiles;
         const int split = (int)(rest / p.batch);
@@ -249,11 +249,7 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % C::STAGES;
           const uint32_t ph = (it / C::STAGES) & 1;
-          if (!ready && !mbar_wait(&full[s], ph, p.status, 0x103)) { ok = false; break; }
-          {   // probe the next stage now; the answer arrives while this stage's MMAs are issued
-            const uint32_t it2 = it + 1;
-            ready = mbar_test(&full[it2 % C::STAGES], (it2 / C::STAGES) & 1);
-          }
+          if (!mbar_wait(&full[s], ph, p.status, 0x103)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_lo = a_lo0 + s * (A_STAGE_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + s * (C::B_STAGE_BYTES >> 4);
@@ -407,7 +403,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // uniform for the compiler
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();           // 0 = leader
   const long long pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -443,7 +439,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (long long item = pair; item < items && ok; item += npairs) {
@@ -472,7 +468,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_tf32(256, P2_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       constexpr uint32_t A_HI = A_MN ? smem_desc_hi(512, LAYOUT_SW128_BASE32B) : smem_desc_hi(1024);
       constexpr uint32_t B_HI = B_MN ? smem_desc_hi(512, LAYOUT_SW128_BASE32B) : smem_desc_hi(1024);
