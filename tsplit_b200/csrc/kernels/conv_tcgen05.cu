@@ -62,13 +62,15 @@ struct ConvParams {
   unsigned long long* prof;   // role-time counters (only written when built with -DTSB_CONV_PROF)
 };
 
-// Narrow tiles (BN <= 128) of the TMA-only kernels run two CTAs per SM: a stage's four MMAs cost
-// the single issuing thread about as much time for a 64-wide tile as for a 256-wide one, so a second
-// CTA's issue thread fills the tensor pipe that one CTA leaves idle.  Each of the two gets half the
-// stages (2 x ~97 KB of shared memory) and its own TMEM columns (2 x 128 or 2 x 256 of 512).
-template <int BN, bool IM2COL>
+// Narrow tiles (BN <= 128) of the TMA-only kernels run two CTAs per SM where there are more tiles than SMs: one's epilogue
+// and waits are covered by the other.  Each of the two gets half the stages (2 x ~97 KB of shared memory) and its own TMEM
+// columns (2 x 128 or 2 x 256 of 512).  A launch of no more tiles than SMs (OCC = 1) has all the stages for its one CTA: with
+// three of them a TMA round trip was not covered.  3x3 256 -> 256 at 14 x 14, batch 32: 22.5 -> 17.6 us; 1x1 1024 -> 256 there:
+// 13.1 -> 11.1; the stem's filter gradient (128 CTAs): 79.3 -> 59.5.
+constexpr int max_ctas(int bn, bool im2col) { return im2col && bn <= 128 ? 2 : 1; }
+template <int BN, bool IM2COL, int CTAS>
 struct Cfg {
-  static constexpr int OCC = (IM2COL && BN <= 128) ? 2 : 1;       // CTAs per SM
+  static constexpr int OCC = CTAS;                                // CTAs per SM
   static constexpr int B_STAGE_BYTES = BN * BK * 4;
   static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   static constexpr int STAGES = ((BN == 256) ? 4 : (BN == 128 ? 6 : 8)) / OCC;
@@ -175,11 +177,11 @@ __device__ __forceinline__ Item decode_item(const ConvParams& p, long long item,
 // IM2COL: the patch operand also arrives by TMA (im2col-mode tensor map `tmi`), so the CTA has no
 // gather warps at all; needs the gathered tensor's channel count to be a multiple of 32 and is not
 // used for strided dgrad.  Otherwise the eight cp.async warps below gather it.
-template <int MODE, int BN, bool IM2COL>
-__global__ void __launch_bounds__(IM2COL ? (MODE == 2 ? 288 : 192) : NUM_THREADS, Cfg<BN, IM2COL>::OCC)
+template <int MODE, int BN, bool IM2COL, int OCC>
+__global__ void __launch_bounds__(IM2COL ? (MODE == 2 ? 288 : 192) : NUM_THREADS, OCC)
 conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmi,
                  const __grid_constant__ CUtensorMap tmo, const ConvParams p) {
-  using C = Cfg<BN, IM2COL>;
+  using C = Cfg<BN, IM2COL, OCC>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_stg = smem;
@@ -1315,19 +1317,16 @@ int sm_count() {
   return n;
 }
 
-template <int MODE, int BN, bool IM2COL>
-int launch(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo, const ConvParams& p,
-           cudaStream_t st) {
-  using C = Cfg<BN, IM2COL>;
-  auto kern = conv_tf32_kernel<MODE, BN, IM2COL>;
+template <int MODE, int BN, bool IM2COL, int OCC>
+int launch_occ(int grid, const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo, const ConvParams& p,
+               cudaStream_t st) {
+  using C = Cfg<BN, IM2COL, OCC>;
+  auto kern = conv_tf32_kernel<MODE, BN, IM2COL, OCC>;
   constexpr int threads = IM2COL ? (MODE == 2 ? 288 : 192) : NUM_THREADS;   // wgrad: three extra producer warps
   static tsb_launch::SmemLimit limit;
   if (limit.raise(kern, C::SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
-  const long long items = (long long)p.tiles_m * p.tiles_n * p.taps * p.splits;
-  const long long slots = (long long)sm_count() * C::OCC;
-  int grid = (int)(items < slots ? items : slots);
-  if (p.stats && grid > p.tiles_n) grid -= grid % p.tiles_n;    // every CTA then sees one column tile only
 #ifdef TSB_CONV_PROF
+  const long long items = (long long)p.tiles_m * p.tiles_n * p.taps * p.splits;
   static unsigned long long* prof = nullptr;
   if (!prof) cudaMalloc(reinterpret_cast<void**>(&prof), 16 * sizeof(unsigned long long));
   cudaMemsetAsync(prof, 0, 16 * sizeof(unsigned long long), st);
@@ -1350,6 +1349,17 @@ int launch(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo
 #endif
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
+}
+
+template <int MODE, int BN, bool IM2COL>
+int launch(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo, const ConvParams& p, cudaStream_t st) {
+  constexpr int most = max_ctas(BN, IM2COL);
+  const long long items = (long long)p.tiles_m * p.tiles_n * p.taps * p.splits;
+  const long long slots = (long long)sm_count() * most;
+  int grid = (int)(items < slots ? items : slots);
+  if (p.stats && grid > p.tiles_n) grid -= grid % p.tiles_n;    // every CTA then sees one column tile only
+  if (most == 2 && items > sm_count()) return launch_occ<MODE, BN, IM2COL, most>(grid, tm, tmi, tmo, p, st);
+  return launch_occ<MODE, BN, IM2COL, 1>(grid, tm, tmi, tmo, p, st);
 }
 
 template <int MODE, bool IM2COL>
@@ -1775,7 +1785,7 @@ int tsb_stem_pack_filters(const float* w, long long so, long long sc, long long 
 // convolution over 32 channels whose positions along a row are s pixels apart and overlap: the patch operand comes as
 // im2col boxes like that of any wide convolution, where the gather path copies 16 bytes at a time.  Pixels and K ranges
 // are taken in the same order as there, so the sums are the same bits.  7x7 stride 2 over 32 x 224 x 224, 64 filters:
-// 170.9 us gathered (64 SMs, bound by the copying warps' instructions) -> 83.7.
+// 170.9 us gathered (64 SMs, bound by the copying warps' instructions) -> 59.5.
 // dw is addressed through element strides (output channel, input channel, kh, kw).
 int tsb_stem_wgrad(const float* xp, const float* dy, float* dw, long long so, long long sc, long long sh, long long sw, int N,
                    int C, int H, int Wp, int O, int KH, int KW, int OH, int OW, int ph, int stride, void* stream) {
