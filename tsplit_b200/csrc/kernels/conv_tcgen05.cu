@@ -35,7 +35,7 @@ constexpr int BK = 32;
 constexpr int UMMA_K = 8;
 constexpr int A_STAGE_BYTES = BM * BK * 4;
 constexpr int STORE_STAGING_BYTES = 4 * 2048;   // per epilogue warp: 32 rows x 16 columns on their way to a TMA store
-constexpr int GATHER_WARPS = 8;        // two per scheduler, so one warp's address arithmetic hides the other's
+constexpr int GATHER_WARPS = 8;        // (16 of them take the same time: what bounds the path is what the copies cost)
 constexpr int GATHER_THREADS = GATHER_WARPS * 32;
 constexpr int NUM_THREADS = 6 * 32 + GATHER_THREADS;   // warp0 TMA, warp1 MMA, warps2-5 epilogue, then gather
 
@@ -79,9 +79,12 @@ struct Cfg {
   static constexpr int TMEM_COLS = (2 * BN <= 128) ? 128 : (2 * BN <= 256 ? 256 : 512);
 };
 
+// Through L1: neighbouring pixels of a tile share most of their patch, and a piece that comes from L2 costs a whole
+// 32-byte sector.  7x7 stride 2 over 32 x 224 x 224 x 4, 64 filters: 102 us past L1, 78 through it; with the bookkeeping
+// of the gather loops as it was (a loop per row and tap), 130.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
   const int sz = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(sz) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(sz) : "memory");
 }
 // Arrival on `bar` that the hardware performs once every cp.async issued so far by this thread has
 // written shared memory.  `.noinc`: the barrier's expected count already includes this arrival.
@@ -161,8 +164,9 @@ struct Item {
 __device__ __forceinline__ Item decode_item(const ConvParams& p, long long item, int BN_) {
   Item it;
   const int tiles = p.tiles_m * p.tiles_n * p.taps;
-  const int tile = (int)(item % tiles);
-  it.split = (int)(item / tiles);
+  // (64-bit divisions take some hundred cycles of every role and tile)
+  it.split = p.splits == 1 ? 0 : (item >> 32) == 0 ? (int)((unsigned)item / (unsigned)tiles) : (int)(item / tiles);
+  const int tile = (int)(item - (long long)it.split * tiles);
   const int per_m = p.tiles_n * p.taps;
   it.m0 = (tile / per_m) * BM;
   const int r = tile % per_m;
@@ -534,6 +538,16 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
     PROF_DECL(ge); PROF_DECL(gt);
     PROF_BEGIN(gt);
     const int ntaps = p.KH * p.KW;
+    // Filter taps that read inside the image as bits (up to 64 taps): of columns c_lo .. c_hi - 1 and rows r_lo .. r_hi - 1.
+    unsigned long long all_rows = 0;          // one bit at the start of every filter row
+    if (ntaps <= 64)
+      for (int kh = 0; kh < p.KH; ++kh) all_rows |= 1ull << (kh * p.KW);
+    auto taps_inside = [&](int c_lo, int c_hi, int r_lo, int r_hi) -> unsigned long long {
+      c_lo = max(c_lo, 0); c_hi = min(c_hi, p.KW); r_lo = max(r_lo, 0); r_hi = min(r_hi, p.KH);
+      if (c_lo >= c_hi || r_lo >= r_hi) return 0;
+      const unsigned long long cols = ((2ull << (c_hi - 1)) - 1) & ~((1ull << c_lo) - 1);
+      return cols * (all_rows & ((2ull << ((r_hi - 1) * p.KW)) - 1) & ~((1ull << (r_lo * p.KW)) - 1));
+    };
     for (long long item = blockIdx.x; item < items && ok; item += gridDim.x) {
       const Item w = decode_item(p, item, BN);
       if (MODE == 0 || MODE == 1) {
@@ -546,34 +560,33 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
         const int SH = (MODE == 0) ? p.H : p.OH, SW = (MODE == 0) ? p.W : p.OW;   // grid of the gathered tensor
         const int SC = (MODE == 0) ? p.C : p.O;                                   // its channel count
         const bool masked = ntaps <= 64 && (MODE == 0 || p.stride == 1);
+        const int tap_step = (MODE == 0) ? BK / p.C : 0, ch_step = (MODE == 0) ? BK - tap_step * p.C : 0;
         const float* rowptr[RPT];      // origin of the row's patch (may point outside; never read when invalid)
         int a0[RPT], b0[RPT];
         unsigned long long vmask[RPT]; // bit tap = that filter tap reads inside the image for this row
+        // image, row and column of the thread's first row; the next ones are RSTEP pixels on
+        int n = (w.m0 + rg) / (PH * PW), x = w.m0 + rg - n * (PH * PW);
+        int y = x / PW;
+        x -= y * PW;
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
+          if (i > 0) {
+            x += RSTEP;
+            while (x >= PW) { x -= PW; ++y; }
+            while (y >= PH) { y -= PH; ++n; }
+          }
           const int pix = w.m0 + rg + RSTEP * i;
           vmask[i] = 0;
           if (pix < p.M) {
-            const int n = pix / (PH * PW);
-            const int rem = pix - n * (PH * PW);
-            const int y = rem / PW, x = rem - y * PW;
             if (MODE == 0) { a0[i] = y * p.stride - p.ph; b0[i] = x * p.stride - p.pw; }
             else           { a0[i] = y + p.ph;            b0[i] = x + p.pw; }
             if (MODE == 0 || p.stride == 1)
               rowptr[i] = p.src + (((long long)n * SH + a0[i]) * SW + b0[i]) * SC;
             else
               rowptr[i] = p.src + (long long)n * SH * SW * SC;
-            if (masked) {
-              unsigned long long colm = 0;
-              for (int kw = 0; kw < p.KW; ++kw) {
-                const int xx = (MODE == 0) ? b0[i] + kw : b0[i] - kw;
-                if ((unsigned)xx < (unsigned)SW) colm |= 1ull << kw;
-              }
-              for (int kh = 0; kh < p.KH; ++kh) {
-                const int yy = (MODE == 0) ? a0[i] + kh : a0[i] - kh;
-                if ((unsigned)yy < (unsigned)SH) vmask[i] |= colm << (kh * p.KW);
-              }
-            }
+            if (masked)
+              vmask[i] = (MODE == 0) ? taps_inside(-b0[i], SW - b0[i], -a0[i], SH - a0[i])
+                                     : taps_inside(b0[i] - SW + 1, b0[i] + 1, a0[i] - SH + 1, a0[i] + 1);
           } else {
             rowptr[i] = p.src; a0[i] = -(1 << 28); b0[i] = -(1 << 28);
           }
@@ -629,11 +642,11 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
           cp_async_arrive(&full[s]);     // this thread's arrival fires when its copies above have landed
           // advance to the next k-block
           if (MODE == 0) {
-            ch += BK;
-            while (ch >= p.C) {
-              ch -= p.C; ++tap;
-              if (++kw == p.KW) { kw = 0; ++kh; }
-            }
+            int more = tap_step;
+            ch += ch_step;
+            if (ch >= p.C) { ch -= p.C; ++more; }
+            tap += more; kw += more;
+            while (kw >= p.KW) { kw -= p.KW; ++kh; }
           } else {
             ch += BK;
             if (++ob == p.ocb) {
@@ -683,14 +696,8 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
           const bool pvalid = pix < mpix;
           const float* rowptr = p.src + (((long long)n * p.H + y0) * p.W + x0) * p.C;
           if (masked) {
-            unsigned long long tapmask = 0;    // bit tap = that tap of this pixel reads inside the image
-            if (pvalid) {
-              unsigned long long colm = 0;
-              for (int kw = 0; kw < p.KW; ++kw)
-                if ((unsigned)(x0 + kw) < (unsigned)p.W) colm |= 1ull << kw;
-              for (int kh = 0; kh < p.KH; ++kh)
-                if ((unsigned)(y0 + kh) < (unsigned)p.H) tapmask |= colm << (kh * p.KW);
-            }
+            // bit tap = that tap of this pixel reads inside the image
+            const unsigned long long tapmask = pvalid ? taps_inside(-x0, p.W - x0, -y0, p.H - y0) : 0;
 #pragma unroll
             for (int i = 0; i < PPT; ++i) {
               const bool v = ptap[i] >= 0 && ((tapmask >> (ptap[i] & 63)) & 1ull);
