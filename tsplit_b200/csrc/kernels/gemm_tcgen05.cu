@@ -83,6 +83,48 @@ __device__ __forceinline__ void store_block(const CUtensorMap* tmC, uint8_t* blo
   which ^= 1;
 }
 
+// The last tile of a CTA: no operand is on its way any more, so the stages hold the whole of a warp's 32 x BN outputs, and
+// a fence (some 250 cycles) and a group of stores are for 128 columns, not 32.  Nothing hides this epilogue, and for a
+// product of one tile per CTA it took nearly as long as the MMAs of K = 512: 6100 cycles, 3600 now (the stores of 128 CTAs at
+// 7 TB/s).  8192 x 512 x 512: 11.7 -> 10.8 us; 256 of 256 x 64 x 256: 16.3 -> 14.1; 1024 x 1024 x 128: 6.5 -> 5.6.
+template <int BN>
+__device__ __forceinline__ void store_last_tile(const CUtensorMap* tmC, uint8_t* blocks, uint32_t tmem, bool has_k, int lane,
+                                                int n0, int n, int row0, int m, int z, int w) {
+  constexpr int STEP = BN < 128 ? BN : 128;
+  if (row0 >= m) return;
+#pragma unroll 1
+  for (int c0 = 0; c0 < BN && n0 + c0 < n; c0 += STEP) {
+#pragma unroll
+    for (int c = 0; c < STEP; c += 64) {
+      float v[2][32];
+      if (has_k) {
+        tmem_ld_32x32(tmem + c0 + c, v[0]);
+        tmem_ld_32x32(tmem + c0 + c + 32, v[1]);
+        tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[0][j] = v[1][j] = 0.f;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint8_t* dst = blocks + ((c0 + c) / 32 + h) * STORE_BLOCK_BYTES + lane * 128;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<float4*>(dst + ((j ^ (lane & 7)) << 4)) =
+              make_float4(v[h][4 * j], v[h][4 * j + 1], v[h][4 * j + 2], v[h][4 * j + 3]);
+      }
+    }
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+      for (int c = 0; c < STEP; c += 32)
+        if (n0 + c0 + c < n) tma_store_4d(tmC, blocks + (c0 + c) / 32 * STORE_BLOCK_BYTES, n0 + c0 + c, row0, z, w);
+      bulk_commit();
+    }
+  }
+}
+
 // Order in which the persistent CTAs walk the output tiles: groups of TILE_GROUP_M tile rows, column by column
 // inside a group.  The CTAs that run at the same time (consecutive tile indices) then share TILE_GROUP_M row
 // panels of A and a handful of column panels of B, which together stay in L2, instead of one or two rows of A
@@ -295,6 +337,11 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
         crow = p.c + at.c_off + (long long)row * p.ldc;
         accumulate = p.accumulate != 0;
       }
+      if (p.tma_store && item + step >= last) {
+        store_last_tile<BN>(&tmC, smem_a + q * (BN / 32) * STORE_BLOCK_BYTES, tmem_base + acc * BN + ((uint32_t)(q * 32) << 16),
+                            has_k, lane, n0, p.n, row - lane, p.m, cz, cw);
+        break;
+      }
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         float v[32];
@@ -330,7 +377,7 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[acc]);
+      if (lane == 0 && item + 2 * step < last) mbar_arrive(&tempty[acc]);      // (nobody waits for the last two)
     }
     if (p.tma_store && lane == 0) bulk_wait_all();     // this lane's stores are complete before the CTA exits
   }
@@ -428,7 +475,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();                                 // the peer's barriers exist before anything signals them
+  cluster_sync_relaxed();                                 // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   tsb_launch::enter();              // barriers and TMEM are set up under the tail of the previous kernel
@@ -522,6 +569,11 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const int cz = at.cz, cw = at.cw;
       float* crow = p.c + at.c_off + (long long)row * p.ldc;
       const bool accumulate = p.accumulate != 0;
+      if (p.tma_store && item + npairs >= items) {
+        store_last_tile<P2_BN>(&tmC, smem_a + q * (P2_BN / 32) * STORE_BLOCK_BYTES,
+                               tmem_base + acc * P2_BN + ((uint32_t)(q * 32) << 16), true, lane, n0, p.n, row - lane, p.m, cz, cw);
+        break;
+      }
 #pragma unroll 1
       for (int c0 = 0; c0 < P2_BN; c0 += 32) {
         float v[32];
@@ -552,7 +604,8 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_leader(&tempty[acc]);   // the leader's MMA thread counts both CTAs' warps
+      // the leader's MMA thread counts both CTAs' warps; nobody waits for the last two tiles
+      if (lane == 0 && item + 2 * npairs < items) mbar_arrive_leader(&tempty[acc]);
     }
     if (p.tma_store && lane == 0) bulk_wait_all();
   }
@@ -560,7 +613,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   // Nobody leaves (and nobody frees TMEM) while the partner may still signal or read.
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();
+  cluster_sync_relaxed();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_2sm(tmem_base, 512);
