@@ -98,3 +98,21 @@ def test_batches_and_head_layout(heads, rows, keys, d):
                                             I64(d), I64(d), 0, 0, 1, _stream()) == 0
             assert torch.equal(o[b * rows:(b + 1) * rows, h * d:(h + 1) * d], om)
     assert lib.tsb_device_status(_stream()) == 0
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [(512, 2048, 4 * 32 * 32), (1024, 1000, 9000), (2016, 1056, 2112)])
+def test_long_ranges_on_pairs_have_the_bits_of_single_tiles(monkeypatch, m, n, k, ta, tb):
+    """K ranges of 32 k-blocks and more run on CTA pairs: whole tiles, ragged columns, a ragged last range."""
+    lib = _lib()
+    a, b = _matrix(k if ta else m, m if ta else k, m if ta else k, 1), _matrix(n if tb else k, k if tb else n, k if tb else n, 2)
+    c = [_matrix(m, n, n, 3) for _ in range(2)]
+    for pair, out in zip(("1", "0"), c):
+        monkeypatch.setenv("TSB_GEMM_PAIR", pair)
+        for accumulate in (0, 1):
+            assert lib.tsb_gemm_tf32(PTR(a.data_ptr()), PTR(b.data_ptr()), PTR(out.data_ptr()), m, n, k, I64(a.shape[1]),
+                                     I64(b.shape[1]), I64(n), ta, tb, 1, I64(0), I64(0), I64(0), accumulate, _stream()) == 0
+    assert torch.equal(*c)
+    ref = (a.double().t() if ta else a.double()) @ (b.double().t() if tb else b.double())
+    assert (c[0].double() - 2 * ref).norm() < 2e-3 * ref.norm()          # operands are cut to 10 bits
+    assert lib.tsb_device_status(_stream()) == 0

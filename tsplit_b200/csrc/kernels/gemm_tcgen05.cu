@@ -482,7 +482,8 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   const int ptm = (p.m + 255) / 256, ptn = (p.n + P2_BN - 1) / P2_BN;
   const int tiles = ptm * ptn;
-  const long long items = (long long)tiles * p.batch;
+  const long long items = (long long)tiles * p.batch * p.splits;      // (a tile of a batch of a K range)
+  const int kb_per_split = (p.kblocks + p.splits - 1) / p.splits;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -491,13 +492,15 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       bool ok = true;
       for (long long item = pair; item < items && ok; item += npairs) {
         const int tile = (int)(item % tiles);
-        const int b = (int)(item / tiles);
+        const long long rest = item / tiles;
+        const int b = (int)(rest % p.batch), split = (int)(rest / p.batch);
+        const int kb0 = split * kb_per_split, kb1 = min(p.kblocks, kb0 + kb_per_split);
         int tm, tn;
         tile_mn(tile, ptm, ptn, tm, tn);
         const int m0 = tm * 256 + (int)rank * 128;           // this CTA's rows of A
         const int n0 = tn * P2_BN + (int)rank * P2_BNH;      // this CTA's columns of B
         const BatchAt at = batch_at(p, b);
-        for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % P2_STAGES;
           const uint32_t ph = (it / P2_STAGES) & 1;
           if (!mbar_wait(&empty[s], ph ^ 1, p.status, 0x111)) { ok = false; break; }
@@ -530,7 +533,8 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (!mbar_wait(&tempty[acc], acc_ph ^ 1, p.status, 0x112)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * P2_BN;
-        for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
+        const int kb0 = (int)(item / tiles / p.batch) * kb_per_split, kb1 = min(p.kblocks, kb0 + kb_per_split);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % P2_STAGES;
           const uint32_t ph = (it / P2_STAGES) & 1;
           if (!mbar_wait(&full[s], ph, p.status, 0x113)) { ok = false; break; }
@@ -540,7 +544,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
             umma_tf32_2sm(d_tmem, smem_desc_join(A_HI, a_lo + k * A_KSTEP), smem_desc_join(B_HI, b_lo + k * B_KSTEP),
-                          idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                          idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           umma_commit_2sm(&empty[s], 3);      // both CTAs may refill this stage once the MMAs retire
         }
         if (ok) umma_commit_2sm(&tfull[acc], 3);
@@ -555,7 +559,8 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     bool ok = true;
     for (long long item = pair; item < items && ok; item += npairs, ++acc_it) {
       const int tile = (int)(item % tiles);
-      const int b = (int)(item / tiles);
+      const long long rest = item / tiles;
+      const int b = (int)(rest % p.batch), split = (int)(rest / p.batch);
       int tm, tn;
       tile_mn(tile, ptm, ptn, tm, tn);
       const int m0 = tm * 256 + (int)rank * 128;
@@ -566,9 +571,10 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       tc_fence_after();
       const int row = m0 + q * 32 + lane;
       const BatchAt at = batch_at(p, b);
-      const int cz = at.cz, cw = at.cw;
-      float* crow = p.c + at.c_off + (long long)row * p.ldc;
-      const bool accumulate = p.accumulate != 0;
+      const int cz = p.splits > 1 ? split * p.batch + b : at.cz, cw = p.splits > 1 ? 0 : at.cw;
+      float* crow = p.splits > 1 ? p.ws + ((long long)(split * p.batch + b) * p.m + row) * p.n
+                                 : p.c + at.c_off + (long long)row * p.ldc;
+      const bool accumulate = p.splits == 1 && p.accumulate != 0;
       if (p.tma_store && item + npairs >= items) {
         store_last_tile<P2_BN>(&tmC, smem_a + q * (P2_BN / 32) * STORE_BLOCK_BYTES,
                                tmem_base + acc * P2_BN + ((uint32_t)(q * 32) << 16), true, lane, n0, p.n, row - lane, p.m, cz, cw);
@@ -923,7 +929,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   auto kern = gemm_tf32_pair_kernel<A_MN, B_MN>;
   static tsb_launch::SmemLimit limit;
   if (limit.raise(kern, P2_SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
-  const long long items = (long long)((p.m + 255) / 256) * ((p.n + P2_BN - 1) / P2_BN) * p.batch;
+  const long long items = (long long)((p.m + 255) / 256) * ((p.n + P2_BN - 1) / P2_BN) * p.batch * p.splits;
   long long pairs = sm_count() / 2;
   if (pairs > items) pairs = items;
   cudaError_t e = tsb_launch::launch_cluster(2u, kern, dim3((unsigned)(2 * pairs)), dim3(192), P2_SMEM_BYTES, st, ta, tb, tc, p);
@@ -1110,13 +1116,16 @@ static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorM
       return TSB_ERR_SCRATCH;
     }
   }
-  // CTA pairs (256 x 256 tiles on SM pairs) when the problem has enough of them and no split-K
+  // CTA pairs (256 x 256 tiles on SM pairs) when the problem has enough of them.  A split K too: a k-block of a 128 x 256
+  // tile is 48 KB, 670 cycles of what one SM takes from L2 when all do, for 512 cycles of MMAs; a CTA of a pair takes 32 KB.
+  // Ranges of at least 32 k-blocks: 4096 x 512 x 32000 (2 ranges) 205 -> 194 us, 512 x 2048 x 8192 (4) 34.6 -> 32.3; shorter
+  // ones are over before that counts: 512 x 512 x 8192 (18 of 15) 14.0 and 14.4, 512 x 1023 x 4000 (9 of 14) 33.5 and 35.9.
   use_pair = false;
   {
-    const long long pair_items = (long long)((m + 255) / 256) * ((n + 255) / 256) * batch;
+    const long long pair_items = (long long)((m + 255) / 256) * ((n + 255) / 256) * batch * p.splits;
     const char* e = getenv("TSB_GEMM_PAIR");              // "0" selects the one-CTA tiles everywhere
     const bool enabled = !(e && e[0] == '0');
-    use_pair = enabled && bn == 256 && p.splits == 1 && m >= 256 && pair_items * 4 >= sm_count() &&
+    use_pair = enabled && bn == 256 && (p.splits == 1 || kr.per >= 32) && m >= 256 && pair_items * 4 >= sm_count() &&
                (!trans_a || m % 32 == 0) && (trans_b || n % 32 == 0);
   }
   if (group_bn) {
