@@ -94,8 +94,31 @@ __device__ __forceinline__ float4 load_cluster(uint32_t local, uint32_t rank) {
   return v;
 }
 
-// `count` > 0 of four outputs; `vec`: 16-byte accesses are aligned.
-__device__ __forceinline__ void store4(float* dst, int count, bool vec, bool accumulate, float4 s) {
+// `count` > 0 of four outputs; `vec`: 16-byte accesses are aligned.  bias: of these columns; relu: where max(output, 0) goes.
+__device__ __forceinline__ void store4(float* dst, int count, bool vec, bool accumulate, float4 s, const float* bias,
+                                       float* relu) {
+  if (bias) {                        // (16-byte aligned; past the last column it is not read)
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (count >= 4) {
+      x = tsb_launch::load(reinterpret_cast<const float4*>(bias));
+    } else {
+      x.x = tsb_launch::load(bias);
+      if (count > 1) x.y = tsb_launch::load(bias + 1);
+      if (count > 2) x.z = tsb_launch::load(bias + 2);
+    }
+    s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+  }
+  if (relu) {
+    const float4 r = make_float4(fmaxf(s.x, 0.f), fmaxf(s.y, 0.f), fmaxf(s.z, 0.f), fmaxf(s.w, 0.f));
+    if (vec && count >= 4) {
+      *reinterpret_cast<float4*>(relu) = r;
+    } else {
+      relu[0] = r.x;
+      if (count > 1) relu[1] = r.y;
+      if (count > 2) relu[2] = r.z;
+      if (count > 3) relu[3] = r.w;
+    }
+  }
   if (vec && count >= 4) {
     if (accumulate) {
       const float4 old = *reinterpret_cast<const float4*>(dst);
@@ -151,6 +174,8 @@ __global__ void __launch_bounds__(COPY_THREADS) gemm_small_kernel(const __grid_c
   const int rows_left = p.m - m0, cols_left = p.n - n0;
   const long long ldc = p.ldc;
   float* c = p.c + o * p.sc2 + in * p.sc + m0 * ldc + n0;
+  const float* bias = p.bias ? p.bias + n0 : nullptr;
+  float* relu = p.relu ? p.relu + o * p.sc2 + in * p.sc + m0 * ldc + n0 : nullptr;
   int* status = grp.status;
   tc_fence_before();
   __syncthreads();
@@ -255,14 +280,15 @@ __global__ void __launch_bounds__(COPY_THREADS) gemm_small_kernel(const __grid_c
         const int col = (lane & 7) * 4;
         int row = warp * 16 + (lane >> 3);
         float* dst = c + row * ldc + col;
-        if (vec_c && cols_left >= TN && !accumulate) {
+        if (vec_c && cols_left >= TN && !accumulate && !bias && !relu) {
 #pragma unroll
           for (int j = 0; j < 4; ++j, row += 4, dst += 4 * ldc)
             if (row < rows_left) *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(part + row * PART_LD + col);
         } else {
           for (int j = 0; j < 4; ++j, row += 4, dst += 4 * ldc)
             if (row < rows_left && col < cols_left)
-              store4(dst, cols_left - col, vec_c, accumulate, *reinterpret_cast<const float4*>(part + row * PART_LD + col));
+              store4(dst, cols_left - col, vec_c, accumulate, *reinterpret_cast<const float4*>(part + row * PART_LD + col),
+                     bias ? bias + col : nullptr, relu ? relu + (dst - c) : nullptr);
         }
       }
       tc_fence_before();
@@ -282,7 +308,8 @@ __global__ void __launch_bounds__(COPY_THREADS) gemm_small_kernel(const __grid_c
 #pragma unroll
       for (int u = 0; u < MAX_SPLITS; ++u)
         if (u < splits) { s.x += v[u].x; s.y += v[u].y; s.z += v[u].z; s.w += v[u].w; }
-      store4(c + row * ldc + col, cols_left - col, vec_c, accumulate, s);
+      store4(c + row * ldc + col, cols_left - col, vec_c, accumulate, s, bias ? bias + col : nullptr,
+             relu ? relu + row * ldc + col : nullptr);
     }
     __syncwarp();
     cluster_sync_all();              // the partial sums stay until everybody has read them
@@ -318,7 +345,7 @@ cudaError_t run_group(Product* p, const CUtensorMap* ta, const CUtensorMap* tb, 
     Product& q = p[i];
     q.tiles_m = (q.m + TM - 1) / TM;
     q.tiles_n = (q.n + TN - 1) / TN;
-    q.vec_c = (reinterpret_cast<uintptr_t>(q.c) & 15) == 0 && q.ldc % 4 == 0 &&
+    q.vec_c = ((reinterpret_cast<uintptr_t>(q.c) | reinterpret_cast<uintptr_t>(q.relu)) & 15) == 0 && q.ldc % 4 == 0 &&
               (q.batch == 1 || (q.sc % 4 == 0 && q.sc2 % 4 == 0));
     g.p[i] = q;
     copies = copies || !q.a.tma || !q.b.tma;

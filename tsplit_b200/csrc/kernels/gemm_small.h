@@ -17,6 +17,8 @@ struct Operand {
 struct Product {
   Operand a, b;
   float* c;
+  const float* bias;             // [n], added to every row; may be null
+  float* relu;                   // second output max(c, 0), strides of c; may be null
   long long ldc, sc, sc2;
   int m, n, k, inner, batch;     // batch = outer * inner
   int accumulate;

@@ -56,6 +56,26 @@ struct GemmParams {
   int a_shift, b_shift;       // rows per outer batch of A / B in memory (M or K rows, N or K rows)
   long long sc2;              // C stride of the outer batch when c_heads (sc is then the head stride)
   int tma_store;              // the output leaves through shared memory and TMA stores (map tmC)
+  const float* bias;          // [n], added to every row (with tma_store and one K range only); may be null
+};
+
+// The bias of 32 columns from `col` on (the same for every row: one line, from L1).
+struct Bias32 {
+  float4 b[8];
+  __device__ __forceinline__ Bias32(const float* bias, int col, int n) {
+    if (col + 32 <= n) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) b[j] = tsb_launch::load(reinterpret_cast<const float4*>(bias + col) + j);
+    } else {               // (n is a multiple of four)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        b[j] = col + 4 * j < n ? tsb_launch::load(reinterpret_cast<const float4*>(bias + col) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  __device__ __forceinline__ void add_to(float* v) const {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { v[4 * j] += b[j].x; v[4 * j + 1] += b[j].y; v[4 * j + 2] += b[j].z; v[4 * j + 3] += b[j].w; }
+  }
 };
 
 // Output blocks of 32 rows x 32 columns on their way to a TMA store, two per epilogue warp.  A thread of the
@@ -89,7 +109,7 @@ __device__ __forceinline__ void store_block(const CUtensorMap* tmC, uint8_t* blo
 // 7 TB/s).  8192 x 512 x 512: 11.7 -> 10.8 us; 256 of 256 x 64 x 256: 16.3 -> 14.1; 1024 x 1024 x 128: 6.5 -> 5.6.
 template <int BN>
 __device__ __forceinline__ void store_last_tile(const CUtensorMap* tmC, uint8_t* blocks, uint32_t tmem, bool has_k, int lane,
-                                                int n0, int n, int row0, int m, int z, int w) {
+                                                int n0, int n, int row0, int m, int z, int w, const float* bias) {
   constexpr int STEP = BN < 128 ? BN : 128;
   if (row0 >= m) return;
 #pragma unroll 1
@@ -104,6 +124,10 @@ __device__ __forceinline__ void store_last_tile(const CUtensorMap* tmC, uint8_t*
       } else {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[0][j] = v[1][j] = 0.f;
+      }
+      if (bias) {
+        Bias32(bias, n0 + c0 + c, n).add_to(v[0]);
+        Bias32(bias, n0 + c0 + c + 32, n).add_to(v[1]);
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -339,7 +363,7 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
       }
       if (p.tma_store && item + step >= last) {
         store_last_tile<BN>(&tmC, smem_a + q * (BN / 32) * STORE_BLOCK_BYTES, tmem_base + acc * BN + ((uint32_t)(q * 32) << 16),
-                            has_k, lane, n0, p.n, row - lane, p.m, cz, cw);
+                            has_k, lane, n0, p.n, row - lane, p.m, cz, cw, p.splits == 1 ? p.bias : nullptr);
         break;
       }
 #pragma unroll 1
@@ -354,7 +378,10 @@ __device__ __forceinline__ void gemm_items(const CUtensorMap& tmA, const CUtenso
         }
         const int col = n0 + c0;
         if (p.tma_store) {
-          if (col < p.n && row - lane < p.m) store_block(&tmC, blocks, which, v, lane, col, row - lane, cz, cw);
+          if (col < p.n && row - lane < p.m) {
+            if (p.bias && p.splits == 1) Bias32(p.bias, col, p.n).add_to(v);
+            store_block(&tmC, blocks, which, v, lane, col, row - lane, cz, cw);
+          }
         } else if (row < p.m && col < p.n) {
           float* dst = crow + col;
           const bool vec_ok = (col + 32 <= p.n) && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0);
@@ -577,7 +604,8 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const bool accumulate = p.splits == 1 && p.accumulate != 0;
       if (p.tma_store && item + npairs >= items) {
         store_last_tile<P2_BN>(&tmC, smem_a + q * (P2_BN / 32) * STORE_BLOCK_BYTES,
-                               tmem_base + acc * P2_BN + ((uint32_t)(q * 32) << 16), true, lane, n0, p.n, row - lane, p.m, cz, cw);
+                               tmem_base + acc * P2_BN + ((uint32_t)(q * 32) << 16), true, lane, n0, p.n, row - lane, p.m, cz, cw,
+                               p.splits == 1 ? p.bias : nullptr);
         break;
       }
 #pragma unroll 1
@@ -587,7 +615,10 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         tmem_ld_wait();
         const int col = n0 + c0;
         if (p.tma_store) {
-          if (col < p.n && row - lane < p.m) store_block(&tmC, blocks, which, v, lane, col, row - lane, cz, cw);
+          if (col < p.n && row - lane < p.m) {
+            if (p.bias && p.splits == 1) Bias32(p.bias, col, p.n).add_to(v);
+            store_block(&tmC, blocks, which, v, lane, col, row - lane, cz, cw);
+          }
         } else if (row < p.m && col < p.n) {
           float* dst = crow + col;
           const bool vec_ok = (col + 32 <= p.n) && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0);
@@ -647,12 +678,16 @@ __global__ void splitk_reduce_kernel(const float* ws, float* __restrict__ c, int
 // The same with 16-byte lanes, for rows of whole float4 on both sides (5.6 -> 4.4 us each in a Transformer block).
 __global__ void __launch_bounds__(256) splitk_reduce_v4(const float4* ws, float4* __restrict__ c, int splits,
                                                         long long per_split4, int m, int n4, long long ldc4,
-                                                        long long sc4, int accumulate) {
+                                                        long long sc4, int accumulate, const float4* bias) {
   tsb_launch::enter();
   const long long i = blockIdx.x * 256ll + threadIdx.x;
   if (i >= per_split4) return;
-  const float4 acc = tsb::sum_splits(ws + i, splits, per_split4);
+  float4 acc = tsb::sum_splits(ws + i, splits, per_split4);
   const long long row = i / n4;
+  if (bias) {
+    const float4 b = bias[i - row * n4];
+    acc.x += b.x; acc.y += b.y; acc.z += b.z; acc.w += b.w;
+  }
   float4* dst = c + row / m * sc4 + row % m * ldc4 + (i - row * n4);
   float4 o = accumulate ? *dst : make_float4(0.f, 0.f, 0.f, 0.f);
   *dst = accumulate ? make_float4(o.x + acc.x, o.y + acc.y, o.z + acc.z, o.w + acc.w) : acc;
@@ -1092,6 +1127,7 @@ static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorM
   bn = n > 128 ? 256 : (n > 64 ? 128 : 64);
   p.c = c; p.m = m; p.n = n; p.k = k; p.batch = batch; p.ldc = ldc; p.sc = sc;
   p.accumulate = accumulate;
+  p.bias = nullptr;
   p.heads = head_mask ? heads : 0;
   p.a_heads = a_heads; p.b_heads = b_heads; p.c_heads = c_heads;
   p.a_shift = trans_a ? k : m;
@@ -1171,12 +1207,21 @@ static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorM
   return TSB_OK;
 }
 
+// What a product's epilogue does besides storing.  Refused (TSB_ERR_UNSUPPORTED, nothing launched) where the outputs do not
+// leave through a path that has it; `relu` is for products that gemm_small.cu takes.
+struct Epilogue {
+  const float* bias = nullptr;      // [n], 16-byte aligned: added to every row
+  float* relu = nullptr;            // a second output max(c, 0), laid out as c
+  bool any() const { return bias || relu; }
+};
+
 // Core entry shared by the allocating and the non-allocating front ends.
 //   ws / ws_bytes : split-K scratch supplied by the caller (may be null when splits resolves to 1)
 int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, int k, long long lda,
                        long long ldb, long long ldc, int trans_a, int trans_b, int batch, long long sa,
                        long long sb, long long sc, int accumulate, int forced_splits, float* ws,
-                       size_t ws_bytes, bool may_alloc, cudaStream_t st, int heads = 0, int head_mask = 0) {
+                       size_t ws_bytes, bool may_alloc, cudaStream_t st, int heads = 0, int head_mask = 0,
+                       const Epilogue& ex = Epilogue()) {
   if (m <= 0 || n <= 0 || k <= 0 || batch <= 0) return TSB_ERR_ARG;
   if (heads < 0 || (heads > 0 && (batch % heads) != 0)) return TSB_ERR_ARG;
   if (heads == 0) head_mask = 0;
@@ -1189,12 +1234,14 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
       CUtensorMap ta, tb;
       const int rc = small_product(&q, &ta, &tb, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, batch, sa, sb, sc,
                                    accumulate, heads, head_mask, kr.per);
+      q.bias = ex.bias; q.relu = ex.relu;
       return rc ? rc : run_small(&q, &ta, &tb, 1, kr.splits, trans_a, trans_b, st);
     }
   }
   if (head_mask) forced_splits = 1;       // the split-K scratch and its reduction address C by one batch stride
   const bool aligned = (lda % 4 == 0) && (ldb % 4 == 0) && (sa % 4 == 0) && (sb % 4 == 0) &&
                        ((reinterpret_cast<uintptr_t>(a) & 15) == 0) && ((reinterpret_cast<uintptr_t>(b) & 15) == 0);
+  if (ex.relu || (ex.any() && !aligned)) return TSB_ERR_UNSUPPORTED;
   // Only the row strides are off (e.g. 255-wide attention matrices): pad the operand rows into scratch
   // once (one pass over the operand) and run the tensor-core kernel on the padded copy.
   if (!aligned && may_alloc && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0) {
@@ -1257,6 +1304,9 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
   int rc = prepare_tc(p, ta, tb, tc, bn, use_pair, 0, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, batch, sa, sb, sc,
                       accumulate, forced_splits, ws, ws_bytes, may_alloc, st, heads, head_mask);
   if (rc) return rc;
+  p.bias = ex.bias;
+  if (ex.bias && !(p.tma_store && n % 4 == 0 && ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0))
+    return TSB_ERR_UNSUPPORTED;
   const bool a_mn = trans_a != 0, b_mn = trans_b == 0;
   if (use_pair) rc = dispatch_pair(a_mn, b_mn, ta, tb, tc, p, st);
   else if (bn == 256) rc = dispatch_major<256>(a_mn, b_mn, ta, tb, tc, p, st);
@@ -1268,7 +1318,7 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
     if (n % 4 == 0 && ldc % 4 == 0 && (batch == 1 || sc % 4 == 0) && (reinterpret_cast<uintptr_t>(c) & 15) == 0) {
       tsb_launch::launch(splitk_reduce_v4, dim3((unsigned)((per_split / 4 + 255) / 256)), 256, 0, st,
                          reinterpret_cast<const float4*>(p.ws), reinterpret_cast<float4*>(c), p.splits, per_split / 4,
-                         m, n / 4, ldc / 4, batch > 1 ? sc / 4 : 0, accumulate);
+                         m, n / 4, ldc / 4, batch > 1 ? sc / 4 : 0, accumulate, reinterpret_cast<const float4*>(ex.bias));
       const cudaError_t e4 = cudaGetLastError();
       if (e4 != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e4 << 8);
       const int late4 = tsb_host::peek_status();
@@ -1319,9 +1369,9 @@ int tsb_gemm_tf32_splitk(const float* a, const float* b, float* c, int m, int n,
 // Up to 16 products C = op(A) op(B) of the same transposition as one launch.  TSB_ERR_UNSUPPORTED when one of them is no
 // candidate (rows that TMA cannot read in a group that gemm_small.cu does not take, split-K, CTA pairs) or the tiles are
 // more than two waves.
-int tsb_gemm_tf32_group(int count, const float** a, const float** b, float** c, const int* m, const int* n, const int* k,
-                        const long long* lda, const long long* ldb, const long long* ldc, int trans_a, int trans_b,
-                        void* stream) {
+static int gemm_group(int count, const float** a, const float** b, float** c, const int* m, const int* n, const int* k,
+                      const long long* lda, const long long* ldb, const long long* ldc, int trans_a, int trans_b,
+                      const float** bias, float** relu, void* stream) {
   if (count < 1 || count > MAX_GROUP) return TSB_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   long long wide = 0;
@@ -1342,10 +1392,13 @@ int tsb_gemm_tf32_group(int count, const float** a, const float** b, float** c, 
       const int rc = small_product(&q[i], &ta[i], &tb[i], a[i], b[i], c[i], m[i], n[i], k[i], lda[i], ldb[i], ldc[i], trans_a,
                                    trans_b, 1, 0, 0, 0, 0, 0, 0, (k[i] + BK - 1) / BK);
       if (rc) return rc;
+      q[i].bias = bias ? bias[i] : nullptr;
+      q[i].relu = relu ? relu[i] : nullptr;
     }
     return run_small(q, ta, tb, count, 1, trans_a, trans_b, st);
   }
   for (int i = 0; i < count; ++i) {
+    if (relu && relu[i]) return TSB_ERR_UNSUPPORTED;
     if ((lda[i] | ldb[i]) % 4 || ((reinterpret_cast<uintptr_t>(a[i]) | reinterpret_cast<uintptr_t>(b[i])) & 15))
       return TSB_ERR_UNSUPPORTED;
     wide += (((long long)m[i] + BM - 1) / BM) * ((n[i] + 2 * GROUP_BN - 1) / (2 * GROUP_BN));
@@ -1360,6 +1413,8 @@ int tsb_gemm_tf32_group(int count, const float** a, const float** b, float** c, 
     const int rc = prepare_tc(g.p[i], g.ta[i], g.tb[i], g.tc[i], width, pair, GROUP_BN, a[i], b[i], c[i], m[i], n[i], k[i],
                               lda[i], ldb[i], ldc[i], trans_a, trans_b, 1, 0, 0, 0, 0, 0, nullptr, 0, false, st, 0, 0);
     if (rc) return rc == TSB_ERR_SCRATCH ? TSB_ERR_UNSUPPORTED : rc;
+    g.p[i].bias = bias ? bias[i] : nullptr;
+    if (g.p[i].bias && !g.p[i].tma_store) return TSB_ERR_UNSUPPORTED;
     g.first[i] = ctas;
     ctas += g.p[i].tiles_m * g.p[i].tiles_n;
   }
@@ -1368,6 +1423,30 @@ int tsb_gemm_tf32_group(int count, const float** a, const float** b, float** c, 
   if (rc) return rc;
   const int late = tsb_host::peek_status();
   return late ? TSB_ERR_TIMEOUT | (late << 8) : TSB_OK;
+}
+
+int tsb_gemm_tf32_group(int count, const float** a, const float** b, float** c, const int* m, const int* n, const int* k,
+                        const long long* lda, const long long* ldb, const long long* ldc, int trans_a, int trans_b,
+                        void* stream) {
+  return gemm_group(count, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, nullptr, nullptr, stream);
+}
+
+// One product (count 1) or a group as above whose outputs get bias[i] (or null) added to every row, and whose max(c, 0)
+// goes to relu[i] as well (or null).  The sums are rounded before the bias is added, as the separate operators do.
+// TSB_ERR_UNSUPPORTED, with nothing launched: a bias that is not 16-byte aligned, a relu of a product that is not small, rows
+// that TMA cannot store.
+int tsb_gemm_tf32_dense(int count, const float** a, const float** b, float** c, const int* m, const int* n, const int* k,
+                        const long long* lda, const long long* ldb, const long long* ldc, int trans_a, int trans_b,
+                        const float** bias, float** relu, void* stream) {
+  if (count < 1 || count > MAX_GROUP) return TSB_ERR_ARG;
+  for (int i = 0; i < count; ++i)
+    if (reinterpret_cast<uintptr_t>(bias[i]) & 15) return TSB_ERR_UNSUPPORTED;
+  if (count > 1) return gemm_group(count, a, b, c, m, n, k, lda, ldb, ldc, trans_a, trans_b, bias, relu, stream);
+  Epilogue ex;
+  ex.bias = bias[0];
+  ex.relu = relu[0];
+  return tsb_gemm_tf32_impl(a[0], b[0], c[0], m[0], n[0], k[0], lda[0], ldb[0], ldc[0], trans_a, trans_b, 1, 0, 0, 0, 0, 0,
+                            nullptr, 0, true, static_cast<cudaStream_t>(stream), 0, 0, ex);
 }
 
 // Synchronise the stream and return (then clear) the device-side wait status:

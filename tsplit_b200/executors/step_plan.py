@@ -1,6 +1,6 @@
 """The order in which the keep-all executors issue a step on the GPU, worked out once per feed shape.
 
-Five things are taken out of the node-by-node loop.  They change no value, but for the rounding of a loss whose labels
+Six things are taken out of the node-by-node loop.  They change no value, but for the rounding of a loss whose labels
 come from class ids (the last one: the same sum, added up in another order):
 
 * element-wise operators over the same elements are collected and run as one ``tsb_pointwise`` program, at the first
@@ -8,6 +8,7 @@ come from class ids (the last one: the same sum, added up in another order):
 * a reshape of a row-major array is a view of it;
 * the small parameter gradients that a normalisation operator hands out from its own buffers are copied in one launch;
 * small matrix products that are ready together run as one launch, and so do column sums of a few rows;
+* the bias of a product, and the ReLU behind it, are added where the product stores its outputs;
 * one-hot labels, scaled and shifted (label smoothing), that only a cross-entropy reads are not made: it takes the ids.
 
 Element-wise nodes are taken as soon as their inputs are there, the others in creation order, and nothing moves past a
@@ -22,7 +23,7 @@ import numpy as np
 
 from .. import ndarray
 from ..ops import _gpu as G
-from ..ops.elementwise import AddConstOp, MulConstOp, _Binary, _Unary, _is_scalar_shape
+from ..ops.elementwise import AddConstOp, MulConstOp, ReluOp, _Binary, _Unary, _is_scalar_shape
 from ..ops.linalg import MatMulOp, _mm_shape
 from ..ops.loss import SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp
 from ..ops.misc import OneHotOp, PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
@@ -152,6 +153,11 @@ class StepPlan(object):
         for n in ex.topo_order:
             if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
                 self._smooth_labels(n)
+        self.dense, self.stored = {}, set()      # product -> (its bias node or None, its ReLU or None), see _dense
+        self.refused = {}                        # product -> what its launch does not take: 1 the ReLU, 2 the bias either
+        for n in ex.topo_order:
+            if n not in self.external and isinstance(n.op, MatMulOp):
+                self._dense(n)
         self.root = {}                    # view -> the node whose array it looks at
         self.actions = []
         self.open = {}                    # key -> Program that still collects
@@ -173,7 +179,7 @@ class StepPlan(object):
         self._schedule(segment)
         self._flush_all()
         del self.users, self.shapes, self.external, self.root, self.open, self.home, self.copies     # planning only
-        del self.copied, self.layouts, self.group_of, self.queues, self.gone, self.kinds
+        del self.copied, self.layouts, self.group_of, self.queues, self.gone, self.kinds, self.stored
 
     def _kind(self, n):
         """What nodes of this operator type may become; "effects": they stay where they are."""
@@ -258,6 +264,26 @@ class StepPlan(object):
         for u in readers:
             self.smooth[u] = (cur.inputs[0], consts[::-1], chain[::-1])
 
+    def _dense(self, product):
+        """``product + row`` that nothing else reads the product of, and the one ReLU of the result (or of the product
+        itself): the product's launch can store them.  The row is there from the start (a parameter)."""
+        result, bias, readers = product, None, self.users.get(product, [])
+        if (len(readers) == 1 and isinstance(readers[0].op, AddBroadcastOp) and readers[0].inputs[0] is product
+                and product not in self.evals and not self._has_effects(readers[0])):
+            row = readers[0].inputs[1]
+            cols = self.shapes[product][-1]
+            if row in self.external and row is not product and tuple(self.shapes[row]) == (cols,):
+                result = bias = readers[0]
+        relus = [u for u in self.users.get(result, ()) if isinstance(u.op, ReluOp) and not self._has_effects(u)]
+        relu = relus[0] if len(relus) == 1 else None
+        made = [n for n in (bias, relu) if n is not None]
+        own = self.arrays.get(product)
+        if made and own is not None and own.is_contiguous() and all(
+                self.arrays.get(n) is not None and self.arrays[n].is_contiguous()
+                and tuple(self.shapes[n]) == tuple(self.shapes[product]) for n in made):
+            self.dense[product] = (bias, relu)
+            self.stored.update(made)
+
     # -- scheduling ------------------------------------------------------------------------
     def _schedule(self, nodes):
         inside = set(nodes)
@@ -267,7 +293,7 @@ class StepPlan(object):
         self.queues, self.gone = {}, set()
 
         def ready(n):
-            cls, ops = "elided" if n in self.elided else self._kind(n), None
+            cls, ops = "elided" if n in self.elided or n in self.stored else self._kind(n), None
             if cls == "element":
                 ops = self._operands(n)
                 cls = None if ops is None else cls
@@ -314,7 +340,8 @@ class StepPlan(object):
                 if n in self.smooth:
                     self._need(self.smooth[n][0])
                 self.actions.append((self.group_of[n][0][0], taken) if len(taken) > 1 else
-                                    ("smooth" if n in self.smooth else "node", n))
+                                    ("smooth", n) if n in self.smooth else
+                                    ("products", taken) if n in self.dense else ("node", n))
                 for m in taken[1:]:
                     done(m)
             done(n)
@@ -479,6 +506,9 @@ class StepPlan(object):
 
     def _products(self, nodes, vals, stream):
         ta, tb = nodes[0].attrs["trans_A"], nodes[0].attrs["trans_B"]
+        if (self.refused.get(nodes[0], 0) < 2 and any(n in self.dense for n in nodes)
+                and self._dense_products(nodes, ta, tb, vals, stream)):
+            return
         items, alone = [], []
         for n in nodes:
             a, b, out = vals[n.inputs[0]], vals[n.inputs[1]], self.arrays[n]
@@ -493,6 +523,43 @@ class StepPlan(object):
             alone = nodes
         for n in alone:
             self._node(n, vals, stream)
+        for n in nodes:
+            for m in self.dense.get(n, ()):
+                if m is not None:
+                    self._node(m, vals, stream)
+
+    def _dense_products(self, nodes, ta, tb, vals, stream):
+        """The products with what their launches store besides; False: not taken.  (The array of a product whose bias is
+        added there is not written; the sums alone would be read by nobody.)"""
+        items = []
+        for n in nodes:
+            bias, relu = self.dense.get(n, (None, None))
+            a, b = vals[n.inputs[0]], vals[n.inputs[1]]
+            row = vals[bias.inputs[1]] if bias is not None else None
+            if not (a.is_contiguous() and b.is_contiguous() and (row is None or row.is_contiguous())):
+                return False
+            items.append((a, b, self.arrays[n if bias is None else bias]) + _mm_shape(a.shape, b.shape, ta, tb)
+                         + (row, None if relu is None else self.arrays[relu]))
+        if len(items) > 1 and not all(G.gemm_group_takes(*i[:2]) for i in items):
+            return False
+        first, late = nodes[0], []
+        has_relu, has_bias = (any(i[j] is not None for i in items) for j in (7, 6))
+        taken = first not in self.refused and G.gemm_dense(items, ta, tb, stream)
+        if not taken and has_relu and has_bias and self.refused.get(first, 1) < 2:
+            # a ReLU is stored by small products only: without it
+            self.refused[first] = 1
+            late = [self.dense[n][1] for n in nodes if n in self.dense and self.dense[n][1] is not None]
+            taken = G.gemm_dense([i[:7] + (None,) for i in items], ta, tb, stream)
+        if not taken:
+            self.refused[first] = 2
+            return False
+        for n in nodes:
+            for m in (n,) + self.dense.get(n, ()):
+                if m is not None:
+                    vals[m] = self.arrays[m]
+        for m in late:
+            self._node(m, vals, stream)
+        return True
 
     def _sums(self, nodes, vals, stream):
         items = [(vals[n.inputs[0]], self.arrays[n]) for n in nodes]

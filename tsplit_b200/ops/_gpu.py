@@ -477,6 +477,23 @@ def gemm_group(products, trans_a, trans_b, stream):
     return rc == 0
 
 
+def gemm_dense(products, trans_a, trans_b, stream):
+    """Products ``(a, b, c, m, n, k, bias, relu)`` of row-major arrays with ``bias`` (or None) added to every row of ``c`` and
+    ``max(c, 0)`` stored in ``relu`` (or None), as one launch (more than one: a group of small ones).  False: not taken,
+    nothing was computed."""
+    cnt = len(products)
+    if not all(p[2].is_cuda for p in products):
+        return False
+    ptr = lambda j: (c_void_p * cnt)(*[p[j].ptr if p[j] is not None else None for p in products])
+    num = lambda j: (c_int * cnt)(*[p[j] for p in products])
+    ld = lambda j: (c_int64 * cnt)(*[p[j].shape[1] for p in products])
+    rc = lib().tsb_gemm_tf32_dense(c_int(cnt), ptr(0), ptr(1), ptr(2), num(3), num(4), num(5), ld(0), ld(1), ld(2),
+                                   c_int(int(trans_a)), c_int(int(trans_b)), ptr(6), ptr(7), _s(stream))
+    if rc != 2:
+        _check(rc, "gemm_tf32_dense")
+    return rc == 0
+
+
 def conv2d(kind, x, w, y, ph, pw, stride, stream):
     """kind 0: y = conv(x, w); 1: x(dx) = dgrad(y(dy), w); 2: w(dw) = wgrad(x, y(dy)).
     All operands channels-last; logical shapes x[N,C,H,W], w[O,C,KH,KW], y[N,O,OH,OW]."""
