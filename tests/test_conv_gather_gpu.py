@@ -24,6 +24,20 @@ def _rand(*shape, seed):
     (2, 8, 12, 11, 12, 9, 9, 4, 4, 1), (3, 100, 5, 3, 68, 3, 3, 1, 1, 1), (7, 12, 2, 2, 36, 1, 3, 0, 1, 1),
     (2, 44, 15, 17, 60, 3, 1, 1, 0, 2), (300, 4, 1, 1, 8, 1, 1, 0, 0, 1), (1, 24, 33, 130, 12, 1, 7, 0, 6, 3)])
 def test_forward_and_gradients(n, c, h, w, o, kh, kw, ph, pw, stride):
+    _check(n, c, h, w, o, kh, kw, ph, pw, stride)
+
+
+# both channel counts multiples of 32, where the data gradient reads the filters in place: one tile, ragged tiles, CTA pairs,
+# filters larger than the padding, a pointwise and an asymmetric one, the four parities of stride 2
+@pytest.mark.parametrize("n,c,h,w,o,kh,kw,ph,pw,stride", [
+    (2, 32, 9, 9, 32, 3, 3, 1, 1, 1), (3, 96, 17, 19, 64, 5, 3, 2, 0, 1), (4, 320, 60, 61, 64, 3, 3, 1, 1, 1),
+    (4, 256, 50, 47, 96, 1, 1, 0, 0, 1), (2, 224, 17, 17, 192, 1, 7, 0, 3, 1), (2, 32, 9, 9, 32, 7, 7, 3, 3, 2),
+    (3, 96, 17, 20, 64, 5, 5, 2, 2, 2), (8, 512, 28, 28, 128, 1, 1, 0, 0, 2)])
+def test_data_gradient_from_filters_in_place(n, c, h, w, o, kh, kw, ph, pw, stride):
+    _check(n, c, h, w, o, kh, kw, ph, pw, stride)
+
+
+def _check(n, c, h, w, o, kh, kw, ph, pw, stride):
     oh, ow = (h + 2 * ph - kh) // stride + 1, (w + 2 * pw - kw) // stride + 1
     x, wt, dy = _rand(n, h, w, c, seed=1), _rand(o, kh, kw, c, seed=2), _rand(n, oh, ow, o, seed=3)
     xd, wd, dyd = x.double().permute(0, 3, 1, 2), wt.double().permute(0, 3, 1, 2), dy.double().permute(0, 3, 1, 2)

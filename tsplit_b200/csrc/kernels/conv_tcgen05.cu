@@ -58,6 +58,7 @@ struct ConvParams {
   float* stats;        // forward only, may be null: per-CTA column sums / sums of squares of the output
   long long stats_plane;   // floats between the plane of sums and the plane of sums of squares
   int a3d;             // wgrad: dy arrives through the 3-D (32 channels, pixel, chunk) view
+  int f_step, f_rh, f_rw, f_kw;   // data gradient as a forward launch: where the filters lie (see filter_tap); f_step 0: plain filters
   int* status;
   unsigned long long* prof;   // role-time counters (only written when built with -DTSB_CONV_PROF)
 };
@@ -200,6 +201,15 @@ __device__ __forceinline__ void store_last_tile(const CUtensorMap* tmo, const Co
   }
 }
 
+// A data gradient runs as a forward launch over dy with flipped filters whose channel roles are exchanged (and, with
+// stride 2, with the taps of one parity).  They are read where they lie, w[o][kh][kw][c]: the operand's columns are the c of
+// one tap, contiguous, and its k are the o, so it is an MN-major one, and flipping is a matter of the tap's coordinate.
+// (Transposing them into scratch first was a launch of 3 to 4 us for each gradient, 61 of them in a ResNet-50 step.)
+// This is the tap of the filters that tap (kh, kw) of the launch multiplies.
+__device__ __forceinline__ int filter_tap(const ConvParams& p, int kh, int kw) {
+  return (p.f_step * (p.KH - 1 - kh) + p.f_rh) * p.f_kw + p.f_step * (p.KW - 1 - kw) + p.f_rw;
+}
+
 struct Item {
   int m0, n0, tap, split, kb0, kb1;
 };
@@ -224,7 +234,7 @@ __device__ __forceinline__ Item decode_item(const ConvParams& p, long long item,
 // IM2COL: the patch operand also arrives by TMA (im2col-mode tensor map `tmi`), so the CTA has no
 // gather warps at all; needs the gathered tensor's channel count to be a multiple of 32 and is not
 // used for strided dgrad.  Otherwise the eight cp.async warps below gather it.
-template <int MODE, int BN, bool IM2COL, int OCC>
+template <int MODE, int BN, bool IM2COL, int OCC, bool FLIP>
 __global__ void __launch_bounds__(IM2COL ? (MODE == 2 ? 288 : 192) : NUM_THREADS, OCC)
 conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmi,
                  const __grid_constant__ CUtensorMap tmo, const ConvParams p) {
@@ -368,7 +378,10 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
             mbar_expect_tx(&full[s], C::STAGE_BYTES);
             tma_load_im2col_4d(smem_a + s * A_STAGE_BYTES, &tmi, &full[s], cb * 32, bw, bh, n, (uint16_t)kw,
                                (uint16_t)kh);
-            tma_load_2d(smem_b + s * C::B_STAGE_BYTES, &tm, &full[s], kb * BK, w.n0);
+            if (FLIP)
+              tma_load_4d(smem_b + s * C::B_STAGE_BYTES, &tm, &full[s], 0, cb * 32, w.n0 >> 5, filter_tap(p, kh, kw));
+            else
+              tma_load_2d(smem_b + s * C::B_STAGE_BYTES, &tm, &full[s], kb * BK, w.n0);
             if (++cb == cpb) {
               cb = 0;
               if (++kw == p.KW) { kw = 0; ++kh; }
@@ -417,7 +430,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
     // ---------------------------------------------------------------- MMA issuer
     if (elect_one()) {
       constexpr int A_MN = (MODE == 2) ? 1 : 0;
-      constexpr int B_MN = (MODE == 0) ? 0 : 1;
+      constexpr int B_MN = (MODE == 0 && !FLIP) ? 0 : 1;
       constexpr uint32_t idesc = make_idesc_tf32(BM, BN, A_MN, B_MN);
       // shared-memory descriptors: MN-major operands use the 32-byte-atom 128B swizzle (chunks of 32
       // columns BK*128 bytes apart, 1024 bytes per K step), K-major ones the plain 128B swizzle
@@ -809,7 +822,7 @@ struct PairCfg {
   static constexpr int TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;    // two accumulators; 128, 256 or 512 columns
 };
 
-template <int BN>
+template <int BN, bool FLIP>
 __global__ void __launch_bounds__(192, 1)
 conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmi,
                      const __grid_constant__ CUtensorMap tmo, const ConvParams p) {
@@ -881,7 +894,10 @@ conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
           if (rank == 0) mbar_expect_tx(&full[s], 2 * PC::STAGE_BYTES);
           tma_load_im2col_4d_2sm(smem_a + s * A_STAGE_BYTES, &tmi, &full[s], cb * 32, bw, bh, n, (uint16_t)kw,
                                  (uint16_t)kh);
-          tma_load_2d_2sm(smem_b + s * PC::B_STAGE_BYTES, &tm, &full[s], kb * BK, n0);
+          if (FLIP)
+            tma_load_4d_2sm(smem_b + s * PC::B_STAGE_BYTES, &tm, &full[s], 0, cb * 32, n0 >> 5, filter_tap(p, kh, kw));
+          else
+            tma_load_2d_2sm(smem_b + s * PC::B_STAGE_BYTES, &tm, &full[s], kb * BK, n0);
           if (++cb == cpb) {
             cb = 0;
             if (++kw == p.KW) { kw = 0; ++kh; }
@@ -893,11 +909,11 @@ conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     if (rank == 0 && elect_one()) {
-      constexpr uint32_t idesc = make_idesc_tf32(256, BN, 0, 0);
-      constexpr uint32_t HI = smem_desc_hi(1024);
-      constexpr uint32_t KSTEP = (UMMA_K * 4) >> 4;
+      constexpr uint32_t idesc = make_idesc_tf32(256, BN, 0, FLIP);
+      constexpr uint32_t HI = smem_desc_hi(1024), B_HI = FLIP ? smem_desc_hi(512, LAYOUT_SW128_BASE32B) : HI;
+      constexpr uint32_t KSTEP = (UMMA_K * 4) >> 4, B_KSTEP = FLIP ? 1024 >> 4 : KSTEP;
       const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem_a), 16);
-      const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem_b), 16);
+      const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem_b), FLIP ? BK * 128 : 16);
       uint32_t it = 0, acc_it = 0;
       bool ok = true;
       for (int item = pair; item < items && ok; item += npairs, ++acc_it) {
@@ -915,7 +931,7 @@ conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
           const uint32_t b_lo = b_lo0 + s * (PC::B_STAGE_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_tf32_2sm(d_tmem, smem_desc_join(HI, a_lo + k * KSTEP), smem_desc_join(HI, b_lo + k * KSTEP), idesc,
+            umma_tf32_2sm(d_tmem, smem_desc_join(HI, a_lo + k * KSTEP), smem_desc_join(B_HI, b_lo + k * B_KSTEP), idesc,
                           (kb > 0 || k > 0) ? 1u : 0u);
           umma_commit_2sm(&empty[s], 3);
         }
@@ -1384,11 +1400,11 @@ int sm_count() {
   return n;
 }
 
-template <int MODE, int BN, bool IM2COL, int OCC>
+template <int MODE, int BN, bool IM2COL, int OCC, bool FLIP>
 int launch_occ(int grid, const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo, const ConvParams& p,
                cudaStream_t st) {
   using C = Cfg<BN, IM2COL, OCC>;
-  auto kern = conv_tf32_kernel<MODE, BN, IM2COL, OCC>;
+  auto kern = conv_tf32_kernel<MODE, BN, IM2COL, OCC, FLIP>;
   constexpr int threads = IM2COL ? (MODE == 2 ? 288 : 192) : NUM_THREADS;   // wgrad: three extra producer warps
   static tsb_launch::SmemLimit limit;
   if (limit.raise(kern, C::SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
@@ -1418,30 +1434,30 @@ int launch_occ(int grid, const CUtensorMap& tm, const CUtensorMap& tmi, const CU
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
 
-template <int MODE, int BN, bool IM2COL>
+template <int MODE, int BN, bool IM2COL, bool FLIP>
 int launch(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo, const ConvParams& p, cudaStream_t st) {
   constexpr int most = max_ctas(BN, IM2COL);
   const long long items = (long long)p.tiles_m * p.tiles_n * p.taps * p.splits;
   const long long slots = (long long)sm_count() * most;
   int grid = (int)(items < slots ? items : slots);
   if (p.stats && grid > p.tiles_n) grid -= grid % p.tiles_n;    // every CTA then sees one column tile only
-  if (most == 2 && items > sm_count()) return launch_occ<MODE, BN, IM2COL, most>(grid, tm, tmi, tmo, p, st);
-  return launch_occ<MODE, BN, IM2COL, 1>(grid, tm, tmi, tmo, p, st);
+  if (most == 2 && items > sm_count()) return launch_occ<MODE, BN, IM2COL, most, FLIP>(grid, tm, tmi, tmo, p, st);
+  return launch_occ<MODE, BN, IM2COL, 1, FLIP>(grid, tm, tmi, tmo, p, st);
 }
 
-template <int MODE, bool IM2COL>
+template <int MODE, bool IM2COL, bool FLIP = false>
 int launch_bn(int bn, const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo, const ConvParams& p,
               cudaStream_t st) {
-  if (bn == 256) return launch<MODE, 256, IM2COL>(tm, tmi, tmo, p, st);
-  if (bn == 128) return launch<MODE, 128, IM2COL>(tm, tmi, tmo, p, st);
-  return launch<MODE, 64, IM2COL>(tm, tmi, tmo, p, st);
+  if (bn == 256) return launch<MODE, 256, IM2COL, FLIP>(tm, tmi, tmo, p, st);
+  if (bn == 128) return launch<MODE, 128, IM2COL, FLIP>(tm, tmi, tmo, p, st);
+  return launch<MODE, 64, IM2COL, FLIP>(tm, tmi, tmo, p, st);
 }
 
-template <int BN>
+template <int BN, bool FLIP>
 int launch_fwd_pair_bn(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo, const ConvParams& p,
                        cudaStream_t st) {
   using PC = PairCfg<BN>;
-  auto kern = conv_fwd_pair_kernel<BN>;
+  auto kern = conv_fwd_pair_kernel<BN, FLIP>;
   static tsb_launch::SmemLimit limit;
   if (limit.raise(kern, PC::SMEM_BYTES) != cudaSuccess) return TSB_ERR_LAUNCH | ((int)cudaGetLastError() << 8);
   const int ptn = (p.NC + BN - 1) / BN;
@@ -1452,13 +1468,6 @@ int launch_fwd_pair_bn(const CUtensorMap& tm, const CUtensorMap& tmi, const CUte
   cudaError_t e = tsb_launch::launch_cluster(2u, kern, dim3((unsigned)(2 * pairs)), dim3(192), PC::SMEM_BYTES, st, tm,
                                              tmi, tmo, p);
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
-}
-
-int launch_fwd_pair(int bn, const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo,
-                    const ConvParams& p, cudaStream_t st) {
-  if (bn == 256) return launch_fwd_pair_bn<256>(tm, tmi, tmo, p, st);
-  if (bn == 128) return launch_fwd_pair_bn<128>(tm, tmi, tmo, p, st);
-  return launch_fwd_pair_bn<64>(tm, tmi, tmo, p, st);
 }
 
 int launch_wgrad_pair(const CUtensorMap& tm, const CUtensorMap& tmi, const CUtensorMap& tmo, const ConvParams& p,
@@ -1480,7 +1489,7 @@ ConvParams base_params(int N, int C, int H, int W, int O, int KH, int KW, int OH
   p.ph = ph; p.pw = pw; p.stride = p.step_w = stride;
   p.src = nullptr; p.out = nullptr; p.ws = nullptr; p.accumulate = 0; p.splits = 1; p.taps = 1;
   p.K = KH * KW * C; p.ocb = (O + 31) / 32; p.status = nullptr; p.prof = nullptr; p.a3d = 0; p.tma_store = 0; p.stats = nullptr; p.stats_plane = 0;
-  p.M = 0; p.NC = 0; p.kblocks = 0; p.tiles_m = 0; p.tiles_n = 0; p.ldc = 0;
+  p.f_step = p.f_rh = p.f_rw = p.f_kw = 0; p.M = 0; p.NC = 0; p.kblocks = 0; p.tiles_m = 0; p.tiles_n = 0; p.ldc = 0;
   return p;
 }
 
@@ -1501,6 +1510,12 @@ int im2col_map(CUtensorMap* out, const float* a, int N, int C, int H, int W, int
   return tsb_host::make_tmap_im2col_f32(out, a, C, W, H, N, lower, upper, 32, pixels, stride, stride, atom32);
 }
 
+// The filters of a data gradient where they lie, w[o][KH][KW][c]: tap (kh, kw) of the launch is their tap
+// (step * (T - 1 - kh) + rh, step * (T' - 1 - kw) + rw).
+struct FlippedFilters {
+  int KH, KW, step, rh, rw;
+};
+
 // out[N,OH,OW,O] = conv(src[N,H,W,C], wts[O,KH,KW,C]).  Serves forward, and stride-1 dgrad with
 // flipped and transposed filters.
 // stats / stats_plane / max_chunks / chunks_out (optional): also leave per-CTA column sums and sums of
@@ -1509,7 +1524,7 @@ int im2col_map(CUtensorMap* out, const float* a, int N, int C, int H, int W, int
 int run_forward(const float* src, const float* wts, float* out, int N, int C, int H, int W, int O, int KH, int KW,
                 int OH, int OW, int ph, int pw, int stride, cudaStream_t st, float* stats = nullptr,
                 long long stats_plane = 0, int max_chunks = 0, int* chunks_out = nullptr, int ph_end = INT_MIN,
-                int pw_end = INT_MIN) {
+                int pw_end = INT_MIN, const FlippedFilters* flip = nullptr) {
   if (chunks_out) *chunks_out = 0;
   if (ph_end == INT_MIN) ph_end = ph;      // symmetric padding unless the caller says otherwise
   if (pw_end == INT_MIN) pw_end = pw;
@@ -1522,9 +1537,23 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
   p.tiles_m = (p.M + BM - 1) / BM;
   p.tiles_n = (p.NC + bn - 1) / bn;
   CUtensorMap tm, tmi;
-  uint64_t d[2] = {(uint64_t)p.K, (uint64_t)O}, s[1] = {(uint64_t)p.K * 4};
-  uint32_t bx[2] = {BK, (uint32_t)bn};
-  int rc = tsb_host::make_tmap_f32(&tm, wts, 2, d, s, bx, false);
+  // filters of `rows` output channels per box
+  auto filter_map = [&](CUtensorMap* out_map, int rows) {
+    if (flip) {      // (32 channels, k = o, chunk of 32 channels, tap)
+      const uint64_t row = (uint64_t)flip->KH * flip->KW * O * 4;
+      uint64_t d[4] = {32, (uint64_t)C, (uint64_t)O / 32, (uint64_t)flip->KH * flip->KW}, s[3] = {row, 128, (uint64_t)O * 4};
+      uint32_t bx[4] = {32, BK, (uint32_t)rows / 32, 1};
+      return tsb_host::make_tmap_f32(out_map, wts, 4, d, s, bx, true);
+    }
+    uint64_t d[2] = {(uint64_t)p.K, (uint64_t)O}, s[1] = {(uint64_t)p.K * 4};
+    uint32_t bx[2] = {BK, (uint32_t)rows};
+    return tsb_host::make_tmap_f32(out_map, wts, 2, d, s, bx, false);
+  };
+  if (flip) {
+    if (C % 32 || O % 32) return TSB_ERR_UNSUPPORTED;
+    p.f_step = flip->step; p.f_rh = flip->rh; p.f_rw = flip->rw; p.f_kw = flip->KW;
+  }
+  int rc = filter_map(&tm, bn);
   if (rc) return rc;
   // output [M][O] leaves through TMA stores of 32 rows x 16 columns (64-byte rows, 64B swizzle)
   CUtensorMap tmo;
@@ -1543,8 +1572,7 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
     // (narrow tiles stay on the one-CTA kernel, whose column statistics come in twice as many chunks)
     if (!(e && e[0] == '0') && bn == 256 && pair_items * 4 >= sm_count()) {
       CUtensorMap tmh;          // filters, bn / 2 rows per CTA
-      uint32_t hb[2] = {BK, (uint32_t)bn / 2};
-      rc = tsb_host::make_tmap_f32(&tmh, wts, 2, d, s, hb, false);
+      rc = filter_map(&tmh, bn / 2);
       if (rc) return rc;
       if (stats) {              // same grid arithmetic as launch_fwd_pair_bn
         long long pairs = sm_count() / 2;
@@ -1556,15 +1584,14 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
           if (chunks_out) *chunks_out = chunks;
         }
       }
-      return launch_fwd_pair(bn, tmh, tmi, tmo, p, st);
+      return p.f_step ? launch_fwd_pair_bn<256, true>(tmh, tmi, tmo, p, st) : launch_fwd_pair_bn<256, false>(tmh, tmi, tmo, p, st);
     }
     // few tiles: narrower ones (here only: the gather path below keeps its width, which was not measured)
     const int nbn = tsb_host::narrow_tile(bn, (long long)p.tiles_m * p.tiles_n, sm_count());
     if (nbn != bn) {
       bn = nbn;
       p.tiles_n = (p.NC + bn - 1) / bn;
-      bx[1] = (uint32_t)bn;
-      rc = tsb_host::make_tmap_f32(&tm, wts, 2, d, s, bx, false);
+      rc = filter_map(&tm, bn);
       if (rc) return rc;
     }
     if (stats) {                // same grid arithmetic as launch<>
@@ -1578,9 +1605,9 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
         if (chunks_out) *chunks_out = chunks;
       }
     }
-    return launch_bn<0, true>(bn, tm, tmi, tmo, p, st);
+    return p.f_step ? launch_bn<0, true, true>(bn, tm, tmi, tmo, p, st) : launch_bn<0, true>(bn, tm, tmi, tmo, p, st);
   }
-  if (rc != TSB_ERR_UNSUPPORTED) return rc;
+  if (rc != TSB_ERR_UNSUPPORTED || flip) return rc;
   return launch_bn<0, false>(bn, tm, tm, tmo, p, st);
 }
 
@@ -1647,10 +1674,8 @@ int run_dgrad_parity(float* dx, const float* w, const float* dy, int N, int C, i
       ptotal += ((size_t)N * ax[a].R * bx[b].R * C * sizeof(float) + 255) & ~size_t(255);
     }
   if (ptotal > (size_t(4) << 30)) return TSB_ERR_UNSUPPORTED;
-  // every class has its own filter buffer: the four launches are queued back to back
-  float* wt = wmax ? get_ws(st, 1, 4 * wmax, size_t(16) << 20) : nullptr;
   float* parts = ptotal ? get_ws(st, 2, ptotal, size_t(64) << 20) : nullptr;
-  if ((wmax && !wt) || (ptotal && !parts)) return TSB_ERR_OOM;
+  if (ptotal && !parts) return TSB_ERR_OOM;
   ParityParts pp;
   for (int a = 0; a < 2; ++a)
     for (int b = 0; b < 2; ++b) {
@@ -1659,14 +1684,21 @@ int run_dgrad_parity(float* dx, const float* w, const float* dy, int N, int C, i
       pp.part[k] = nullptr;
       pp.R[k][0] = A.R; pp.R[k][1] = B.R;
       if (!live[k]) continue;
-      float* wk = wt + (size_t)k * (wmax / sizeof(float));
       float* part = reinterpret_cast<float*>(reinterpret_cast<char*>(parts) + poff[k]);
-      dim3 grid((C + 31) / 32, (O + 31) / 32, A.T * B.T);
-      tsb_launch::launch(parity_filters, grid, dim3(32, 8), 0, st, w, wk, O, C, KH, KW, A.r, A.T, B.r, B.T);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
-      const int rc = run_forward(dy, wk, part, N, O, OH, OW, C, A.T, B.T, A.R, B.R, A.pad_lead, B.pad_lead, 1, st,
-                                 nullptr, 0, 0, nullptr, A.pad_trail, B.pad_trail);
+      const FlippedFilters flip = {KH, KW, 2, A.r, B.r};
+      int rc = run_forward(dy, w, part, N, O, OH, OW, C, A.T, B.T, A.R, B.R, A.pad_lead, B.pad_lead, 1, st, nullptr, 0, 0, nullptr,
+                           A.pad_trail, B.pad_trail, &flip);
+      if (rc == TSB_ERR_UNSUPPORTED) {      // channels of no 32: filters transposed in scratch
+        float* wk = get_ws(st, 1, 4 * wmax, size_t(16) << 20);
+        if (!wk) return TSB_ERR_OOM;
+        wk += (size_t)k * (wmax / sizeof(float));      // every class has its own: the four launches are queued back to back
+        dim3 grid((C + 31) / 32, (O + 31) / 32, A.T * B.T);
+        tsb_launch::launch(parity_filters, grid, dim3(32, 8), 0, st, w, wk, O, C, KH, KW, A.r, A.T, B.r, B.T);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
+        rc = run_forward(dy, wk, part, N, O, OH, OW, C, A.T, B.T, A.R, B.R, A.pad_lead, B.pad_lead, 1, st, nullptr, 0, 0, nullptr,
+                         A.pad_trail, B.pad_trail);
+      }
       if (rc) return rc;
       pp.part[k] = part;
     }
@@ -1710,6 +1742,14 @@ int tsb_conv2d(int kind, float* x, float* w, float* y, int N, int C, int H, int 
     rc = run_forward(x, w, y, N, C, H, W, O, KH, KW, OH, OW, ph, pw, stride, st);
   } else if (kind == 1 && stride == 1 && (O % 32) == 0 && ph <= KH - 1 && pw <= KW - 1) {
     // stride-1 dgrad = forward convolution of dy with the flipped, transposed filters
+    const FlippedFilters flip = {KH, KW, 1, 0, 0};
+    rc = run_forward(y, w, x, N, O, OH, OW, C, KH, KW, H, W, KH - 1 - ph, KW - 1 - pw, 1, st, nullptr, 0, 0, nullptr, INT_MIN,
+                     INT_MIN, &flip);
+    if (rc != TSB_ERR_UNSUPPORTED) {
+      if (rc) return rc;
+      const int late = tsb_host::peek_status();
+      return late ? TSB_ERR_TIMEOUT | (late << 8) : TSB_OK;
+    }
     const size_t wbytes = (size_t)C * KH * KW * O * sizeof(float);
     float* wt = get_ws(st, 1, wbytes, size_t(16) << 20);
     if (!wt) return TSB_ERR_OOM;
