@@ -1,7 +1,7 @@
 """The order in which the keep-all executors issue a step on the GPU, worked out once per feed shape.
 
-Six things are taken out of the node-by-node loop.  They change no value, but for the rounding of a loss whose labels
-come from class ids (the last one: the same sum, added up in another order):
+Seven things are taken out of the node-by-node loop.  They change no value, but for the rounding of a loss whose labels
+come from class ids (the same sum, added up in another order):
 
 * element-wise operators over the same elements are collected and run as one ``tsb_pointwise`` program, at the first
   node that needs one of their results; results that nobody outside the program reads are not stored;
@@ -9,7 +9,8 @@ come from class ids (the last one: the same sum, added up in another order):
 * the small parameter gradients that a normalisation operator hands out from its own buffers are copied in one launch;
 * small matrix products that are ready together run as one launch, and so do column sums of a few rows;
 * the bias of a product, and the ReLU behind it, are added where the product stores its outputs;
-* one-hot labels, scaled and shifted (label smoothing), that only a cross-entropy reads are not made: it takes the ids.
+* one-hot labels, scaled and shifted (label smoothing), that only a cross-entropy reads are not made: it takes the ids;
+* a loss and its gradient come from one pass over the logits, when the gradient is due.
 
 Element-wise nodes are taken as soon as their inputs are there, the others in creation order, and nothing moves past a
 node with effects of its own (an optimizer update, a collective, a swap).  The memory-planning executors have
@@ -153,6 +154,11 @@ class StepPlan(object):
         for n in ex.topo_order:
             if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
                 self._smooth_labels(n)
+        self.both = {}                           # gradient of a loss -> the loss that is computed with it
+        for n in ex.topo_order:
+            if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
+                self._loss_with_gradient(n)
+        self.late = set(self.both.values())
         self.dense, self.stored = {}, set()      # product -> (its bias node or None, its ReLU or None), see _dense
         self.refused = {}                        # product -> what its launch does not take: 1 the ReLU, 2 the bias either
         for n in ex.topo_order:
@@ -264,6 +270,18 @@ class StepPlan(object):
         for u in readers:
             self.smooth[u] = (cur.inputs[0], consts[::-1], chain[::-1])
 
+    def _loss_with_gradient(self, loss):
+        """When nobody needs ``loss`` before its one gradient is due (a seed of ones takes its shape only)."""
+        logits, labels = loss.inputs
+        grads = [u for u in self.users.get(logits, ()) if isinstance(u.op, SoftmaxCrossEntropyGradientOp)
+                 and u.inputs[0] is logits and u.inputs[1] is labels]
+        others = [u for u in self.users.get(logits, ()) if isinstance(u.op, SoftmaxCrossEntropyOp) and u.inputs[1] is labels]
+        if (len(grads) == 1 and len(others) == 1 and all(isinstance(u.op, _FillLike) for u in self.users.get(loss, ()))
+                and (loss in self.smooth) == (grads[0] in self.smooth) and not self._has_effects(loss)
+                and not self._has_effects(grads[0]) and self.arrays.get(loss) is not None
+                and self.arrays.get(grads[0]) is not None):
+            self.both[grads[0]] = loss
+
     def _dense(self, product):
         """``product + row`` that nothing else reads the product of, and the one ReLU of the result (or of the product
         itself): the product's launch can store them.  The row is there from the start (a parameter)."""
@@ -341,6 +359,7 @@ class StepPlan(object):
                     self._need(self.smooth[n][0])
                 self.actions.append((self.group_of[n][0][0], taken) if len(taken) > 1 else
                                     ("smooth", n) if n in self.smooth else
+                                    ("loss", n) if n in self.both or n in self.late else
                                     ("products", taken) if n in self.dense else ("node", n))
                 for m in taken[1:]:
                     done(m)
@@ -480,8 +499,13 @@ class StepPlan(object):
                 self._node(x, vals, stream)
             elif what == "view":
                 vals[x] = self.arrays[x]
-            elif what == "smooth":
-                self._smooth(x, vals, stream, made)
+            elif what in ("loss", "smooth"):
+                if x in self.late:
+                    vals[x] = self.arrays[x]         # (a seed of ones takes its shape)
+                elif x in self.both:
+                    self._loss(x, vals, stream, made)
+                else:
+                    self._smooth(x, vals, stream, made)
             elif what == "products":
                 self._products(x, vals, stream)
             elif what == "sums":
@@ -570,13 +594,37 @@ class StepPlan(object):
             for n in nodes:
                 self._node(n, vals, stream)
 
-    def _smooth(self, n, vals, stream, made):
-        ids, consts, chain = self.smooth[n]
-        on, off = np.float32(1), np.float32(0)               # what the operators make of a one and of a zero
-        for m in consts:
+    def _loss(self, n, vals, stream, made):
+        """A gradient and the loss that waited for it."""
+        loss = self.both[n]
+        x, g, out, grad = vals[n.inputs[0]], vals[n.inputs[2]], self.arrays[loss], self.arrays[n]
+        if x.is_contiguous() and grad.is_contiguous():
+            if n in self.smooth:
+                ids = vals[self.smooth[n][0]]
+                ok = ids.is_contiguous() and G.softmax_ce_both_smooth(x, ids, *self._on_off(n), g, out, grad, stream)
+            else:
+                labels = vals[n.inputs[1]]
+                ok = labels.is_contiguous() and G.softmax_ce_both(x, labels, g, out, grad, stream)
+            if ok:
+                vals[loss], vals[n] = out, grad
+                return
+        for m in (loss, n):
+            if m in self.smooth:
+                self._smooth(m, vals, stream, made)
+            else:
+                self._node(m, vals, stream)
+
+    def _on_off(self, n):
+        """What the operators of smoothed labels make of a one and of a zero."""
+        on, off = np.float32(1), np.float32(0)
+        for m in self.smooth[n][1]:
             c = np.float32(_constant(m))
             on, off = (on * c, off * c) if isinstance(m.op, MulConstOp) else (on + c, off + c)
-        on, off = float(on), float(off)
+        return float(on), float(off)
+
+    def _smooth(self, n, vals, stream, made):
+        ids, _, chain = self.smooth[n]
+        on, off = self._on_off(n)
         x, i, out = vals[n.inputs[0]], vals[ids], self.arrays[n]
         ok = x.is_contiguous() and i.is_contiguous() and out.is_contiguous()
         if ok and isinstance(n.op, SoftmaxCrossEntropyOp):

@@ -264,6 +264,27 @@ def softmax_ce_smooth(logits, ids, on, off, loss, stream):
     return rc == 0
 
 
+def softmax_ce_both(logits, labels, g, loss, dx, stream):
+    """Loss and gradient, the logits read once; False: not on a GPU."""
+    if not logits.is_cuda:
+        return False
+    rows, cols = logits.shape
+    _check(lib().tsb_softmax_ce_both(_p(logits), _p(labels), _p(g), _p(loss), _p(dx), c_int64(rows), c_int64(cols), _s(stream)),
+           "softmax_ce_both")
+    return True
+
+
+def softmax_ce_both_smooth(logits, ids, on, off, g, loss, dx, stream):
+    if not logits.is_cuda:
+        return False
+    rows, cols = logits.shape
+    rc = lib().tsb_softmax_ce_both_smooth(_p(logits), _p(ids), c_float(on), c_float(off), _p(g), _p(loss), _p(dx), c_int64(rows),
+                                          c_int64(cols), _s(stream))
+    if rc != 2:
+        _check(rc, "softmax_ce_both_smooth")
+    return rc == 0
+
+
 def softmax_ce_grad_smooth(logits, ids, on, off, g, dx, stream):
     rows, cols = logits.shape
     rc = lib().tsb_softmax_ce_grad_smooth(_p(logits), _p(ids), c_float(on), c_float(off), _p(g), _p(dx), c_int64(rows),
