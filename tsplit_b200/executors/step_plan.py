@@ -5,9 +5,10 @@ come from class ids (the same sum, added up in another order):
 
 * element-wise operators over the same elements are collected and run as one ``tsb_pointwise`` program, at the first
   node that needs one of their results; results that nobody outside the program reads are not stored;
-* a reshape of a row-major array is a view of it;
+* a reshape of a row-major array is a view of it, and so is a slice that only products read;
 * the small parameter gradients that a normalisation operator hands out from its own buffers are copied in one launch;
-* small matrix products that are ready together run as one launch, and so do column sums of a few rows;
+* small matrix products that are ready together run as one launch, and so do column sums of a few rows, which wait until
+  there is a launch of them or nothing else is left to do;
 * the bias of a product, and the ReLU behind it, are added where the product stores its outputs;
 * one-hot labels, scaled and shifted (label smoothing), that only a cross-entropy reads are not made: it takes the ids;
 * a loss and its gradient come from one pass over the logits, when the gradient is due.
@@ -29,7 +30,7 @@ from ..ops.linalg import MatMulOp, _mm_shape
 from ..ops.loss import SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp
 from ..ops.misc import OneHotOp, PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
 from ..ops.norm import BatchNormGradScaleOp
-from ..ops.shape import AddBroadcastOp, ReduceSumOp, ReshapeOp, ReshapeGradientOp
+from ..ops.shape import AddBroadcastOp, ReduceSumOp, ReshapeOp, ReshapeGradientOp, SliceOp
 
 FULL, ROW, SCALAR = 0, 1, 2
 _BINARY = 32                       # instruction code of binary operator 0
@@ -49,6 +50,13 @@ def _key(arr):
     if t.is_contiguous():
         return ("rows", t.numel())
     return (arr.shape, arr.strides) if arr.is_dense() else None
+
+
+def _row_stride(arr):
+    """Of a matrix whose rows are contiguous, dense or a slice of wider ones; 0: another layout."""
+    if arr.is_contiguous():
+        return arr.shape[-1]
+    return arr.strides[0] if len(arr.shape) == 2 and arr.strides[1] == 1 and arr.strides[0] >= arr.shape[1] else 0
 
 
 def _code(node):
@@ -154,6 +162,7 @@ class StepPlan(object):
         for n in ex.topo_order:
             if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
                 self._smooth_labels(n)
+        self.sliced = {n for n in ex.topo_order if n not in self.external and isinstance(n.op, SliceOp) and self._is_sliced(n)}
         self.both = {}                           # gradient of a loss -> the loss that is computed with it
         for n in ex.topo_order:
             if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
@@ -215,6 +224,12 @@ class StepPlan(object):
         src, arr = self.arrays.get(n.inputs[0]), self.arrays.get(n)
         return (src is not None and arr is not None and n.inputs[0] not in self.evals and src.t.is_contiguous()
                 and arr.t.is_contiguous() and src.t.numel() == arr.t.numel())
+
+    def _is_sliced(self, n):
+        """Rows and columns of a value that is there from the start, for products, which take any row stride."""
+        users = self.users.get(n, ())
+        return (n not in self.evals and n.inputs[0] in self.external and len(self.shapes[n]) == 2 and len(users) > 0
+                and all(isinstance(u.op, MatMulOp) and not self._has_effects(u) for u in users))
 
     def _operands(self, n):
         """[(node, kind)] when ``n`` can be part of a program, else None."""
@@ -307,21 +322,27 @@ class StepPlan(object):
         inside = set(nodes)
         waits = {n: sum(1 for i in set(n.inputs) if i in inside) for n in nodes}
         users = self.users
-        light, heavy = [], []             # ready nodes: those that cost no launch of their own, the others
+        # ready nodes: those that cost no launch of their own, the others, and of these the column sums that may wait
+        light, heavy, sums, waiting = [], [], [], 0
         self.queues, self.gone = {}, set()
 
         def ready(n):
+            nonlocal waiting
             cls, ops = "elided" if n in self.elided or n in self.stored else self._kind(n), None
             if cls == "element":
                 ops = self._operands(n)
                 cls = None if ops is None else cls
+            elif n in self.sliced:
+                cls = "slice"
             elif cls == "other" or cls == "view" and not self._is_view(n):
                 cls = None
             if cls:
                 heapq.heappush(light, (n.id, n, cls, ops))
                 return
-            heapq.heappush(heavy, (n.id, n))
             group = self.group_of[n] = self._group(n)
+            may_wait = group is not None and group[0] == ("sums",)
+            heapq.heappush(sums if may_wait else heavy, (n.id, n))
+            waiting += may_wait
             if group:
                 heapq.heappush(self.queues.setdefault(group[0], []), (n.id, n, group[1]))
 
@@ -334,11 +355,13 @@ class StepPlan(object):
         for n in nodes:
             if waits[n] == 0:
                 ready(n)
-        while light or heavy:
+        while light or heavy or sums:
             if light:
                 _, n, cls, ops = heapq.heappop(light)
                 if cls == "elided":
                     pass
+                elif cls == "slice":
+                    self.actions.append(("slice", n))
                 elif cls == "view":
                     self._view(n)
                 elif cls == "copy":
@@ -348,10 +371,12 @@ class StepPlan(object):
                 else:
                     self._collect(n, ops)
             else:
-                _, n = heapq.heappop(heavy)
+                _, n = heapq.heappop(heavy if heavy and waiting < MAX_GROUP else sums or heavy)
                 if n in self.gone:
                     continue
                 taken = self._mates(n)
+                if self.group_of[n] and self.group_of[n][0] == ("sums",):
+                    waiting -= len(taken)
                 for m in taken:
                     for i in m.inputs:
                         self._need(i)
@@ -360,7 +385,8 @@ class StepPlan(object):
                 self.actions.append((self.group_of[n][0][0], taken) if len(taken) > 1 else
                                     ("smooth", n) if n in self.smooth else
                                     ("loss", n) if n in self.both or n in self.late else
-                                    ("products", taken) if n in self.dense else ("node", n))
+                                    ("products", taken) if n in self.dense or not self.sliced.isdisjoint(n.inputs) else
+                                    ("node", n))
                 for m in taken[1:]:
                     done(m)
             done(n)
@@ -499,6 +525,8 @@ class StepPlan(object):
                 self._node(x, vals, stream)
             elif what == "view":
                 vals[x] = self.arrays[x]
+            elif what == "slice":
+                vals[x] = self._slice(x, vals[x.inputs[0]], vals, stream)
             elif what in ("loss", "smooth"):
                 if x in self.late:
                     vals[x] = self.arrays[x]         # (a seed of ones takes its shape)
@@ -528,6 +556,18 @@ class StepPlan(object):
                     for n in x:
                         self._node(n, vals, stream)
 
+    def _slice(self, n, src, vals, stream):
+        """A view of ``src`` that products read in place, or else ``n``'s own array with the values in it."""
+        begin, own = n.attrs["begin"], self.arrays[n]
+        if src.is_contiguous() and src.shape[1] % 4 == 0 and own.is_contiguous():
+            at = src.t.storage_offset() + begin[0] * src.shape[1] + begin[1]
+            view = ndarray.NDArray(src.t.as_strided(own.shape, (src.shape[1], 1), at), src.ctx, owns=False)
+            view._base = src
+            if view.ptr % 16 == 0:
+                return view
+        n.op.compute(n, [src], own, False, stream)
+        return own
+
     def _products(self, nodes, vals, stream):
         ta, tb = nodes[0].attrs["trans_A"], nodes[0].attrs["trans_B"]
         if (self.refused.get(nodes[0], 0) < 2 and any(n in self.dense for n in nodes)
@@ -536,11 +576,13 @@ class StepPlan(object):
         items, alone = [], []
         for n in nodes:
             a, b, out = vals[n.inputs[0]], vals[n.inputs[1]], self.arrays[n]
-            if a.is_contiguous() and b.is_contiguous() and out.is_contiguous() and G.gemm_group_takes(a, b):
+            if _row_stride(a) and _row_stride(b) and out.is_contiguous() and G.gemm_group_takes(a, b):
                 items.append((n, (a, b, out) + _mm_shape(a.shape, b.shape, ta, tb)))
             else:
                 alone.append(n)            # (a row of 10 classes needs padding, which a group does not do)
-        if len(items) > 1 and G.gemm_group([i for _, i in items], ta, tb, stream):
+        one = len(items) == 1 and not self.sliced.isdisjoint(items[0][0].inputs)
+        if (len(items) > 1 and G.gemm_group([i for _, i in items], ta, tb, stream)
+                or one and G.gemm_dense([i + (None, None) for _, i in items], ta, tb, stream)):
             for n, _ in items:
                 vals[n] = self.arrays[n]
         else:
@@ -560,7 +602,7 @@ class StepPlan(object):
             bias, relu = self.dense.get(n, (None, None))
             a, b = vals[n.inputs[0]], vals[n.inputs[1]]
             row = vals[bias.inputs[1]] if bias is not None else None
-            if not (a.is_contiguous() and b.is_contiguous() and (row is None or row.is_contiguous())):
+            if not (_row_stride(a) and _row_stride(b) and (row is None or row.is_contiguous())):
                 return False
             items.append((a, b, self.arrays[n if bias is None else bias]) + _mm_shape(a.shape, b.shape, ta, tb)
                          + (row, None if relu is None else self.arrays[relu]))
@@ -641,6 +683,10 @@ class StepPlan(object):
         self._node(n, vals, stream)
 
     def _node(self, n, vals, stream):
+        for i in n.inputs:
+            if i in self.sliced and not vals[i].is_contiguous():       # an operator that reads whole arrays only
+                i.op.compute(i, [vals[i.inputs[0]]], self.arrays[i], False, stream)
+                vals[i] = self.arrays[i]
         out = self.arrays.get(n)
         n.op.compute(n, [vals[i] for i in n.inputs], out, False, stream)
         vals[n] = out

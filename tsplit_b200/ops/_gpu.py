@@ -480,9 +480,14 @@ def gemm(a, b, c, trans_a, trans_b, stream, batch=1, sa=0, sb=0, sc=0, m=None, n
     _check(rc, "gemm_tf32")
 
 
+def _ld(a):
+    """Row stride of a matrix with contiguous rows."""
+    return a.shape[1] if a.is_contiguous() else a.strides[0]
+
+
 def gemm_group_takes(a, b):
     """Whether a product of these operands may be in a group: TMA reads them where they are."""
-    return not ((a.shape[1] | b.shape[1]) & 3 or (a.ptr | b.ptr) & 15)
+    return not ((_ld(a) | _ld(b)) & 3 or (a.ptr | b.ptr) & 15)
 
 
 def gemm_group(products, trans_a, trans_b, stream):
@@ -490,7 +495,7 @@ def gemm_group(products, trans_a, trans_b, stream):
     cnt = len(products)
     ptr = lambda j: (c_void_p * cnt)(*[p[j].ptr for p in products])
     num = lambda j: (c_int * cnt)(*[p[j] for p in products])
-    ld = lambda j: (c_int64 * cnt)(*[p[j].shape[1] for p in products])
+    ld = lambda j: (c_int64 * cnt)(*[_ld(p[j]) for p in products])
     rc = lib().tsb_gemm_tf32_group(c_int(cnt), ptr(0), ptr(1), ptr(2), num(3), num(4), num(5), ld(0), ld(1), ld(2),
                                    c_int(int(trans_a)), c_int(int(trans_b)), _s(stream))
     if rc != 2:
@@ -507,7 +512,7 @@ def gemm_dense(products, trans_a, trans_b, stream):
         return False
     ptr = lambda j: (c_void_p * cnt)(*[p[j].ptr if p[j] is not None else None for p in products])
     num = lambda j: (c_int * cnt)(*[p[j] for p in products])
-    ld = lambda j: (c_int64 * cnt)(*[p[j].shape[1] for p in products])
+    ld = lambda j: (c_int64 * cnt)(*[_ld(p[j]) for p in products])
     rc = lib().tsb_gemm_tf32_dense(c_int(cnt), ptr(0), ptr(1), ptr(2), num(3), num(4), num(5), ld(0), ld(1), ld(2),
                                    c_int(int(trans_a)), c_int(int(trans_b)), ptr(6), ptr(7), _s(stream))
     if rc != 2:
