@@ -24,6 +24,7 @@
 namespace {
 
 using tsb_launch::load;
+using tsb_launch::load_last;
 
 using namespace tsb_pw;
 
@@ -54,7 +55,7 @@ __global__ void __launch_bounds__(256) unary_flat(const float* x, float* __restr
     float4 v[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u)
-      if (OP != UN_FILL && j + u * 256 < n4) v[u] = load(reinterpret_cast<const float4*>(x) + j + u * 256);
+      if (OP != UN_FILL && j + u * 256 < n4) v[u] = load_last(reinterpret_cast<const float4*>(x) + j + u * 256);
 #pragma unroll
     for (int u = 0; u < 2; ++u)
       if (j + u * 256 < n4) {
@@ -82,8 +83,8 @@ __global__ void __launch_bounds__(256) binary_flat(const float* p, const float* 
 #pragma unroll
     for (int u = 0; u < 2; ++u)
       if (j + u * 256 < n4) {
-        a[u] = load(reinterpret_cast<const float4*>(p) + j + u * 256);
-        b[u] = load(reinterpret_cast<const float4*>(q) + j + u * 256);
+        a[u] = load_last(reinterpret_cast<const float4*>(p) + j + u * 256);
+        b[u] = load_last(reinterpret_cast<const float4*>(q) + j + u * 256);
       }
 #pragma unroll
     for (int u = 0; u < 2; ++u)
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(256) bias_add_v4(const float4* x, const float4
   for (int u = 0; u < 2; ++u) {
     const long long j = i + u * 256;
     if (j < n4) {
-      v[u] = load(x + j);
+      v[u] = load_last(x + j);
       w[u] = load(b + ((n4 >> 32) == 0 ? (unsigned)j % cols4 : (unsigned)(j % cols4)));
     }
   }

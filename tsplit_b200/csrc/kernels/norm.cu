@@ -28,6 +28,7 @@
 namespace {
 
 using tsb_launch::load;
+using tsb_launch::load_last;
 
 constexpr int MAX_CHUNKS = 128;
 constexpr long long PLANE_FLOATS = (long long)MAX_CHUNKS * 8192;   // one partial plane: chunks x channels
@@ -240,12 +241,14 @@ __device__ __forceinline__ void row_col(long long i, int C4, long long total, lo
   }
 }
 
+// Forward from the end of the tensor: the convolution that wrote x wrote its end last, and the one that reads y reads
+// its beginning first (32 x 56 x 56 x 256 37.1 -> 34.8 us with the hint on x, a 3 x 3 max pool after it 27.2 -> 22.9).
 __global__ void __launch_bounds__(256) bn_apply_fwd(const float* x, const float* scale,
                              const float* bias, const float* mean,
                              const float* invstd, float* __restrict__ y, long long rows, int C,
                              long long ldx, long long ldy, int relu) {
   tsb_launch::enter();
-  const long long total = rows * (C >> 2), i = blockIdx.x * (long long)APPLY_TILE + threadIdx.x;
+  const long long total = rows * (C >> 2), i = (gridDim.x - 1 - blockIdx.x) * (long long)APPLY_TILE + threadIdx.x;
   long long r[2];
   int c[2];
   float4 v[2];
@@ -253,7 +256,7 @@ __global__ void __launch_bounds__(256) bn_apply_fwd(const float* x, const float*
   for (int u = 0; u < 2; ++u)
     if (i + u * 256 < total) {
       row_col(i + u * 256, C >> 2, total, r[u], c[u]);
-      v[u] = load(reinterpret_cast<const float4*>(x + r[u] * ldx + c[u]));
+      v[u] = load_last(reinterpret_cast<const float4*>(x + r[u] * ldx + c[u]));
     }
 #pragma unroll
   for (int u = 0; u < 2; ++u)
@@ -285,8 +288,8 @@ __global__ void __launch_bounds__(256) bn_apply_bwd(const float* dy, const float
   for (int u = 0; u < 2; ++u)
     if (i + u * 256 < total) {
       row_col(i + u * 256, C >> 2, total, r[u], c[u]);
-      g[u] = load(reinterpret_cast<const float4*>(dy + r[u] * lddy + c[u]));
-      v[u] = load(reinterpret_cast<const float4*>(x + r[u] * ldx + c[u]));
+      g[u] = load_last(reinterpret_cast<const float4*>(dy + r[u] * lddy + c[u]));
+      v[u] = load_last(reinterpret_cast<const float4*>(x + r[u] * ldx + c[u]));
     }
 #pragma unroll
   for (int u = 0; u < 2; ++u)

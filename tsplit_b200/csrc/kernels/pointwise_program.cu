@@ -58,6 +58,8 @@ __global__ void __launch_bounds__(256) pointwise_program(const __grid_constant__
   const long long i = blockIdx.x * (long long)T + threadIdx.x;
   if (i >= p.n4) return;
   const unsigned in_row = (p.n4 >> 32) == 0 ? (unsigned)i % p.cols4 : (unsigned)(i % p.cols4);
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
   for (int k = 0; k < p.n_in; ++k) {
     if (p.kind[k] == 2) {
       const float v = load(p.in[k]);
@@ -65,7 +67,7 @@ __global__ void __launch_bounds__(256) pointwise_program(const __grid_constant__
     } else {
       const float4* src = reinterpret_cast<const float4*>(p.in[k]) + (p.kind[k] == 0 ? i : in_row);
       const uint32_t dst = (uint32_t)__cvta_generic_to_shared(r + k * T);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+      asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");

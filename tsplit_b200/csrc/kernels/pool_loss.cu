@@ -31,6 +31,7 @@ namespace cg = cooperative_groups;
 namespace {
 
 using tsb_launch::load;
+using tsb_launch::load_last;
 
 int sm_count() {
   static int n = 0;
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(WIN_COLS * WIN_LANES) avg_pool_window(const fl
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int q = i + u * WIN_LANES, qy = q / ww, qx = q - qy * ww;
-        v[u] = q < end ? load(reinterpret_cast<const float4*>(base + (y0 + qy) * p.xsh + (x0 + qx) * p.xsw))
+        v[u] = q < end ? load_last(reinterpret_cast<const float4*>(base + (y0 + qy) * p.xsh + (x0 + qx) * p.xsw))
                        : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
@@ -330,7 +331,7 @@ __global__ void pool_bwd_tiled(const float* x, const float* dy, float* __restric
 #pragma unroll
     for (int a = 0; a < K; ++a)
 #pragma unroll
-      for (int b = 0; b < K; ++b) v[a * K + b] = *reinterpret_cast<const float4*>(x + base + a * p.xsh + b * p.xsw);
+      for (int b = 0; b < K; ++b) v[a * K + b] = load_last(reinterpret_cast<const float4*>(x + base + a * p.xsh + b * p.xsw));
     int ax = 0, ay = 0, az = 0, aw = 0;          // index of the first maximum per channel
     float4 m = v[0];
 #pragma unroll
@@ -771,7 +772,7 @@ __global__ void __launch_bounds__(256) masked_softmax_warp_rows_v4(const float4*
       const int i = lane + 32 * j;
       v[j] = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
       keys[j] = make_float4(1.f, 1.f, 1.f, 1.f);
-      if (i < nvec) v[j] = load(xr + i);
+      if (i < nvec) v[j] = load_last(xr + i);
       if (i < nvec && kt) keys[j] = load(kt + i);
     }
 #pragma unroll
@@ -873,7 +874,7 @@ __global__ void __launch_bounds__(256) scaled_softmax_grad_warp_rows_v4(const fl
     for (int j = 0; j < NV; ++j) {
       const int i = lane + 32 * j;
       a[j] = i < nvec ? load(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      g[j] = i < nvec ? load(gr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      g[j] = i < nvec ? load_last(gr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
       s += (a[j].x * g[j].x + a[j].y * g[j].y) + (a[j].z * g[j].z + a[j].w * g[j].w);
     }
 #pragma unroll
