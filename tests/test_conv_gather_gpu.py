@@ -29,10 +29,12 @@ def test_forward_and_gradients(n, c, h, w, o, kh, kw, ph, pw, stride):
 
 # both channel counts multiples of 32, where the data gradient reads the filters in place: one tile, ragged tiles, CTA pairs,
 # filters larger than the padding, a pointwise and an asymmetric one, the four parities of stride 2
+# (which write their pixels of dx: tiles that cross rows and images, several to a CTA, classes without rows or taps)
 @pytest.mark.parametrize("n,c,h,w,o,kh,kw,ph,pw,stride", [
     (2, 32, 9, 9, 32, 3, 3, 1, 1, 1), (3, 96, 17, 19, 64, 5, 3, 2, 0, 1), (4, 320, 60, 61, 64, 3, 3, 1, 1, 1),
     (4, 256, 50, 47, 96, 1, 1, 0, 0, 1), (2, 224, 17, 17, 192, 1, 7, 0, 3, 1), (2, 32, 9, 9, 32, 7, 7, 3, 3, 2),
-    (3, 96, 17, 20, 64, 5, 5, 2, 2, 2), (8, 512, 28, 28, 128, 1, 1, 0, 0, 2)])
+    (3, 96, 17, 20, 64, 5, 5, 2, 2, 2), (8, 512, 28, 28, 128, 1, 1, 0, 0, 2),
+    (24, 256, 56, 55, 32, 3, 3, 1, 1, 2), (5, 288, 33, 31, 32, 2, 3, 0, 1, 2), (2, 32, 1, 9, 32, 1, 1, 0, 0, 2)])
 def test_data_gradient_from_filters_in_place(n, c, h, w, o, kh, kw, ph, pw, stride):
     _check(n, c, h, w, o, kh, kw, ph, pw, stride)
 

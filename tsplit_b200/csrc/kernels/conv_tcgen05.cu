@@ -59,6 +59,8 @@ struct ConvParams {
   long long stats_plane;   // floats between the plane of sums and the plane of sums of squares
   int a3d;             // wgrad: dy arrives through the 3-D (32 channels, pixel, chunk) view
   int f_step, f_rh, f_rw, f_kw;   // data gradient as a forward launch: where the filters lie (see filter_tap); f_step 0: plain filters
+  long long out_sn, out_sh;    // floats between images, rows and pixels of an output that is not dense (a parity class of a
+  int out_sw;                  // strided data gradient); out_sw 0: it is
   int* status;
   unsigned long long* prof;   // role-time counters (only written when built with -DTSB_CONV_PROF)
 };
@@ -208,6 +210,48 @@ __device__ __forceinline__ void store_last_tile(const CUtensorMap* tmo, const Co
 // This is the tap of the filters that tap (kh, kw) of the launch multiplies.
 __device__ __forceinline__ int filter_tap(const ConvParams& p, int kh, int kw) {
   return (p.f_step * (p.KH - 1 - kh) + p.f_rh) * p.f_kw + p.f_step * (p.KW - 1 - kw) + p.f_rw;
+}
+
+// A tile of one parity class of a strided data gradient: its rows are every other pixel of every other row of dx, out of a
+// TMA store's reach (a block of 32 crosses the ends of rows).  The warp turns 32 rows x 16 columns in shared memory and
+// writes 64 bytes of eight rows at a time.  Whole data gradients of 32 images, against dense classes and a pass that interleaved
+// them: 3x3 128 to 56 x 56 61.1 -> 35.7 us, 256 to 28 x 28 43.9 -> 30.1; 1x1 512 to 56 x 56 x 256 53.8 -> 34.0.
+template <int BN>
+__device__ __forceinline__ void store_class_tile(const ConvParams& p, uint8_t* stg, uint32_t tmem, int lane, int n0, int row0) {
+  const int row = row0 + lane, pixels = p.OH * p.OW, n = row / pixels, rem = row - n * pixels, y = rem / p.OW, x = rem - y * p.OW;
+  const long long off = row < p.M ? n * p.out_sn + y * p.out_sh + (long long)x * p.out_sw : -1;
+  float* at[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const long long o = __shfl_sync(0xffffffffu, off, i * 8 + (lane >> 2));
+    at[i] = o < 0 ? nullptr : p.out + o + n0 + (lane & 3) * 4;
+  }
+  const uint32_t base = smem_u32(stg), srow = base + lane * 64, sx = (uint32_t)(lane >> 1) & 3;
+#pragma unroll 1
+  for (int c0 = 0; c0 < BN && n0 + c0 < p.NC; c0 += 32) {
+    float v[32];
+    tmem_ld_32x32(tmem + c0, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      __syncwarp();                        // everybody has read the block before
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int j = half * 16 + c * 4;
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(srow + (((uint32_t)c ^ sx) << 4)), "f"(v[j]), "f"(v[j + 1]),
+                     "f"(v[j + 2]), "f"(v[j + 3]) : "memory");
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t r = i * 8 + (lane >> 2);
+        float4 o;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w)
+                     : "r"(base + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4)) : "memory");
+        if (at[i]) *reinterpret_cast<float4*>(at[i] + c0 + half * 16) = o;
+      }
+    }
+  }
 }
 
 struct Item {
@@ -511,6 +555,13 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__
       } else {
         crow = p.out + (long long)row * p.ldc + coloff;
         accumulate = p.accumulate != 0;
+      }
+      if (FLIP && p.out_sw) {
+        store_class_tile<BN>(p, smem_stg + q * 2048, tmem_base + acc * BN + ((uint32_t)(q * 32) << 16), lane, w.n0, w.m0 + q * 32);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0 && item + 2 * (long long)gridDim.x < items) mbar_arrive(&tempty[acc]);
+        continue;
       }
       if (p.tma_store && item + gridDim.x >= items) {
         store_last_tile<BN>(&tmo, p, smem_a + q * BN * 128, tmem_base + acc * BN + ((uint32_t)(q * 32) << 16), has_k, lane, w.n0,
@@ -961,6 +1012,13 @@ conv_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
       if (!mbar_wait(&tfull[acc], acc_ph, p.status, 0x214)) { ok = false; break; }
       tc_fence_after();
       const int row0 = m0 + q * 32;
+      if (FLIP && p.out_sw) {
+        store_class_tile<BN>(p, stg, tmem_base + acc * BN + ((uint32_t)(q * 32) << 16), lane, n0, row0);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0 && item + 2 * npairs < items) mbar_arrive_leader(&tempty[acc]);
+        continue;
+      }
       if (item + npairs >= items) {
         store_last_tile<BN>(&tmo, p, smem_a + q * BN * 128, tmem_base + acc * BN + ((uint32_t)(q * 32) << 16), true, lane, n0, row0,
                             row0, p.stats ? my_stat : nullptr);
@@ -1278,7 +1336,8 @@ __global__ void upsample_zero_insert(const float* dy, float* __restrict__ up, in
 //     dx_a[i] = sum_t dy[i + q - t] * w[2t + r]
 // which is the data gradient of a STRIDE-1 convolution with the sub-filter w[2t + r] (T taps) and padding q.  So
 // each of the four (row parity, column parity) classes is one stride-1 forward launch over dy with the class's
-// flipped, transposed sub-filter; the four dense results are then interleaved into dx by one kernel.  The launch
+// flipped, transposed sub-filter, which writes its pixels of dx (channels of no 32: dense results, interleaved into dx
+// by one kernel).  The launch
 // pads dy by T - 1 - q at the leading edge and by R - OH + q at the trailing edge (R = ceil((H - a) / 2) rows of
 // the class; the two differ, and the trailing one may be negative), so it produces exactly R rows.
 // 3x3 / pad 1: 1 + 2 taps per axis, 9 tap-positions per 2x2 block of dx against 36 on the zero-inserted
@@ -1345,6 +1404,16 @@ __global__ void parity_interleave(const ParityParts pp, float* __restrict__ dx, 
       v = tsb_launch::load_last(reinterpret_cast<const float4*>(src + (((long long)n * pp.R[k][0] + (y >> 1)) * pp.R[k][1] + (x >> 1)) * C + c));
     *reinterpret_cast<float4*>(dx + i * 4) = v;
   }
+}
+
+// Zeros in the pixels of dx whose class (2 * row parity + column parity) is a bit of `zero`; a block per row.
+__global__ void __launch_bounds__(256) parity_zeros(float* __restrict__ dx, int zero, int H, int W, int C4) {
+  tsb_launch::enter();
+  const int classes = zero >> ((blockIdx.x % (unsigned)H & 1) * 2) & 3;
+  if (!classes) return;
+  float4* row = reinterpret_cast<float4*>(dx) + (long long)blockIdx.x * W * C4;
+  for (int i = threadIdx.x; i < W * C4; i += 256)
+    if (classes >> (i / C4 & 1) & 1) row[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // (Channel counts are multiples of four, so filters are whole float4.)  Eight partial sums in flight per thread instead
@@ -1494,7 +1563,7 @@ ConvParams base_params(int N, int C, int H, int W, int O, int KH, int KW, int OH
   p.ph = ph; p.pw = pw; p.stride = p.step_w = stride;
   p.src = nullptr; p.out = nullptr; p.ws = nullptr; p.accumulate = 0; p.splits = 1; p.taps = 1;
   p.K = KH * KW * C; p.ocb = (O + 31) / 32; p.status = nullptr; p.prof = nullptr; p.a3d = 0; p.tma_store = 0; p.stats = nullptr; p.stats_plane = 0;
-  p.f_step = p.f_rh = p.f_rw = p.f_kw = 0; p.M = 0; p.NC = 0; p.kblocks = 0; p.tiles_m = 0; p.tiles_n = 0; p.ldc = 0;
+  p.f_step = p.f_rh = p.f_rw = p.f_kw = p.out_sw = 0; p.out_sn = p.out_sh = 0; p.M = 0; p.NC = 0; p.kblocks = 0; p.tiles_m = 0; p.tiles_n = 0; p.ldc = 0;
   return p;
 }
 
@@ -1519,6 +1588,8 @@ int im2col_map(CUtensorMap* out, const float* a, int N, int C, int H, int W, int
 // (step * (T - 1 - kh) + rh, step * (T' - 1 - kw) + rw).
 struct FlippedFilters {
   int KH, KW, step, rh, rw;
+  long long out_sn = 0, out_sh = 0;      // floats between images, rows and pixels of the output; out_sw 0: it is dense
+  int out_sw = 0;
 };
 
 // out[N,OH,OW,O] = conv(src[N,H,W,C], wts[O,KH,KW,C]).  Serves forward, and stride-1 dgrad with
@@ -1557,6 +1628,7 @@ int run_forward(const float* src, const float* wts, float* out, int N, int C, in
   if (flip) {
     if (C % 32 || O % 32) return TSB_ERR_UNSUPPORTED;
     p.f_step = flip->step; p.f_rh = flip->rh; p.f_rw = flip->rw; p.f_kw = flip->KW;
+    p.out_sn = flip->out_sn; p.out_sh = flip->out_sh; p.out_sw = flip->out_sw;
   }
   int rc = filter_map(&tm, bn);
   if (rc) return rc;
@@ -1666,6 +1738,25 @@ int run_dgrad_parity(float* dx, const float* w, const float* dy, int N, int C, i
   for (int a = 0; a < 2; ++a) {
     if (!parity_axis(H, OH, KH, ph, a, &ax[a]) || !parity_axis(W, OW, KW, pw, a, &bx[a])) return TSB_ERR_UNSUPPORTED;
   }
+  // Channels in whole 32s: every class reads the filters in place and writes its own pixels of dx.
+  if (C % 32 == 0) {
+    int rc = TSB_OK, zero = 0;
+    for (int k = 0; k < 4 && rc == TSB_OK; ++k) {
+      const ParityAxis &A = ax[k >> 1], &B = bx[k & 1];
+      if (A.R == 0 || B.R == 0) continue;
+      if (A.empty || B.empty) { zero |= 1 << k; continue; }
+      FlippedFilters flip = {KH, KW, 2, A.r, B.r};
+      flip.out_sn = (long long)H * W * C; flip.out_sh = 2ll * W * C; flip.out_sw = 2 * C;
+      rc = run_forward(dy, w, dx + ((long long)(k >> 1) * W + (k & 1)) * C, N, O, OH, OW, C, A.T, B.T, A.R, B.R, A.pad_lead,
+                       B.pad_lead, 1, st, nullptr, 0, 0, nullptr, A.pad_trail, B.pad_trail, &flip);
+    }
+    if (rc == TSB_OK && zero) {
+      tsb_launch::launch(parity_zeros, dim3((unsigned)((long long)N * H)), 256, 0, st, dx, zero, H, W, C / 4);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
+    }
+    if (rc != TSB_ERR_UNSUPPORTED) return rc;
+  }
   size_t wmax = 0, ptotal = 0, poff[4] = {0, 0, 0, 0};
   bool live[4];
   for (int a = 0; a < 2; ++a)
@@ -1690,20 +1781,15 @@ int run_dgrad_parity(float* dx, const float* w, const float* dy, int N, int C, i
       pp.R[k][0] = A.R; pp.R[k][1] = B.R;
       if (!live[k]) continue;
       float* part = reinterpret_cast<float*>(reinterpret_cast<char*>(parts) + poff[k]);
-      const FlippedFilters flip = {KH, KW, 2, A.r, B.r};
-      int rc = run_forward(dy, w, part, N, O, OH, OW, C, A.T, B.T, A.R, B.R, A.pad_lead, B.pad_lead, 1, st, nullptr, 0, 0, nullptr,
-                           A.pad_trail, B.pad_trail, &flip);
-      if (rc == TSB_ERR_UNSUPPORTED) {      // channels of no 32: filters transposed in scratch
-        float* wk = get_ws(st, 1, 4 * wmax, size_t(16) << 20);
-        if (!wk) return TSB_ERR_OOM;
-        wk += (size_t)k * (wmax / sizeof(float));      // every class has its own: the four launches are queued back to back
-        dim3 grid((C + 31) / 32, (O + 31) / 32, A.T * B.T);
-        tsb_launch::launch(parity_filters, grid, dim3(32, 8), 0, st, w, wk, O, C, KH, KW, A.r, A.T, B.r, B.T);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
-        rc = run_forward(dy, wk, part, N, O, OH, OW, C, A.T, B.T, A.R, B.R, A.pad_lead, B.pad_lead, 1, st, nullptr, 0, 0, nullptr,
-                         A.pad_trail, B.pad_trail);
-      }
+      float* wk = get_ws(st, 1, 4 * wmax, size_t(16) << 20);
+      if (!wk) return TSB_ERR_OOM;
+      wk += (size_t)k * (wmax / sizeof(float));      // every class has its own: the four launches are queued back to back
+      dim3 grid((C + 31) / 32, (O + 31) / 32, A.T * B.T);
+      tsb_launch::launch(parity_filters, grid, dim3(32, 8), 0, st, w, wk, O, C, KH, KW, A.r, A.T, B.r, B.T);
+      cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return TSB_ERR_LAUNCH | ((int)e << 8);
+      const int rc = run_forward(dy, wk, part, N, O, OH, OW, C, A.T, B.T, A.R, B.R, A.pad_lead, B.pad_lead, 1, st, nullptr, 0, 0,
+                                 nullptr, A.pad_trail, B.pad_trail);
       if (rc) return rc;
       pp.part[k] = part;
     }
