@@ -158,29 +158,28 @@ col_partial(const float* a, const float* b, const float* mean,
   }
 }
 
-// Sum of the chunk partials of one channel, in double and in a fixed order: block = 32 channels
-// x FIN_LANES lanes; lane y adds chunks y, y+FIN_LANES, ... (four independent loads in flight),
-// lane 0 then adds the lane sums.
-constexpr int FIN_LANES = 32;
+// Sum of the chunk partials of one channel, in double and in a fixed order: block = FIN_CHANNELS channels x FIN_LANES
+// lanes; lane y adds chunks y, y + FIN_LANES, ... (four loads of each plane in flight), lane 0 then adds the lane sums.
+// Bound by the launch and a few round trips to L2, so blocks are short: with 32 channels one took a whole SM's threads and
+// could not be placed before the kernel ahead had left it (the 53 of a ResNet-50 step 222 -> 206 us forward, 194 -> 165
+// backward; 16 channels 222 and 194; with ten loads in flight, and the registers for them, 231 and 203).
+constexpr int FIN_CHANNELS = 8, FIN_LANES = 32;
 __device__ __forceinline__ void reduce_partials(const float* part, int chunks, int C, int c,
                                                 double& s, double& ss, long long plane = PLANE_FLOATS) {
-  __shared__ double sh0[FIN_LANES][33], sh1[FIN_LANES][33];
+  __shared__ double sh0[FIN_LANES][FIN_CHANNELS + 1], sh1[FIN_LANES][FIN_CHANNELS + 1];
   double a = 0.0, b = 0.0;
   if (c < C) {
-    int ch = threadIdx.y;
-    for (; ch + 3 * FIN_LANES < chunks; ch += 4 * FIN_LANES) {
+    for (int ch = threadIdx.y; ch < chunks; ch += 4 * FIN_LANES) {
       float x[4], y[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        x[u] = part[(long long)(ch + u * FIN_LANES) * C + c];
-        y[u] = part[plane + (long long)(ch + u * FIN_LANES) * C + c];
-      }
+      for (int u = 0; u < 4; ++u)
+        if (ch + u * FIN_LANES < chunks) {
+          x[u] = part[(long long)(ch + u * FIN_LANES) * C + c];
+          y[u] = part[plane + (long long)(ch + u * FIN_LANES) * C + c];
+        }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) { a += x[u]; b += y[u]; }
-    }
-    for (; ch < chunks; ch += FIN_LANES) {
-      a += part[(long long)ch * C + c];
-      b += part[plane + (long long)ch * C + c];
+      for (int u = 0; u < 4; ++u)
+        if (ch + u * FIN_LANES < chunks) { a += x[u]; b += y[u]; }
     }
   }
   sh0[threadIdx.y][threadIdx.x] = a;
@@ -193,13 +192,14 @@ __device__ __forceinline__ void reduce_partials(const float* part, int chunks, i
   }
 }
 
-// Forward finalise: mean / invstd from the partial sums (+ running statistics).  Block (32, FIN_LANES).
-__global__ void bn_finalize_fwd(const float* part, int chunks, int C, double count, float eps,
-                                float momentum, float* __restrict__ mean, float* __restrict__ invstd,
-                                float* __restrict__ run_mean, float* __restrict__ run_var,
-                                long long plane = PLANE_FLOATS) {
+// Forward finalise: mean / invstd from the partial sums (+ running statistics).  Block (FIN_CHANNELS, FIN_LANES).
+__global__ void __launch_bounds__(FIN_CHANNELS * FIN_LANES)
+bn_finalize_fwd(const float* part, int chunks, int C, double count, float eps,
+                float momentum, float* __restrict__ mean, float* __restrict__ invstd,
+                float* __restrict__ run_mean, float* __restrict__ run_var,
+                long long plane = PLANE_FLOATS) {
   tsb_launch::enter();
-  const int c = blockIdx.x * 32 + threadIdx.x;
+  const int c = blockIdx.x * FIN_CHANNELS + threadIdx.x;
   double s, ss;
   reduce_partials(part, chunks, C, c, s, ss, plane);
   if (threadIdx.y != 0 || c >= C) return;
@@ -214,10 +214,11 @@ __global__ void bn_finalize_fwd(const float* part, int chunks, int C, double cou
   }
 }
 
-__global__ void bn_finalize_bwd(const float* part, int chunks, int C, float* __restrict__ dscale,
-                                float* __restrict__ dbias, long long plane = PLANE_FLOATS) {
+__global__ void __launch_bounds__(FIN_CHANNELS * FIN_LANES)
+bn_finalize_bwd(const float* part, int chunks, int C, float* __restrict__ dscale,
+                float* __restrict__ dbias, long long plane = PLANE_FLOATS) {
   tsb_launch::enter();
-  const int c = blockIdx.x * 32 + threadIdx.x;
+  const int c = blockIdx.x * FIN_CHANNELS + threadIdx.x;
   double s, ss;
   reduce_partials(part, chunks, C, c, s, ss, plane);
   if (threadIdx.y != 0 || c >= C) return;
@@ -354,7 +355,7 @@ StatGeom stat_geom(long long rows, int C, long long chunk_cap = 1 << 30) {
   g.grid = dim3((unsigned)col_blocks, (unsigned)g.chunks);
   return g;
 }
-inline unsigned fin_blocks(long long C) { return (unsigned)((C + 31) / 32); }
+inline unsigned fin_blocks(long long C) { return (unsigned)((C + FIN_CHANNELS - 1) / FIN_CHANNELS); }
 
 unsigned apply_grid(long long rows, long long C) { return (unsigned)((rows * (C / 4) + APPLY_TILE - 1) / APPLY_TILE); }
 
@@ -550,7 +551,7 @@ int tsb_bn_forward(const float* x, const float* scale, const float* bias, float*
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<0>, sg.grid, STAT_THREADS, 0, st, x, nullptr, nullptr, nullptr, part, rows, (int)C,
                      ldx, 0, sg.chunks, sg.cw, nullptr, nullptr, PLANE_FLOATS);
-  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C, (double)rows,
+  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, sg.chunks, (int)C, (double)rows,
                      eps, momentum, save_mean, save_invstd, run_mean, run_var, PLANE_FLOATS);
   tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y, rows,
                      (int)C, ldx, ldy, relu);
@@ -566,7 +567,7 @@ int tsb_bn_forward_from_partials(const float* part, int chunks, long long plane,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows <= 0 || C <= 0 || chunks <= 0 || !part) return TSB_ERR_ARG;
   if ((C % 4) || (ldx % 4) || (ldy % 4)) return TSB_ERR_UNSUPPORTED;
-  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, chunks, (int)C, (double)rows,
+  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, chunks, (int)C, (double)rows,
                      eps, momentum, save_mean, save_invstd, run_mean, run_var, plane);
   tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y, rows,
                      (int)C, ldx, ldy, relu);
@@ -603,7 +604,7 @@ int tsb_bn_forward_static(const float* x, const float* scale, const float* bias,
   // same call, so nothing in the shared array has to be cleared between calls
   tsb_launch::launch(col_partial<0>, sg.grid, STAT_THREADS, 0, st, x, nullptr, nullptr, nullptr, part, rows, (int)C,
                      ldx, 0, sg.chunks, sg.cw, nullptr, nullptr, PLANE_FLOATS);
-  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C, (double)rows,
+  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, sg.chunks, (int)C, (double)rows,
                      eps, momentum, save_mean, save_invstd, run_mean, run_var, PLANE_FLOATS);
   tsb_launch::launch(bn_apply_fwd, apply_grid(rows, C), 256, 0, st, x, scale, bias, save_mean, save_invstd, y, rows,
                      (int)C, ldx, ldy, relu);
@@ -621,7 +622,7 @@ int tsb_bn_backward(const float* dy, const float* x, const float* scale, const f
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<1>, sg.grid, STAT_THREADS, 0, st, dy, x, save_mean, save_invstd, part, rows, (int)C,
                      lddy, ldx, sg.chunks, sg.cw, nullptr, nullptr, PLANE_FLOATS);
-  tsb_launch::launch(bn_finalize_bwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C, dscale,
+  tsb_launch::launch(bn_finalize_bwd, fin_blocks(C), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, sg.chunks, (int)C, dscale,
                      dbias, PLANE_FLOATS);
   tsb_launch::launch(bn_apply_bwd, apply_grid(rows, C), 256, 0, st, dy, x, scale, save_mean, save_invstd, dscale,
                      dbias, dx, rows, (int)C, lddy, ldx, lddx, 1.f / (float)rows, nullptr);
@@ -642,7 +643,7 @@ int tsb_bn_relu_backward(const float* dy, const float* x, const float* scale, co
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<1>, sg.grid, STAT_THREADS, 0, st, dy, x, save_mean, save_invstd, part, rows, (int)C,
                      lddy, ldx, sg.chunks, sg.cw, scale, bias, PLANE_FLOATS);
-  tsb_launch::launch(bn_finalize_bwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, sg.chunks, (int)C, dscale,
+  tsb_launch::launch(bn_finalize_bwd, fin_blocks(C), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, sg.chunks, (int)C, dscale,
                      dbias, PLANE_FLOATS);
   tsb_launch::launch(bn_apply_bwd, apply_grid(rows, C), 256, 0, st, dy, x, scale, save_mean, save_invstd, dscale,
                      dbias, dx, rows, (int)C, lddy, ldx, lddx, 1.f / (float)rows, bias);
@@ -675,7 +676,7 @@ int tsb_bn_stats_finalize(const float* part, long long plane, int chunks, double
                           void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (chunks <= 0 || C <= 0 || count <= 0 || !part) return TSB_ERR_ARG;
-  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, chunks, (int)C, count, eps,
+  tsb_launch::launch(bn_finalize_fwd, fin_blocks(C), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, chunks, (int)C, count, eps,
                      momentum, mean, invstd, run_mean, run_var, plane);
   return done();
 }
@@ -701,7 +702,7 @@ int tsb_bn_bwd_finalize(const float* part, long long plane, int chunks, long lon
                         void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (chunks <= 0 || C <= 0 || !part) return TSB_ERR_ARG;
-  tsb_launch::launch(bn_finalize_bwd, fin_blocks(C), dim3(32, FIN_LANES), 0, st, part, chunks, (int)C, dscale, dbias,
+  tsb_launch::launch(bn_finalize_bwd, fin_blocks(C), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, chunks, (int)C, dscale, dbias,
                      plane);
   return done();
 }
@@ -762,13 +763,13 @@ int tsb_layer_norm_grad(const float* dy, const float* x, const float* scale, con
     dim3 grid4((unsigned)((D4 + bt - 1) / bt), chunks);
     tsb_launch::launch(ln_bwd_params_partial_v4, grid4, bt, 0, st, reinterpret_cast<const float4*>(dy),
                        reinterpret_cast<const float4*>(x), mean, invstd, part, rows, D4, chunks);
-    tsb_launch::launch(bn_finalize_bwd, fin_blocks(D), dim3(32, FIN_LANES), 0, st, part, chunks, (int)D, dscale, dbias,
+    tsb_launch::launch(bn_finalize_bwd, fin_blocks(D), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, chunks, (int)D, dscale, dbias,
                        PLANE_FLOATS);
     return done();
   }
   dim3 grid((unsigned)((D + 127) / 128), chunks);
   tsb_launch::launch(ln_bwd_params_partial, grid, 128, 0, st, dy, x, mean, invstd, part, rows, (int)D, chunks);
-  tsb_launch::launch(bn_finalize_bwd, fin_blocks(D), dim3(32, FIN_LANES), 0, st, part, chunks, (int)D, dscale, dbias,
+  tsb_launch::launch(bn_finalize_bwd, fin_blocks(D), dim3(FIN_CHANNELS, FIN_LANES), 0, st, part, chunks, (int)D, dscale, dbias,
                      PLANE_FLOATS);
   return done();
 }
