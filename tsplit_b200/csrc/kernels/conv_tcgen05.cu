@@ -1416,13 +1416,12 @@ __global__ void __launch_bounds__(256) parity_zeros(float* __restrict__ dx, int 
     if (classes >> (i / C4 & 1) & 1) row[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// (Channel counts are multiples of four, so filters are whole float4.)  Eight partial sums in flight per thread instead
-// of one float after another.  Whole filter gradients of 32 images: 512 x 512 x 3 x 3 at 7 x 7 29.2 -> 26.9 us, 512 x 128 at
-// 28 x 28 21.9 -> 20.7, 64 x 64 x 3 x 3 at 56 x 56 38.9 -> 39.0.
-__global__ void __launch_bounds__(256) conv_splitk_reduce(const float4* ws, float4* __restrict__ out,
+// (Channel counts are multiples of four, so filters are whole float4.)  Short blocks, since many filters are: with 256
+// threads the 52 of a ResNet-50 step take 231 us, with 128 226.
+__global__ void __launch_bounds__(128) conv_splitk_reduce(const float4* ws, float4* __restrict__ out,
                                                           int splits, long long per_split4) {
   tsb_launch::enter();
-  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  const long long i = blockIdx.x * 128ll + threadIdx.x;
   if (i < per_split4) out[i] = tsb::sum_splits(ws + i, splits, per_split4);
 }
 
@@ -1945,7 +1944,7 @@ int tsb_conv2d(int kind, float* x, float* w, float* y, int N, int C, int H, int 
     if (rc) return rc;
     if (p.splits > 1) {
       const long long per_split4 = (long long)O * KH * KW * C / 4;
-      tsb_launch::launch(conv_splitk_reduce, dim3((unsigned)((per_split4 + 255) / 256)), 256, 0, st,
+      tsb_launch::launch(conv_splitk_reduce, dim3((unsigned)((per_split4 + 127) / 128)), 128, 0, st,
                          reinterpret_cast<const float4*>(p.ws), reinterpret_cast<float4*>(p.out), p.splits,
                          per_split4);
       cudaError_t e = cudaGetLastError();

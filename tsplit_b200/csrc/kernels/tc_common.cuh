@@ -275,16 +275,19 @@ __host__ __device__ constexpr uint32_t make_idesc_tf32(int M, int N, int a_mn_ma
          ((uint32_t)(M >> 4) << 24);
 }
 
-// Sum of `splits` partial results, four floats of each, in their order; eight loads in flight.
+// Sum of `splits` partial results, four floats of each, in their order.  The kernels around it last 3 to 5 us, which is
+// their launch and a few round trips to L2.  Loads in flight, us of the 52 conv_splitk_reduce of a ResNet-50 step and of
+// the 17 splitk_reduce_v4 of a Transformer block: 4 258 and 72, 5 248 and 69, 6 231 and 65, 7 237 and 67, 8 264 and 75,
+// 16 283 and 87 (registers and code that every launch places and fetches anew).
 __device__ __forceinline__ float4 sum_splits(const float4* ws, int splits, long long per_split4) {
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s = 0; s < splits; s += 8) {
-    float4 v[8];
+  for (int s = 0; s < splits; s += 6) {
+    float4 v[6];
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
+    for (int u = 0; u < 6; ++u)
       if (s + u < splits) v[u] = __ldcs(ws + (s + u) * per_split4);
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
+    for (int u = 0; u < 6; ++u)
       if (s + u < splits) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
   }
   return acc;
