@@ -59,3 +59,21 @@ def test_pixels_of_four_channels(n, c, h, w):
     y = _arr(torch.full((n, 4, h, w), 7.0, device="cuda"))
     G._to_pixels(x, y, _stream())
     assert torch.equal(y.t[:, :c], x.t) and not y.t[:, c:].any()
+
+
+# windows of 3 x 3 two apart: one pixel, tiles cut in both axes and at a window's middle, a ragged channel block, rows that no
+# window reaches; many ties, and values below any finite one
+@pytest.mark.parametrize("pad", [0, 1])
+@pytest.mark.parametrize("n,c,h,w", [(1, 4, 3, 3), (2, 36, 16, 33), (1, 8, 15, 18), (2, 4, 34, 47), (3, 68, 4, 5)])
+def test_max_gradient_of_3x3_windows(n, c, h, w, pad):
+    from tsplit_b200.ops.pool import np_max_pool_grad
+    x = torch.round(_rand(n, c, h, w) * 2) / 2
+    x[x < -0.75] = -float("inf")
+    y = torch.nn.functional.max_pool2d(x, 3, 2, pad)
+    dy = torch.round(_rand(*y.shape, seed=1) * 8) / 8                # sums of four eighths are exact
+    dx = _arr(torch.full((n, c, h, w), 7.0, device="cuda"))
+    G.pool_grad(0, _arr(x), _arr(y), _arr(dy), dx, 3, 3, pad, 2, _stream())
+    # (the oracle pads with -inf, which must not tie with a place inside)
+    low = torch.where(torch.isinf(x), torch.full_like(x, -1e9), x).cpu().numpy()
+    want = np_max_pool_grad(low, None, dy.cpu().numpy(), 3, 3, pad, 2)
+    assert torch.equal(dx.t.cpu(), torch.from_numpy(want))
