@@ -25,11 +25,11 @@ import numpy as np
 
 from .. import ndarray
 from ..ops import _gpu as G
-from ..ops.elementwise import AddConstOp, MulConstOp, ReluOp, _Binary, _Unary, _is_scalar_shape
+from ..ops.elementwise import AddConstOp, AddReluOp, MulConstOp, ReluOp, _Binary, _Unary, _is_scalar_shape
 from ..ops.linalg import MatMulOp, _mm_shape
 from ..ops.loss import SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp
 from ..ops.misc import OneHotOp, PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
-from ..ops.norm import BatchNormGradScaleOp
+from ..ops.norm import BatchNormGradScaleOp, BatchNormOp
 from ..ops.shape import AddBroadcastOp, ReduceSumOp, ReshapeOp, ReshapeGradientOp, SliceOp
 
 FULL, ROW, SCALAR = 0, 1, 2
@@ -173,6 +173,15 @@ class StepPlan(object):
         for n in ex.topo_order:
             if n not in self.external and isinstance(n.op, MatMulOp):
                 self._dense(n)
+        self.joined = {}                  # residual addition with its ReLU -> the batch norm that it is computed with
+        place, segments = {}, 0
+        for n in ex.topo_order:
+            place[n] = segments
+            if n not in self.external:
+                segments += self._has_effects(n)
+                if type(n.op) is AddReluOp:
+                    self._join(n, place)
+        self.norms = set(self.joined.values())
         self.root = {}                    # view -> the node whose array it looks at
         self.actions = []
         self.open = {}                    # key -> Program that still collects
@@ -317,6 +326,16 @@ class StepPlan(object):
             self.dense[product] = (bias, relu)
             self.stored.update(made)
 
+    def _join(self, n, place):
+        """``relu(a + batch_norm(x))`` that alone reads the batch norm (its gradient does not): one apply pass for both."""
+        for b in sorted(set(n.inputs), key=lambda i: -i.id):
+            if (type(b.op) is BatchNormOp and b not in self.external and b not in self.evals and self.users.get(b) == [n]
+                    and n.inputs.count(b) == 1 and place[b] == place[n] and not self._has_effects(n)
+                    and self.arrays.get(b) is not None and self.arrays.get(n) is not None
+                    and all(tuple(self.shapes[i]) == tuple(self.shapes[n]) for i in n.inputs)):
+                self.joined[n] = b
+                return
+
     # -- scheduling ------------------------------------------------------------------------
     def _schedule(self, nodes):
         inside = set(nodes)
@@ -329,7 +348,11 @@ class StepPlan(object):
         def ready(n):
             nonlocal waiting
             cls, ops = "elided" if n in self.elided or n in self.stored else self._kind(n), None
-            if cls == "element":
+            if n in self.norms:
+                cls = "elided"
+            elif n in self.joined:
+                cls = None
+            elif cls == "element":
                 ops = self._operands(n)
                 cls = None if ops is None else cls
             elif n in self.sliced:
@@ -380,11 +403,15 @@ class StepPlan(object):
                 for m in taken:
                     for i in m.inputs:
                         self._need(i)
+                if n in self.joined:
+                    for i in self.joined[n].inputs:
+                        self._need(i)
                 if n in self.smooth:
                     self._need(self.smooth[n][0])
                 self.actions.append((self.group_of[n][0][0], taken) if len(taken) > 1 else
                                     ("smooth", n) if n in self.smooth else
                                     ("loss", n) if n in self.both or n in self.late else
+                                    ("join", n) if n in self.joined else
                                     ("products", taken) if n in self.dense or not self.sliced.isdisjoint(n.inputs) else
                                     ("node", n))
                 for m in taken[1:]:
@@ -538,6 +565,8 @@ class StepPlan(object):
                 self._products(x, vals, stream)
             elif what == "sums":
                 self._sums(x, vals, stream)
+            elif what == "join":
+                self._joined(x, vals, stream)
             elif what == "program":
                 if x.run(vals, self.arrays, stream):
                     for m in x.members:
@@ -635,6 +664,16 @@ class StepPlan(object):
         else:
             for n in nodes:
                 self._node(n, vals, stream)
+
+    def _joined(self, n, vals, stream):
+        """(The batch norm's own array is not written: nobody else reads it.)"""
+        norm = self.joined[n]
+        add = vals[n.inputs[0] if n.inputs[1] is norm else n.inputs[1]]
+        if norm.op.forward_add(norm, [vals[i] for i in norm.inputs], add, self.arrays[n], stream):
+            vals[norm], vals[n] = self.arrays[norm], self.arrays[n]
+        else:
+            self._node(norm, vals, stream)
+            self._node(n, vals, stream)
 
     def _loss(self, n, vals, stream, made):
         """A gradient and the loss that waited for it."""

@@ -581,6 +581,20 @@ def bn_forward_from_partials(part, chunks, x, scale, bias, y, save_mean, save_in
                                               _s(stream)), "bn_forward_from_partials")
 
 
+def bn_forward_add(part, chunks, x, scale, bias, add, y, save_mean, save_invstd, run_mean, run_var, momentum, eps, stream):
+    """``relu(bn(x) + add)``; ``part``: column sums that the convolution left, or None.  False: arrays it does not take."""
+    if not (y.t.is_cuda and x.t.is_cuda and add.t.is_cuda and x.same_layout(add) and x.same_layout(y)):
+        return False
+    rows, c, ldx = _rows_c(x)
+    if rows == 0 or c % 4 or c > 8192 or ldx % 4 or any(a.ptr & 15 for a in (x, add, y)):
+        return False
+    _check(lib().tsb_bn_forward_add(_p(part) if part is not None else None, c_int(chunks), c_int64(CONV_STAT_MAX_CHUNKS * c),
+                                    _p(x), _p(scale), _p(bias), _p(add), _p(y), _p(save_mean), _p(save_invstd), _p(run_mean),
+                                    _p(run_var), c_int64(rows), c_int64(c), c_int64(ldx), c_int64(ldx), c_int64(ldx),
+                                    c_float(momentum), c_float(eps), _s(stream)), "bn_forward_add")
+    return True
+
+
 _PAD_CACHE = {}
 
 

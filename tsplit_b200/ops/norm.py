@@ -64,17 +64,21 @@ class BatchNormOp(Op):
             x.attrs["bn_consumer"] = node      # the convolution's epilogue then supplies the column statistics
         return node
 
-    def _forward(self, node, iv, out, stream, relu):
-        x, scale, bias = iv
-        st = node.state
-        c = x.shape[1]
+    def _statistics(self, node, x):
+        """The node's side buffers, and the column sums that a convolution left in them: (state, chunks)."""
+        st, c = node.state, x.shape[1]
         if "mean" not in st or st["mean"].shape != (c,):
             st["mean"], st["invstd"] = _small((c,), x.ctx), _small((c,), x.ctx)
             st["run_mean"], st["run_var"] = _small((c,), x.ctx, 0.0), _small((c,), x.ctx, 1.0)
+        chunks = 0 if st.get("rematerialise") else st.pop("conv_chunks", 0)
+        return st, chunks if st.get("conv_rows") == x.shape[0] * x.shape[2] * x.shape[3] else 0
+
+    def _forward(self, node, iv, out, stream, relu):
+        x, scale, bias = iv
+        st, chunks = self._statistics(node, x)
         if st.get("rematerialise"):      # same step, statistics known: normalise only, leave running stats alone
             return G.bn_apply(x, scale, bias, out, st["mean"], st["invstd"], relu, stream)
-        chunks = st.pop("conv_chunks", 0)
-        if chunks and st.get("conv_rows") == x.shape[0] * x.shape[2] * x.shape[3]:
+        if chunks:
             return G.bn_forward_from_partials(st["conv_part"], chunks, x, scale, bias, out, st["mean"], st["invstd"],
                                               st["run_mean"], st["run_var"], node.attrs["momentum"],
                                               node.attrs["eps"], relu, stream)
@@ -110,6 +114,19 @@ class BatchNormOp(Op):
 
     def gpu_compute(self, node, iv, out, stream):
         self._forward(node, iv, out, stream, False)
+
+    def forward_add(self, node, iv, add, out, stream):
+        """``relu(batch_norm(x) + add)`` in one pass, without the batch norm's own result; False: not taken."""
+        x, scale, bias = iv
+        if node.state.get("rematerialise") or len(x.shape) != 4 or not x.t.is_cuda:
+            return False
+        left = node.state.get("conv_chunks", 0)
+        st, chunks = self._statistics(node, x)
+        if G.bn_forward_add(st["conv_part"] if chunks else None, chunks, x, scale, bias, add, out, st["mean"], st["invstd"],
+                            st["run_mean"], st["run_var"], node.attrs["momentum"], node.attrs["eps"], stream):
+            return True
+        st["conv_chunks"] = left
+        return False
 
     def gradient(self, node, g):
         x, scale, bias = node.inputs
