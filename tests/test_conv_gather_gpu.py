@@ -57,3 +57,17 @@ def _check(n, c, h, w, o, kh, kw, ph, pw, stride):
         err = (out.double().permute(0, 3, 1, 2) - refs[kind]).abs().max().item()
         assert err <= 2 ** -23 * terms * max(refs[kind].abs().max().item(), 1.0), (kind, err)
     assert lib.tsb_device_status(st) == 0
+
+
+# classes without taps, all four with some, ragged tiles and several per CTA; channels of no 32, which it leaves alone
+@pytest.mark.parametrize("n,c,h,w,o,kh,kw,ph,pw", [(2, 32, 9, 9, 32, 1, 1, 0, 0), (3, 96, 17, 20, 64, 3, 3, 1, 1),
+                                                   (24, 256, 56, 55, 32, 1, 1, 0, 0), (2, 100, 9, 9, 32, 1, 1, 0, 0)])
+def test_strided_data_gradient_added_to_another(n, c, h, w, o, kh, kw, ph, pw):
+    oh, ow = (h + 2 * ph - kh) // 2 + 1, (w + 2 * pw - kw) // 2 + 1
+    wt, dy, first = _rand(o, kh, kw, c, seed=2), _rand(n, oh, ow, o, seed=3), _rand(n, h, w, c, seed=4)
+    lib, st = _base.kernels(), PTR(torch.cuda.current_stream().cuda_stream)
+    alone, both = torch.empty_like(first), first.clone()
+    assert lib.tsb_conv2d(1, *[PTR(a.data_ptr()) for a in (alone, wt, dy)], n, c, h, w, o, kh, kw, oh, ow, ph, pw, 2, st) == 0
+    rc = lib.tsb_conv2d_dgrad_add(*[PTR(a.data_ptr()) for a in (both, wt, dy)], n, c, h, w, o, kh, kw, oh, ow, ph, pw, st)
+    assert rc == (2 if c % 32 else 0)
+    assert torch.equal(both, first if c % 32 else first + alone)           # one addition, rounded once either way

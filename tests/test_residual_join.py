@@ -1,4 +1,5 @@
-"""A residual addition with its ReLU computed by the batch norm before it: the plan on the host, the kernel on the GPU."""
+"""A residual addition with its ReLU computed by the batch norm before it, and the sum of two gradients by the later
+convolution: the plan on the host, the kernels on the GPU."""
 import numpy as np
 import pytest
 import torch
@@ -7,6 +8,7 @@ import test_step_plan as base
 from tsplit_b200 import gpu_ops as ad, ndarray
 from tsplit_b200.models import resnet
 from tsplit_b200.ops import _gpu as G
+from tsplit_b200.ops.conv import Conv2dGradDataOp
 from tsplit_b200.ops.norm import BatchNormOp, np_bn_forward
 
 
@@ -21,9 +23,19 @@ def test_resnet(monkeypatch, taken):
             out.numpy_view()[...] = np.maximum(self.np_compute(node, [x, scale, bias]) + add, 0)
         return taken
     monkeypatch.setattr(BatchNormOp, "forward_add", forward_add)
+    added = []
+
+    def add_to(self, node, iv, out, stream):
+        added.append(node)
+        if taken:
+            out.numpy_view()[...] += self.np_compute(node, [v.numpy_view() for v in iv])
+        return taken
+    monkeypatch.setattr(Conv2dGradDataOp, "add_to", add_to)
     plan = base._compare(monkeypatch, lambda: base._model(resnet(26, num_classes=10, image=32, width_div=8), 2), steps=2)
-    assert len(plan.joined) == 8 and len(joins) == 16
-    assert all(n.inputs.count(b) == 1 for n, b in plan.joined.items())
+    assert len(joins) == 16
+    # eight blocks; in three of them the input's two gradients, one of stride 2
+    assert sorted(type(b.op).name for b in plan.joined.values()) == ["BatchNorm"] * 8 + ["Conv2dGradData"] * 3
+    assert len(added) == 6 and all(n.inputs.count(b) == 1 for n, b in plan.joined.items())
 
 
 def test_what_stays(monkeypatch):

@@ -25,7 +25,8 @@ import numpy as np
 
 from .. import ndarray
 from ..ops import _gpu as G
-from ..ops.elementwise import AddConstOp, AddReluOp, MulConstOp, ReluOp, _Binary, _Unary, _is_scalar_shape
+from ..ops.conv import Conv2dGradDataOp
+from ..ops.elementwise import AddConstOp, AddOp, AddReluOp, MulConstOp, ReluOp, _Binary, _Unary, _is_scalar_shape
 from ..ops.linalg import MatMulOp, _mm_shape
 from ..ops.loss import SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp
 from ..ops.misc import OneHotOp, PlaceholderOp, _FillLike, SwapInOp, SwapOutOp
@@ -173,7 +174,7 @@ class StepPlan(object):
         for n in ex.topo_order:
             if n not in self.external and isinstance(n.op, MatMulOp):
                 self._dense(n)
-        self.joined = {}                  # residual addition with its ReLU -> the batch norm that it is computed with
+        self.joined = {}                  # addition -> the batch norm or the gradient that it is computed with
         place, segments = {}, 0
         for n in ex.topo_order:
             place[n] = segments
@@ -181,7 +182,9 @@ class StepPlan(object):
                 segments += self._has_effects(n)
                 if type(n.op) is AddReluOp:
                     self._join(n, place)
-        self.norms = set(self.joined.values())
+                elif type(n.op) is AddOp:
+                    self._add_gradients(n, place)
+        self.inner = set(self.joined.values())   # computed with the node that reads them
         self.root = {}                    # view -> the node whose array it looks at
         self.actions = []
         self.open = {}                    # key -> Program that still collects
@@ -336,6 +339,22 @@ class StepPlan(object):
                 self.joined[n] = b
                 return
 
+    def _add_gradients(self, n, place):
+        """The sum of two convolutions' gradients that alone reads them, one of stride 2: the other one's result is written
+        where the sum goes, and this one adds to it."""
+        def alone(i):
+            return (type(i.op) is Conv2dGradDataOp and i not in self.external and i not in self.evals and self.users.get(i) == [n]
+                    and place[i] == place[n] and i not in self.joined.values()
+                    and self.arrays.get(i) is not None and tuple(self.shapes[i]) == tuple(self.shapes[n]))
+        a, b = n.inputs
+        if a is b or self.arrays.get(n) is None or self._has_effects(n) or not (alone(a) and alone(b)):
+            return
+        late = b if b.attrs["stride"] == 2 else a
+        first = a if late is b else b
+        if late.attrs["stride"] == 2 and self.arrays[first].same_layout(self.arrays[n]):
+            self.joined[n] = late
+            self.arrays[first] = self.arrays[n]
+
     # -- scheduling ------------------------------------------------------------------------
     def _schedule(self, nodes):
         inside = set(nodes)
@@ -348,7 +367,7 @@ class StepPlan(object):
         def ready(n):
             nonlocal waiting
             cls, ops = "elided" if n in self.elided or n in self.stored else self._kind(n), None
-            if n in self.norms:
+            if n in self.inner:
                 cls = "elided"
             elif n in self.joined:
                 cls = None
@@ -666,13 +685,14 @@ class StepPlan(object):
                 self._node(n, vals, stream)
 
     def _joined(self, n, vals, stream):
-        """(The batch norm's own array is not written: nobody else reads it.)"""
-        norm = self.joined[n]
-        add = vals[n.inputs[0] if n.inputs[1] is norm else n.inputs[1]]
-        if norm.op.forward_add(norm, [vals[i] for i in norm.inputs], add, self.arrays[n], stream):
-            vals[norm], vals[n] = self.arrays[norm], self.arrays[n]
+        """(The inner node's own array is not written: nobody else reads it.)"""
+        inner, out = self.joined[n], self.arrays[n]
+        other = vals[n.inputs[0] if n.inputs[1] is inner else n.inputs[1]]
+        ins = [vals[i] for i in inner.inputs]
+        if (inner.op.forward_add(inner, ins, other, out, stream) if type(n.op) is AddReluOp else inner.op.add_to(inner, ins, out, stream)):
+            vals[inner], vals[n] = self.arrays[inner], out
         else:
-            self._node(norm, vals, stream)
+            self._node(inner, vals, stream)
             self._node(n, vals, stream)
 
     def _loss(self, n, vals, stream, made):

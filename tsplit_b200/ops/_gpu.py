@@ -570,6 +570,21 @@ def conv2d_fwd_stats(x, w, y, ph, pw, stride, part, stream, chunk_offset=0, plan
     return int(chunks.value)
 
 
+def conv2d_dgrad_add(dx, w, dy, ph, pw, stride, stream):
+    """``dx += dgrad(dy, w)``; False: not taken, and ``dx`` is as it was."""
+    if stride != 2 or not (dx.t.is_cuda and all(a.is_channels_last() for a in (dx, w, dy))):
+        return False
+    n, c, h, wd = dx.shape
+    o, _, kh, kw = w.shape
+    _, _, oh, ow = dy.shape
+    rc = lib().tsb_conv2d_dgrad_add(_p(dx), _p(w), _p(dy), c_int(n), c_int(c), c_int(h), c_int(wd), c_int(o), c_int(kh), c_int(kw),
+                                    c_int(oh), c_int(ow), c_int(ph), c_int(pw), _s(stream))
+    if rc == 2:          # sizes that it does not cover
+        return False
+    _check(rc, "conv2d_dgrad_add")
+    return True
+
+
 def bn_forward_from_partials(part, chunks, x, scale, bias, y, save_mean, save_invstd, run_mean, run_var, momentum,
                              eps, relu, stream):
     rows, c, ldx = _rows_c(x)

@@ -154,6 +154,11 @@ class Conv2dGradDataOp(Op):
             h, w = h + 1, w + 1
         return (n, c, h, w)
 
+    def add_to(self, node, iv, out, stream):
+        """Adds the gradient to what ``out`` holds; False: not taken."""
+        ph, pw = _pads(node)
+        return G.conv2d_dgrad_add(out, iv[0], iv[1], ph, pw, node.attrs["stride"], stream)
+
     def np_compute(self, node, iv):
         ph, pw = _pads(node)
         xs = self._xshape(node, iv[0].shape, iv[1].shape)
