@@ -1,6 +1,6 @@
 """The order in which the keep-all executors issue a step on the GPU, worked out once per feed shape.
 
-Seven things are taken out of the node-by-node loop.  They change no value, but for the rounding of a loss whose labels
+Nine things are taken out of the node-by-node loop.  They change no value, but for the rounding of a loss whose labels
 come from class ids (the same sum, added up in another order):
 
 * element-wise operators over the same elements are collected and run as one ``tsb_pointwise`` program, at the first
@@ -11,7 +11,10 @@ come from class ids (the same sum, added up in another order):
   there is a launch of them or nothing else is left to do;
 * the bias of a product, and the ReLU behind it, are added where the product stores its outputs;
 * one-hot labels, scaled and shifted (label smoothing), that only a cross-entropy reads are not made: it takes the ids;
-* a loss and its gradient come from one pass over the logits, when the gradient is due.
+* a loss and its gradient come from one pass over the logits, when the gradient is due;
+* a residual addition and its ReLU are taken by the batch norm before them, where nothing else reads that;
+* of two convolutions' gradients that only their sum reads, the first is written where the sum goes, and the other, if its
+  stride is 2, adds itself to it.
 
 Element-wise nodes are taken as soon as their inputs are there, the others in creation order, and nothing moves past a
 node with effects of its own (an optimizer update, a collective, a swap).  The memory-planning executors have
