@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import test_step_plan as base
-from tsplit_b200 import gpu_ops as ad, ndarray
+from tsplit_b200 import gpu_ops as ad, ndarray, optimizer
 from tsplit_b200.executors import step_plan
 from tsplit_b200.models import lstm
 from tsplit_b200.ops import _gpu as G
@@ -49,6 +49,31 @@ def test_which_slices_are_copied(monkeypatch):
                 {x: r.standard_normal((8, 12), np.float32), w: r.standard_normal((4, 12), np.float32)})
     monkeypatch.setattr(G, "gemm_dense", _dense)
     assert len(base._compare(monkeypatch, build).sliced) == 1
+
+
+@pytest.mark.parametrize("steps", [1, 2])
+def test_a_slice_is_older_than_the_update_behind_it(monkeypatch, steps):
+    """A product behind the update reads what was sliced before it; slices that are read on one side only stay in place."""
+    r = np.random.default_rng(0)
+    xv, zv, wv = (r.standard_normal(s).astype(np.float32) for s in ((4, 8), (4, 8), (8, 12)))
+    made = []
+
+    def compute(self, node, ins, out, *rest):
+        out, x = (v.numpy_view() if isinstance(v, ndarray.NDArray) else v for v in (out, ins[0]))
+        out[...] = self.np_compute(node, [x])
+    monkeypatch.setattr(step_plan.SliceOp, "compute", compute)
+    monkeypatch.setattr(G, "gemm_dense", _dense)
+
+    def build():
+        x, z, w = ad.Variable("x"), ad.Variable("z"), ad.Variable("w", value=wv.copy())
+        both, early = ad.slice_op(w, (0, 4), (8, 4)), ad.slice_op(w, (0, 0), (8, 4))
+        h = ad.matmul_op(x, both) + ad.matmul_op(x, early)
+        train = optimizer.SGDOptimizer(0.05).minimize(ad.reduce_sum_op(ad.mul_op(h, h), [0, 1]), [w])
+        late = ad.slice_op(w, (0, 8), (8, 4))
+        made[:] = [both, early, late]
+        return [h, train, ad.matmul_op(z, both), ad.matmul_op(z, late)], {x: xv, z: zv}
+    plan = base._compare(monkeypatch, build, steps=steps)
+    assert plan.sliced == set(made[1:])
 
 
 @pytest.mark.gpu

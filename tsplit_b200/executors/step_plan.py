@@ -162,6 +162,13 @@ class StepPlan(object):
                 for i in n.inputs:
                     self.users.setdefault(i, []).append(n)
         self.kinds = {}                   # operator type -> _kind
+        # how many nodes with effects stand before a node: what a rule takes together must have the same number, or one of
+        # its operands may be another by then
+        self.place, effects = {}, 0
+        for n in ex.topo_order:
+            self.place[n] = effects
+            if n not in self.external:
+                effects += self._has_effects(n)
         self.smooth, self.elided = {}, set()
         for n in ex.topo_order:
             if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
@@ -178,15 +185,12 @@ class StepPlan(object):
             if n not in self.external and isinstance(n.op, MatMulOp):
                 self._dense(n)
         self.joined = {}                  # addition -> the batch norm or the gradient that it is computed with
-        place, segments = {}, 0
         for n in ex.topo_order:
-            place[n] = segments
             if n not in self.external:
-                segments += self._has_effects(n)
                 if type(n.op) is AddReluOp:
-                    self._join(n, place)
+                    self._join(n)
                 elif type(n.op) is AddOp:
-                    self._add_gradients(n, place)
+                    self._add_gradients(n)
         self.inner = set(self.joined.values())   # computed with the node that reads them
         self.root = {}                    # view -> the node whose array it looks at
         self.actions = []
@@ -209,7 +213,7 @@ class StepPlan(object):
         self._schedule(segment)
         self._flush_all()
         del self.users, self.shapes, self.external, self.root, self.open, self.home, self.copies     # planning only
-        del self.copied, self.layouts, self.group_of, self.queues, self.gone, self.kinds, self.stored
+        del self.copied, self.layouts, self.group_of, self.queues, self.gone, self.kinds, self.stored, self.place
 
     def _kind(self, n):
         """What nodes of this operator type may become; "effects": they stay where they are."""
@@ -241,10 +245,11 @@ class StepPlan(object):
                 and arr.t.is_contiguous() and src.t.numel() == arr.t.numel())
 
     def _is_sliced(self, n):
-        """Rows and columns of a value that is there from the start, for products, which take any row stride."""
+        """Rows and columns of a value that is there from the start, for products, which take any row stride.  (The value
+        may be a parameter: behind its update a view would show the new one.)"""
         users = self.users.get(n, ())
         return (n not in self.evals and n.inputs[0] in self.external and len(self.shapes[n]) == 2 and len(users) > 0
-                and all(isinstance(u.op, MatMulOp) and not self._has_effects(u) for u in users))
+                and all(isinstance(u.op, MatMulOp) and not self._has_effects(u) and self.place[u] == self.place[n] for u in users))
 
     def _operands(self, n):
         """[(node, kind)] when ``n`` can be part of a program, else None."""
@@ -332,22 +337,22 @@ class StepPlan(object):
             self.dense[product] = (bias, relu)
             self.stored.update(made)
 
-    def _join(self, n, place):
+    def _join(self, n):
         """``relu(a + batch_norm(x))`` that alone reads the batch norm (its gradient does not): one apply pass for both."""
         for b in sorted(set(n.inputs), key=lambda i: -i.id):
             if (type(b.op) is BatchNormOp and b not in self.external and b not in self.evals and self.users.get(b) == [n]
-                    and n.inputs.count(b) == 1 and place[b] == place[n] and not self._has_effects(n)
+                    and n.inputs.count(b) == 1 and self.place[b] == self.place[n] and not self._has_effects(n)
                     and self.arrays.get(b) is not None and self.arrays.get(n) is not None
                     and all(tuple(self.shapes[i]) == tuple(self.shapes[n]) for i in n.inputs)):
                 self.joined[n] = b
                 return
 
-    def _add_gradients(self, n, place):
+    def _add_gradients(self, n):
         """The sum of two convolutions' gradients that alone reads them, one of stride 2: the other one's result is written
         where the sum goes, and this one adds to it."""
         def alone(i):
             return (type(i.op) is Conv2dGradDataOp and i not in self.external and i not in self.evals and self.users.get(i) == [n]
-                    and place[i] == place[n] and i not in self.joined.values()
+                    and self.place[i] == self.place[n] and i not in self.joined.values()
                     and self.arrays.get(i) is not None and tuple(self.shapes[i]) == tuple(self.shapes[n]))
         a, b = n.inputs
         if a is b or self.arrays.get(n) is None or self._has_effects(n) or not (alone(a) and alone(b)):
