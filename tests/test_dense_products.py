@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import test_step_plan as base
-from tsplit_b200 import gpu_ops as ad, ndarray
+from tsplit_b200 import gpu_ops as ad, ndarray, optimizer
 from tsplit_b200.models import mlp, transformer
 from tsplit_b200.ops import _gpu as G
 
@@ -64,6 +64,26 @@ def test_what_is_not_a_bias(monkeypatch):
     monkeypatch.setattr(G, "gemm_dense", _dense(calls, True))
     plan = base._compare(monkeypatch, build)
     assert not plan.dense and not calls
+
+
+def test_what_stands_behind_an_update_is_not_stored_before_it(monkeypatch):
+    """A bias that an update between the product and the addition changes, and a ReLU of a value behind an update; the
+    products in front of one keep theirs."""
+    r = np.random.default_rng(0)
+    xv, wv, bv = (r.standard_normal(s).astype(np.float32) for s in ((4, 8), (8, 12), (12,)))
+    made = []
+
+    def build():
+        x, w, b = ad.Variable("x"), ad.Variable("w"), ad.Variable("b", value=bv.copy())
+        p, plain = ad.matmul_op(x, w), ad.matmul_op(x, w)
+        q = ad.matmul_op(x, w)
+        early = q + ad.broadcasttoTF_op(b, q)
+        train = optimizer.SGDOptimizer(0.5).minimize(ad.reduce_sum_op(ad.mul_op(early, early), [0, 1]), [b])
+        made[:] = [q]
+        return [early, train, ad.relu_op(p + ad.broadcasttoTF_op(b, p)), ad.relu_op(plain), ad.relu_op(early)], {x: xv, w: wv}
+    monkeypatch.setattr(G, "gemm_dense", _dense([], True))
+    plan = base._compare(monkeypatch, build, steps=2)
+    assert [(q, relu) for q, (bias, relu) in plan.dense.items()] == [(made[0], None)]
 
 
 # one tile; a K that is split, by a cluster and by two kernels; rows of no whole 16 bytes; tiles of 64, 128 and 256 columns,

@@ -319,15 +319,17 @@ class StepPlan(object):
 
     def _dense(self, product):
         """``product + row`` that nothing else reads the product of, and the one ReLU of the result (or of the product
-        itself): the product's launch can store them.  The row is there from the start (a parameter)."""
+        itself): the product's launch can store them.  The row is there from the start, a parameter: an addition behind its
+        update has to read the new one."""
         result, bias, readers = product, None, self.users.get(product, [])
         if (len(readers) == 1 and isinstance(readers[0].op, AddBroadcastOp) and readers[0].inputs[0] is product
-                and product not in self.evals and not self._has_effects(readers[0])):
+                and product not in self.evals and not self._has_effects(readers[0]) and self.place[readers[0]] == self.place[product]):
             row = readers[0].inputs[1]
             cols = self.shapes[product][-1]
             if row in self.external and row is not product and tuple(self.shapes[row]) == (cols,):
                 result = bias = readers[0]
-        relus = [u for u in self.users.get(result, ()) if isinstance(u.op, ReluOp) and not self._has_effects(u)]
+        relus = [u for u in self.users.get(result, ())
+                 if isinstance(u.op, ReluOp) and not self._has_effects(u) and self.place[u] == self.place[product]]
         relu = relus[0] if len(relus) == 1 else None
         made = [n for n in (bias, relu) if n is not None]
         own = self.arrays.get(product)
