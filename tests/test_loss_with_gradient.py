@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import test_step_plan as base
-from tsplit_b200 import gpu_ops as ad, ndarray
+from tsplit_b200 import gpu_ops as ad, ndarray, optimizer
 from tsplit_b200.ops import _gpu as G
 
 
@@ -58,6 +58,22 @@ def test_one_pass_for_both(monkeypatch, smoothed, taken):
 
 def test_a_loss_that_is_read_is_not_late(monkeypatch):
     assert not base._compare(monkeypatch, _net(False, True)).both
+
+
+def test_a_loss_does_not_wait_for_a_gradient_behind_an_update(monkeypatch):
+    """Its labels are a variable that an optimizer trains between the two."""
+    r = np.random.default_rng(0)
+    xv, tv, lv = (r.standard_normal((6, 12)).astype(np.float32) for _ in range(3))
+    dense, _ = _both([])
+    monkeypatch.setattr(G, "softmax_ce_both", dense)
+
+    def build():
+        x, t, lab = ad.Variable("x"), ad.Variable("t"), ad.Variable("lab", value=np.abs(lv))
+        loss = ad.softmaxcrossentropy_op(x, lab)
+        diff = lab + ad.opposite_op(t)
+        train = optimizer.SGDOptimizer(0.1).minimize(ad.reduce_sum_op(ad.mul_op(diff, diff), [0, 1]), [lab])
+        return [loss, train] + ad.gradients(loss, [x]), {x: xv, t: tv}
+    assert not base._compare(monkeypatch, build, steps=2).both
 
 
 # a row of a few classes, more than a thread keeps, long rows: from L2, staged in shared memory, too long for that; ids

@@ -306,12 +306,14 @@ class StepPlan(object):
             self.smooth[u] = (cur.inputs[0], consts[::-1], chain[::-1])
 
     def _loss_with_gradient(self, loss):
-        """When nobody needs ``loss`` before its one gradient is due (a seed of ones takes its shape only)."""
+        """When nobody needs ``loss`` before its one gradient is due (a seed of ones takes its shape only), and no update of
+        its logits or labels stands between the two."""
         logits, labels = loss.inputs
         grads = [u for u in self.users.get(logits, ()) if isinstance(u.op, SoftmaxCrossEntropyGradientOp)
                  and u.inputs[0] is logits and u.inputs[1] is labels]
         others = [u for u in self.users.get(logits, ()) if isinstance(u.op, SoftmaxCrossEntropyOp) and u.inputs[1] is labels]
-        if (len(grads) == 1 and len(others) == 1 and all(isinstance(u.op, _FillLike) for u in self.users.get(loss, ()))
+        if (len(grads) == 1 and len(others) == 1 and self.place[grads[0]] == self.place[loss]
+                and all(isinstance(u.op, _FillLike) for u in self.users.get(loss, ()))
                 and (loss in self.smooth) == (grads[0] in self.smooth) and not self._has_effects(loss)
                 and not self._has_effects(grads[0]) and self.arrays.get(loss) is not None
                 and self.arrays.get(grads[0]) is not None):
