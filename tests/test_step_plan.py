@@ -373,6 +373,21 @@ def test_labels_that_are_refused_are_made_once_a_step(monkeypatch):
         np.testing.assert_allclose(g, w, rtol=1e-5, atol=1e-6)
 
 
+def test_labels_are_older_than_an_update_of_their_ids(monkeypatch):
+    """A cross-entropy behind the update reads the labels that were made in front of it."""
+    xv, = _arrays((6, 12))
+    old, new = np.array([0, 3, 11, 5, 5, 2], np.float32), np.array([1, 2, 3, 4, 5, 6], np.float32)
+
+    def build():
+        x, t, i = ad.Variable("x"), ad.Variable("t"), ad.Variable("i", value=old.copy())
+        lab = ad.addbyconst_op(ad.mul_byconst_op(ad.one_hot_op(i, 12), 0.9), 0.01)
+        early = ad.softmaxcrossentropy_op(x, lab)
+        diff = i + ad.opposite_op(t)
+        train = optimizer.SGDOptimizer(0.5).minimize(ad.reduce_sum_op(ad.mul_op(diff, diff), [0]), [i])     # i = t
+        return [early, train, ad.softmaxcrossentropy_op(ad.mul_byconst_op(x, 2.0), lab)], {x: xv, t: new}
+    assert not _compare(monkeypatch, build).smooth
+
+
 # one group of four; a row length that is no power of two; the last size of the short blocks and the first of the long
 # ones; a tensor past the limit for many values
 @pytest.mark.gpu

@@ -294,12 +294,14 @@ class StepPlan(object):
             cur = cur.inputs[0]
             if tuple(self.shapes[cur])[-1:] != tuple(self.shapes[labels])[-1:]:
                 return
-        readers = [u for u in self.users.get(labels, ())]
+        readers = self.users.get(labels, [])
         if len(self.shapes[labels]) != 2 or not all(
                 isinstance(u.op, (SoftmaxCrossEntropyOp, SoftmaxCrossEntropyGradientOp)) and u.inputs[1] is labels
                 and u.inputs.count(labels) == 1 for u in readers):
             return
         if any(u not in chain for m in chain[1:] for u in self.users.get(m, ())):
+            return
+        if len({self.place[u] for u in chain + readers}) > 1:       # an update may change the ids in between
             return
         self.elided.update(chain)
         for u in readers:
