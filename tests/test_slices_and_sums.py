@@ -97,3 +97,12 @@ def test_step_on_the_gpu(monkeypatch, steps, features, batch):
         outs.append([o.t.clone() for o in ex.run(feed)])
     for other in outs[1:]:
         assert all(torch.equal(a, b) for a, b in zip(outs[0], other))
+
+
+@pytest.mark.gpu
+def test_operators_are_timed_after_a_step_with_slices_in_place():
+    m = lstm(steps=3, features=8, hidden=32, num_classes=12)
+    x, y = m.synthetic_batch(16)
+    ex = ad.recomputeExecutor([m.loss] + ad.gradients(m.loss, list(m.variables)), ctx=ndarray.gpu(0), policy="speed")
+    table = ex.measure_ops({m.X: x, m.y_: y}, repeats=1)
+    assert {"Slice", "MatMul"} <= {n.op.name for n in table} and min(table.values()) > 0

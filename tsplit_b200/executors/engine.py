@@ -839,6 +839,8 @@ class MemoryExecutor(Executor):
                 ms = a.elapsed_time(b)
                 best = ms if best is None else min(best, ms)
             table[n] = best
+            if out is not None:
+                vals[n] = out          # (a slice that the planned step read in place was a view of wider rows)
         self.measured_op_ms = table
         return table
 
