@@ -530,8 +530,8 @@ int done() {
   return e == cudaSuccess ? TSB_OK : (TSB_ERR_LAUNCH | ((int)e << 8));
 }
 
-float* colsum_scratch() {   // 64 chunks x up to 64K columns
-  return static_cast<float*>(tsb_scratch::get(nullptr, tsb_scratch::COLSUM_PARTIALS, 64ull * 65536 * 4));
+float* colsum_scratch(cudaStream_t st) {   // 64 chunks x up to 64K columns
+  return static_cast<float*>(tsb_scratch::get(st, tsb_scratch::COLSUM_PARTIALS, 64ull * 65536 * 4));
 }
 
 }  // namespace
@@ -765,7 +765,7 @@ int tsb_reduce_sum(const float* x, float* y, int nk, const long long* kshape, co
     return done();
   }
   if (nk == 1 && nr == 1 && kxs[0] == 1 && nkeep <= 65536 && nred >= 64) {
-    float* part = colsum_scratch();
+    float* part = colsum_scratch(st);
     if (part) {
       if ((nkeep & 3) == 0 && (rxs[0] & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
         // scratch: 64 x 65536 floats, so up to 256 chunks for 16384 columns or fewer

@@ -34,8 +34,8 @@ constexpr int MAX_CHUNKS = 128;
 constexpr long long PLANE_FLOATS = (long long)MAX_CHUNKS * 8192;   // one partial plane: chunks x channels
 constexpr long long SCRATCH_FLOATS = 2 * PLANE_FLOATS;              // two planes (up to 8192 channels at MAX_CHUNKS)
 
-float* scratch() {
-  return static_cast<float*>(tsb_scratch::get(nullptr, tsb_scratch::NORM_PARTIALS, SCRATCH_FLOATS * sizeof(float)));
+float* scratch(cudaStream_t st) {
+  return static_cast<float*>(tsb_scratch::get(st, tsb_scratch::NORM_PARTIALS, SCRATCH_FLOATS * sizeof(float)));
 }
 
 int sm_count() {
@@ -552,7 +552,7 @@ int tsb_bn_forward(const float* x, const float* scale, const float* bias, float*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows <= 0 || C <= 0) return TSB_ERR_ARG;
   if ((C % 4) || (ldx % 4) || (ldy % 4) || C > 8192) return TSB_ERR_UNSUPPORTED;
-  float* part = scratch();
+  float* part = scratch(st);
   if (!part) return TSB_ERR_OOM;
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<0>, sg.grid, STAT_THREADS, 0, st, x, nullptr, nullptr, nullptr, part, rows, (int)C,
@@ -589,7 +589,7 @@ int tsb_bn_forward_add(const float* part, int chunks, long long plane, const flo
   if (rows <= 0 || C <= 0 || !add || (part && chunks <= 0)) return TSB_ERR_ARG;
   if ((C % 4) || (ldx % 4) || (ldadd % 4) || (ldy % 4) || C > 8192) return TSB_ERR_UNSUPPORTED;
   if (!part) {
-    float* own = scratch();
+    float* own = scratch(st);
     if (!own) return TSB_ERR_OOM;
     const StatGeom sg = stat_geom(rows, (int)C);
     tsb_launch::launch(col_partial<0>, sg.grid, STAT_THREADS, 0, st, x, nullptr, nullptr, nullptr, own, rows, (int)C, ldx, 0,
@@ -646,7 +646,7 @@ int tsb_bn_backward(const float* dy, const float* x, const float* scale, const f
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows <= 0 || C <= 0) return TSB_ERR_ARG;
   if ((C % 4) || (ldx % 4) || (lddy % 4) || (lddx % 4) || C > 8192) return TSB_ERR_UNSUPPORTED;
-  float* part = scratch();
+  float* part = scratch(st);
   if (!part) return TSB_ERR_OOM;
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<1>, sg.grid, STAT_THREADS, 0, st, dy, x, save_mean, save_invstd, part, rows, (int)C,
@@ -667,7 +667,7 @@ int tsb_bn_relu_backward(const float* dy, const float* x, const float* scale, co
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows <= 0 || C <= 0 || !bias) return TSB_ERR_ARG;
   if ((C % 4) || (ldx % 4) || (lddy % 4) || (lddx % 4) || C > 8192) return TSB_ERR_UNSUPPORTED;
-  float* part = scratch();
+  float* part = scratch(st);
   if (!part) return TSB_ERR_OOM;
   const StatGeom sg = stat_geom(rows, (int)C);
   tsb_launch::launch(col_partial<1>, sg.grid, STAT_THREADS, 0, st, dy, x, save_mean, save_invstd, part, rows, (int)C,
@@ -765,7 +765,7 @@ int tsb_layer_norm_grad(const float* dy, const float* x, const float* scale, con
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows <= 0 || D <= 0) return TSB_ERR_ARG;
   if (D > 8192) return TSB_ERR_UNSUPPORTED;
-  float* part = scratch();
+  float* part = scratch(st);
   if (!part) return TSB_ERR_OOM;
   const long long threads = rows * 32;
   const int d4 = (int)(D / 4);

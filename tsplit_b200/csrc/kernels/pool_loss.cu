@@ -563,8 +563,8 @@ __global__ void __launch_bounds__(256) max_pool_bwd_3s2(const float* x, const fl
   }
 }
 
-unsigned char* argmax_scratch(size_t bytes) {
-  return static_cast<unsigned char*>(tsb_scratch::get(nullptr, tsb_scratch::POOL_ARGMAX, bytes, size_t(32) << 20));
+unsigned char* argmax_scratch(size_t bytes, cudaStream_t st) {
+  return static_cast<unsigned char*>(tsb_scratch::get(st, tsb_scratch::POOL_ARGMAX, bytes, size_t(32) << 20));
 }
 
 // ------------------------------------------------------------------ softmax family
@@ -1289,8 +1289,8 @@ int launch_rows(K plain, K staged, long long rows, int nvec, cudaStream_t st, A.
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-float* row_scratch(long long rows) {
-  return static_cast<float*>(tsb_scratch::get(nullptr, tsb_scratch::LOSS_ROWS, (size_t)rows * sizeof(float),
+float* row_scratch(long long rows, cudaStream_t st) {
+  return static_cast<float*>(tsb_scratch::get(st, tsb_scratch::LOSS_ROWS, (size_t)rows * sizeof(float),
                                               size_t(65536) * sizeof(float)));
 }
 
@@ -1381,9 +1381,8 @@ int tsb_pool_bwd(int kind, const float* x, const float* y, const float* dy, floa
         tsb_launch::launch(max_pool_bwd_tile, blocks, 256, smem, st, x, dy, dx, p, (int)tiles_x, nw);
       return done();
     }
-    // overlapping windows: positions of the maxima first, then a gather per input pixel (one scratch
-    // buffer per device: pooling backward passes of one device must not overlap on different streams)
-    unsigned char* idx = argmax_scratch((size_t)n * oh * ow * c);
+    // overlapping windows: positions of the maxima first, then a gather per input pixel
+    unsigned char* idx = argmax_scratch((size_t)n * oh * ow * c, st);
     if (idx) {
       tsb_launch::launch(pool_argmax, ew_grid((long long)n * oh * ow * (c / 4)), 256, 0, st, x, idx, p);
       tsb_launch::launch(pool_bwd_from_argmax, grid, 256, 0, st, idx, dy, dx, p);
@@ -1527,9 +1526,9 @@ int tsb_scaled_softmax_grad(const float* y, const float* dy, float* dx, long lon
 
 int tsb_softmax_ce(const float* x, const float* labels, float* loss, long long rows, long long cols, void* stream) {
   if (rows <= 0 || cols <= 0) return TSB_ERR_ARG;
-  float* rl = row_scratch(rows);
-  if (!rl) return TSB_ERR_OOM;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  float* rl = row_scratch(rows, st);
+  if (!rl) return TSB_ERR_OOM;
   const int grid = (int)(rows < 148 * 16 ? rows : 148 * 16);
   if (cols >= 512 && cols % 4 == 0 && cols / 4 < (1ll << 30) && aligned16(x) && aligned16(labels)) {
     const int rc = launch_rows(ce_rows_v4<DenseLabels, false>, ce_rows_v4<DenseLabels, true>, rows, (int)(cols / 4), st,
@@ -1554,9 +1553,9 @@ int tsb_softmax_ce_grad(const float* x, const float* labels, const float* g, flo
 int tsb_softmax_ce_both(const float* x, const float* labels, const float* g, float* loss, float* dx, long long rows,
                         long long cols, void* stream) {
   if (rows <= 0 || cols <= 0) return TSB_ERR_ARG;
-  float* rl = row_scratch(rows);
-  if (!rl) return TSB_ERR_OOM;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  float* rl = row_scratch(rows, st);
+  if (!rl) return TSB_ERR_OOM;
   const int rc = ce_grad(x, labels, g, dx, rows, cols, rl, st);
   if (rc) return rc;
   tsb_launch::launch(mean_rows, 1, 1024, 0, st, rl, loss, rows);
@@ -1569,9 +1568,9 @@ int tsb_softmax_ce_smooth(const float* x, const float* ids, float on, float off,
                           long long cols, void* stream) {
   if (rows <= 0 || cols <= 0) return TSB_ERR_ARG;
   if (cols < 512 || cols % 4 || cols / 4 >= (1ll << 30) || !aligned16(x)) return TSB_ERR_UNSUPPORTED;
-  float* rl = row_scratch(rows);
-  if (!rl) return TSB_ERR_OOM;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  float* rl = row_scratch(rows, st);
+  if (!rl) return TSB_ERR_OOM;
   tsb_launch::launch(ce_smooth_rows_v4, dim3((unsigned)(rows < 148 * 16 ? rows : 148 * 16)),
                      dim3(cols >= 8192 ? 512 : 256), 0, st, reinterpret_cast<const float4*>(x),
                      SmoothLabels{ids, on, off, 0}, rl, rows, (int)(cols / 4));
@@ -1592,9 +1591,9 @@ int tsb_softmax_ce_both_smooth(const float* x, const float* ids, float on, float
                                long long rows, long long cols, void* stream) {
   if (rows <= 0 || cols <= 0) return TSB_ERR_ARG;
   if (cols < 512 || cols % 4 || cols / 4 >= (1ll << 30) || !aligned16(x) || !aligned16(dx)) return TSB_ERR_UNSUPPORTED;
-  float* rl = row_scratch(rows);
-  if (!rl) return TSB_ERR_OOM;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  float* rl = row_scratch(rows, st);
+  if (!rl) return TSB_ERR_OOM;
   const int rc = launch_rows(ce_grad_rows_v4<SmoothLabels, false, true>, ce_grad_rows_v4<SmoothLabels, true, true>, rows,
                              (int)(cols / 4), st, reinterpret_cast<const float4*>(x), SmoothLabels{ids, on, off, 0}, g,
                              reinterpret_cast<float4*>(dx), rows, (int)(cols / 4), rl);
