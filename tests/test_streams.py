@@ -1,5 +1,6 @@
 """Executors on streams of their own share no scratch: what one launch leaves for the next belongs to their stream."""
 import ctypes
+import types
 
 import pytest
 import torch
@@ -65,3 +66,40 @@ def test_each_stream_has_scratch_of_its_own(run):
         outs.append([o.t.clone() for o in (run(stream), torch.cuda.synchronize())[0]])
         assert held() > before
     assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+def _pointers(monkeypatch, shape, pads, stride, streams):
+    """The calls of a stem's forward pass and filter gradient on each stream: [(entry, address of the packed image)]."""
+    calls = []
+
+    class Lib(object):
+        def __getattr__(self, name):
+            def entry(*args):
+                at = {"tsb_pack_pixels": 1, "tsb_pack_pixel_rows": 1, "tsb_stem_wgrad": 0, "tsb_conv2d": 1}.get(name)
+                calls.append((name, None if at is None else args[at].value))
+                return 0
+            return entry
+    monkeypatch.setattr(G, "lib", lambda: Lib())
+    monkeypatch.setattr(G, "_PAD_CACHE", {})
+
+    def empty(shape, ctx, **kw):                  # channels last, as on a GPU
+        t = torch.empty(shape)
+        return ndarray.from_tensor(t if t.dim() != 4 else t.to(memory_format=torch.channels_last), ctx)
+    monkeypatch.setattr(ndarray, "empty", empty)
+    n, c, h, w, o, k = shape
+    oh, ow = (h + 2 * pads - k) // stride + 1, (w + 2 * pads - k) // stride + 1
+    x, f, y = (ndarray.empty(s, ndarray.cpu(0)) for s in ((n, c, h, w), (o, c, k, k), (n, o, oh, ow)))
+    res = []
+    for handle in streams:
+        for kind in (0, 2):
+            G.conv2d(kind, x, f, y, pads, pads, stride, types.SimpleNamespace(handle=handle))
+        res.append([c for c in calls if c[1] is not None])
+        del calls[:]
+    return res, sum(b[1].t.numel() if isinstance(b, tuple) else b.t.numel() for k, b in G._PAD_CACHE.items() if k[0] not in ("w", "stem_w"))
+
+
+@pytest.mark.parametrize("shape,pads,stride", [((4, 3, 64, 64, 16, 7), 3, 2), ((4, 3, 64, 64, 16, 7), 3, 1),
+                                               ((4, 5, 64, 64, 16, 7), 3, 2)])
+def test_packed_images_belong_to_a_stream(monkeypatch, shape, pads, stride):
+    (first, second, again), _ = _pointers(monkeypatch, shape, pads, stride, (11, 12, 11))
+    assert first == again and not {p for _, p in first} & {p for _, p in second}

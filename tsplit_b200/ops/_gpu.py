@@ -610,32 +610,39 @@ def bn_forward_add(part, chunks, x, scale, bias, add, y, save_mean, save_invstd,
     return True
 
 
+# Copies of operands that the kernels read in another layout.  A buffer belongs to a stream: what a call leaves in one is
+# read by the launches behind it, and executors on other streams may run in between.
 _PAD_CACHE = {}
+
+
+def _buffer(key, arr, stream, make):
+    key += (arr.ctx.device_id, stream.handle if stream is not None else 0)
+    buf = _PAD_CACHE.get(key)
+    if buf is None:
+        buf = _PAD_CACHE[key] = make()
+    return buf
 
 
 def _as_channels_last(arr, tag, stream):
     from .. import ndarray
-    key = (tag, arr.shape, arr.ctx.device_id)
-    buf = _PAD_CACHE.get(key)
-    if buf is None:
-        buf = _PAD_CACHE[key] = ndarray.empty(arr.shape, arr.ctx, use_pool=False, channels_last=True)
+    buf = _buffer((tag, arr.shape), arr, stream,
+                  lambda: ndarray.empty(arr.shape, arr.ctx, use_pool=False, channels_last=True))
     copy(arr, buf, stream)
     return buf
 
 
-def _padded(arr, c4, tag):
+def _padded(arr, c4, tag, stream):
     """Cached channels-last scratch with the channel count rounded up to a
     multiple of 4 (the gather moves 16-byte pieces).  The padding lanes are
     zeroed once at creation; every use rewrites only the real channels."""
     from .. import ndarray
-    shape = (arr.shape[0], c4, arr.shape[2], arr.shape[3])
-    key = (tag, shape, arr.ctx.device_id)
-    buf = _PAD_CACHE.get(key)
-    if buf is None:
-        buf = ndarray.empty(shape, arr.ctx, use_pool=False)
+    n, c, h, w = arr.shape
+
+    def make():
+        buf = ndarray.empty((n, c4, h, w), arr.ctx, use_pool=False)
         buf.t.zero_()
-        _PAD_CACHE[key] = buf
-    return buf
+        return buf
+    return _buffer((tag, n, c, c4, h, w), arr, stream, make)
 
 
 def _to_pixels(x, x4, stream):
@@ -664,7 +671,7 @@ def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
         return _conv2d_packed_stem(kind, x, w, y, ph, pw, stream)
     if kind == 2 and stride > 1 and _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
         return
-    x4, w4 = _padded(x, c4, "x"), _padded(w, c4, "w")
+    x4, w4 = _padded(x, c4, "x", stream), _padded(w, c4, "w", stream)
     xs, ws = x4.strides, w4.strides
     if kind in (0, 2):
         _to_pixels(x, x4, stream)
@@ -687,10 +694,7 @@ def _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
     if c > 3 or kh > 8 or kw > 8 or o % 4 or not x.is_channels_last():
         return False
     wp = max((ow - 1) * stride + 8, wd + pw)
-    key = ("windows", (n, h, wp), x.ctx.device_id)
-    xp = _PAD_CACHE.get(key)
-    if xp is None:
-        xp = _PAD_CACHE[key] = ndarray.empty((n * h * wp * 4,), x.ctx, use_pool=False)
+    xp = _buffer(("windows", n, h, wp), x, stream, lambda: ndarray.empty((n * h * wp * 4,), x.ctx, use_pool=False))
     rc = lib().tsb_pack_pixel_rows(_p(x), _p(xp), c_int(c), c_int64(n * h), c_int(wd), c_int(wp), c_int(pw), _s(stream))
     if rc == 0:
         so, sc, sh, sw = w.strides
@@ -714,12 +718,9 @@ def _conv2d_packed_stem(kind, x, w, y, ph, pw, stream):
     n, c, h, wd = x.shape
     o, _, kh, kw = w.shape
     _, _, oh, ow = y.shape
-    x4 = _padded(x, 4, "x")
+    x4 = _padded(x, 4, "x", stream)
     _to_pixels(x, x4, stream)
-    key = ("stem_w", (o, kh), x.ctx.device_id)
-    packed = _PAD_CACHE.get(key)
-    if packed is None:
-        packed = _PAD_CACHE[key] = ndarray.empty((8 * o * kh * 3 * 32,), x.ctx, use_pool=False)
+    packed = _buffer(("stem_w", o, kh), x, stream, lambda: ndarray.empty((8 * o * kh * 3 * 32,), x.ctx, use_pool=False))
     so, sc, sh, sw = w.strides
     if kind == 0:
         _check(lib().tsb_stem_pack_filters(_p(w), c_int64(so), c_int64(sc), c_int64(sh), c_int64(sw), _p(packed),
