@@ -103,3 +103,17 @@ def _pointers(monkeypatch, shape, pads, stride, streams):
 def test_packed_images_belong_to_a_stream(monkeypatch, shape, pads, stride):
     (first, second, again), _ = _pointers(monkeypatch, shape, pads, stride, (11, 12, 11))
     assert first == again and not {p for _, p in first} & {p for _, p in second}
+
+
+def test_windows_take_the_room_of_the_packed_image(monkeypatch):
+    (calls,), floats = _pointers(monkeypatch, (4, 3, 64, 64, 16, 7), 3, 2, (11,))
+    assert [name for name, _ in calls] == ["tsb_pack_pixels", "tsb_conv2d", "tsb_pack_pixel_rows", "tsb_stem_wgrad"]
+    assert len({p for _, p in calls}) == 1 and floats == 4 * 64 * (31 * 2 + 8) * 4          # the wider rows
+
+
+@pytest.mark.parametrize("shape,stride", [((1, 3, 16, 16, 8, 3), 2), ((4, 3, 64, 64, 10, 3), 2), ((4, 3, 64, 64, 16, 9), 2)])
+def test_nothing_is_packed_for_a_refusal(monkeypatch, shape, stride):
+    """Images too small for the windows' tensor maps, filters of no whole 16 bytes, of nine taps."""
+    (calls,), floats = _pointers(monkeypatch, shape, 1, stride, (11,))
+    assert [name for name, _ in calls] == ["tsb_pack_pixels", "tsb_conv2d"] * 2
+    assert floats == shape[0] * shape[2] * shape[3] * 4

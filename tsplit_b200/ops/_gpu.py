@@ -645,6 +645,19 @@ def _padded(arr, c4, tag, stream):
     return _buffer((tag, n, c, c4, h, w), arr, stream, make)
 
 
+def _pixels(x, wide, stream):
+    """Room for ``x`` as pixels of four channels, in rows of up to ``wide`` of them: (the dense image, all of the buffer).
+    One buffer for the copy that a forward pass reads and for the windows of the filter gradient, which are made anew."""
+    from .. import ndarray
+    n, c, h, w = x.shape
+
+    def make():
+        flat = ndarray.empty((n * h * max(w, wide) * 4,), x.ctx, use_pool=False)
+        flat.t.zero_()
+        return ndarray.from_tensor(flat.t.as_strided((n, 4, h, w), (h * w * 4, 1, w * 4, 4)), x.ctx), flat
+    return _buffer(("pixels", n, c, h, w, wide), x, stream, make)
+
+
 def _to_pixels(x, x4, stream):
     """``x`` into the first channels of its padded copy."""
     n, c, h, w = x.shape
@@ -671,7 +684,8 @@ def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
         return _conv2d_packed_stem(kind, x, w, y, ph, pw, stream)
     if kind == 2 and stride > 1 and _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
         return
-    x4, w4 = _padded(x, c4, "x", stream), _padded(w, c4, "w", stream)
+    x4 = _pixels(x, _window_row(x, w, y, ph, pw, stride), stream)[0] if c < 4 else _padded(x, c4, "x", stream)
+    w4 = _padded(w, c4, "w", stream)
     xs, ws = x4.strides, w4.strides
     if kind in (0, 2):
         _to_pixels(x, x4, stream)
@@ -684,17 +698,29 @@ def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
         copy_raw(w4.ptr, ws, w.ptr, w.strides, w.shape, stream)
 
 
-def _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
-    """Filter gradient of a strided few-channel stem through TMA windows of eight pixels (``tsb_stem_wgrad``); False for
-    a shape it does not cover."""
-    from .. import ndarray
+def _window_row(x, w, y, ph, pw, stride):
+    """Pixels of a row of windows for ``tsb_stem_wgrad``, or 0 where that does not take the filter gradient: known before
+    anything is packed for it.  (Its tensor maps want 128 KB.)"""
     n, c, h, wd = x.shape
     o, _, kh, kw = w.shape
     _, _, oh, ow = y.shape
-    if c > 3 or kh > 8 or kw > 8 or o % 4 or not x.is_channels_last():
-        return False
+    if stride < 2 or c > 3 or kh > 8 or kw > 8 or o % 4 or ph > 127 or h + 2 * ph < kh or (h + 2 * ph - kh) // stride + 1 != oh:
+        return 0
     wp = max((ow - 1) * stride + 8, wd + pw)
-    xp = _buffer(("windows", n, h, wp), x, stream, lambda: ndarray.empty((n * h * wp * 4,), x.ctx, use_pool=False))
+    small = n * h * min(wp * 16, ow * 128) < 128 << 10
+    return 0 if small or wp >= 1 << 16 or n * h >= 1 << 24 or n * oh * ow >= 1 << 31 else wp
+
+
+def _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
+    """Filter gradient of a strided few-channel stem through TMA windows of eight pixels (``tsb_stem_wgrad``); False for
+    a shape it does not cover."""
+    n, c, h, wd = x.shape
+    o, _, kh, kw = w.shape
+    _, _, oh, ow = y.shape
+    wp = _window_row(x, w, y, ph, pw, stride) if x.is_channels_last() else 0
+    if not wp:
+        return False
+    xp = _pixels(x, wp, stream)[1]
     rc = lib().tsb_pack_pixel_rows(_p(x), _p(xp), c_int(c), c_int64(n * h), c_int(wd), c_int(wp), c_int(pw), _s(stream))
     if rc == 0:
         so, sc, sh, sw = w.strides
@@ -718,7 +744,7 @@ def _conv2d_packed_stem(kind, x, w, y, ph, pw, stream):
     n, c, h, wd = x.shape
     o, _, kh, kw = w.shape
     _, _, oh, ow = y.shape
-    x4 = _padded(x, 4, "x", stream)
+    x4 = _pixels(x, 0, stream)[0]
     _to_pixels(x, x4, stream)
     packed = _buffer(("stem_w", o, kh), x, stream, lambda: ndarray.empty((8 * o * kh * 3 * 32,), x.ctx, use_pool=False))
     so, sc, sh, sw = w.strides
