@@ -117,3 +117,13 @@ def test_nothing_is_packed_for_a_refusal(monkeypatch, shape, stride):
     (calls,), floats = _pointers(monkeypatch, shape, 1, stride, (11,))
     assert [name for name, _ in calls] == ["tsb_pack_pixels", "tsb_conv2d"] * 2
     assert floats == shape[0] * shape[2] * shape[3] * 4
+
+
+@pytest.mark.parametrize("shape,stride,zeroed", [((4, 3, 64, 64, 16, 7), 2, 1), ((4, 5, 64, 64, 16, 7), 2, 2)])
+def test_padding_is_zeroed_in_the_order_of_the_stream(monkeypatch, shape, stride, zeroed):
+    """(Another stream's pass over a new buffer may come behind what this one has put there.)"""
+    streams = []
+    monkeypatch.setattr(torch.Tensor, "zero_", None)
+    monkeypatch.setattr(G, "fill", lambda y, value, stream: streams.append((value, stream.handle)))
+    _pointers(monkeypatch, shape, 3, stride, (11,))
+    assert streams == [(0.0, 11)] * zeroed            # padded filters, and images of more than four channels

@@ -640,7 +640,7 @@ def _padded(arr, c4, tag, stream):
 
     def make():
         buf = ndarray.empty((n, c4, h, w), arr.ctx, use_pool=False)
-        buf.t.zero_()
+        fill(buf, 0.0, stream)
         return buf
     return _buffer((tag, n, c, c4, h, w), arr, stream, make)
 
@@ -653,21 +653,17 @@ def _pixels(x, wide, stream):
 
     def make():
         flat = ndarray.empty((n * h * max(w, wide) * 4,), x.ctx, use_pool=False)
-        flat.t.zero_()
         return ndarray.from_tensor(flat.t.as_strided((n, 4, h, w), (h * w * 4, 1, w * 4, 4)), x.ctx), flat
     return _buffer(("pixels", n, c, h, w, wide), x, stream, make)
 
 
 def _to_pixels(x, x4, stream):
-    """``x`` into the first channels of its padded copy."""
+    """``x`` into the first channels of its padded copy, zeros into the others of a copy by :func:`_pixels`."""
     n, c, h, w = x.shape
-    if x.is_channels_last() and c < 4:
-        rc = lib().tsb_pack_pixels(_p(x), _p(x4), c_int(c), c_int64(n * h * w), _s(stream))
-        if rc == 0:
-            return
-        if rc != 2:      # 2: sizes that the strided copy takes
-            _check(rc, "pack_pixels")
-    copy_raw(x.ptr, x.strides, x4.ptr, x4.strides, x.shape, stream)
+    if c < 4:
+        _check(lib().tsb_pack_pixels(_p(x), _p(x4), c_int(c), c_int64(n * h * w), _s(stream)), "pack_pixels")
+    else:
+        copy_raw(x.ptr, x.strides, x4.ptr, x4.strides, x.shape, stream)
 
 
 def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
