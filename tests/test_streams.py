@@ -1,6 +1,7 @@
 """Executors on streams of their own share no scratch: what one launch leaves for the next belongs to their stream."""
 import ctypes
 import types
+import weakref
 
 import pytest
 import torch
@@ -80,8 +81,6 @@ def _pointers(monkeypatch, shape, pads, stride, streams):
                 return 0
             return entry
     monkeypatch.setattr(G, "lib", lambda: Lib())
-    monkeypatch.setattr(G, "_PAD_CACHE", {})
-
     def empty(shape, ctx, **kw):                  # channels last, as on a GPU
         t = torch.empty(shape)
         return ndarray.from_tensor(t if t.dim() != 4 else t.to(memory_format=torch.channels_last), ctx)
@@ -89,13 +88,14 @@ def _pointers(monkeypatch, shape, pads, stride, streams):
     n, c, h, w, o, k = shape
     oh, ow = (h + 2 * pads - k) // stride + 1, (w + 2 * pads - k) // stride + 1
     x, f, y = (ndarray.empty(s, ndarray.cpu(0)) for s in ((n, c, h, w), (o, c, k, k), (n, o, oh, ow)))
-    res = []
+    res, by_handle = [], {}
     for handle in streams:
+        stream = by_handle.setdefault(handle, types.SimpleNamespace(handle=handle, buffers={}))
         for kind in (0, 2):
-            G.conv2d(kind, x, f, y, pads, pads, stride, types.SimpleNamespace(handle=handle))
+            G.conv2d(kind, x, f, y, pads, pads, stride, stream)
         res.append([c for c in calls if c[1] is not None])
         del calls[:]
-    return res, sum(b[1].t.numel() if isinstance(b, tuple) else b.t.numel() for k, b in G._PAD_CACHE.items() if k[0] not in ("w", "stem_w"))
+    return res, sum(b[1].t.numel() for s in by_handle.values() for b in s.buffers.values() if isinstance(b, tuple))
 
 
 @pytest.mark.parametrize("shape,pads,stride", [((4, 3, 64, 64, 16, 7), 3, 2), ((4, 3, 64, 64, 16, 7), 3, 1),
@@ -127,3 +127,24 @@ def test_padding_is_zeroed_in_the_order_of_the_stream(monkeypatch, shape, stride
     monkeypatch.setattr(G, "fill", lambda y, value, stream: streams.append((value, stream.handle)))
     _pointers(monkeypatch, shape, 3, stride, (11,))
     assert streams == [(0.0, 11)] * zeroed            # padded filters, and images of more than four channels
+
+
+@pytest.mark.gpu
+def test_buffers_are_given_back_with_their_stream():
+    ctx = ndarray.gpu(0)
+    x, f, y = _image(4, 3, 64, 64), _image(16, 3, 7, 7, seed=1), _image(4, 16, 32, 32)
+    stream = Stream(ctx)
+    other = Stream(ctx, torch_stream=stream.torch_stream)
+    handle = weakref.ref(stream.buffers)
+    G.conv2d(0, x, f, y, 3, 3, 2, stream)
+    assert len(other.buffers) == 2 and Stream(ctx).buffers is not other.buffers
+    want = y.t.clone()
+    del stream
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    G.conv2d(0, x, f, y, 3, 3, 2, other)                       # the same ones
+    assert torch.cuda.memory_allocated() == held
+    del other
+    assert handle() is None and held - torch.cuda.memory_allocated() >= 4 * 64 * 64 * 16
+    torch.cuda.synchronize()
+    assert torch.equal(y.t, want)

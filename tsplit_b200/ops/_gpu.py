@@ -612,14 +612,18 @@ def bn_forward_add(part, chunks, x, scale, bias, add, y, save_mean, save_invstd,
 
 # Copies of operands that the kernels read in another layout.  A buffer belongs to a stream: what a call leaves in one is
 # read by the launches behind it, and executors on other streams may run in between.
-_PAD_CACHE = {}
+_NO_STREAM = {}
 
 
 def _buffer(key, arr, stream, make):
-    key += (arr.ctx.device_id, stream.handle if stream is not None else 0)
-    buf = _PAD_CACHE.get(key)
+    held = _NO_STREAM if stream is None else stream.buffers
+    key += (arr.ctx.device_id,)
+    buf = held.get(key)
     if buf is None:
-        buf = _PAD_CACHE[key] = make()
+        buf = held[key] = make()
+        for part in buf if isinstance(buf, tuple) else (buf,):
+            if part.is_cuda and stream is not None:      # (its memory was asked for on torch's current stream)
+                part.t.record_stream(stream.torch_stream)
     return buf
 
 

@@ -9,6 +9,8 @@ inspects, so stream discipline is testable without a GPU.
 from __future__ import annotations
 
 import itertools
+import threading
+import weakref
 from ctypes import c_void_p
 
 import torch
@@ -26,6 +28,16 @@ def _native(name):
     return getattr(_base.kernels()._lib, name)
 
 
+class Buffers(dict):
+    """Device memory that operators keep for the launches of one stream.  All objects of a ``cudaStream_t`` share it, and
+    it is given back with the last of them."""
+    __slots__ = ("__weakref__",)
+
+
+_BUFFERS = weakref.WeakValueDictionary()         # (device, cudaStream_t) -> Buffers
+_BUFFERS_LOCK = threading.Lock()
+
+
 def _is_cuda(ctx):
     return ctx is not None and ctx.device_type == 2
 
@@ -38,6 +50,11 @@ class Stream(object):
         if _is_cuda(ctx):
             self.torch_stream = torch_stream or torch.cuda.Stream(
                 device=ctx.torch_device, priority=priority)
+        if self.torch_stream is None:
+            self.buffers = Buffers()
+        else:
+            with _BUFFERS_LOCK:
+                self.buffers = _BUFFERS.setdefault((ctx.device_id, self.handle), Buffers())
 
     @property
     def handle(self):
