@@ -6,6 +6,7 @@ import torch
 
 import test_step_plan as base
 from tsplit_b200 import gpu_ops as ad, ndarray
+from tsplit_b200.executors import step_plan
 from tsplit_b200.models import resnet
 from tsplit_b200.ops import _gpu as G
 from tsplit_b200.ops.conv import Conv2dGradDataOp
@@ -48,6 +49,25 @@ def test_what_stays(monkeypatch):
                 {x: r.standard_normal((2, 4, 6, 6), np.float32), s: np.ones((1, 4, 1, 1), np.float32),
                  b: np.zeros((1, 4, 1, 1), np.float32)})
     assert not base._compare(monkeypatch, build).joined
+
+
+def test_planning_searches_no_list_of_additions(monkeypatch):
+    """Counted in comparisons of nodes, which do not depend on the machine."""
+    def comparisons(inputs):
+        w, xs, count = ad.Variable("w"), [ad.Variable("x%d" % i) for i in range(inputs)], [0]
+        sums = [ad.conv2d_op(x, w, padding=1, stride=2) + ad.conv2d_op(x, w, padding=1, stride=2) for x in xs]
+        nodes = [g for s, x in zip(sums, xs) for g in ad.gradients(ad.reduce_sum_op(s, [0, 1, 2, 3]), [x])]
+        shapes = {x: (1, 2, 8, 8) for x in xs}
+        shapes[w] = (2, 2, 3, 3)
+        ex = ad.Executor(nodes, ctx=ndarray.cpu(0))
+        ex.infer_shape(shapes)
+        ex.memory_plan(shapes)
+        with monkeypatch.context() as m:
+            m.setattr(type(w), "__eq__", lambda a, b: (count.__setitem__(0, count[0] + 1), a is b)[1], raising=False)
+            plan = step_plan.StepPlan(ex, set(shapes))
+        assert len(plan.joined) == inputs
+        return count[0]
+    assert comparisons(80) <= 4 * comparisons(20) + 100
 
 
 # one row, part of a tile, a last tile of one thread's half, channels of no power of two; column sums of its own

@@ -156,42 +156,39 @@ class StepPlan(object):
         self.placeholders = [n for n in ex.topo_order if isinstance(n.op, PlaceholderOp) and n not in fed]
         self.evals = set(ex.eval_node_list)
         self.external = set(self.placeholders) | set(fed)
-        self.users = {}
+        self.kinds = {}                   # operator type -> _kind
+        # place: how many nodes with effects stand before a node.  What a rule takes together must have the same number, or
+        # one of its operands may be another by then.
+        self.users, self.place, own, effects = {}, {}, {}, set()      # own: operator type -> nodes
         for n in ex.topo_order:
+            self.place[n] = len(effects)
             if n not in self.external:
+                own.setdefault(type(n.op), []).append(n)
                 for i in n.inputs:
                     self.users.setdefault(i, []).append(n)
-        self.kinds = {}                   # operator type -> _kind
-        # how many nodes with effects stand before a node: what a rule takes together must have the same number, or one of
-        # its operands may be another by then
-        self.place, effects = {}, 0
-        for n in ex.topo_order:
-            self.place[n] = effects
-            if n not in self.external:
-                effects += self._has_effects(n)
+                if self._has_effects(n):
+                    effects.add(n)
+
+        def of(op):
+            return [n for t, nodes in own.items() if issubclass(t, op) for n in nodes]
+        losses = of(SoftmaxCrossEntropyOp)
         self.smooth, self.elided = {}, set()
-        for n in ex.topo_order:
-            if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
-                self._smooth_labels(n)
-        self.sliced = {n for n in ex.topo_order if n not in self.external and isinstance(n.op, SliceOp) and self._is_sliced(n)}
+        for n in losses:
+            self._smooth_labels(n)
+        self.sliced = {n for n in of(SliceOp) if self._is_sliced(n)}
         self.both = {}                           # gradient of a loss -> the loss that is computed with it
-        for n in ex.topo_order:
-            if n not in self.external and isinstance(n.op, SoftmaxCrossEntropyOp):
-                self._loss_with_gradient(n)
+        for n in losses:
+            self._loss_with_gradient(n)
         self.late = set(self.both.values())
         self.dense, self.stored = {}, set()      # product -> (its bias node or None, its ReLU or None), see _dense
         self.refused = {}                        # product -> what its launch does not take: 1 the ReLU, 2 the bias either
-        for n in ex.topo_order:
-            if n not in self.external and isinstance(n.op, MatMulOp):
-                self._dense(n)
-        self.joined = {}                  # addition -> the batch norm or the gradient that it is computed with
-        for n in ex.topo_order:
-            if n not in self.external:
-                if type(n.op) is AddReluOp:
-                    self._join(n)
-                elif type(n.op) is AddOp:
-                    self._add_gradients(n)
-        self.inner = set(self.joined.values())   # computed with the node that reads them
+        for n in of(MatMulOp):
+            self._dense(n)
+        self.joined, self.inner = {}, set()      # addition -> the batch norm or the gradient that it is computed with; these
+        for n in own.get(AddReluOp, ()):
+            self._join(n)
+        for n in own.get(AddOp, ()):
+            self._add_gradients(n)
         self.root = {}                    # view -> the node whose array it looks at
         self.actions = []
         self.open = {}                    # key -> Program that still collects
@@ -203,7 +200,7 @@ class StepPlan(object):
         for n in ex.topo_order:
             if n in self.external:
                 continue
-            if self._has_effects(n):
+            if n in effects:
                 self._schedule(segment)
                 segment = []
                 self._flush_all()
@@ -351,6 +348,7 @@ class StepPlan(object):
                     and self.arrays.get(b) is not None and self.arrays.get(n) is not None
                     and all(tuple(self.shapes[i]) == tuple(self.shapes[n]) for i in n.inputs)):
                 self.joined[n] = b
+                self.inner.add(b)
                 return
 
     def _add_gradients(self, n):
@@ -358,7 +356,7 @@ class StepPlan(object):
         where the sum goes, and this one adds to it."""
         def alone(i):
             return (type(i.op) is Conv2dGradDataOp and i not in self.external and i not in self.evals and self.users.get(i) == [n]
-                    and self.place[i] == self.place[n] and i not in self.joined.values()
+                    and self.place[i] == self.place[n] and i not in self.inner
                     and self.arrays.get(i) is not None and tuple(self.shapes[i]) == tuple(self.shapes[n]))
         a, b = n.inputs
         if a is b or self.arrays.get(n) is None or self._has_effects(n) or not (alone(a) and alone(b)):
@@ -367,6 +365,7 @@ class StepPlan(object):
         first = a if late is b else b
         if late.attrs["stride"] == 2 and self.arrays[first].same_layout(self.arrays[n]):
             self.joined[n] = late
+            self.inner.add(late)
             self.arrays[first] = self.arrays[n]
 
     # -- scheduling ------------------------------------------------------------------------
@@ -517,7 +516,7 @@ class StepPlan(object):
             new = len({r for r, _ in operands if home.get(r) is not prog})
             limit = MAX_SLOTS_LARGE if numel >= LARGE else MAX_SLOTS
             if (len(prog.inputs) + new > min(MAX_IN, limit - 4) or len(prog.members) >= MAX_INS
-                    or (cols and prog.cols and prog.cols != cols) or self._slots_with(prog, n) > limit):
+                    or (cols and prog.cols and prog.cols != cols) or self._too_many_slots(prog, n, limit)):
                 self._flush(prog)
                 prog = None
         if prog is None:
@@ -545,10 +544,11 @@ class StepPlan(object):
         prog.live += readers > 0
 
     @staticmethod
-    def _slots_with(prog, n):
-        """Upper bound of the slots after one more member: every value still read later holds one."""
-        done = sum(1 for i in set(n.inputs) if prog.left.get(i) == n.inputs.count(i))       # read by nobody after n
-        return len(prog.inputs) + prog.live - done + 3
+    def _too_many_slots(prog, n, limit):
+        """After one more member: every value still read later holds one."""
+        most = len(prog.inputs) + prog.live + 3
+        return most > limit and most - sum(          # (less those that are read by nobody after n)
+            1 for i in set(n.inputs) if prog.left.get(i) == n.inputs.count(i)) > limit
 
     def _flush(self, prog):
         del self.open[prog.key]
