@@ -93,3 +93,27 @@ def test_gemm_odd_row_stride_is_padded_not_simt():
     assert _run(255, 64, 255, 1, 0, batch=16) < 5e-3
     assert _run(130, 255, 64, 0, 1, batch=3) < 5e-3
     assert _run(100, 37, 72, 0, 0) < 5e-3            # ldb = 37
+
+
+@pytest.mark.parametrize("rows", [40, 520])
+def test_heads_of_no_whole_16_bytes(rows):
+    """Rows of whole 16 bytes, heads inside them that are not: copied where TMA would have to read them, head by head."""
+    from tsplit_b200 import gpu_ops as ad, ndarray
+    n, heads, d = 3, 2, 6
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v = (torch.randn((n, rows, heads, d), generator=gen, device="cuda") for _ in range(3))
+    p = torch.randn((n, heads, rows, rows), generator=gen, device="cuda")
+    Q, K, V, P = (ad.Variable(name) for name in "QKVP")
+    ex = ad.Executor([ad.batch_matmul_op(Q, K, trans_B=True, heads_A=True, heads_B=True),
+                      ad.batch_matmul_op(P, V, heads_B=True, heads_out=True),
+                      ad.batch_matmul_op(P, V, trans_A=True, heads_B=True, heads_out=True)], ctx=ndarray.gpu(0))
+
+    def arr(t):
+        a = ndarray.empty(tuple(t.shape), ndarray.gpu(0), use_pool=False, channels_last=False)
+        a.t.copy_(t)
+        return a
+    got = [o.t.double() for o in ex.run({Q: arr(q), K: arr(k), V: arr(v), P: arr(p)})]
+    q, k, v, p = (t.double() for t in (q, k, v, p))
+    want = [torch.einsum("nqhd,nkhd->nhqk", q, k), torch.einsum("nhqk,nkhd->nqhd", p, v), torch.einsum("nhkq,nkhd->nqhd", p, v)]
+    for g, w in zip(got, want):
+        assert (g - w).norm() < 2e-3 * w.norm()              # operands of 10 bits

@@ -972,9 +972,10 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
 }
 
 // Copy of a [batch][rows][cols] operand whose row stride is not a multiple of four floats into a
-// scratch array with the row stride rounded up (pad columns zero), so that TMA can address it.
-__global__ void pad_rows_kernel(const float* src, float* __restrict__ dst, int batch, int rows,
-                                int cols, long long lds, long long ss, long long ldd, long long sd) {
+// scratch array with the row stride rounded up (pad columns zero), so that TMA can address it.  Matrix (o, i) of the
+// batch, i < inner, begins o * so + i * ss in.
+__global__ void pad_rows_kernel(const float* src, float* __restrict__ dst, int batch, int rows, int cols, long long lds,
+                                int inner, long long so, long long ss, long long ldd, long long sd) {
   tsb_launch::enter();
   const long long total = (long long)batch * rows * ldd;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -993,7 +994,8 @@ __global__ void pad_rows_kernel(const float* src, float* __restrict__ dst, int b
       row = (int)(r % rows);
       b = r / rows;
     }
-    dst[b * sd + row * ldd + c] = c < cols ? src[b * ss + row * lds + c] : 0.f;
+    const int o = inner < batch ? (int)b / inner : 0;
+    dst[b * sd + row * ldd + c] = c < cols ? src[o * so + (b - (long long)o * inner) * ss + row * lds + c] : 0.f;
   }
 }
 
@@ -1261,8 +1263,8 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
         const long long total = (long long)batch * rows_a * lda2;
         long long blocks = (total + 255) / 256;
         if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-        tsb_launch::launch(pad_rows_kernel, (unsigned)blocks, 256, 0, st, a, buf, batch, rows_a, cols_a, lda,
-                           batch > 1 ? sa : 0, lda2, sa2);
+        tsb_launch::launch(pad_rows_kernel, (unsigned)blocks, 256, 0, st, a, buf, batch, rows_a, cols_a, lda, a_heads ? heads : batch,
+                           rows_a * lda, sa, lda2, sa2);
         ap = buf;
       }
     }
@@ -1275,8 +1277,8 @@ int tsb_gemm_tf32_impl(const float* a, const float* b, float* c, int m, int n, i
         const long long total = (long long)batch * rows_b * ldb2;
         long long blocks = (total + 255) / 256;
         if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-        tsb_launch::launch(pad_rows_kernel, (unsigned)blocks, 256, 0, st, b, buf, batch, rows_b, cols_b, ldb,
-                           batch > 1 ? sb : 0, ldb2, sb2);
+        tsb_launch::launch(pad_rows_kernel, (unsigned)blocks, 256, 0, st, b, buf, batch, rows_b, cols_b, ldb, b_heads ? heads : batch,
+                           rows_b * ldb, sb, ldb2, sb2);
         bp = buf;
       }
     }
