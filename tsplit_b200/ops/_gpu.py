@@ -11,6 +11,7 @@ There is no fallback: on a CUDA context a missing library is an error.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_void_p, c_int, c_int64, c_float
 
 from .. import _base
@@ -615,22 +616,23 @@ def bn_forward_add(part, chunks, x, scale, bias, add, y, save_mean, save_invstd,
 _NO_STREAM = {}
 
 
-def _buffer(key, arr, stream, make):
-    held = _NO_STREAM if stream is None else stream.buffers
-    key += (arr.ctx.device_id,)
-    buf = held.get(key)
-    if buf is None:
-        buf = held[key] = make()
-        for part in buf if isinstance(buf, tuple) else (buf,):
-            if part.is_cuda and stream is not None:      # (its memory was asked for on torch's current stream)
-                part.t.record_stream(stream.torch_stream)
+def _held(stream):
+    return _NO_STREAM if stream is None else stream.buffers
+
+
+def _kept(shape, arr, stream):
+    from .. import ndarray
+    buf = ndarray.empty(shape, arr.ctx, use_pool=False, channels_last=True)
+    if buf.is_cuda and stream is not None:           # (the memory was asked for on torch's current stream)
+        buf.t.record_stream(stream.torch_stream)
     return buf
 
 
 def _as_channels_last(arr, tag, stream):
-    from .. import ndarray
-    buf = _buffer((tag, arr.shape), arr, stream,
-                  lambda: ndarray.empty(arr.shape, arr.ctx, use_pool=False, channels_last=True))
+    held, key = _held(stream), (tag, arr.shape, arr.ctx.device_id)
+    buf = held.get(key)
+    if buf is None:
+        buf = held[key] = _kept(arr.shape, arr, stream)
     copy(arr, buf, stream)
     return buf
 
@@ -639,26 +641,26 @@ def _padded(arr, c4, tag, stream):
     """Cached channels-last scratch with the channel count rounded up to a
     multiple of 4 (the gather moves 16-byte pieces).  The padding lanes are
     zeroed once at creation; every use rewrites only the real channels."""
-    from .. import ndarray
-    n, c, h, w = arr.shape
-
-    def make():
-        buf = ndarray.empty((n, c4, h, w), arr.ctx, use_pool=False)
+    held, key = _held(stream), (tag, arr.shape, c4, arr.ctx.device_id)
+    buf = held.get(key)
+    if buf is None:
+        n, _, h, w = arr.shape
+        buf = held[key] = _kept((n, c4, h, w), arr, stream)
         fill(buf, 0.0, stream)
-        return buf
-    return _buffer((tag, n, c, c4, h, w), arr, stream, make)
+    return buf
 
 
 def _pixels(x, wide, stream):
     """Room for ``x`` as pixels of four channels, in rows of up to ``wide`` of them: (the dense image, all of the buffer).
     One buffer for the copy that a forward pass reads and for the windows of the filter gradient, which are made anew."""
-    from .. import ndarray
-    n, c, h, w = x.shape
-
-    def make():
-        flat = ndarray.empty((n * h * max(w, wide) * 4,), x.ctx, use_pool=False)
-        return ndarray.from_tensor(flat.t.as_strided((n, 4, h, w), (h * w * 4, 1, w * 4, 4)), x.ctx), flat
-    return _buffer(("pixels", n, c, h, w, wide), x, stream, make)
+    held, key = _held(stream), ("pixels", x.shape, wide, x.ctx.device_id)
+    bufs = held.get(key)
+    if bufs is None:
+        from .. import ndarray
+        n, c, h, w = x.shape
+        flat = _kept((n * h * max(w, wide) * 4,), x, stream)
+        bufs = held[key] = ndarray.from_tensor(flat.t.as_strided((n, 4, h, w), (h * w * 4, 1, w * 4, 4)), x.ctx), flat
+    return bufs
 
 
 def _to_pixels(x, x4, stream):
@@ -684,7 +686,7 @@ def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
         return _conv2d_packed_stem(kind, x, w, y, ph, pw, stream)
     if kind == 2 and stride > 1 and _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
         return
-    x4 = _pixels(x, _window_row(x, w, y, ph, pw, stride), stream)[0] if c < 4 else _padded(x, c4, "x", stream)
+    x4 = _pixels(x, _window_row(x.shape, w.shape, y.shape, ph, pw, stride), stream)[0] if c < 4 else _padded(x, c4, "x", stream)
     w4 = _padded(w, c4, "w", stream)
     xs, ws = x4.strides, w4.strides
     if kind in (0, 2):
@@ -698,12 +700,13 @@ def _conv2d_padded_channels(kind, x, w, y, ph, pw, stride, stream):
         copy_raw(w4.ptr, ws, w.ptr, w.strides, w.shape, stream)
 
 
+@functools.lru_cache(maxsize=1024)
 def _window_row(x, w, y, ph, pw, stride):
-    """Pixels of a row of windows for ``tsb_stem_wgrad``, or 0 where that does not take the filter gradient: known before
-    anything is packed for it.  (Its tensor maps want 128 KB.)"""
-    n, c, h, wd = x.shape
-    o, _, kh, kw = w.shape
-    _, _, oh, ow = y.shape
+    """Pixels of a row of windows for ``tsb_stem_wgrad``, of the operands' shapes, or 0 where that does not take the filter
+    gradient: known before anything is packed for it.  (Its tensor maps want 128 KB.)"""
+    n, c, h, wd = x
+    o, _, kh, kw = w
+    _, _, oh, ow = y
     if stride < 2 or c > 3 or kh > 8 or kw > 8 or o % 4 or ph > 127 or h + 2 * ph < kh or (h + 2 * ph - kh) // stride + 1 != oh:
         return 0
     wp = max((ow - 1) * stride + 8, wd + pw)
@@ -717,7 +720,7 @@ def _strided_stem_wgrad(x, w, y, ph, pw, stride, stream):
     n, c, h, wd = x.shape
     o, _, kh, kw = w.shape
     _, _, oh, ow = y.shape
-    wp = _window_row(x, w, y, ph, pw, stride) if x.is_channels_last() else 0
+    wp = _window_row(x.shape, w.shape, y.shape, ph, pw, stride) if x.is_channels_last() else 0
     if not wp:
         return False
     xp = _pixels(x, wp, stream)[1]
@@ -740,13 +743,15 @@ def _packed_stem_ok(x, w, y, c4, pw, stride):
 
 
 def _conv2d_packed_stem(kind, x, w, y, ph, pw, stream):
-    from .. import ndarray
     n, c, h, wd = x.shape
     o, _, kh, kw = w.shape
     _, _, oh, ow = y.shape
     x4 = _pixels(x, 0, stream)[0]
     _to_pixels(x, x4, stream)
-    packed = _buffer(("stem_w", o, kh), x, stream, lambda: ndarray.empty((8 * o * kh * 3 * 32,), x.ctx, use_pool=False))
+    held, key = _held(stream), ("stem_w", o, kh, x.ctx.device_id)
+    packed = held.get(key)
+    if packed is None:
+        packed = held[key] = _kept((8 * o * kh * 3 * 32,), x, stream)
     so, sc, sh, sw = w.strides
     if kind == 0:
         _check(lib().tsb_stem_pack_filters(_p(w), c_int64(so), c_int64(sc), c_int64(sh), c_int64(sw), _p(packed),
