@@ -1,5 +1,6 @@
 """Executors on streams of their own share no scratch: what one launch leaves for the next belongs to their stream."""
 import ctypes
+import gc
 import types
 import weakref
 
@@ -8,16 +9,20 @@ import torch
 
 from tsplit_b200 import _base, ndarray
 from tsplit_b200.ops import _gpu as G
+from tsplit_b200.runtime import cudagraph
 from tsplit_b200.stream import Stream
 
 
 def _rand(*shape, seed=0):
-    return ndarray.from_tensor(torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda"), ndarray.gpu(0))
+    t = torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda")
+    torch.cuda.synchronize()                       # (read on other streams)
+    return ndarray.from_tensor(t, ndarray.gpu(0))
 
 
 def _image(*shape, seed=0):
     a = ndarray.empty(shape, ndarray.gpu(0), use_pool=False)
     a.t.copy_(_rand(*shape, seed=seed).t)
+    torch.cuda.synchronize()
     return a
 
 
@@ -57,6 +62,8 @@ def _wide_max_pool_grad(stream):
 def test_each_stream_has_scratch_of_its_own(run):
     held = _base.kernels().tsb_scratch_bytes
     held.restype = ctypes.c_longlong
+    torch.cuda.synchronize()
+    _base.kernels().tsb_scratch_trim()             # (given-back buffers would be taken)
     outs = []
     for _ in range(2):
         handle = ctypes.c_void_p()                 # (a new one: torch's streams come from a pool)
@@ -148,3 +155,28 @@ def test_buffers_are_given_back_with_their_stream():
     assert handle() is None and held - torch.cuda.memory_allocated() >= 4 * 64 * 64 * 16
     torch.cuda.synchronize()
     assert torch.equal(y.t, want)
+
+
+@pytest.mark.gpu
+def test_scratch_of_a_finished_stream_is_for_the_next_one():
+    """Handed on once the stream, and what was captured on it, has gone; another stream's stays its own."""
+    ctx = ndarray.gpu(0)
+    held = _base.kernels().tsb_scratch_bytes
+    held.restype = ctypes.c_longlong
+    torch.cuda.synchronize()
+    gc.collect()
+    _base.kernels().tsb_scratch_trim()
+    first, other = Stream(ctx), Stream(ctx)
+    want = [o.t.clone() for o in (_losses(first), torch.cuda.synchronize())[0]]
+    graph = cudagraph.capture(first, lambda: None)
+    del first
+    before = held()
+    _losses(other)
+    torch.cuda.synchronize()
+    assert held() > before                         # the graph may still be replayed
+    del graph
+    before = held()
+    third = Stream(ctx)
+    got = (_losses(third), torch.cuda.synchronize())[0]
+    assert held() == before and all(torch.equal(g.t, w) for g, w in zip(got, want))
+    assert (_losses(Stream(ctx)), torch.cuda.synchronize())[0] and held() > before

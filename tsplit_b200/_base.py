@@ -52,6 +52,11 @@ def _load(name):
     return lib
 
 
+def loaded(name):
+    """The library, or None where nothing has asked for it yet."""
+    return _cache.get(name)
+
+
 def runtime():
     lib = _load("libtsplit_runtime.so")
     return lib

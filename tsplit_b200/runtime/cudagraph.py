@@ -7,8 +7,8 @@ from .. import _base
 
 
 class CapturedGraph(object):
-    def __init__(self, handle):
-        self.handle = handle
+    def __init__(self, handle, buffers=None):
+        self.handle, self.buffers = handle, buffers          # (what the captured launches read and write stays)
 
     def launch(self, stream):
         rc = _base.kernels().tsb_graph_launch(self.handle, ctypes.c_void_p(stream.handle))
@@ -40,4 +40,4 @@ def capture(stream, fn):
     rc = lib.tsb_graph_end(ctypes.c_void_p(stream.handle), ctypes.byref(exec_handle))
     if rc:
         raise RuntimeError("graph capture failed: " + _base.error_string(rc))
-    return CapturedGraph(exec_handle)
+    return CapturedGraph(exec_handle, stream.buffers)

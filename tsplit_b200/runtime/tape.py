@@ -23,7 +23,7 @@ ACTIVE = [None]
 
 #: entries that are queries or graph control, never actions of a step
 NOT_ACTIONS = {"tsb_graph_begin", "tsb_graph_end", "tsb_graph_launch", "tsb_graph_destroy", "tsb_mem_info",
-               "tsb_scratch_bytes", "tsb_scratch_trim", "tsb_device_status", "tsb_comm_status"}
+               "tsb_scratch_bytes", "tsb_scratch_trim", "tsb_scratch_give_back", "tsb_device_status", "tsb_comm_status"}
 
 _INT32 = (ctypes.c_int, ctypes.c_short, ctypes.c_byte, ctypes.c_bool)
 _UINT32 = (ctypes.c_uint, ctypes.c_ushort, ctypes.c_ubyte)

@@ -30,12 +30,32 @@ def _native(name):
 
 class Buffers(dict):
     """Device memory that operators keep for the launches of one stream.  All objects of a ``cudaStream_t`` share it, and
-    it is given back with the last of them."""
-    __slots__ = ("__weakref__",)
+    what was captured on it, and it is given back with the last of them; so is the kernel library's own scratch of a stream
+    that was made here (another one may be gone by then)."""
+    __slots__ = ("__weakref__", "scratch_too")
 
 
 _BUFFERS = weakref.WeakValueDictionary()         # (device, cudaStream_t) -> Buffers
-_BUFFERS_LOCK = threading.Lock()
+_BUFFERS_LOCK = threading.RLock()                # (a collection inside it may give back another stream's)
+
+
+def _give_back(device, handle):
+    lib = _base.loaded("libtsplit_kernels.so")
+    with _BUFFERS_LOCK:
+        if lib is not None and (device, handle) not in _BUFFERS:
+            lib.tsb_scratch_give_back(device, c_void_p(handle))
+
+
+def _buffers(device, handle, made_here):
+    with _BUFFERS_LOCK:
+        held = _BUFFERS.get((device, handle))
+        if held is None:
+            held = _BUFFERS[device, handle] = Buffers()
+            held.scratch_too = False
+        if made_here and not held.scratch_too:
+            held.scratch_too = True
+            weakref.finalize(held, _give_back, device, handle).atexit = False
+    return held
 
 
 def _is_cuda(ctx):
@@ -50,11 +70,7 @@ class Stream(object):
         if _is_cuda(ctx):
             self.torch_stream = torch_stream or torch.cuda.Stream(
                 device=ctx.torch_device, priority=priority)
-        if self.torch_stream is None:
-            self.buffers = Buffers()
-        else:
-            with _BUFFERS_LOCK:
-                self.buffers = _BUFFERS.setdefault((ctx.device_id, self.handle), Buffers())
+        self.buffers = Buffers() if self.torch_stream is None else _buffers(ctx.device_id, self.handle, torch_stream is None)
 
     @property
     def handle(self):
