@@ -1,6 +1,4 @@
 """Bias and ReLU stored by the product's own launch: the plan on the host, the kernels on the GPU against separate operators."""
-import ctypes
-
 import numpy as np
 import pytest
 import torch

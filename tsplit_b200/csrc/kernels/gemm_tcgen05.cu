@@ -1187,7 +1187,6 @@ static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorM
   if (rc) return rc;
   rc = operand_map(&tb, &p.b_chunked, b, trans_b == 0, n, k, ldb, b_rows, b_bat, sbb, bbox);
   if (rc) return rc;
-  // (rows of whole 16-byte units only: a box is clipped to them, and would write into the gap behind a row of 1023)
   // C (or the split-K partial sums) as [outer][head or batch][row][column], where its strides allow a tensor map
   tc = ta;
   {
@@ -1196,6 +1195,7 @@ static int prepare_tc(GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, CUtensorM
     const long long mat = p.splits > 1 ? (long long)m * n : (batch > 1 ? sc : (long long)m * ldc);
     const uint64_t mats = c_heads ? (uint64_t)heads : (uint64_t)batch * p.splits;
     const long long top = c_heads ? p.sc2 : (long long)mats * mat;
+    // (rows of whole 16-byte units only: a box is clipped to them, and would write into the gap behind a row of 1023)
     p.tma_store = (p.splits > 1 || !accumulate) && n % 4 == 0 && row % 4 == 0 && mat % 4 == 0 && top % 4 == 0 && row > 0 && mat > 0 &&
                   (reinterpret_cast<uintptr_t>(base) & 15) == 0 && top < (1ll << 37);
     if (p.tma_store) {

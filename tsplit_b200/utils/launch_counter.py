@@ -12,7 +12,8 @@ _count = [0]
 #: kernels launched per entry point (entries not listed launch one)
 KERNELS_PER_ENTRY = {
     "tsb_bn_forward": 3, "tsb_bn_backward": 3, "tsb_softmax_ce": 2, "tsb_softmax_ce_smooth": 2,
-    "tsb_layer_norm_grad": 3,
+    "tsb_layer_norm_grad": 3, "tsb_softmax_ce_both": 2, "tsb_softmax_ce_both_smooth": 2, "tsb_bn_forward_add": 2,
+    "tsb_stem_wgrad": 2,
     "tsb_graph_begin": 0, "tsb_graph_end": 0, "tsb_graph_destroy": 0, "tsb_device_status": 0,
     "tsb_mem_info": 0, "tsb_scratch_bytes": 0, "tsb_scratch_trim": 0, "tsb_scratch_give_back": 0,
     "tsb_graph_launch": 0,
