@@ -1112,7 +1112,7 @@ __device__ __forceinline__ MaxSum smooth_row_loss(const float4* x, const float4*
   }
   return sum.finish(lab, nvec, sh, loss);
 }
-// 4096 x 32000 with the mean of the rows: 91 us (90 to 100 on three boxes), bound by DRAM.  (The row is walked here and not by the
+// 4096 x 32000 with the mean of the rows: 91 us, bound by DRAM.  (The row is walked here and not by the
 // function above, whose code for it takes 3 to 5 % longer.)
 __global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* x, SmoothLabels lab,
                                                          float* __restrict__ row_loss, long long rows, int nvec) {
@@ -1139,7 +1139,7 @@ __global__ void __launch_bounds__(512) ce_smooth_rows_v4(const float4* x, Smooth
 }
 
 // row_loss (LOSS): the loss as well, as the kernels above make it; a training step that takes both reads its logits once.
-// 4096 x 32000 with labels from ids, one after the other on one box: 91 us of loss, 198 of gradient, 297 of the two in turn
+// 4096 x 32000 with labels from ids, in one run: 91 us of loss, 198 of gradient, 297 of the two in turn
 // -> 220 (the step that takes both 1187 -> 1127 us at the power cap).
 template <class Labels, bool STAGED, bool LOSS>
 __global__ void __launch_bounds__(512) ce_grad_rows_v4(const float4* x, Labels lab,
