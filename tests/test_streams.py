@@ -4,10 +4,11 @@ import gc
 import types
 import weakref
 
+import numpy as np
 import pytest
 import torch
 
-from tsplit_b200 import _base, ndarray
+from tsplit_b200 import _base, gpu_ops as ad, ndarray
 from tsplit_b200.ops import _gpu as G
 from tsplit_b200.runtime import cudagraph
 from tsplit_b200.stream import Stream
@@ -180,3 +181,31 @@ def test_scratch_of_a_finished_stream_is_for_the_next_one():
     got = (_losses(third), torch.cuda.synchronize())[0]
     assert held() == before and all(torch.equal(g.t, w) for g, w in zip(got, want))
     assert (_losses(Stream(ctx)), torch.cuda.synchronize())[0] and held() > before
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("executor", ["Executor", "microopExecutor"])
+def test_first_step_behind_work_on_the_current_stream(executor):
+    """Running statistics, step counter, padded operands and slots of a first step do not wait for one another by luck."""
+    ctx, results = ndarray.gpu(0), []
+    for busy in (False, True):
+        r = np.random.default_rng(0)
+        val = lambda *shape: (0.2 * r.standard_normal(shape)).astype(np.float32)
+        x, y, w, s, b, wd = (ad.Variable(n, value=v) for n, v in (
+            ("x", None), ("y", None), ("w", val(16, 5, 3, 3)), ("s", val(1, 16, 1, 1)), ("b", val(1, 16, 1, 1)), ("wd", val(1024, 12))))
+        norm = ad.batch_normalization_op(ad.conv2d_op(x, w, padding=1, stride=2), s, b)
+        drop = ad.dropout_op(norm, 0.7)
+        drop.attrs["seed"] = 5
+        loss = ad.softmaxcrossentropy_op(ad.matmul_op(ad.array_reshape_op(drop, (-1, 1024)), wd), y)
+        grads = ad.gradients(loss, [w])
+        feed = {x: ndarray.array(val(8, 5, 16, 16), ctx), y: ndarray.array(np.eye(12, dtype=np.float32)[np.arange(8)], ctx)}
+        for v in (w, s, b, wd):
+            v.tensor_value = ndarray.array(v.tensor_value, ctx)
+        torch.cuda.synchronize()
+        if busy:
+            torch.cuda._sleep(200_000_000)                  # a tenth of a second
+        ex = getattr(ad, executor)([loss, norm] + grads, ctx=ctx)
+        results.append([o.t.clone() for _ in range(2) for o in ex.run(feed)])
+        torch.cuda.synchronize()
+        results[-1] += [norm.state[k].t.clone() for k in ("run_mean", "run_var")]
+    assert all(torch.equal(p, q) for p, q in zip(*results))

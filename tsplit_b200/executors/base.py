@@ -244,6 +244,8 @@ class Executor(object):
             if self.__dict__.get("_step_dev") is None:
                 self._step_dev = torch.full((1,), misc.STEP[0] - 1, dtype=torch.int64,
                                             device=self.ctx.torch_device)
+                # (this, like optimizer slots and parameters, is written on torch's current stream)
+                self.stream.torch_stream.wait_stream(torch.cuda.current_stream(self.ctx.torch_device))
             misc.STEP_DEV[0] = self._step_dev.data_ptr()
         else:
             misc.STEP_DEV[0] = 0

@@ -242,10 +242,10 @@ def _bn_state(orig):
     return st
 
 
-def _side(shape, ctx, value=None):
+def _side(shape, ctx, value=None, stream=None):
     a = ndarray.empty(shape, ctx, use_pool=False)
     if value is not None:
-        a.t.fill_(value)
+        G.fill(a, value, stream)
     return a
 
 
@@ -299,7 +299,7 @@ class BnFinalizeOp(_MicroBase):
         c = int(np.prod(scale.shape))
         if "mean" not in st or st["mean"].shape != (c,):
             st["mean"], st["invstd"] = _side((c,), scale.ctx), _side((c,), scale.ctx)
-            st["run_mean"], st["run_var"] = _side((c,), scale.ctx, 0.0), _side((c,), scale.ctx, 1.0)
+            st["run_mean"], st["run_var"] = _side((c,), scale.ctx, 0.0, stream), _side((c,), scale.ctx, 1.0, stream)
         G.bn_stats_finalize(st["micro_part"], st["micro_part"].shape[0] // 2, st["micro_chunks"], st["micro_rows"], c,
                             eps, mom, st["mean"], st["invstd"], st["run_mean"], st["run_var"], stream)
         st["stats_open"] = False        # pieces rebuilt from here on are plain convolutions

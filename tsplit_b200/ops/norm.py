@@ -45,12 +45,12 @@ def np_bn_backward(gy, x, scale, mean, invstd):
     return dx.astype(np.float32), dscale.astype(np.float32), dbias.astype(np.float32)
 
 
-def _small(shape, ctx, value=None):
+def _small(shape, ctx, value=None, stream=None):
     """Per-node side buffer (statistics, parameter gradients): tiny, so it lives
-    outside the capped activation pool."""
+    outside the capped activation pool.  Filled on the stream that uses it."""
     a = ndarray.empty(shape, ctx, use_pool=False)
     if value is not None:
-        a.t.fill_(value)
+        G.fill(a, value, stream)
     return a
 
 
@@ -64,18 +64,18 @@ class BatchNormOp(Op):
             x.attrs["bn_consumer"] = node      # the convolution's epilogue then supplies the column statistics
         return node
 
-    def _statistics(self, node, x):
+    def _statistics(self, node, x, stream):
         """The node's side buffers, and the column sums that a convolution left in them: (state, chunks)."""
         st, c = node.state, x.shape[1]
         if "mean" not in st or st["mean"].shape != (c,):
             st["mean"], st["invstd"] = _small((c,), x.ctx), _small((c,), x.ctx)
-            st["run_mean"], st["run_var"] = _small((c,), x.ctx, 0.0), _small((c,), x.ctx, 1.0)
+            st["run_mean"], st["run_var"] = _small((c,), x.ctx, 0.0, stream), _small((c,), x.ctx, 1.0, stream)
         chunks = 0 if st.get("rematerialise") else st.pop("conv_chunks", 0)
         return st, chunks if st.get("conv_rows") == x.shape[0] * x.shape[2] * x.shape[3] else 0
 
     def _forward(self, node, iv, out, stream, relu):
         x, scale, bias = iv
-        st, chunks = self._statistics(node, x)
+        st, chunks = self._statistics(node, x, stream)
         if st.get("rematerialise"):      # same step, statistics known: normalise only, leave running stats alone
             return G.bn_apply(x, scale, bias, out, st["mean"], st["invstd"], relu, stream)
         if chunks:
@@ -121,7 +121,7 @@ class BatchNormOp(Op):
         if node.state.get("rematerialise") or len(x.shape) != 4 or not x.t.is_cuda:
             return False
         left = node.state.get("conv_chunks", 0)
-        st, chunks = self._statistics(node, x)
+        st, chunks = self._statistics(node, x, stream)
         if G.bn_forward_add(st["conv_part"] if chunks else None, chunks, x, scale, bias, add, out, st["mean"], st["invstd"],
                             st["run_mean"], st["run_var"], node.attrs["momentum"], node.attrs["eps"], stream):
             return True
